@@ -84,7 +84,7 @@ struct DeviceScope {
 // The tick kernel of the handle's engine for `nreg` regions: one CTA per region.
 // The parallel sweep uses only the parallel member of TickSmem's union: its launch asks for that
 // much shared memory, which leaves the rest of the SM's 256 KB to L1.
-constexpr int PAR_SMEM_BYTES = (int)((offsetof(TickSmem, u) + sizeof(ParSmem) + 127) / 128 * 128);
+constexpr int PAR_SMEM_BYTES = (int)((offsetof(TickSmem, u) + sizeof(LvSmem) + 127) / 128 * 128);
 static_assert(PAR_SMEM_BYTES <= (int)sizeof(TickSmem), "parallel sweep shared memory");
 
 cudaError_t launch_tick(const Tune& t, Region* regs, int nreg, int n_ticks, int smem, cudaStream_t st) {
@@ -444,31 +444,18 @@ int vf_fluid_upload_world(vf_fluid* h, int32_t nx, int32_t ny, int32_t nz, int32
   if ((rc = dalloc(h, &R.stamp, ncells, false))) return rc;
   if ((rc = dalloc(h, &R.last_woken, cap))) return rc;
   CK(cudaMemsetAsync(R.stamp, 0xFF, ncells * 4, h->stream));
-  // parallel sweep: per-cell records, rows, pull stamps and versions
-  if ((rc = dalloc(h, &R.rec, MAX_CELLS_PER_TICK))) return rc;
-  if ((rc = dalloc(h, &R.rowstart, MAX_CELLS_PER_TICK + 1))) return rc;
-  if ((rc = dalloc(h, &R.rowof, MAX_CELLS_PER_TICK))) return rc;
-  if ((rc = dalloc(h, &R.rowprog, MAX_CELLS_PER_TICK))) return rc;
-  if ((rc = dalloc(h, &R.pcnt, MAX_CELLS_PER_TICK + 1))) return rc;
-  if ((rc = dalloc(h, &R.zrow, (uint64_t)R.PY * R.PZ, false))) return rc;
-  CK(cudaMemsetAsync(R.zrow, 0xFF, (uint64_t)R.PY * R.PZ * 4, h->stream));
-  if ((rc = dalloc(h, &R.preader, ncells))) return rc;
-  if ((rc = dalloc(h, &R.ptbits, words))) return rc;
-  if ((rc = dalloc(h, &R.ptlist, MAX_PULLS_PER_TICK + 64))) return rc;
-  if ((rc = dalloc(h, &R.ptreg, PTREG_CAP))) return rc;
-  if ((rc = dalloc(h, &R.pextra, (MAX_CELLS_PER_TICK + 31) / 32))) return rc;
-  if ((rc = dalloc(h, &R.pxlist, MAX_CELLS_PER_TICK))) return rc;
+  // parallel sweep: per-cell records, events, lists
+  if ((rc = dalloc(h, &R.lv, MAX_CELLS_PER_TICK, false))) return rc;
+  if ((rc = dalloc(h, &R.lv_old, MAX_CELLS_PER_TICK, false))) return rc;
+  if ((rc = dalloc(h, &R.lv_ev, MAX_CELLS_PER_TICK, false))) return rc;
+  if ((rc = dalloc(h, &R.lv_src, MAX_CELLS_PER_TICK, false))) return rc;
+  if ((rc = dalloc(h, &R.lv_over, 2 * MAX_CELLS_PER_TICK, false))) return rc;
+  if ((rc = dalloc(h, &R.lv_park, 2 * MAX_CELLS_PER_TICK, false))) return rc;
+  if ((rc = dalloc(h, &R.pextra, (MAX_CELLS_PER_TICK + 31) / 32, false))) return rc;
+  if ((rc = dalloc(h, &R.pxlist, MAX_CELLS_PER_TICK, false))) return rc;
   if ((rc = dalloc(h, &R.rb, ncells, false))) return rc;
   if (ring_w && (rc = dalloc(h, &R.detbits, words))) return rc;
-  if ((rc = dalloc(h, &R.deps, (uint64_t)MAX_CELLS_PER_TICK * 16, false))) return rc;
-  // the warps' search contexts in global memory: visited sets empty (every search empties its own
-  // before it returns)
-  if ((rc = dalloc(h, &R.pcg, MAX_WARPS, false))) return rc;
-  static_assert(EMPTY_ID == 0xFFFFFFFFu, "a visited-set slot of 0xFF bytes is free");
-  CK(cudaMemsetAsync(R.pcg, 0xFF, MAX_WARPS * sizeof(PullCtx), h->stream));
   CK(cudaMemsetAsync(R.rb, 0xFF, ncells * 4, h->stream));
-  // the parallel sweep packs search-queue coordinates in 16 bits per axis
-  if (R.PX >= 65536 || R.PZ >= 65536 || R.PY >= 65536) h->tune.engine = 0;
   R.chg_cap = 1u << 22;
   if ((rc = dalloc(h, &R.chg, R.chg_cap, false))) return rc;
   uint64_t qcap = next_pow2(std::max<uint64_t>({h->want_queue, std::min<uint64_t>(ncells, 1ull << 22), 1ull << 16}));
@@ -576,15 +563,7 @@ int vf_fluid_tick_async(vf_fluid* h, int32_t n_ticks) {
   h->hzero[0] = 0u;
   CK(cudaMemcpyAsync(&h->R.ctl->changed, h->hzero, sizeof(unsigned), cudaMemcpyHostToDevice, h->stream));
   if (n_ticks > 0) {
-    if (h->auto_engine) {
-      // pull-heavy water (deep lakes, many pressure searches per cell) runs faster on the one-warp
-      // sweep; everything else on the parallel sweep. Counters as of the last synchronisation.
-      const uint64_t dc = h->hctl->cells_total - h->auto_cells, db = h->hctl->bfs_visits - h->auto_bfs;
-      const bool wide_ok = h->R.PX < 65536 && h->R.PZ < 65536 && h->R.PY < 65536;
-      if (dc > 0) h->tune.engine = (wide_ok && 2 * db <= 3 * dc) ? 1 : 0;
-      h->auto_cells = h->hctl->cells_total;
-      h->auto_bfs = h->hctl->bfs_visits;
-    }
+    if (h->auto_engine) h->tune.engine = 1;
     CK(launch_tick(h->tune, h->dR, 1, n_ticks, h->smem_bytes, h->stream));
   }
   return VF_OK;
@@ -1019,8 +998,6 @@ int vf_fluid_reset(vf_fluid* h) {  // fluid.rs:318-320: the fluid's tables only
   CK(cudaMemsetAsync(R.mark_tflag, 0, tiles * 4, h->stream));
   // per-tick maps a failed tick may have left set (cell positions, rows, pull-written cells)
   CK(cudaMemsetAsync(R.stamp, 0xFF, (size_t)R.ncells * 4, h->stream));
-  CK(cudaMemsetAsync(R.zrow, 0xFF, (size_t)R.PY * R.PZ * 4, h->stream));
-  CK(cudaMemsetAsync(R.ptbits, 0, words * 4, h->stream));
   if (R.detbits) CK(cudaMemsetAsync(R.detbits, 0, words * 4, h->stream));  // kept entries go with the rest
   h->det.clear();
   Ctl c = *h->hctl;

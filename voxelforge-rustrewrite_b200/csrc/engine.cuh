@@ -82,40 +82,8 @@ struct Ctl {
 };
 constexpr int NPROF = 16;
 
-// Per drained cell of the parallel sweep (global memory, indexed by sorted position). The old
-// footprint values serve readers that must see the state before this cell (multi-version reads)
-// and the rollback of a segment; the event fields are committed in sorted order at the tick's end.
-struct __align__(16) CellRec {
-  float opart[7];          // footprint partials when the cell started (self, below, up, +x, -x, +z, -z)
-  unsigned char omat[7];   // footprint materials when the cell started
-  unsigned char wmask;     // footprint cells the cell's flow wrote
-  unsigned char cmask;     // cells whose material changed: footprint bits 0..6, bit 7 the pull source
-  unsigned char amask;     // activation slots in program order (0 source, 1 self after the pull,
-                           // 2 below, 3..6 sides, 7 self)
-  unsigned char flags;     // RF_*
-  signed char pdelta;      // partial-entry count delta
-  unsigned src;            // pull source cell id
-  float src_opart;         // the source's partial before the pull wrote it
-  unsigned char src_omat;  // and its material
-  unsigned char pad0;
-  unsigned short entries;  // pressure-search queue entries examined
-  unsigned tk_main;        // execution ticket of the flow's writes (segment-wide order of writes)
-  unsigned tk_src;         // execution ticket of the pull's source write
-};
-constexpr unsigned RF_ATTEMPT = 1u, RF_SUCCESS = 2u, RF_CHANGED = 4u, RF_SEED_SELF = 8u, RF_SEED_SRC = 16u, RF_SRCW = 32u;
-
-// A pull's write of its source cell, kept for readers earlier in sorted order that read the cell
-// after the write (open addressing by cell id; a slot belongs to the segment whose epoch it holds).
-struct __align__(16) PullTarget {
-  unsigned epoch;   // segment epoch owning the slot (claimed by CAS)
-  unsigned ready;   // == epoch once the fields below are written
-  unsigned id;      // source cell id
-  unsigned writer;  // sorted position of the pulling cell
-  float opart;      // the source's partial before the write
-  unsigned omat;    // the source's material before the write
-  unsigned pad[2];
-};
-constexpr unsigned PTREG_CAP = 16384;  // > 4 x the pulls one segment can make
+struct LvCell;
+struct LvOld;
 
 struct Region {
   // ---- geometry (voxel dims, brick dims, ring width; padded scheduler domain)
@@ -153,23 +121,20 @@ struct Region {
   unsigned int ev_act_cap, ev_seed_cap, ev_chg_cap;
   unsigned int* stamp;       // ncells: first event index per cell during a commit (0xFFFFFFFF idle)
   unsigned int* last_woken;  // atlas_cap: last tick a cell of the slot's brick was drained (0 = never)
-  // ---- parallel sweep (per tick; `stamp` doubles as the cell -> sorted position map)
-  CellRec* rec;          // MAX_CELLS_PER_TICK
-  unsigned* rowstart;    // MAX_CELLS_PER_TICK + 1: first sorted position of each row (y, z)
-  unsigned* rowof;       // MAX_CELLS_PER_TICK: row of each cell, bit 31 may attempt a pull, bit 30 solid
-  unsigned* rowprog;     // MAX_CELLS_PER_TICK: cells of the row finished
-  unsigned* pcnt;        // MAX_CELLS_PER_TICK + 1: exclusive prefix count of possible attempts
-  unsigned* zrow;        // PY * PZ: row of (y, z) this tick, NOSLOT otherwise
-  unsigned* preader;     // ncells: latest pull read (segment epoch << 16 | position + 1)
-  unsigned* ptbits;      // ncells bits: a pull wrote the cell this tick
-  unsigned* ptlist;      // MAX_PULLS_PER_TICK + 64 cells whose ptbits are set
-  PullTarget* ptreg;     // PTREG_CAP
-  unsigned* pextra;      // MAX_CELLS_PER_TICK bits: later cells a pull took below 1 - 1e-4 (not counted in pcnt)
-  unsigned* pxlist;      // MAX_CELLS_PER_TICK: the positions whose pextra bit is set
-  unsigned* rb;          // ncells: earliest writer during a segment's rollback (0xFFFFFFFF idle)
-  unsigned* deps;        // MAX_CELLS_PER_TICK * 16: earlier conflicting cells of each cell (10 used)
-  unsigned* detbits;     // ring worlds: ncells bits, the cell's partial entry is kept for an evicted chunk
-  struct PullCtx* pcg;   // one pressure-search context per sweep warp (used when the shared pool is empty)
+  // ---- parallel sweep (per tick; `stamp` doubles as the cell -> sorted position map), all of
+  // MAX_CELLS_PER_TICK entries (two of the lists)
+  LvCell* lv;              // what a round reads of each drained cell
+  LvOld* lv_old;           // the volumes a cell of the gate layer replaced
+  unsigned* lv_ev;         // events: bits 0-7 activation slots in program order (0 source, 1 self after the
+                           // pull, 2 below, 3..6 sides, 7 self), 8-15 cells whose material changed
+                           // (footprint slots, 15 the pull source), 16 seeds itself, 17 seeds the source
+  unsigned* lv_src;        // pull source cell id
+  unsigned short* lv_over; // the rounds' lists past what shared memory holds (two)
+  unsigned short* lv_park; // ready cells above the gate layer (two)
+  unsigned* pextra;        // bits: full cells a pull took below 1 - 1e-4
+  unsigned* pxlist;        // their positions
+  unsigned* rb;            // ncells: claims of the levelling's flood fill (0xFFFFFFFF idle)
+  unsigned* detbits;       // ring worlds: ncells bits, the cell's partial entry is kept for an evicted chunk
   Ctl* ctl;
 };
 

@@ -5,7 +5,7 @@
 #include <cuda_fp16.h>
 
 #include "engine_dev.cuh"
-#include "sweep_par.cuh"
+#include "sweep_lvl.cuh"
 
 namespace vfe {
 
@@ -19,8 +19,6 @@ namespace vfe {
 constexpr int TICK_THREADS = 256;
 constexpr int TICK_WARPS = TICK_THREADS / 32;
 constexpr int PAR_THREADS = MAX_WARPS * 32;
-constexpr int PEXPOSE = 3;            // water cells over a full cell that pulls may empty in one tick
-constexpr unsigned PAR_MAX_SPLITS = 6;  // conflicts at one position before it runs in order
 
 // ---------------------------------------------------------------- CTA radix sort (LSD, 8 bit)
 // Stable within each warp's contiguous chunk; chunks in order -> stable overall. Sorts n unique
@@ -169,7 +167,7 @@ struct TickSmem {
   unsigned scan[MAX_WARPS + 1];
   union {
     SeqSmem s;  // one-warp sweep
-    ParSmem p;  // parallel sweep
+    LvSmem p;   // parallel sweep
   } u;
 };
 
@@ -568,25 +566,6 @@ __device__ void sweep(const Region& R, TickSmem& sm, WS& sW, const int* ring, un
   __syncthreads();
 }
 // ------------------------------------------------------------------- the parallel sweep
-// Segment end for `room` more attempts from `pos` (one thread): the largest e <= n with at most
-// `room` cells in [pos, e) that may attempt a pull. `extra` cells at or after pos, taken below full
-// by earlier pulls of the tick although not counted in pcnt, are charged up front.
-__device__ unsigned seg_end_for(const Region& R, unsigned pos, unsigned n, unsigned room, unsigned extra, float ratio, float factor) {
-  if (extra >= room) return pos + 1u;
-  // sized for `factor` times the attempts expected at `ratio` per possible attempter; a segment
-  // that overshoots the budget is undone and cut at its room-th attempt (exact either way)
-  unsigned span = room - extra;
-  if (span > 32u && ratio * (1.0f / factor) < 1.0f) span = (unsigned)fminf(4.0e9f, factor * (float)span / ratio);
-  const unsigned lim = R.pcnt[pos] + span;
-  unsigned lo = pos + 1u, hi = n;  // answer in [pos + 1, n]
-  while (lo < hi) {
-    const unsigned m = (lo + hi + 1u) >> 1;
-    if (R.pcnt[m] <= lim) lo = m;
-    else hi = m - 1u;
-  }
-  return lo;
-}
-
 // Sum of a per-thread value over the CTA (all threads call).
 __device__ unsigned long long cta_sum(TickSmem& sm, unsigned long long v) {
   for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(FULLMASK, v, o);
@@ -599,13 +578,17 @@ __device__ unsigned long long cta_sum(TickSmem& sm, unsigned long long v) {
   return t;
 }
 
-// The sweep of one tick by every warp of the CTA (sweep_par.cuh describes the schedule). On return
-// the tick's activation, seed and change logs hold the sweep's events in program order and sW its
-// counters, exactly as the one-warp sweep leaves them.
-__device__ __noinline__ void sweep_parallel(const Region& R, TickSmem& sm, WS& sW, const int* ring, unsigned n, bool flip, Tune tune) {
-  ParSmem& ps = sm.u.p;
+// The sweep of one tick by the CTA (sweep_lvl.cuh describes the schedule). On return the tick's
+// activation, seed and change logs hold the sweep's events in program order and sW its counters.
+__device__ __noinline__ void sweep_levels(const Region& Rs, TickSmem& sm, WS& sW, const int* ring, unsigned n, bool flip, Tune tune) {
+  LvSmem& L = sm.u.p;
+  // The region's constants in registers: a round is a chain of dependent instructions, and behind
+  // every store the compiler would read them from shared memory again (~30 cycles each).
+  const Region R = Rs;
   const unsigned tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
   const float FULL = full_level();
+  const unsigned long long cap = tune.spin_cap;
+  const unsigned ngrp = (n + 31u) / 32u;
   long long tp0 = clock64();
   auto plap = [&](int k) {
     if (tid == 0) {
@@ -614,335 +597,213 @@ __device__ __noinline__ void sweep_parallel(const Region& R, TickSmem& sm, WS& s
       tp0 = now;
     }
   };
-  ParProf pf{0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
-  unsigned long long w_fetch = 0, w_total = 0;
-  // ---- positions, rows and the cells that may attempt a pull (fluid.rs:594)
-  __shared__ unsigned s_rows, s_pc;
+  int pd = 0;
+  // ---- positions, footprints, and the cells that attempt a pull or may find a start cell
+  for (unsigned g = tid; g <= NGROUPS; g += NT_) {
+    L.pend[g] = 0u;
+    if (g >= ngrp) L.att[g] = L.pp[g] = 0u;
+  }
+  for (unsigned g = tid; g < ngrp; g += NT_) R.pextra[g] = 0u;
   if (tid == 0) {
-    s_rows = 0;
-    s_pc = 0;
+    L.cnt[0] = L.cnt[1] = L.cnt[2] = 0u;
+    L.park_n[0] = L.park_n[1] = 0u;
+    L.nx = 0u;
+    L.kp = n;
+    L.head = n;
+    L.hword = 0u;
+    L.hblk = 0u;
+    L.gate = -1;
+    L.lend = 0u;
+    L.nsearch = 0u;
+    L.n_succ = L.n_searches = L.n_again = 0u;
+    L.n_entries = 0ull;
   }
-  __syncthreads();
-  for (unsigned base = 0; base < n; base += NT_) {
-    const unsigned i = base + tid;
-    const bool valid = i < n;
-    unsigned rowflag = 0, P = 0, S = 0;
-    int x = 0, y = 0, z = 0;
-    if (valid) {
-      const unsigned key = R.cells[i];
-      const unsigned cid = key_to_id(R, key, flip);
-      R.stamp[cid] = i;
-      rowflag = (i == 0u || udiv(key, (unsigned)R.PX, R.mx) != udiv(R.cells[i - 1u], (unsigned)R.PX, R.mx)) ? 1u : 0u;
-      dom_xyz(R, cid, x, y, z);
-      // the cell and the PEXPOSE + 1 cells over it, loads issued together
-      CD col[PEXPOSE + 2];
-#pragma unroll
-      for (int d = 0; d <= PEXPOSE + 1; ++d) col[d] = load_cell(R, ring, x, y + d, z);
-      const CD c = col[0];
-      S = cd_solid(c) ? 1u : 0u;
-      if (!S) {
-        // A cell attempts only below 1 - 1e-4. One full at the tick's start gets there only as a
-        // pull's source, which must be a surface cell (up solid, outside or empty) when the pull
-        // runs; a cell under water becomes one after pulls empty the cells above it, one pull per
-        // cell. Cells with at most PEXPOSE water cells over them are counted; a deeper exposure
-        // in one tick is caught when the pull runs (a conflict).
-        P = cd_volume(c) < FULL ? 1u : 0u;
-#pragma unroll
-        for (int d = 1; d <= PEXPOSE + 1; ++d)
-          if (!P && (cd_solid(col[d]) || cd_volume(col[d]) <= 0.0f)) P = 1u;
-      }
-    }
-    unsigned trow, tp;
-    const unsigned orow = cta_scan_count(sm, rowflag, &trow);
-    const unsigned op = cta_scan_count(sm, P, &tp);
-    const unsigned rows0 = s_rows, pc0 = s_pc;
-    if (valid) {
-      const unsigned row = rows0 + orow + rowflag - 1u;
-      R.rowof[i] = row | (P << 31) | (S << 30);
-      R.pcnt[i] = pc0 + op;
-      if (rowflag) {
-        R.rowstart[row] = i;
-        R.rowprog[row] = 0u;
-        R.zrow[(size_t)y * (unsigned)R.PZ + (unsigned)(z - R.pz0)] = row;
-      }
-    }
-    __syncthreads();
-    if (tid == 0) {
-      s_rows += trow;
-      s_pc += tp;
-    }
-    __syncthreads();
-  }
-  if (tid == 0) {
-    R.rowstart[s_rows] = n;
-    R.pcnt[n] = s_pc;
-    R.ctl->ptn = 0u;
-  }
-  // earlier conflicting cells of every cell (the position map is complete now)
-  for (unsigned i = tid; i < n; i += NT_) {  // one cell per thread: ten position loads in flight
-    const unsigned cid = key_to_id(R, R.cells[i], flip);
-    int x, y, z;
-    dom_xyz(R, cid, x, y, z);
-    unsigned d[16];
-#pragma unroll
-    for (unsigned l = 0; l < 10u; ++l) {
-      int dx, dy, dz;
-      dep_offset(l, flip, dx, dy, dz);
-      const unsigned r = rank_at(R, x + dx, y + dy, z + dz);
-      d[l] = r < i ? r : NOSLOT;
-    }
-#pragma unroll
-    for (unsigned l = 10u; l < 16u; ++l) d[l] = NOSLOT;
-    uint4* o = reinterpret_cast<uint4*>(R.deps + (size_t)i * 16u);
-#pragma unroll
-    for (int q = 0; q < 4; ++q) o[q] = make_uint4(d[4 * q], d[4 * q + 1], d[4 * q + 2], d[4 * q + 3]);
-  }
-  for (unsigned w = tid; w < (n + 3u) / 4u; w += NT_) ps.state[w] = 0u;
-  for (unsigned w = tid; w < (n + 31u) / 32u; w += NT_) R.pextra[w] = 0u;
-  if (tid == 0) R.ctl->pxn = 0u;
-  for (unsigned t = tid; t < NPC_SMEM * PV_CAP; t += NT_) ps.pc[t / PV_CAP].vis[t % PV_CAP] = EMPTY_ID;
-  if (tid == 0) ps.pc_free = ((tune.gate >> 21) & 1) ? 0u : (1u << NPC_SMEM) - 1u;  // bit 21: global contexts only
-  __syncthreads();
-  plap(0);
-  // ---- budget segments
-  __shared__ unsigned s_pos, s_c, s_end, s_mode, s_epoch, s_go, s_cap, s_split;
-  if (tid == 0) {
-    s_pos = 0;
-    s_c = 0;
-    s_cap = n;    // a segment split by a conflict ends here
-    s_split = 0;  // splits of the current position so far
-  }
-  __syncthreads();
-  const int gate = max(0, min(tune.gate & 0xFF, GATE_MAX));
-  const int cone = (tune.gate >> 8) & 0xFF ? min((tune.gate >> 8) & 0xFF, GATE_MAX) : gate;
-  __shared__ unsigned s_extra;
-  // attempts per possible attempter over this tick's completed pull segments (the last tick's to
-  // start with), for sizing the next segment
-  __shared__ unsigned long long s_att_acc, s_p_acc;
-  __shared__ unsigned s_pull_end, s_nseg;
-  if (tid == 0) {
-    s_att_acc = 0ull;
-    s_p_acc = 0ull;
-    s_pull_end = n;  // known once a segment overshot the budget: its room-th attempt's cell + 1
-    s_nseg = 0;
-  }
-  while (true) {
-    // cells at or after the position that earlier pulls took below full (not counted in pcnt)
-    {
-      const unsigned nx = min(__ldcg(&R.ctl->pxn), MAX_CELLS_PER_TICK);
-      unsigned long long c = 0;
-      for (unsigned q = tid; q < nx; q += NT_) c += __ldcg(R.pxlist + q) >= s_pos ? 1u : 0u;
-      c = cta_sum(sm, c);
-      if (tid == 0) s_extra = (unsigned)c;
-    }
-    if (tid == 0) {
-      const unsigned pos = s_pos;
-      s_go = pos < n ? 1u : 0u;
-      if (s_go) {
-        if (s_c >= MAX_PULLS_PER_TICK) {
-          s_end = n;
-          s_mode = PM_NOPULL;
-        } else {
-          float ratio = 1.0f;
-          if (s_p_acc >= 256ull) ratio = (float)s_att_acc / (float)s_p_acc;
-          else if (R.ctl->att_ratio) ratio = (float)R.ctl->att_ratio * (1.0f / 65536.0f);
-          ratio = fminf(1.0f, fmaxf(ratio, 0.125f));
-          // the tick's first segment stops short of the expected budget end; later ones reach past
-          // it, so that an overshoot finds the exact end, after which one segment runs the rest
-          // with pulls up to that end and none after it
-          if (s_pull_end < n) s_end = n;
-          else s_end = seg_end_for(R, pos, n, MAX_PULLS_PER_TICK - s_c, s_extra, ratio, s_nseg == 0u ? 0.9f : 1.25f);
-          s_mode = PM_PULL;
-        }
-        s_end = min(s_end, max(s_cap, pos + 1u));
-        // a position split too often runs its (short) segment in order on one warp
-        if (s_split >= PAR_MAX_SPLITS) s_mode = PM_SEQ;
-        unsigned ep = R.ctl->seg_epoch + 1u;
-        if ((ep & 0xFFFFu) == 0u) ep += 1u;  // epoch 0 marks free version slots and unstamped reads
-        R.ctl->seg_epoch = ep;
-        s_epoch = ep;
-        ps.next_task = R.rowof[pos] & 0x3FFFFFFFu;
-        ps.task_end = R.rowof[s_end - 1u] & 0x3FFFFFFFu;
-        ps.abort = 0u;
-        ps.viol = 0u;
-        ps.viol_pos = 0xFFFFFFFFu;
-        ps.ticket = 0u;
-        for (int w = 0; w < MAX_WARPS; ++w) ps.wrow[w] = WROW_IDLE;
-        R.ctl->par_segments += 1ull;
-      }
-    }
-    __syncthreads();
-    if (!s_go) break;
-    ParTick T;
-    T.seg_start = s_pos;
-    T.seg_end = s_end;
-    T.pull_end = s_pull_end;
-    T.epoch = s_epoch;
-    T.gate = gate;
-    T.cone = cone;
-    T.flip = flip;
-    T.spin_cap = tune.spin_cap;
-    const int mode = (int)s_mode;
-    unsigned seq_pulls = 0;
-    if (mode == PM_SEQ) {
-      // one warp, in sorted order, the budget counted exactly
-      if (warp == 0) {
-        unsigned sp = s_c;
-        unsigned cgi = 0xFFFFFFFFu, cg = 0u;
-        for (unsigned i = T.seg_start; i < T.seg_end; ++i) process_cell_par(R, ps, R.pcg[0], ring, T, PM_SEQ, i, sp, pf, NOSLOT, cgi, cg, NOSLOT, 0u, R.cells[i]);
-        if (lane == 0) R.ctl->par_replayed += T.seg_end - T.seg_start;
-      }
-      __syncthreads();
-      if (vld((const unsigned*)&R.ctl->status) != 0u) return;
-    } else {
-      // ---- row workers
-      const long long w0 = clock64();
-      while (true) {
-        const long long f0 = clock64();
-        unsigned t = 0;
-        if (lane == 0) t = atomicAdd(&ps.next_task, 1u);
-        t = __shfl_sync(FULLMASK, t, 0);
-        if (t > ps.task_end) break;
-        const unsigned rs = R.rowstart[t];
-        const unsigned a = max(rs, T.seg_start), b = min(R.rowstart[t + 1u], T.seg_end);
-        // publish the row and its next cell for cone_wait (key / PX = y * PZ + sorted z)
-        const unsigned ka = R.cells[a];
-        const unsigned yz = udiv(ka, (unsigned)R.PX, R.mx), yy = udiv(yz, (unsigned)R.PZ, R.mz), zs = yz - yy * (unsigned)R.PZ;
-        const unsigned zr = flip ? (unsigned)R.PZ - 1u - zs : zs;
-        const unsigned long long rowtag = ((unsigned long long)yy << 48) | ((unsigned long long)zr << 32);
-        w_fetch += (unsigned long long)(clock64() - f0);
-        bool ok = true;
-        unsigned cgi = 0xFFFFFFFFu, cg = 0u;
-        unsigned jr_next = R.deps[a * 16u + (lane & 15u)];
-        unsigned key_next = ka;
-        for (unsigned i = a; i < b && ok; ++i) {
-          const unsigned jr = jr_next, key = key_next;
-          if (i + 1u < b) {  // used by the next cell
-            jr_next = R.deps[(i + 1u) * 16u + (lane & 15u)];
-            key_next = R.cells[i + 1u];
-          }
-          if (lane == 0) *(volatile unsigned long long*)&ps.wrow[warp] = rowtag | (key - yz * (unsigned)R.PX);
-          ok = process_cell_par(R, ps, R.pcg[warp], ring, T, mode, i, seq_pulls, pf, jr, cgi, cg, t, rs, key);
-        }
-        if (lane == 0) *(volatile unsigned long long*)&ps.wrow[warp] = WROW_IDLE;
-        if (!ok || vld(&ps.abort)) break;
-      }
-      w_total += (unsigned long long)(clock64() - w0);
-      __syncthreads();
-      plap(1);
-      if (vld((const unsigned*)&R.ctl->status) != 0u) return;  // a wait or a capacity ran out: the tick fails
-      if (ps.viol) {
-        // a conflict the schedule could not order at pull position k: undo the segment and run it
-        // again up to k + 1 (the late reader is then outside it), the rest afterwards
-        rollback_segment(R, ps, ring, T.seg_start, T.seg_end, flip);
-        for (unsigned i = T.seg_start + tid; i < T.seg_end; i += NT_) atomicAnd(&ps.state[i >> 2], ~(0xFFu << ((i & 3u) * 8u)));
-        const unsigned r0 = R.rowof[T.seg_start] & 0x3FFFFFFFu, r1 = R.rowof[T.seg_end - 1u] & 0x3FFFFFFFu;
-        for (unsigned r = r0 + tid; r <= r1; r += NT_) {
-          const unsigned st = R.rowstart[r];
-          R.rowprog[r] = T.seg_start > st ? T.seg_start - st : 0u;
-        }
-        __syncthreads();
-        plap(2);
-        if (tid == 0) {
-          R.ctl->par_rollbacks += 1ull;
-          s_cap = min(ps.viol_pos, T.seg_end - 1u) + 1u;
-          s_split += 1u;
-        }
-        __syncthreads();
-        continue;
-      }
-    }
-    // ---- attempts made in the segment (exact: every cell of it has finished)
-    unsigned long long att = 0;
-    for (unsigned i = T.seg_start + tid; i < T.seg_end; i += NT_) att += (R.rec[i].flags & RF_ATTEMPT) ? 1u : 0u;
-    att = cta_sum(sm, att);
-    const unsigned room = MAX_PULLS_PER_TICK - min(s_c, MAX_PULLS_PER_TICK);
-    if (mode == PM_PULL && att > room) {
-      // more cells attempted than the budget left (cells that pulls took below full beyond the
-      // counted ones): the cells up to the room-th attempt were right. Undo the segment and run it
-      // again up to that cell; the rest follows with the budget spent.
-      __shared__ unsigned s_cut;
-      if (tid == 0) s_cut = T.seg_end;
-      __syncthreads();
-      unsigned run = 0;
-      for (unsigned base = T.seg_start; base < T.seg_end; base += NT_) {
-        const unsigned i = base + tid;
-        const unsigned f = (i < T.seg_end && (R.rec[i].flags & RF_ATTEMPT)) ? 1u : 0u;
-        unsigned tot;
-        const unsigned off = cta_scan_count(sm, f, &tot);
-        if (f && run + off + 1u == room) s_cut = i + 1u;
-        run += tot;
-        __syncthreads();
-        if (run >= room) break;
-      }
-      rollback_segment(R, ps, ring, T.seg_start, T.seg_end, flip);
-      for (unsigned i = T.seg_start + tid; i < T.seg_end; i += NT_) atomicAnd(&ps.state[i >> 2], ~(0xFFu << ((i & 3u) * 8u)));
-      const unsigned r0 = R.rowof[T.seg_start] & 0x3FFFFFFFu, r1 = R.rowof[T.seg_end - 1u] & 0x3FFFFFFFu;
-      for (unsigned r = r0 + tid; r <= r1; r += NT_) {
-        const unsigned st = R.rowstart[r];
-        R.rowprog[r] = T.seg_start > st ? T.seg_start - st : 0u;
-      }
-      __syncthreads();
-      if (tid == 0) {
-        R.ctl->par_rollbacks += 1ull;
-        R.ctl->par_conflicts[2] += 1ull;
-        s_pull_end = s_cut;
-        s_cap = n;
-      }
-      __syncthreads();
-      continue;
-    }
-    if (tid == 0) {
-      if (mode == PM_PULL) {
-        s_att_acc += att;
-        s_p_acc += R.pcnt[min(T.seg_end, T.pull_end)] - R.pcnt[T.seg_start];
-        s_nseg += 1u;
-      }
-      s_c += (unsigned)att;
-      s_pos = T.seg_end;
-      s_cap = n;
-      s_split = 0;
-    }
-    __syncthreads();
-  }
-  if (tid == 0 && s_p_acc >= 256ull) R.ctl->att_ratio = (unsigned)(65536.0 * (double)s_att_acc / (double)s_p_acc);
-  if (lane == 0) {
-    unsigned long long* q = R.ctl->pprof;
-    atomicAdd(q + 4, pf.dep);
-    atomicAdd(q + 5, pf.start);
-    atomicAdd(q + 6, pf.load);
-    atomicAdd(q + 7, pf.pull);
-    atomicAdd(q + 8, pf.write);
-    atomicAdd(q + 9, pf.cells);
-    atomicAdd(q + 10, w_fetch);
-    atomicAdd(q + 11, w_total);
-    atomicAdd(q + 12, pf.cone);
-    atomicAdd(q + 13, pf.gate);
-    atomicAdd(q + 14, pf.npull);
-    atomicAdd(q + 15, pf.rounds);
-    atomicAdd(q + 16, pf.tread);
-    atomicAdd(q + 17, pf.tpw);
-  }
-  tp0 = clock64();
-  // ---- per-tick maps back to idle: positions, rows, pull-written cells
-  for (unsigned i = tid; i < n; i += NT_) {
-    const unsigned key = R.cells[i];
-    const unsigned cid = key_to_id(R, key, flip);
-    R.stamp[cid] = 0xFFFFFFFFu;
-    if (i == 0u || udiv(key, (unsigned)R.PX, R.mx) != udiv(R.cells[i - 1u], (unsigned)R.PX, R.mx)) {
+  for (unsigned g = warp; g < ngrp; g += NW_) {
+    const unsigned i = g * 32u + lane;
+    bool att = false, pp = false;
+    if (i < n) {
+      const unsigned cid = key_to_id(R, R.cells[i], flip);
       int x, y, z;
       dom_xyz(R, cid, x, y, z);
-      R.zrow[(size_t)y * (unsigned)R.PZ + (unsigned)(z - R.pz0)] = NOSLOT;
+      CD c[7];
+#pragma unroll
+      for (int l = 0; l < 7; ++l) {
+        int ox, oy, oz;
+        fp_off(l, ox, oy, oz);
+        c[l] = load_cell(R, ring, x + ox, y + oy, z + oz);
+      }
+      R.lv_ev[i] = 0u;
+      if (cd_solid(c[0])) {  // fluid.rs:586-589; nothing reads a solid cell's partial volume
+        if (c[0].slot != NOSLOT && c[0].part > 0.0f) {
+          R.avol[(size_t)c[0].slot * 512u + local_index(x, y, z)] = 0.0f;
+          pd -= 1;
+        }
+        reinterpret_cast<unsigned char*>(L.dep)[i] = DONE;
+      } else {
+        reinterpret_cast<unsigned char*>(L.dep)[i] = 0;
+        R.stamp[cid] = i;
+        unsigned fl = local_index(x, y, z) << 16;
+        unsigned sl[7];
+        att = cd_volume(c[0]) < FULL;
+#pragma unroll
+        for (int l = 0; l < 7; ++l) {
+          const bool so = cd_solid(c[l]);
+          sl[l] = c[l].slot != NOSLOT ? c[l].slot : (UNIFORM | c[l].mat);
+          fl |= so ? (1u << l) : 0u;
+          if (l >= 2) {
+            int ox, oy, oz;
+            fp_off(l, ox, oy, oz);
+            const bool st = !so && x + ox >= 0 && z + oz >= 0;
+            fl |= st ? (1u << (6 + l)) : 0u;
+            pp |= att && st && cd_volume(c[l]) >= FULL;
+          }
+        }
+        uint4* o = reinterpret_cast<uint4*>(R.lv + i);
+        o[0] = make_uint4(sl[0], sl[1], sl[2], sl[3]);
+        o[1] = make_uint4(sl[4], sl[5], sl[6], cid);
+        reinterpret_cast<uint2*>(o)[7] = make_uint2(fl, (unsigned)y);
+      }
+    }
+    const unsigned ab = __ballot_sync(FULLMASK, att), pb = __ballot_sync(FULLMASK, pp);
+    if (lane == 0) {
+      L.att[g] = ab;
+      L.pp[g] = pb;
     }
   }
+  __syncthreads();
+  // ---- attempts before each group, and the position from which the budget is spent at the latest
+  unsigned total_att;
   {
-    const unsigned np = min(R.ctl->ptn, MAX_PULLS_PER_TICK + 64u);
-    for (unsigned t = tid; t < np; t += NT_) {
-      const unsigned id = R.ptlist[t];
-      atomicAnd(R.ptbits + (id >> 5), ~(1u << (id & 31u)));
+    const unsigned per = (ngrp + NT_ - 1u) / NT_, g0 = min(ngrp, tid * per), g1 = min(ngrp, g0 + per);
+    unsigned c = 0;
+    for (unsigned g = g0; g < g1; ++g) c += (unsigned)__popc(L.att[g]);
+    unsigned run = cta_scan_count(sm, c, &total_att);
+    for (unsigned g = g0; g < g1; ++g) {
+      const unsigned a = L.att[g], k = (unsigned)__popc(a);
+      L.gpre[g] = (unsigned short)run;
+      if (run < MAX_PULLS_PER_TICK && run + k >= MAX_PULLS_PER_TICK) {
+        unsigned b = a;
+        for (unsigned r = run + 1u; r < MAX_PULLS_PER_TICK; ++r) b &= b - 1u;
+        L.kp = g * 32u + (unsigned)__ffs(b);  // after the last attempt of the budget
+      }
+      run += k;
     }
   }
-  // ---- the records in sorted order -> the tick's event logs (program order) and counters
+  __syncthreads();
+  const unsigned kp = L.kp;
+  for (unsigned g = kp / 32u + tid; g < ngrp; g += NT_) L.pp[g] &= g == kp / 32u ? (1u << (kp & 31u)) - 1u : 0u;
+  // ---- the later conflicting cells of every cell, and how many earlier ones each waits for
+  const int sgn = flip ? -1 : 1;
+  for (unsigned i = tid; i < n; i += NT_) {
+    if (reinterpret_cast<volatile unsigned char*>(L.dep)[i] == DONE) continue;
+    int x, y, z;
+    dom_xyz(R, R.lv[i].cid, x, y, z);
+    unsigned s[12];
+#pragma unroll
+    for (int q = 0; q < 12; ++q) {
+      int dx, dy, dz;
+      succ_offset(q, sgn, dx, dy, dz);
+      const unsigned r = (q < 11 || i < kp) ? rank_at(R, x + dx, y + dy, z + dz) : NOSLOT;
+      s[q] = r == NOSLOT ? NOSUCC : r;
+    }
+#pragma unroll
+    for (int q = 0; q < 12; ++q)
+      if (s[q] != NOSUCC) atomicAdd(&L.dep[s[q] >> 2], 1u << ((s[q] & 3u) * 8u));
+    uint4* o = reinterpret_cast<uint4*>(R.lv + i);
+    o[2] = make_uint4(s[0] | s[1] << 16, s[2] | s[3] << 16, s[4] | s[5] << 16, s[6] | s[7] << 16);
+    reinterpret_cast<uint2*>(o)[6] = make_uint2(s[8] | s[9] << 16, s[10] | s[11] << 16);
+  }
+  const int teams = (int)(NT_ / TEAM_THREADS);
+  __syncthreads();
+  if (warp == 0) lv_head(R, L, n, teams);
+  __syncthreads();
+  int gate = L.gate;
+  // ---- the first round: cells that wait for nobody
+  for (unsigned i = tid; i < n; i += NT_) {
+    if (reinterpret_cast<volatile unsigned char*>(L.dep)[i] != 0) continue;
+    if (R.lv[i].y <= gate) list_put(R, L, 0u, atomicAdd(&L.cnt[0], 1u), i);
+    else R.lv_park[atomicAdd(&L.park_n[0], 1u)] = (unsigned short)i;
+  }
+  __syncthreads();
+  plap(0);
+  // ---- rounds
+  unsigned cur = 0, cc = 0, pb = 0, rounds = 0, idle = 0;  // list, counter, parked list; the same on every thread
+  unsigned fcount = L.cnt[0], nres = 0;
+  bool alive = L.head < n, timeout = false;
+  const LaneSlot ls = lane_slot();
+  long long t_pull = 0;
+  while (true) {
+    const unsigned nb = cur ^ 1u, nc = cc == 2u ? 0u : cc + 1u, zc = nc == 2u ? 0u : nc + 1u;
+    if (tid == 0) L.cnt[zc] = 0u;
+    for (unsigned t0 = warp * 4u; t0 < fcount + nres; t0 += NW_ * 4u) {
+      const unsigned t = t0 + (lane >> 3);
+      const bool has = t < fcount + nres, pulled = has && t < nres;
+      unsigned i = 0, ev = 0;
+      float got = 0.0f;
+      if (pulled) {
+        i = L.s[t].pos;
+        got = L.s[t].got;
+        ev = L.res_ev[t];
+      } else if (has) {
+        i = list_get(R, L, cur, t - nres);
+      }
+      lv_cells(R, L, ls, has, i, pulled, got, ev, gate, kp, nb, nc, pb, pd, cap);
+    }
+    __syncthreads();
+    ++rounds;
+    nres = 0;
+    if (alive) {  // pulls are still possible: whose turn is it, which layers may run
+      if (warp == 0) lv_head(R, L, n, teams);
+      __syncthreads();
+      alive = L.head < n;
+      if (L.gate != gate) {
+        gate = L.gate;
+        const unsigned np = L.park_n[pb];
+        for (unsigned t = tid; t < np; t += NT_) {
+          const unsigned i = R.lv_park[(size_t)pb * MAX_CELLS_PER_TICK + t];
+          if (R.lv[i].y <= gate) list_put(R, L, nb, atomicAdd(&L.cnt[nc], 1u), i);
+          else R.lv_park[(size_t)(pb ^ 1u) * MAX_CELLS_PER_TICK + atomicAdd(&L.park_n[pb ^ 1u], 1u)] = (unsigned short)i;
+        }
+        __syncthreads();
+        if (tid == 0) L.park_n[pb] = 0u;
+        pb ^= 1u;
+      }
+      const int m = (int)L.nsearch;
+      if (m) {
+        const long long c0 = clock64();
+        lv_pulls(R, L, ring, m, pd, cap);
+        nres = L.ncommit;
+        t_pull += clock64() - c0;
+      }
+    }
+    cur = nb;
+    cc = nc;
+    fcount = L.cnt[cc];
+    idle = fcount + nres ? 0u : idle + 1u;
+    if (idle && !alive) break;
+    timeout = rounds >= cap || idle > 4u;  // an idle round with a pull pending cannot last: its search waits for a listed cell
+    if (timeout) break;
+  }
+  __syncthreads();
+  if (timeout) {
+    if (tid == 0) set_status(R, ST_TIMEOUT, 38);
+    __syncthreads();
+    return;
+  }
+  plap(1);
+  if (tid == 0) {
+    unsigned long long* q = R.ctl->pprof;
+    q[7] += (unsigned long long)t_pull;
+    q[9] += n;
+    q[14] += L.n_searches;
+    q[15] += rounds;
+    R.ctl->par_segments += rounds;
+    R.ctl->par_rollbacks += L.n_again;
+    R.ctl->par_replayed += L.n_searches;
+  }
+  // ---- the position map back to idle
+  for (unsigned i = tid; i < n; i += NT_) R.stamp[key_to_id(R, R.cells[i], flip)] = 0xFFFFFFFFu;
+  // ---- the cells' events in sorted order -> the tick's event logs (program order)
   __shared__ unsigned s_na, s_ns, s_nc;
   if (tid == 0) {
     s_na = 0;
@@ -952,24 +813,20 @@ __device__ __noinline__ void sweep_parallel(const Region& R, TickSmem& sm, WS& s
   __syncthreads();
   const unsigned pxy = (unsigned)R.PX * (unsigned)R.PY;
   const bool lr = sW.level_round;
-  unsigned long long c_att = 0, c_succ = 0, c_ent = 0, c_chg = 0, c_pd = 0;
+  unsigned any_chg = 0;
   for (unsigned base = 0; base < n; base += NT_) {
     const unsigned i = base + tid;
     unsigned am = 0, fl = 0, cm = 0, src = 0, cid = 0;
     if (i < n) {
-      const CellRec& rc = R.rec[i];
-      am = rc.amask;
-      fl = rc.flags;
-      cm = rc.cmask;
-      src = rc.src;
+      const unsigned e = R.lv_ev[i];
+      am = e & 0xFFu;
+      cm = (e >> 8) & 0xFFu;
+      fl = e >> 16;
       cid = key_to_id(R, R.cells[i], flip);
-      c_att += (fl & RF_ATTEMPT) ? 1u : 0u;
-      c_succ += (fl & RF_SUCCESS) ? 1u : 0u;
-      c_ent += rc.entries;
-      c_pd += (unsigned long long)(long long)rc.pdelta;
-      c_chg |= (fl & RF_CHANGED) ? 1u : 0u;
+      if (am & 1u) src = R.lv_src[i];
+      any_chg |= cm;
     }
-    const unsigned ns = lr ? 0u : (((fl & RF_SEED_SRC) ? 1u : 0u) + ((fl & RF_SEED_SELF) ? 1u : 0u));
+    const unsigned ns = lr ? 0u : (unsigned)__popc(fl & 3u);
     unsigned ta, ts, tc;
     const unsigned oa = cta_scan_count(sm, (unsigned)__popc(am), &ta);
     const unsigned os = cta_scan_count(sm, ns, &ts);
@@ -994,13 +851,13 @@ __device__ __noinline__ void sweep_parallel(const Region& R, TickSmem& sm, WS& s
         ++pa;
       }
       unsigned psd = s_ns + os;
-      if (ns) {
-        if (fl & RF_SEED_SRC) {
+      if (ns) {  // the pull's source, then the cell itself
+        if (fl & 2u) {
           if (psd < R.ev_seed_cap) R.ev_seed[psd] = src;
           else set_status(R, ST_OOM, 41);
           ++psd;
         }
-        if (fl & RF_SEED_SELF) {
+        if (fl & 1u) {
           if (psd < R.ev_seed_cap) R.ev_seed[psd] = cid;
           else set_status(R, ST_OOM, 41);
         }
@@ -1012,7 +869,6 @@ __device__ __noinline__ void sweep_parallel(const Region& R, TickSmem& sm, WS& s
         switch (l) {
           case 0: id = cid; break;
           case 1: id = cid - (unsigned)R.PX; break;
-          case 2: id = cid + (unsigned)R.PX; break;
           case 3: id = cid + 1u; break;
           case 4: id = cid - 1u; break;
           case 5: id = cid + pxy; break;
@@ -1032,20 +888,17 @@ __device__ __noinline__ void sweep_parallel(const Region& R, TickSmem& sm, WS& s
     }
     __syncthreads();
   }
-  c_att = cta_sum(sm, c_att);
-  c_succ = cta_sum(sm, c_succ);
-  c_ent = cta_sum(sm, c_ent);
-  c_chg = cta_sum(sm, c_chg);
-  c_pd = cta_sum(sm, c_pd);
+  const unsigned long long c_pd = cta_sum(sm, (unsigned long long)(long long)pd);
+  any_chg = __syncthreads_or((int)any_chg);
   if (tid == 0) {
     sW.nact = s_na;
     sW.nseed = s_ns;
     sW.nchg = s_nc;
-    sW.pull_attempts = c_att;
-    sW.pull_success = c_succ;
-    sW.bfs_visits = c_ent;
+    sW.pull_attempts = min(MAX_PULLS_PER_TICK, total_att + L.nx);
+    sW.pull_success = L.n_succ;
+    sW.bfs_visits = L.n_entries;
     sW.pdelta = (long long)c_pd;
-    sW.changed = c_chg != 0;
+    sW.changed = any_chg != 0;
   }
   __syncthreads();
   plap(3);
@@ -1254,8 +1107,8 @@ __device__ __noinline__ void level_finish_cta(const Region& R, TickSmem& sm, WS&
     if (__any_sync(FULLMASK, need)) materialize_par(R, need, c.gi, c.slot, cap);
     bool ch = false;
     if (wv) {
-      const SVPlan p = sv_plan(c, avg);
-      if (c.slot != NOSLOT) sv_apply(R, c, x, y, z, p);
+      const SVPlan p = sv_plan(c.part, c.mat, c.slot != NOSLOT, avg);
+      if (c.slot != NOSLOT) sv_apply(R, (size_t)c.slot * 512u + local_index(x, y, z), p);
       ch = p.ch;
       pd += p.dp;
     }
@@ -1557,7 +1410,7 @@ __device__ void run_ticks(const Region& R, TickSmem& sm, int n_ticks, Tune tune)
     __syncthreads();
     lap(1);
     // ---- the sweep (fluid.rs:584-651)
-    if (par) sweep_parallel(R, sm, sW, ring, n, flip, tune);
+    if (par) sweep_levels(R, sm, sW, ring, n, flip, tune);
     else sweep(R, sm, sW, ring, n, flip, tune);
     lap(2);
     if (par ? vld((const unsigned*)&R.ctl->status) != 0u : sm.u.s.abort != 0u) {
