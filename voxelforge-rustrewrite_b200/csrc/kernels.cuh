@@ -599,22 +599,19 @@ __device__ __noinline__ void sweep_levels(const Region& Rs, TickSmem& sm, WS& sW
   };
   int pd = 0;
   // ---- positions, footprints, and the cells that attempt a pull or may find a start cell
-  for (unsigned g = tid; g <= NGROUPS; g += NT_) {
-    L.pend[g] = 0u;
-    if (g >= ngrp) L.att[g] = L.pp[g] = 0u;
-  }
+  for (unsigned g = ngrp + tid; g <= NGROUPS; g += NT_) L.att[g] = L.pp[g] = 0u;
   for (unsigned g = tid; g < ngrp; g += NT_) R.pextra[g] = 0u;
+  for (unsigned t = tid; t < VIS_SLOTS; t += NT_) {
+    L.s.vkey[t] = EMPTY_ID;
+    L.s.vrank[t] = 0xFFFFFFFFu;
+  }
   if (tid == 0) {
     L.cnt[0] = L.cnt[1] = L.cnt[2] = 0u;
+    L.cur = L.cc = L.pb = 0u;
     L.park_n[0] = L.park_n[1] = 0u;
     L.nx = 0u;
     L.kp = n;
-    L.head = n;
-    L.hword = 0u;
-    L.hblk = 0u;
-    L.gate = -1;
-    L.lend = 0u;
-    L.nsearch = 0u;
+    L.rounds = L.resume = L.timeout = 0u;
     L.n_succ = L.n_searches = L.n_again = 0u;
     L.n_entries = 0ull;
   }
@@ -713,79 +710,78 @@ __device__ __noinline__ void sweep_levels(const Region& Rs, TickSmem& sm, WS& sW
     o[2] = make_uint4(s[0] | s[1] << 16, s[2] | s[3] << 16, s[4] | s[5] << 16, s[6] | s[7] << 16);
     reinterpret_cast<uint2*>(o)[6] = make_uint2(s[8] | s[9] << 16, s[10] | s[11] << 16);
   }
-  const int teams = (int)(NT_ / TEAM_THREADS);
   __syncthreads();
-  if (warp == 0) lv_head(R, L, n, teams);
+  if (warp == 0) {
+    HeadState H{n, 0u, 0u, 0u, -1, 0u};
+    lv_head(R, L, n, H);
+    if (lane == 0) L.h = H;
+  }
   __syncthreads();
-  int gate = L.gate;
+  int gate = L.h.gate;
   // ---- the first round: cells that wait for nobody
   for (unsigned i = tid; i < n; i += NT_) {
     if (reinterpret_cast<volatile unsigned char*>(L.dep)[i] != 0) continue;
     if (R.lv[i].y <= gate) list_put(R, L, 0u, atomicAdd(&L.cnt[0], 1u), i);
-    else R.lv_park[atomicAdd(&L.park_n[0], 1u)] = (unsigned short)i;
+    else park_put(R, 0u, atomicAdd(&L.park_n[0], 1u), i);
   }
   __syncthreads();
   plap(0);
   // ---- rounds
-  unsigned cur = 0, cc = 0, pb = 0, rounds = 0, idle = 0;  // list, counter, parked list; the same on every thread
-  unsigned fcount = L.cnt[0], nres = 0;
-  bool alive = L.head < n, timeout = false;
   const LaneSlot ls = lane_slot();
-  long long t_pull = 0;
+  long long t_wide = 0, t_search = 0;
   while (true) {
-    const unsigned nb = cur ^ 1u, nc = cc == 2u ? 0u : cc + 1u, zc = nc == 2u ? 0u : nc + 1u;
-    if (tid == 0) L.cnt[zc] = 0u;
-    for (unsigned t0 = warp * 4u; t0 < fcount + nres; t0 += NW_ * 4u) {
-      const unsigned t = t0 + (lane >> 3);
-      const bool has = t < fcount + nres, pulled = has && t < nres;
-      unsigned i = 0, ev = 0;
-      float got = 0.0f;
-      if (pulled) {
-        i = L.s[t].pos;
-        got = L.s[t].got;
-        ev = L.res_ev[t];
-      } else if (has) {
-        i = list_get(R, L, cur, t - nres);
-      }
-      lv_cells(R, L, ls, has, i, pulled, got, ev, gate, kp, nb, nc, pb, pd, cap);
-    }
+    // warp 0 alone decides what comes next: nobody else reads the lists' state while it runs
+    if (warp == 0) pd += lv_solo(Rs, L, ring, n, gate, sgn, cap);
     __syncthreads();
-    ++rounds;
-    nres = 0;
-    if (alive) {  // pulls are still possible: whose turn is it, which layers may run
-      if (warp == 0) lv_head(R, L, n, teams);
+    const unsigned req = L.req;
+    if (req == SR_END) break;
+    if (req == SR_SEARCH) {
+      const long long c0 = clock64();
+      search_cta(Rs, L, ring);
+      t_search += clock64() - c0;
+    } else if (req == SR_GATE) {
+      gate = L.h.gate;
+      const unsigned pb = L.pb, np = min(L.park_n[pb], MAX_CELLS_PER_TICK), lb = L.cur, lc = L.cc;
+      for (unsigned t = tid; t < np; t += NT_) {
+        const unsigned i = R.lv_park[(size_t)pb * MAX_CELLS_PER_TICK + t];
+        if (R.lv[i].y <= gate) list_put(R, L, lb, atomicAdd(&L.cnt[lc], 1u), i);
+        else park_put(R, pb ^ 1u, atomicAdd(&L.park_n[pb ^ 1u], 1u), i);
+      }
       __syncthreads();
-      alive = L.head < n;
-      if (L.gate != gate) {
-        gate = L.gate;
-        const unsigned np = L.park_n[pb];
-        for (unsigned t = tid; t < np; t += NT_) {
-          const unsigned i = R.lv_park[(size_t)pb * MAX_CELLS_PER_TICK + t];
-          if (R.lv[i].y <= gate) list_put(R, L, nb, atomicAdd(&L.cnt[nc], 1u), i);
-          else R.lv_park[(size_t)(pb ^ 1u) * MAX_CELLS_PER_TICK + atomicAdd(&L.park_n[pb ^ 1u], 1u)] = (unsigned short)i;
+      if (tid == 0) {
+        L.park_n[pb] = 0u;
+        L.pb = pb ^ 1u;
+      }
+      __syncthreads();
+    } else {
+      const long long c0 = clock64();
+      const bool alive = L.h.head < n;  // pulls are still possible: warp 0 looks after every round
+      unsigned cur = L.cur, cc = L.cc, rounds = L.rounds, fcount = min(L.cnt[cc], MAX_CELLS_PER_TICK);
+      const unsigned pb = L.pb;
+      do {
+        const unsigned nb = cur ^ 1u, nc = cc == 2u ? 0u : cc + 1u, zc = nc == 2u ? 0u : nc + 1u;
+        if (tid == 0) L.cnt[zc] = 0u;
+        for (unsigned t0 = warp * 4u; t0 < fcount; t0 += NW_ * 4u) {
+          const unsigned t = t0 + (lane >> 3);
+          const unsigned i = t < fcount ? list_get(R, L, cur, t) : 0u;
+          lv_cells(R, L, ls, t < fcount && !cell_done(L, i), i, false, 0.0f, 0u, gate, kp, nb, nc, pb, pd, cap);
         }
         __syncthreads();
-        if (tid == 0) L.park_n[pb] = 0u;
-        pb ^= 1u;
+        cur = nb;
+        cc = nc;
+        ++rounds;
+        fcount = min(L.cnt[cc], MAX_CELLS_PER_TICK);
+      } while (!alive && fcount > SOLO_CELLS && rounds < cap);
+      __syncthreads();  // everybody has read the count
+      if (tid == 0) {
+        L.cur = cur;
+        L.cc = cc;
+        L.rounds = rounds;
       }
-      const int m = (int)L.nsearch;
-      if (m) {
-        const long long c0 = clock64();
-        lv_pulls(R, L, ring, m, pd, cap);
-        nres = L.ncommit;
-        t_pull += clock64() - c0;
-      }
+      t_wide += clock64() - c0;
     }
-    cur = nb;
-    cc = nc;
-    fcount = L.cnt[cc];
-    idle = fcount + nres ? 0u : idle + 1u;
-    if (idle && !alive) break;
-    timeout = rounds >= cap || idle > 4u;  // an idle round with a pull pending cannot last: its search waits for a listed cell
-    if (timeout) break;
   }
-  __syncthreads();
-  if (timeout) {
+  if (L.timeout) {
     if (tid == 0) set_status(R, ST_TIMEOUT, 38);
     __syncthreads();
     return;
@@ -793,11 +789,12 @@ __device__ __noinline__ void sweep_levels(const Region& Rs, TickSmem& sm, WS& sW
   plap(1);
   if (tid == 0) {
     unsigned long long* q = R.ctl->pprof;
-    q[7] += (unsigned long long)t_pull;
+    q[7] += (unsigned long long)t_search;
+    q[8] += (unsigned long long)t_wide;
     q[9] += n;
     q[14] += L.n_searches;
-    q[15] += rounds;
-    R.ctl->par_segments += rounds;
+    q[15] += L.rounds;
+    R.ctl->par_segments += L.rounds;
     R.ctl->par_rollbacks += L.n_again;
     R.ctl->par_replayed += L.n_searches;
   }

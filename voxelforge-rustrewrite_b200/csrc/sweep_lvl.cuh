@@ -34,12 +34,11 @@ namespace vfe {
 
 constexpr unsigned GRID_LOCKED = 0xFFFFFFFFu;  // grid word while a warp materialises the brick
 constexpr int MAX_WARPS = 16;                  // warps of a CTA running the sweep
-constexpr int TEAM_WARPS = 4;                  // warps that run one pressure search together
-constexpr int TEAM_THREADS = 32 * TEAM_WARPS;
-constexpr int MAX_TEAMS = MAX_WARPS / TEAM_WARPS;
-constexpr unsigned TEAM_ENTRIES = TEAM_THREADS / 5;  // queue entries a search examines per round
-constexpr unsigned VIS_SLOTS = 1024;  // visited set of one search: <= 6 + 512 + 5 * TEAM_ENTRIES cells
-static_assert(6 + PRESSURE_SEARCH + 5 * TEAM_ENTRIES < VIS_SLOTS, "visited set");
+constexpr unsigned SOLO_CELLS = 4;             // a list this short is run by one warp (eight lanes per cell)
+constexpr unsigned SOLO_ENTRIES = 6;           // queue entries one warp examines per search round
+constexpr unsigned SOLO_WAIT = SOLO_ENTRIES;   // a search with more entries waiting goes to all warps
+constexpr unsigned VIS_SLOTS = 2048;           // visited set of a search: <= 6 + 512 + one round's 5 per entry (512)
+constexpr int VIS_SHIFT = 21;                  // hash bits kept: 32 - log2(VIS_SLOTS)
 constexpr unsigned NGROUPS = (MAX_CELLS_PER_TICK + 31) / 32;
 constexpr unsigned LIST_CAP = 4096;   // a round's list kept in shared memory; the rest goes to global
 constexpr unsigned NOSUCC = 0xFFFFu;
@@ -65,43 +64,50 @@ struct __align__(16) LvOld {
   unsigned wmask;  // footprint slots it wrote
 };
 
-// One pressure search (a team of TEAM_WARPS warps).
-enum SearchStatus { SS_NONE = 0, SS_SUCCESS = 1, SS_BLOCKED = 2 };
+// The pressure search under way.
+enum SearchStatus { SS_NONE = 0, SS_SUCCESS = 1, SS_BLOCKED = 2, SS_MORE = 3 };
 struct Search {
   unsigned q[PRESSURE_SEARCH];  // queued cells, relative to the pulling cell (rel_pack)
   float qv[PRESSURE_SEARCH];    // their volume
-  unsigned vkey[VIS_SLOTS];     // visited cells (EMPTY_ID = free)
+  unsigned vkey[VIS_SLOTS];     // visited cells (EMPTY_ID = free); all free between searches
   unsigned vrank[VIS_SLOTS];    // earliest (entry, direction) that tested the cell
-  float fv[8];                  // the pulling cell's footprint volumes
-  unsigned m_win[TEAM_WARPS], m_side[TEAM_WARPS], m_new[TEAM_WARPS];
+  unsigned short qh[PRESSURE_SEARCH + 8];  // visited slots of the queued cells, the pulling cell's at [512]
+  unsigned m_win[MAX_WARPS], m_side[MAX_WARPS], m_new[MAX_WARPS];
   unsigned blk;                 // 1 + an unfinished earlier cell the search depends on (0: none)
-  unsigned before;              // cells before this one that pulls took below full
-  unsigned pos, status, entries, qlen, hit, full;
-  float got, here;
+  unsigned pos, status, i, qlen, side;  // the cell, and the search's progress
+  float vol, got, here;         // its volume, what the pull takes, the source's volume
   int cx, cy, cz;               // the pulling cell
   int sx, sy, sz;               // the source
 };
+
+// What warp 0 asks of the CTA between rounds.
+enum SoloRequest { SR_LIST = 0, SR_GATE = 1, SR_SEARCH = 2, SR_END = 3 };
+// The first pp cell and what is known about it.
+struct HeadState {
+  unsigned head, word;  // its position (n: none), its group
+  unsigned blk;         // 1 + the cell its search waits for (0: none)
+  unsigned test;        // lv_prune: 0 to be tested, 1 + the cell the test waits for, or TEST_FAILED
+  int gate;             // its layer: cells above it wait
+  unsigned lend;        // first position after that layer
+};
+constexpr unsigned TEST_FAILED = 0xFFFFFFFFu;
 
 struct LvSmem {
   unsigned dep[(MAX_CELLS_PER_TICK + 3) / 4];  // a byte per cell: unfinished earlier conflicting cells, DONE
   unsigned att[NGROUPS + 1];   // bit per cell: not solid and below 1 - 1e-4 at the tick's start
   unsigned pp[NGROUPS + 1];    // bit per unfinished cell that may find a start cell within the budget
-  unsigned pend[NGROUPS + 1];  // bit per cell that reached its turn and has a start cell
   unsigned short gpre[NGROUPS + 1];  // att bits before each group of 32
   unsigned short list[2][LIST_CAP];
   unsigned cnt[3];             // list lengths, rotating: this round's, the next, the one being cleared
-  unsigned park_n[2];          // ready cells above the gate
+  unsigned cur, cc;            // the list and the counter of the next round
+  unsigned park_n[2], pb;      // ready cells above the gate, and which parked list holds them
   unsigned kp;                 // positions from here on cannot pull (budget spent before them)
   unsigned nx;                 // full cells pulls took from (Region::pxlist)
-  unsigned head, hword, hblk;  // first pp cell, its group, 1 + the cell its search waits for
-  int gate;                    // layer of the first pp cell: cells above it wait
-  unsigned lend;               // first position after that layer
-  unsigned nsearch, ncommit;   // pulls whose turn has come, those that commit
-  unsigned cand[MAX_TEAMS];
-  unsigned res_ev[MAX_TEAMS];
+  HeadState h;
+  unsigned req, rounds, resume, timeout;
   unsigned n_succ, n_searches, n_again;
   unsigned long long n_entries;
-  Search s[MAX_TEAMS];
+  Search s;
 };
 
 __device__ __forceinline__ unsigned vld(const unsigned* p) { return *(volatile const unsigned*)p; }
@@ -160,7 +166,15 @@ __device__ __forceinline__ CD load_cell_par(const Region& R, const int* ring, in
 // collective. The first warp to take a brick's grid word (CAS to GRID_LOCKED) allocates and fills the
 // slot and publishes it; the others read the published slot. A warp publishes every brick it has
 // locked before it waits for one, so two warps never wait for each other.
-__device__ void materialize_par(const Region& R, bool need, unsigned gi, unsigned& slot, unsigned long long cap) {
+// (By value: a Region behind a reference would keep the caller's copy out of registers.)
+struct AtlasRef {
+  unsigned* grid;
+  unsigned char* amat;
+  float* avol;
+  Ctl* ctl;
+  unsigned atlas_cap;
+};
+__device__ __noinline__ unsigned materialize_warp(AtlasRef R, bool need, unsigned gi, unsigned slot, unsigned long long cap) {
   const unsigned lane = lane_id();
   const unsigned key = need ? gi : (0xFFFFFFFFu - lane);
   const unsigned peers = __match_any_sync(FULLMASK, key);
@@ -176,7 +190,7 @@ __device__ void materialize_par(const Region& R, bool need, unsigned gi, unsigne
         if (atomicCAS(R.grid + gi, g, GRID_LOCKED) == g) {
           s = atomicAdd(&R.ctl->atlas_used, 1u);
           if (s >= R.atlas_cap) {
-            set_status(R, ST_OOM, 1);
+            if (atomicCAS(&R.ctl->status, 0, ST_OOM) == 0) R.ctl->err_info = 1;
             atomicExch(R.grid + gi, g);
             s = NOSLOT;
             open = false;
@@ -188,7 +202,7 @@ __device__ void materialize_par(const Region& R, bool need, unsigned gi, unsigne
         s = g - 256u;
         open = false;
       } else if (++spins > cap) {
-        set_status(R, ST_TIMEOUT, 31);
+        if (atomicCAS(&R.ctl->status, 0, ST_TIMEOUT) == 0) R.ctl->err_info = 31;
         open = false;
       } else {
         backoff(spins);
@@ -214,8 +228,11 @@ __device__ void materialize_par(const Region& R, bool need, unsigned gi, unsigne
   }
   const int src = need ? (__ffs(peers) - 1) : (int)lane;
   const unsigned s2 = __shfl_sync(FULLMASK, s, src);
-  if (need) slot = s2;
   __syncwarp();
+  return need ? s2 : slot;
+}
+__device__ __forceinline__ void materialize_par(const Region& R, bool need, unsigned gi, unsigned& slot, unsigned long long cap) {
+  slot = materialize_warp(AtlasRef{R.grid, R.amat, R.avol, R.ctl, R.atlas_cap}, need, gi, slot, cap);
 }
 
 // FluidSim::set_volume (fluid.rs:327-355) split into the decision and the stores.
@@ -278,54 +295,20 @@ __device__ __forceinline__ void rel_unpack(unsigned k, int& dx, int& dy, int& dz
   dy = (int)(k >> 22);
 }
 
-// The flow part of a cell's update (fluid.rs:606-650) from its footprint volumes, its solid cells
-// (bits) and its volume `vol` (> 0): 1. fall into the free capacity below, 2. share with lower sides
-// when supported, 3. evaporate crumbs. Every side's flow depends only on the volume after the fall
-// and that side's volume; only the running volume subtracts them in side order.
-struct FlowPlan {
-  float vol;          // the cell's volume afterwards (before the write-back test)
-  float below_new;    // the cell below's new volume when w_below
-  float side_new[4];  // +x, -x, +z, -z new volumes when their bit of wside is set
-  bool w_below;
-  unsigned wside;     // bit i: side i is written
-  unsigned amask;     // activation slots 2 (below) and 3..6 (sides)
-};
-__device__ __forceinline__ FlowPlan flow_plan(const float (&v)[7], unsigned solid, float vol) {
-  const float FULL = full_level();
-  FlowPlan P;
-  const bool below_solid = (solid >> 1) & 1u;
-  const float bv = below_solid ? 0.0f : v[1];
-  const float ff = fminf(vol, __fsub_rn(1.0f, bv));
-  P.w_below = !below_solid && ff > 1e-6f;
-  P.below_new = __fadd_rn(bv, ff);
-  vol = P.w_below ? __fsub_rn(vol, ff) : vol;
-  const float below_after = P.w_below ? (P.below_new >= FULL ? 1.0f : P.below_new) : bv;
-  const bool spread = vol > MIN_SPREAD && (below_solid || below_after >= FULL);
-  const float here = vol;
-  P.wside = 0u;
-  P.amask = P.w_below ? (1u << 2) : 0u;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const bool open = !((solid >> (3 + i)) & 1u);
-    const float nv = open ? v[3 + i] : 0.0f;
-    const float f = __fmul_rn(__fsub_rn(here, nv), 0.2f);
-    const bool ok = spread && open && !(nv >= here) && !(f < MIN_FLOW) && !(__fsub_rn(here, f) < MIN_SPREAD * 0.5f);
-    P.side_new[i] = __fadd_rn(nv, f);
-    P.wside |= ok ? (1u << i) : 0u;
-    vol = ok ? __fsub_rn(vol, f) : vol;
-    P.amask |= (ok && f > SLEEP) ? (1u << (3 + i)) : 0u;
-  }
-  P.vol = vol < EVAPORATE ? 0.0f : vol;
-  return P;
-}
-
 // ------------------------------------------------------------------------------- the lists
+// A cell enters a list once and the parked list once, so neither outgrows the tick's cells; the bounds
+// are checked all the same where an entry goes to global memory.
 __device__ __forceinline__ unsigned list_get(const Region& R, const LvSmem& L, unsigned b, unsigned t) {
   return t < LIST_CAP ? L.list[b][t] : R.lv_over[(size_t)b * MAX_CELLS_PER_TICK + t];
 }
 __device__ __forceinline__ void list_put(const Region& R, LvSmem& L, unsigned b, unsigned t, unsigned i) {
   if (t < LIST_CAP) L.list[b][t] = (unsigned short)i;
-  else R.lv_over[(size_t)b * MAX_CELLS_PER_TICK + t] = (unsigned short)i;
+  else if (t < MAX_CELLS_PER_TICK) R.lv_over[(size_t)b * MAX_CELLS_PER_TICK + t] = (unsigned short)i;
+  else set_status(R, ST_RANGE, 51);
+}
+__device__ __forceinline__ void park_put(const Region& R, unsigned b, unsigned t, unsigned i) {
+  if (t < MAX_CELLS_PER_TICK) R.lv_park[(size_t)b * MAX_CELLS_PER_TICK + t] = (unsigned short)i;
+  else set_status(R, ST_RANGE, 52);
 }
 __device__ __forceinline__ bool cell_done(const LvSmem& L, unsigned i) { return ((vld(&L.dep[i >> 2]) >> ((i & 3u) * 8u)) & 0xFFu) == DONE; }
 __device__ __forceinline__ bool bit_of(const unsigned* w, unsigned i) { return (w[i >> 5] >> (i & 31u)) & 1u; }
@@ -354,14 +337,15 @@ __device__ __forceinline__ LaneSlot lane_slot() {
 
 // Four cells at sorted positions i (fluid.rs:584-651), eight lanes each, warp-collective (groups
 // without a cell: `has` false). `pulled`: the cell's pull has run and took `got` (event bits `ev`);
-// otherwise a cell with a start cell is left pending for its pull. nb / nc: the next round's list and
-// its counter; pb: the parked list.
+// otherwise a cell with a start cell is left for its pull (lv_solo). nb / nc: the list that ready
+// successors join and its counter; pb: the parked list. Returns the cell's volume afterwards.
 //
 // Eight lanes rather than one thread per cell: a round is a latency chain (a few dozen to a few
 // hundred cells on 16 warps), and a lane that holds one slot issues one address, one pair of loads,
-// one set_volume and two successor counts where a thread issues seven, seven, six and twelve. The
-// exchange costs seven shuffles and five ballots.
-__device__ __forceinline__ void lv_cells(const Region& R, LvSmem& L, const LaneSlot& S, bool has, unsigned i, bool pulled, float got, unsigned ev,
+// one set_volume and two successor counts where a thread issues seven, seven, six and twelve. A
+// cell that is sure to run counts its successors down while its volumes are on their way: nobody
+// reads the next list before the round has ended.
+__device__ __forceinline__ float lv_cells(const Region& R, LvSmem& L, const LaneSlot& S, bool has, unsigned i, bool pulled, float got, unsigned ev,
                                          int gate, unsigned kp, unsigned nb, unsigned nc, unsigned pb, int& pd, unsigned long long cap) {
   const float FULL = full_level();
   const unsigned lane = lane_id(), l = lane & 7u, base = lane & 24u;
@@ -372,14 +356,13 @@ __device__ __forceinline__ void lv_cells(const Region& R, LvSmem& L, const LaneS
     w2 = p[8];
   }
   const unsigned flags = __shfl_sync(FULLMASK, w2, 6, 8);
-  const unsigned cid = __shfl_sync(FULLMASK, w1, 7, 8);
   const int y = (int)__shfl_sync(FULLMASK, w2, 7, 8);
   const bool cell = has && l < 7u && !((flags >> l) & 1u);  // the lane holds a cell that is not solid
   const unsigned loc = flags >> 16, at = (loc & ~S.lm) | ((loc + S.la) & S.lm);
   unsigned slot = cell ? w1 : UNIFORM, gi = 0;
   if (cell && (slot & UNIFORM)) {  // uniform at the tick's start: the value, or the slot the brick has now
     int x, yy, z;
-    dom_xyz(R, cid, x, yy, z);
+    dom_xyz(R, R.lv[i].cid, x, yy, z);
     gi = grid_index(R, (x + S.ox) >> 3, (yy + S.oy) >> 3, (z + S.oz) >> 3);
     const unsigned g = grid_word(R, gi, cap);
     slot = g < 256u ? (UNIFORM | g) : g - 256u;
@@ -391,20 +374,45 @@ __device__ __forceinline__ void lv_cells(const Region& R, LvSmem& L, const LaneS
     part = R.avol[o];
     mat = R.amat[o];
   }
-  const float v = part > 0.0f ? part : (cell && mat == WATER ? 1.0f : 0.0f);
   // ---- a cell that attempts a pull and has a start cell waits for the pull
-  const unsigned starts = (__ballot_sync(FULLMASK, cell && l >= 2u && ((flags >> (6u + l)) & 1u) && v >= FULL) >> base) & 0xFFu;
-  const float v0 = __shfl_sync(FULLMASK, v, 0, 8), bv = __shfl_sync(FULLMASK, v, 1, 8);
-  if (has && !pulled && i < kp && v0 < FULL && starts) {
-    if (l == 0u) {
-      atomicOr(&L.pend[i >> 5], 1u << (i & 31u));
-      if (!bit_of(L.pp, i)) set_status(R, ST_RANGE, 50);  // every cell that finds a start cell is in pp
+  if (__any_sync(FULLMASK, has && !pulled && i < kp && bit_of(L.pp, i))) {
+    const float v = part > 0.0f ? part : (cell && mat == WATER ? 1.0f : 0.0f);
+    const unsigned starts = (__ballot_sync(FULLMASK, cell && l >= 2u && ((flags >> (6u + l)) & 1u) && v >= FULL) >> base) & 0xFFu;
+    const float self = __shfl_sync(FULLMASK, v, 0, 8);
+    if (!pulled && i < kp && self < FULL && starts) has = false;
+  }
+  // ---- successors whose last earlier cell this was: to the next list, or parked above the gate
+  {
+    bool r0 = false, r1 = false;
+    if (has && l < 6u) {
+      const unsigned a = w2 & 0xFFFFu, b = w2 >> 16;
+      unsigned oa = 0, ob = 0;
+      if (a != NOSUCC) oa = atomicSub(&L.dep[a >> 2], 1u << ((a & 3u) * 8u)) >> ((a & 3u) * 8u);
+      if (b != NOSUCC) ob = atomicSub(&L.dep[b >> 2], 1u << ((b & 3u) * 8u)) >> ((b & 3u) * 8u);
+      r0 = (oa & 0xFFu) == 1u;
+      r1 = (ob & 0xFFu) == 1u;
     }
-    has = false;
+    const unsigned shut = (y + 1 > gate ? S.open1 : 0u) | (y + 2 > gate ? S.open2 : 0u);
+    const bool p0 = r0 && !(shut & 1u), p1 = r1 && !(shut & 2u);
+    const unsigned g0 = __ballot_sync(FULLMASK, p0), g1 = __ballot_sync(FULLMASK, p1);
+    if (g0 | g1) {
+      unsigned t = 0;
+      if (lane == 0u) t = atomicAdd(&L.cnt[nc], (unsigned)(__popc(g0) + __popc(g1)));
+      t = __shfl_sync(FULLMASK, t, 0);
+      if (p0) list_put(R, L, nb, t + (unsigned)__popc(g0 & lanemask_lt()), w2 & 0xFFFFu);
+      if (p1) list_put(R, L, nb, t + (unsigned)(__popc(g0) + __popc(g1 & lanemask_lt())), w2 >> 16);
+    }
+    if ((r0 && !p0) || (r1 && !p1)) {
+      unsigned t = atomicAdd(&L.park_n[pb], (r0 && !p0 ? 1u : 0u) + (r1 && !p1 ? 1u : 0u));
+      if (r0 && !p0) park_put(R, pb, t++, w2 & 0xFFFFu);
+      if (r1 && !p1) park_put(R, pb, t, w2 >> 16);
+    }
   }
   // ---- 1. fall into the free capacity below, 2. share with lower sides when supported, 3. evaporate
   // crumbs (fluid.rs:606-650). Every side's flow depends on the volume after the fall and its own
   // volume only; the running volume subtracts the flows in side order (a side without one: 0).
+  const float v = part > 0.0f ? part : (cell && mat == WATER ? 1.0f : 0.0f);
+  const float v0 = __shfl_sync(FULLMASK, v, 0, 8), bv = __shfl_sync(FULLMASK, v, 1, 8);
   float vol = pulled && got > 0.0f ? __fadd_rn(v0, got) : v0;
   const bool live = has && vol > 0.0f;  // fluid.rs:602-604
   const bool below_solid = (flags >> 1) & 1u;
@@ -431,58 +439,33 @@ __device__ __forceinline__ void lv_cells(const Region& R, LvSmem& L, const LaneS
     materialize_par(R, need, gi, s, cap);
     if (need && s != NOSLOT) slot = s;
   }
-  const bool hs = !(slot & UNIFORM);
   SVPlan p{};
   if (wr) {
+    const bool hs = !(slot & UNIFORM);
     p = sv_plan(part, (unsigned char)mat, hs, wv);
     if (hs) sv_apply(R, (size_t)slot * 512u + at, p);
     pd += p.dp;
   }
-  const unsigned wm = (__ballot_sync(FULLMASK, wr) >> base) & 0x7Fu;
-  const unsigned cm = (__ballot_sync(FULLMASK, wr && p.ch) >> base) & 0x7Fu;
-  const unsigned am = (__ballot_sync(FULLMASK, l == 1u ? w_below : ok && f > SLEEP) >> base) & 0x7Au;  // slots 1, 3..6
-  bool r0 = false, r1 = false;  // the lane's successors whose last earlier cell this was
+  const unsigned wm = __ballot_sync(FULLMASK, wr) >> base;
+  const unsigned cm = __ballot_sync(FULLMASK, wr && p.ch) >> base;
+  const unsigned am = __ballot_sync(FULLMASK, l == 1u ? w_below : ok && f > SLEEP) >> base;
   if (has) {
     if (y == gate) reinterpret_cast<unsigned*>(R.lv_old + i)[l] = l == 7u ? wm : __float_as_uint(v);
     if (l == 0u) {
       // activation slots: 2 below, 3..6 the sides, 7 the cell itself
       const bool self = live && dv > SLEEP;
-      R.lv_ev[i] = ev | (am & 0x78u) | ((am & 2u) << 1) | (self ? 0x10080u : 0u) | (cm << 8);
-      atomicOr(&L.dep[i >> 2], DONE << ((i & 3u) * 8u));
+      R.lv_ev[i] = ev | (am & 0x78u) | ((am & 2u) << 1) | (self ? 0x10080u : 0u) | ((cm & 0x7Fu) << 8);
+      reinterpret_cast<volatile unsigned char*>(L.dep)[i] = (unsigned char)DONE;
       if (i < kp && bit_of(L.pp, i)) atomicAnd(&L.pp[i >> 5], ~(1u << (i & 31u)));
     }
-    if (l < 6u) {
-      const unsigned a = w2 & 0xFFFFu, b = w2 >> 16;
-      unsigned oa = 0, ob = 0;
-      if (a != NOSUCC) oa = atomicSub(&L.dep[a >> 2], 1u << ((a & 3u) * 8u));
-      if (b != NOSUCC) ob = atomicSub(&L.dep[b >> 2], 1u << ((b & 3u) * 8u));
-      r0 = a != NOSUCC && ((oa >> ((a & 3u) * 8u)) & 0xFFu) == 1u;
-      r1 = b != NOSUCC && ((ob >> ((b & 3u) * 8u)) & 0xFFu) == 1u;
-    }
-  }
-  // ---- the ready ones: to the next round, or parked above the gate
-  const unsigned shut = (y + 1 > gate ? S.open1 : 0u) | (y + 2 > gate ? S.open2 : 0u);
-  const unsigned g0 = __ballot_sync(FULLMASK, r0 && !(shut & 1u)), g1 = __ballot_sync(FULLMASK, r1 && !(shut & 2u));
-  if (g0 | g1) {
-    unsigned t = 0;
-    if (lane == 0u) t = atomicAdd(&L.cnt[nc], (unsigned)(__popc(g0) + __popc(g1)));
-    t = __shfl_sync(FULLMASK, t, 0);
-    if (r0 && !(shut & 1u)) list_put(R, L, nb, t + (unsigned)__popc(g0 & lanemask_lt()), w2 & 0xFFFFu);
-    if (r1 && !(shut & 2u)) list_put(R, L, nb, t + (unsigned)(__popc(g0) + __popc(g1 & lanemask_lt())), w2 >> 16);
-  }
-  if ((r0 && (shut & 1u)) || (r1 && (shut & 2u))) {
-    unsigned t = atomicAdd(&L.park_n[pb], (r0 && (shut & 1u) ? 1u : 0u) + (r1 && (shut & 2u) ? 1u : 0u));
-    if (r0 && (shut & 1u)) R.lv_park[(size_t)pb * MAX_CELLS_PER_TICK + t++] = (unsigned short)(w2 & 0xFFFFu);
-    if (r1 && (shut & 2u)) R.lv_park[(size_t)pb * MAX_CELLS_PER_TICK + t] = (unsigned short)(w2 >> 16);
   }
   __syncwarp();
+  return vol;
 }
 
 // --------------------------------------------------------------------------- pressure search
-__device__ __forceinline__ void team_sync(int team) { asm volatile("bar.sync %0, %1;" ::"r"(1 + team), "r"(TEAM_THREADS) : "memory"); }
-
 __device__ __forceinline__ unsigned vis_slot(Search& C, unsigned key) {
-  unsigned h = (key * 2654435761u) >> 22;  // 10 bits
+  unsigned h = (key * 2654435761u) >> VIS_SHIFT;
   while (true) {
     const unsigned old = atomicCAS(&C.vkey[h], EMPTY_ID, key);
     if (old == EMPTY_ID || old == key) return h;
@@ -490,14 +473,11 @@ __device__ __forceinline__ unsigned vis_slot(Search& C, unsigned key) {
   }
 }
 
-// The volume a cell (a, y, c) of the pulling layer holds at the turn of the cell at position k, given
-// the volume `v` it holds now: later cells that already ran and wrote it are looked through (the
-// earliest such write's old value); an unfinished earlier writer is reported in C.blk.
-__device__ float old_volume(const Region& R, const LvSmem& L, Search& C, unsigned k, int a, int y, int c, float v) {
-  unsigned j[5];
-#pragma unroll
-  for (int q = 0; q < 5; ++q)  // the writers of the cell: itself, and the sides it is a side of
-    j[q] = rank_at(R, a - (q == 1) + (q == 2), y, c - (q == 3) + (q == 4));
+// The volume a cell of the pulling layer holds at the turn of the cell at position k, given the volume
+// `v` it holds now and the positions j of its writers (itself, and the cells it is a side of): later
+// ones that already ran and wrote it are looked through (the earliest such write's old value); an
+// unfinished earlier writer is reported in C.blk.
+__device__ __forceinline__ float old_volume(const Region& R, const LvSmem& L, Search& C, unsigned k, const unsigned (&j)[5], float v) {
   unsigned best = NOSLOT;
 #pragma unroll
   for (int q = 0; q < 5; ++q) {
@@ -508,267 +488,343 @@ __device__ float old_volume(const Region& R, const LvSmem& L, Search& C, unsigne
     } else if (done && j[q] < best) {
       const LvOld& o = R.lv_old[j[q]];
       const int fl = q == 0 ? 0 : q + 2;
-      if ((o.wmask >> fl) & 1u) {
+      const unsigned wm = o.wmask;
+      const float ov = o.vol[fl];
+      if ((wm >> fl) & 1u) {
         best = j[q];
-        v = o.vol[fl];
+        v = ov;
       }
     }
   }
   return v;
 }
 
-// FluidSim::pressure_pull (fluid.rs:511-561) of the cell at position k, by one team; writes nothing but
-// C. TEAM_ENTRIES queue entries per round, one neighbour per thread, the reference's queue order kept
-// exactly: the first surface entry in queue order wins; the 24 side checks at the start level are
-// counted in (entry, direction) order; a cell found by several threads of a round belongs to the
-// earliest (vrank). Entries past the 512th are never examined, so appends stop there.
-__device__ void lv_search(const Region& R, LvSmem& L, const int* ring, int team, unsigned k, unsigned long long cap) {
-  Search& C = L.s[team];
+// What a search round's thread finds: its queue entry's neighbour d.
+struct SearchRead {
+  unsigned key;  // the neighbour, packed
+  float here, v;
+  bool win, cand, side;
+};
+__device__ __forceinline__ SearchRead search_read(const Region& R, LvSmem& L, const int* ring, bool act, unsigned e, unsigned d, bool sides) {
+  Search& C = L.s;
+  SearchRead r{0u, 0.0f, 0.0f, false, false, false};
+  if (act) {
+    int a, b, c, dx, dy, dz;
+    rel_unpack(C.q[e], a, b, c);
+    r.here = C.qv[e];
+    dir5((int)d, dx, dy, dz);
+    dx += a;
+    dy += b;
+    dz += c;
+    const int x = C.cx + dx, y = C.cy + dy, z = C.cz + dz;
+    // (once the 24 side checks at the start level are spent, what its cells hold no longer matters)
+    const bool rd = d == 0u ? y < R.ny : (x >= 0 && z >= 0 && (sides || dy != 0));
+    bool top = true;
+    if (rd && !outside(R, ring, x, y, z)) {
+      // the grid word and, on the pulling layer, the writers' positions: issued together
+      const unsigned g = gld(R.grid + grid_index(R, x >> 3, y >> 3, z >> 3));
+      unsigned j[5] = {NOSLOT, NOSLOT, NOSLOT, NOSLOT, NOSLOT};
+      if (dy == 0) {
+#pragma unroll
+        for (int q = 0; q < 5; ++q) j[q] = rank_at(R, x - (q == 1) + (q == 2), y, z - (q == 3) + (q == 4));
+      }
+      const size_t o = g < 256u ? (size_t)0 : (size_t)(g - 256u) * 512u + local_index(x, y, z);
+      const float part = R.avol[o];
+      const unsigned am = R.amat[o], m = g < 256u ? g : am;
+      if (m == 0u || m == WATER) {
+        r.v = g >= 256u && part > 0.0f ? part : (m == WATER ? 1.0f : 0.0f);
+        if (dy == 0) r.v = old_volume(R, L, C, C.pos, j, r.v);
+        top = r.v <= 0.0f;
+      }
+    }
+    // the surface test of the entry on its up neighbour (fluid.rs:534-535), else an expansion
+    r.win = d == 0u && top && b > 0 && r.here > 0.0f;
+    r.cand = rd && !top;
+    r.side = r.cand && d != 0u && dy == 0;
+    r.key = rel_pack(dx, dy, dz);
+  }
+  return r;
+}
+
+__device__ __forceinline__ void search_won(Search& C, const SearchRead& r, unsigned e) {
+  int a, b, c;
+  rel_unpack(C.q[e], a, b, c);
+  C.sx = C.cx + a;
+  C.sy = C.cy + b;
+  C.sz = C.cz + c;
+  C.here = r.here;
+  C.got = fminf(__fsub_rn(1.0f, C.vol), r.here);
+  C.status = SS_SUCCESS;
+  C.i = e + 1u;
+}
+
+// FluidSim::pressure_pull (fluid.rs:511-561) of the cell at position k: its start, by one warp. Writes
+// nothing but L.s. Returns whether there is anything to examine.
+__device__ __forceinline__ bool search_begin(const Region& R, LvSmem& L, const int* ring, unsigned k, unsigned long long cap) {
+  Search& C = L.s;
   const float FULL = full_level();
-  const unsigned tt = threadIdx.x % TEAM_THREADS, tw = tt >> 5, lane = tt & 31u;
+  const unsigned lane = lane_id();
   const LvCell& rc = R.lv[k];
   const unsigned flags = rc.flags;
   int x, y, z;
   dom_xyz(R, rc.cid, x, y, z);
-  for (unsigned t = tt; t < VIS_SLOTS; t += TEAM_THREADS) {
-    C.vkey[t] = EMPTY_ID;
-    C.vrank[t] = 0xFFFFFFFFu;
-  }
-  if (tt < 7u) {
+  float v = 0.0f;
+  if (lane < 7u && !((flags >> lane) & 1u)) {
     int ox, oy, oz;
-    fp_off((int)tt, ox, oy, oz);
-    const CD c = load_cell_par(R, ring, x + ox, y + oy, z + oz, cap);
-    C.fv[tt] = cd_solid(c) ? 0.0f : cd_volume(c);
+    fp_off((int)lane, ox, oy, oz);
+    v = cd_volume(load_cell_par(R, ring, x + ox, y + oy, z + oz, cap));
   }
-  if (tt == 0) {
-    C.blk = 0u;
-    C.before = 0u;
+  const float vol = __shfl_sync(FULLMASK, v, 0);
+  unsigned starts = (__ballot_sync(FULLMASK, lane >= 2u && lane < 7u && ((flags >> (6u + lane)) & 1u) && v >= FULL) >> 2) & 31u;
+  unsigned before = attempts_before(L, k);
+  if (before + L.nx >= MAX_PULLS_PER_TICK) {  // near the budget: the cells before this one that pulls took below full
+    unsigned c = 0;
+    for (unsigned t = lane; t < L.nx; t += 32u) c += R.pxlist[t] < k ? 1u : 0u;
+    before += __reduce_add_sync(FULLMASK, c);
+  }
+  if (!(vol < FULL) || before >= MAX_PULLS_PER_TICK) starts = 0u;
+  if (lane == 0) {
     C.pos = k;
     C.status = SS_NONE;
-    C.entries = 0u;
-    C.qlen = 0u;
-    C.hit = 0u;
-    C.full = 0u;
+    C.blk = 0u;
+    C.i = 0u;
+    C.side = 0u;
+    C.qlen = (unsigned)__popc(starts);
+    C.vol = vol;
     C.got = 0.0f;
     C.cx = x;
     C.cy = y;
     C.cz = z;
   }
-  team_sync(team);
-  {
-    unsigned c = 0;
-    for (unsigned t = tt; t < L.nx; t += TEAM_THREADS) c += R.pxlist[t] < k ? 1u : 0u;
-    if (c) atomicAdd(&C.before, c);
-  }
-  team_sync(team);
-  const float vol = C.fv[0];
-  unsigned starts = 0u;
-#pragma unroll
-  for (int d = 0; d < 5; ++d) starts |= (((flags >> (8 + d)) & 1u) && C.fv[2 + d] >= FULL) ? (1u << d) : 0u;
-  if (!(vol < FULL) || attempts_before(L, k) + C.before >= MAX_PULLS_PER_TICK || !starts) return;
-  if (tt == 0) {
-    C.vrank[vis_slot(C, rel_pack(0, 0, 0))] = 0u;
-    unsigned p = 0;
-    for (int d = 0; d < 5; ++d) {
-      if (!((starts >> d) & 1u)) continue;
-      int dx, dy, dz;
-      dir5(d, dx, dy, dz);
-      const unsigned key = rel_pack(dx, dy, dz);
-      C.q[p] = key;
-      C.qv[p] = C.fv[2 + d];
-      C.vrank[vis_slot(C, key)] = ++p;
-    }
-  }
-  team_sync(team);
-  const unsigned j = tt / 5u, d = tt - 5u * j;
-  unsigned qlen = (unsigned)__popc(starts), i = 0, side = 0;
-  while (i < qlen && i < PRESSURE_SEARCH) {
-    const unsigned kk = min(TEAM_ENTRIES, min(qlen, PRESSURE_SEARCH) - i);
-    const bool act = j < kk;
-    int a = 0, b = 0, c = 0, dx = 0, dy = 0, dz = 0;
-    float here = 0.0f, v = 0.0f;
-    bool rd = false, so = true;
-    unsigned key = 0;
-    if (act) {
-      key = C.q[i + j];
-      here = C.qv[i + j];
-      rel_unpack(key, a, b, c);
-      dir5((int)d, dx, dy, dz);
-      dx += a;
-      dy += b;
-      dz += c;
-      const int na = x + dx, nb = y + dy, nc = z + dz;
-      rd = d == 0u ? nb < R.ny : (na >= 0 && nc >= 0);
-      if (rd) {
-        const CD cd = load_cell_par(R, ring, na, nb, nc, cap);
-        so = cd_solid(cd);
-        v = so ? 0.0f : cd_volume(cd);
-        if (!so && dy == 0) v = old_volume(R, L, C, k, na, nb, nc, v);
+  if (starts) {
+    // the start cells in direction order; visited ranks 0 (the cell itself), 1..5
+    const unsigned d = lane - 2u;
+    const bool st = lane >= 2u && lane < 7u && ((starts >> d) & 1u);
+    if (st || lane == 0u) {
+      int dx = 0, dy = 0, dz = 0;
+      if (st) dir5((int)d, dx, dy, dz);
+      const unsigned key = rel_pack(dx, dy, dz), h = vis_slot(C, key);
+      C.vrank[h] = st ? d + 1u : 0u;
+      const unsigned p = st ? (unsigned)__popc(starts & ((1u << d) - 1u)) : PRESSURE_SEARCH;
+      C.qh[p] = (unsigned short)h;
+      if (st) {
+        C.q[p] = key;
+        C.qv[p] = v;
       }
     }
-    // surface test of each entry on its up neighbour (fluid.rs:534-535)
-    const bool top = so || v <= 0.0f;
-    const bool win = act && d == 0u && top && b > 0 && here > 0.0f;
-    bool cand = rd && !top;
-    const bool scnt = cand && d >= 1u && dy == 0;
-    const unsigned wmk = __ballot_sync(FULLMASK, win), smk = __ballot_sync(FULLMASK, scnt);
-    if (lane == 0) {
-      C.m_win[tw] = wmk;
-      C.m_side[tw] = smk;
-    }
-    team_sync(team);
-    if (C.blk) {  // an earlier cell has yet to write what the search read: run it again later
-      if (tt == 0) C.status = SS_BLOCKED;
-      return;
-    }
-    int wt = -1;
-    unsigned sbefore = side, sall = side;
-#pragma unroll
-    for (int w = 0; w < TEAM_WARPS; ++w) {
-      const unsigned m = C.m_win[w];
-      if (m && wt < 0) wt = 32 * w + __ffs(m) - 1;
-      const unsigned sc = (unsigned)__popc(C.m_side[w]);
-      if ((unsigned)w < tw) sbefore += sc;
-      sall += sc;
-    }
-    if (wt >= 0) {
-      if ((int)tt == wt) {
-        C.sx = x + a;
-        C.sy = y + b;
-        C.sz = z + c;
-        C.here = here;
-        C.got = fminf(__fsub_rn(1.0f, vol), here);
-        C.status = SS_SUCCESS;
-        C.entries = i + j + 1u;
-        C.qlen = min(qlen, PRESSURE_SEARCH);
-      }
-      team_sync(team);
+  }
+  __syncwarp();
+  return starts != 0u;
+}
+
+// Search rounds by one warp, SOLO_ENTRIES queue entries each, one neighbour per lane, the reference's
+// queue order kept exactly: the first surface entry in queue order wins; the 24 side checks at the
+// start level are counted in (entry, direction) order; a cell several lanes find belongs to the
+// earliest. Ends with C.status, or SS_MORE when many entries wait (all warps take over).
+__device__ __forceinline__ void search_solo(const Region& R, LvSmem& L, const int* ring) {
+  Search& C = L.s;
+  const unsigned lane = lane_id(), j = lane / 5u, d = lane - 5u * j;
+  unsigned i = C.i, qlen = C.qlen, side = C.side, status = SS_NONE;
+  while (i < qlen) {
+    if (qlen - i > SOLO_WAIT || qlen + 5u * SOLO_ENTRIES > PRESSURE_SEARCH) {
+      status = SS_MORE;
       break;
     }
+    const unsigned kk = min(SOLO_ENTRIES, qlen - i);
+    const SearchRead r = search_read(R, L, ring, j < kk, i + j, d, side < 24u);
+    __syncwarp();
+    if (vld(&C.blk)) {  // an earlier cell has yet to write what the search read: run it again later
+      status = SS_BLOCKED;
+      break;
+    }
+    const unsigned wm = __ballot_sync(FULLMASK, r.win);
+    if (wm) {
+      const unsigned wl = (unsigned)__ffs(wm) - 1u;
+      if (lane == wl) {
+        search_won(C, r, i + j);
+        C.qlen = qlen;
+      }
+      __syncwarp();
+      return;
+    }
+    const unsigned sm = __ballot_sync(FULLMASK, r.side);
+    const bool cand = r.cand && !(r.side && side + (unsigned)__popc(sm & lanemask_lt()) + 1u > 24u);
+    side += (unsigned)__popc(sm);
+    const unsigned rank = 6u + (i + j) * 5u + d;
+    unsigned h = 0;
+    if (cand) {
+      h = vis_slot(C, r.key);
+      atomicMin(&C.vrank[h], rank);
+    }
+    __syncwarp();
+    const bool isnew = cand && vld(&C.vrank[h]) == rank;
+    const unsigned nm = __ballot_sync(FULLMASK, isnew);
+    const unsigned pos = qlen + (unsigned)__popc(nm & lanemask_lt());
+    if (isnew && pos < PRESSURE_SEARCH) {
+      C.q[pos] = r.key;
+      C.qv[pos] = r.v;
+      C.qh[pos] = (unsigned short)h;
+    }
+    qlen += (unsigned)__popc(nm);
+    i += kk;
+    __syncwarp();
+  }
+  if (lane == 0) {
+    C.status = status;
+    C.i = i;
+    C.qlen = qlen;
+    C.side = side;
+  }
+  __syncwarp();
+}
+
+// The same rounds by all warps of the CTA, six entries each in queue order, until the search ends.
+// Entries past the 512th are never examined (fluid.rs:530), so appends stop there. All threads; ends
+// with a barrier, the visited set empty.
+__device__ __noinline__ void search_cta(const Region& Rs, LvSmem& L, const int* ring) {
+  const Region R = Rs;
+  Search& C = L.s;
+  const unsigned tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, nw = blockDim.x >> 5;
+  const unsigned jl = lane / 5u, d = lane - 5u * jl, j = warp * SOLO_ENTRIES + jl;  // lanes 30, 31 idle
+  unsigned i = C.i, qlen = C.qlen, side = C.side;
+  while (i < qlen && i < PRESSURE_SEARCH) {
+    const unsigned kk = min(SOLO_ENTRIES * nw, min(qlen, PRESSURE_SEARCH) - i);
+    const SearchRead r = search_read(R, L, ring, jl < SOLO_ENTRIES && j < kk, i + j, d, side < 24u);
+    const unsigned wm = __ballot_sync(FULLMASK, r.win), smk = __ballot_sync(FULLMASK, r.side);
+    // no more than 24 side checks at the start level (fluid.rs:546-549): their order over the warps
+    // matters only in the round that passes the limit
+    if (lane == 0) {
+      C.m_win[warp] = wm;
+      C.m_side[warp] = smk;
+    }
+    __syncthreads();
+    if (C.blk) {
+      if (tid == 0) C.status = SS_BLOCKED;
+      break;
+    }
+    const unsigned wmine = lane < nw ? C.m_win[lane] : 0u, smine = lane < nw ? C.m_side[lane] : 0u;
+    const unsigned wany = __ballot_sync(FULLMASK, wmine != 0u), sany = __ballot_sync(FULLMASK, smine != 0u);
+    if (wany) {
+      if (warp == (unsigned)__ffs(wany) - 1u && lane == (unsigned)__ffs(wm) - 1u) search_won(C, r, i + j);
+      break;
+    }
+    bool cand = r.cand;
+    if (sany) {
+      const unsigned c = (unsigned)__popc(smine);
+      const unsigned before = __reduce_add_sync(FULLMASK, lane < warp ? c : 0u);
+      if (r.side && side + before + (unsigned)__popc(smk & lanemask_lt()) + 1u > 24u) cand = false;
+      side += __reduce_add_sync(FULLMASK, c);
+    }
     if (qlen < PRESSURE_SEARCH) {
-      // expansions (fluid.rs:541-556)
-      if (scnt && sbefore + (unsigned)__popc(smk & lanemask_lt()) + 1u > 24u) cand = false;
-      side = sall;
       const unsigned rank = 6u + (i + j) * 5u + d;
       unsigned h = 0;
       if (cand) {
-        key = rel_pack(dx, dy, dz);
-        h = vis_slot(C, key);
+        h = vis_slot(C, r.key);
         atomicMin(&C.vrank[h], rank);
       }
-      team_sync(team);
+      __syncthreads();
       const bool isnew = cand && vld(&C.vrank[h]) == rank;
-      const unsigned nmk = __ballot_sync(FULLMASK, isnew);
-      if (lane == 0) C.m_new[tw] = nmk;
-      team_sync(team);
-      unsigned pos = qlen + (unsigned)__popc(nmk & lanemask_lt()), all = 0;
-#pragma unroll
-      for (int w = 0; w < TEAM_WARPS; ++w) {
-        const unsigned nw = (unsigned)__popc(C.m_new[w]);
-        if ((unsigned)w < tw) pos += nw;
-        all += nw;
-      }
+      const unsigned nm = __ballot_sync(FULLMASK, isnew);
+      if (lane == 0) C.m_new[warp] = (unsigned)__popc(nm);
+      __syncthreads();
+      const unsigned c = lane < nw ? C.m_new[lane] : 0u;
+      const unsigned before = __reduce_add_sync(FULLMASK, lane < warp ? c : 0u), all = __reduce_add_sync(FULLMASK, c);
+      const unsigned pos = qlen + before + (unsigned)__popc(nm & lanemask_lt());
       if (isnew && pos < PRESSURE_SEARCH) {
-        C.q[pos] = key;
-        C.qv[pos] = v;
+        C.q[pos] = r.key;
+        C.qv[pos] = r.v;
       }
       qlen += all;
     }
     i += kk;
-    team_sync(team);
+    __syncthreads();
   }
-  if (tt == 0) {
-    if (C.status != SS_SUCCESS) {
-      C.entries = i;
-      C.qlen = min(qlen, PRESSURE_SEARCH);
-    } else {
-      // does the pull leave its own cell full? (its flow is planned on the footprint just read)
-      float fv[7];
-#pragma unroll
-      for (int l = 0; l < 7; ++l) fv[l] = C.fv[l];
-      const FlowPlan P = flow_plan(fv, flags & 0x7Fu, __fadd_rn(vol, C.got));
-      C.full = P.vol >= FULL ? 1u : 0u;
+  __syncthreads();
+  if (tid == 0 && C.status == SS_MORE) {
+    C.status = SS_NONE;
+    C.i = i;
+  }
+  for (unsigned t = tid; t < VIS_SLOTS; t += blockDim.x) {
+    C.vkey[t] = EMPTY_ID;
+    C.vrank[t] = 0xFFFFFFFFu;
+  }
+  __syncthreads();
+}
+
+// The end of a pull, one warp: the source's write (fluid.rs:536-540), then the cell itself.
+__device__ __forceinline__ void pull_end(const Region& R, LvSmem& L, const int* ring, const LaneSlot& S, int gate, unsigned kp, unsigned cur, unsigned cc,
+                                         unsigned pb, int& pd, unsigned long long cap) {
+  Search& C = L.s;
+  const unsigned lane = lane_id(), k = C.pos;
+  unsigned ev = 0u;
+  if (C.status == SS_SUCCESS) {
+    const float nv = __fsub_rn(C.here, C.got);
+    CD c = CD{0.0f, NOSLOT, 0u, 0, true};
+    if (lane == 0) c = load_cell_par(R, ring, C.sx, C.sy, C.sz, cap);
+    const bool need = lane == 0 && c.slot == NOSLOT && set_volume_needs_slot(c, nv);
+    if (__any_sync(FULLMASK, need)) materialize_par(R, need, c.gi, c.slot, cap);
+    if (lane == 0) {
+      const unsigned sid = dom_id(R, C.sx, C.sy, C.sz);
+      const unsigned j = R.stamp[sid];
+      const SVPlan p = sv_plan(c.part, c.mat, c.slot != NOSLOT, nv);
+      if (c.slot != NOSLOT) sv_apply(R, (size_t)c.slot * 512u + local_index(C.sx, C.sy, C.sz), p);
+      pd += p.dp;
+      R.lv_src[k] = sid;
+      // activation slots 0 (the source) and 1 (around the cell); bit 17 seeds the source
+      ev = 3u | (p.ch ? 0x8000u : 0u) | (2u << 16);
+      // a drained source that was full attempts a pull of its own when its turn comes
+      if (j != NOSLOT && nv < full_level() && !bit_of(L.att, j) && !((R.pextra[j >> 5] >> (j & 31u)) & 1u)) {
+        R.pextra[j >> 5] |= 1u << (j & 31u);
+        R.pxlist[L.nx] = j;
+        L.nx += 1u;
+        if (j < kp) L.pp[j >> 5] |= 1u << (j & 31u);
+      }
+      L.n_succ += 1u;
     }
+    ev = __shfl_sync(FULLMASK, ev, 0);
   }
-}
-
-// Did the search of team w read the source of team o's pull (as a queue entry or beside one)?
-__device__ void lv_hits(LvSmem& L, int w, int o) {
-  Search& C = L.s[w];
-  const Search& S = L.s[o];
-  const int rx = S.sx - C.cx, ry = S.sy - C.cy, rz = S.sz - C.cz;
-  bool hit = false;
-  for (unsigned t = threadIdx.x % TEAM_THREADS; t < C.qlen; t += TEAM_THREADS) {
-    int a, b, c;
-    rel_unpack(C.q[t], a, b, c);
-    const int ex = abs(rx - a), ey = ry - b, ez = abs(rz - c);
-    hit |= (ey == 0 || ey == 1) && ex + ez + ey <= 1;
-  }
-  if (hit) atomicOr(&C.hit, 1u << o);
-}
-
-// The write of a committed pull's source (fluid.rs:536-540), one warp.
-__device__ void lv_source(const Region& R, LvSmem& L, const int* ring, int team, int& pd, unsigned long long cap) {
-  const Search& C = L.s[team];
-  const unsigned lane = lane_id();
-  const float nv = __fsub_rn(C.here, C.got);
-  CD c = CD{0.0f, NOSLOT, 0u, 0, true};
-  if (lane == 0) c = load_cell_par(R, ring, C.sx, C.sy, C.sz, cap);
-  const bool need = lane == 0 && c.slot == NOSLOT && set_volume_needs_slot(c, nv);
-  if (__any_sync(FULLMASK, need)) materialize_par(R, need, c.gi, c.slot, cap);
   if (lane == 0) {
-    const unsigned sid = dom_id(R, C.sx, C.sy, C.sz);
-    const SVPlan p = sv_plan(c.part, c.mat, c.slot != NOSLOT, nv);
-    if (c.slot != NOSLOT) sv_apply(R, (size_t)c.slot * 512u + local_index(C.sx, C.sy, C.sz), p);
-    pd += p.dp;
-    R.lv_src[C.pos] = sid;
-    // activation slots 0 (the source) and 1 (around the cell); bit 17 seeds the source
-    L.res_ev[team] = 3u | (p.ch ? 0x8000u : 0u) | (2u << 16);
-    // a drained source that was full attempts a pull of its own when its turn comes
-    const unsigned j = R.stamp[sid];
-    if (j != NOSLOT && nv < full_level() && !bit_of(L.att, j) && !(atomicOr(R.pextra + (j >> 5), 1u << (j & 31u)) & (1u << (j & 31u)))) {
-      R.pxlist[atomicAdd(&L.nx, 1u)] = j;
-      if (j < L.kp) atomicOr(&L.pp[j >> 5], 1u << (j & 31u));
+    L.n_entries += C.i;
+    L.n_searches += 1u;
+  }
+  __syncwarp();
+  const float vol = lv_cells(R, L, S, lane < 8u, k, true, C.got, ev, gate, kp, cur, cc, pb, pd, cap);
+  if (lane == 0u && ev && vol >= full_level()) {
+    // a pull that leaves its own cell full gives its later neighbours on the layer a start cell
+    const LvCell& rc = R.lv[k];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const unsigned nb = rc.succ[q == 0 ? 0 : 3];
+      if (nb != NOSUCC && nb < kp && bit_of(L.att, nb)) L.pp[nb >> 5] |= 1u << (nb & 31u);
     }
   }
   __syncwarp();
 }
 
-// After a round, one warp: the first pp cell in sorted order and its layer (the gate), and the pulls
-// whose turn has come: the first pp cells that are all pending, up to one per team (none while the
-// first one waits for an earlier cell).
-__device__ void lv_head(const Region& R, LvSmem& L, unsigned n, int teams) {
+// Finds the first pp cell in sorted order and its layer (the gate), one warp.
+__device__ __forceinline__ void lv_head(const Region& R, LvSmem& L, unsigned n, HeadState& H) {
   const unsigned lane = lane_id(), ngrp = (n + 31u) / 32u;
-  if (L.head < n && bit_of(L.pp, L.head) && (!bit_of(L.pend, L.head) || (L.hblk && !cell_done(L, L.hblk - 1u)))) {
-    if (lane == 0) L.nsearch = 0u;  // the first pp cell has yet to have its turn
-    return;
-  }
-  unsigned w = L.hword;
-  unsigned P = 0, any = 0;
+  unsigned w = H.word, P = 0, any = 0;
   while (w < ngrp) {
-    P = w + lane < ngrp ? L.pp[w + lane] : 0u;
+    P = w + lane < ngrp ? vld(&L.pp[w + lane]) : 0u;
     any = __ballot_sync(FULLMASK, P != 0u);
     if (any) break;
     w += 32u;
   }
+  H.blk = H.test = 0u;
   if (!any) {
-    if (lane == 0) {
-      L.hword = ngrp;
-      L.head = n;
-      L.gate = 0x7FFFFFFF;
-      L.nsearch = 0u;
-    }
+    H.word = ngrp;
+    H.head = n;
+    H.gate = 0x7FFFFFFF;
     return;
   }
   const int fl = __ffs(any) - 1;
-  const unsigned head = (w + (unsigned)fl) * 32u + (unsigned)__ffs(__shfl_sync(FULLMASK, P, fl)) - 1u;
-  const unsigned old = L.head, hblk = head == old ? L.hblk : 0u;
-  int gate = L.gate;
-  unsigned lend = L.lend;
-  if (head >= lend) {  // a new gate layer: its first position after the layer, by a 32-way search
-    gate = R.lv[head].y;
-    const unsigned lim = (unsigned)(gate + 1) * (unsigned)R.PZ * (unsigned)R.PX;
-    unsigned lo = head, hi = n;  // cells[lo] is on the layer; the answer lies in (lo, hi]
+  H.word = w + (unsigned)fl;
+  H.head = H.word * 32u + (unsigned)__ffs(__shfl_sync(FULLMASK, P, fl)) - 1u;
+  if (H.head >= H.lend) {  // a new gate layer: its first position after the layer, by a 32-way search
+    H.gate = R.lv[H.head].y;
+    const unsigned lim = (unsigned)(H.gate + 1) * (unsigned)R.PZ * (unsigned)R.PX;
+    unsigned lo = H.head, hi = n;  // cells[lo] is on the layer; the answer lies in (lo, hi]
     while (hi - lo > 1u) {
       const unsigned st = (hi - lo + 31u) / 32u, p = lo + (lane + 1u) * st;
       const unsigned b = __ballot_sync(FULLMASK, p < hi && R.cells[p] < lim);
@@ -777,88 +833,163 @@ __device__ void lv_head(const Region& R, LvSmem& L, unsigned n, int teams) {
       lo = nlo;
       hi = nhi;
     }
-    lend = hi;
-  }
-  __syncwarp();
-  const bool ready = bit_of(L.pend, head) && (hblk == 0u || cell_done(L, hblk - 1u));
-  unsigned m = 0;
-  if (ready) {
-    const unsigned D = w + lane < ngrp ? L.pend[w + lane] : 0u;
-    const unsigned no = P & ~D;  // pp cells whose turn has not come: candidates end before the first
-    const unsigned nb = __ballot_sync(FULLMASK, no != 0u);
-    const int nl = nb ? __ffs(nb) - 1 : 32;
-    unsigned c = (int)lane < nl ? P : ((int)lane == nl ? P & ((no & (0u - no)) - 1u) : 0u);
-    while (m < (unsigned)teams) {
-      const unsigned cb = __ballot_sync(FULLMASK, c != 0u);
-      if (!cb) break;
-      if ((int)lane == __ffs(cb) - 1) {
-        L.cand[m] = (w + lane) * 32u + (unsigned)__ffs(c) - 1u;
-        c &= c - 1u;
-      }
-      ++m;
-    }
-  }
-  if (lane == 0) {
-    L.hword = w + (unsigned)fl;
-    L.head = head;
-    L.hblk = hblk;
-    L.gate = gate;
-    L.lend = lend;
-    L.nsearch = m;
+    H.lend = hi;
   }
 }
 
-// The searches of the pulls lv_head picked, side by side; the longest prefix whose searches would have
-// found the same one after another commits. All threads; ends with a barrier.
-__device__ void lv_pulls(const Region& R, LvSmem& L, const int* ring, int m, int& pd, unsigned long long cap) {
-  const unsigned tid = threadIdx.x;
-  const int team = (int)(tid / TEAM_THREADS);
-  if (team < m) lv_search(R, L, ring, team, L.cand[team], cap);
-  __syncthreads();
-  if (m > 1) {
-    if (team < m && L.s[team].status != SS_BLOCKED)
-      for (int o = 0; o < team; ++o)
-        if (L.s[o].status == SS_SUCCESS) lv_hits(L, team, o);
-    __syncthreads();
+// 1 + the last unfinished earlier cell of the pulling layer within three rows and columns of the cell
+// at position k (0: none). A search examines at most 24 sides on its own layer, so nearly all it reads
+// there is written by these cells: one probe per lane here instead of a search that finds out.
+__device__ __forceinline__ unsigned lv_near(const Region& R, const LvSmem& L, unsigned k, int sgn) {
+  const unsigned lane = lane_id();
+  int x, y, z;
+  dom_xyz(R, R.lv[k].cid, x, y, z);
+  // lanes 0..20: the three rows before, x - 3 .. x + 3; 21..23: the three cells before in the row
+  const int row = (int)lane / 7, dx = lane < 21u ? (int)lane - 7 * row - 3 : -sgn * ((int)lane - 20);
+  const int dz = lane < 21u ? -sgn * (row + 1) : 0;
+  unsigned w = 0u;
+  if (lane < 24u) {
+    const unsigned p = rank_at(R, x + dx, y, z + dz);
+    if (p != NOSLOT && !cell_done(L, p)) w = p + 1u;
   }
-  if (tid == 0) {
-    int c = 0;
-    unsigned won = 0u;
-    while (c < m) {
-      const Search& S = L.s[c];
-      if (S.status == SS_BLOCKED) {
-        if (c == 0) L.hblk = S.blk;
-        L.n_again += 1u;
-        break;
+  return __reduce_max_sync(FULLMASK, w);
+}
+
+// The first pp cell has yet to have its turn: can it still find a start cell then? A full neighbour
+// stays full unless it runs before the cell does and falls: a side earlier in sorted order, over a
+// cell that no unfinished cell writes and that has room (a full cell makes no attempt, and a fall of
+// 2e-4 leaves it below 1 - 1e-4). A cell whose full neighbours all do that will not pull and leaves
+// pp: later pulls need not wait for it. Returns 0 = it will not pull, 1 + a cell to wait for before
+// the test can tell, or TEST_FAILED.
+__device__ __forceinline__ unsigned lv_prune(const Region& R, LvSmem& L, const int* ring, unsigned k, unsigned long long cap) {
+  const unsigned lane = lane_id();
+  const LvCell& rc = R.lv[k];
+  const unsigned flags = rc.flags;
+  int x, y, z;
+  dom_xyz(R, rc.cid, x, y, z);
+  const float FULL = full_level();
+  // lanes 8m .. 8m + 7 (m = 0..3) look at side m; lane 0 at the cell above too
+  const unsigned m = lane >> 3, q = lane & 7u;
+  const int ax = x + (m == 0u) - (m == 1u), az = z + (m == 2u) - (m == 3u);
+  bool fail = false;
+  unsigned wait = 0u;
+  if (lane == 0u && ((flags >> 8) & 1u)) fail = cd_volume(load_cell_par(R, ring, x, y + 1, z, cap)) >= FULL;
+  if ((flags >> (9u + m)) & 1u) {
+    if (cd_volume(load_cell_par(R, ring, ax, y, az, cap)) >= FULL) {
+      if (q == 0u) {  // the side itself: earlier and unfinished
+        const unsigned p = rank_at(R, ax, y, az);
+        fail |= p == NOSLOT || p > k || cell_done(L, p);
+      } else if (q == 1u) {  // room below it
+        const CD b = load_cell_par(R, ring, ax, y - 1, az, cap);
+        fail |= cd_solid(b) || !(__fsub_rn(1.0f, cd_volume(b)) >= 2e-4f);
       }
-      if (S.hit & won) break;
-      L.res_ev[c] = 0u;
-      L.pend[S.pos >> 5] &= ~(1u << (S.pos & 31u));
-      bool stop = false;
-      if (S.status == SS_SUCCESS) {
-        won |= 1u << c;
-        L.n_succ += 1u;
-        if (S.full) {  // its later neighbours on the layer may start from it
-          const LvCell& rc = R.lv[S.pos];
-#pragma unroll
-          for (int q = 0; q < 2; ++q) {
-            const unsigned nb = rc.succ[q == 0 ? 0 : 3];
-            if (nb == NOSUCC || nb >= L.kp || !bit_of(L.att, nb) || bit_of(L.pp, nb)) continue;
-            L.pp[nb >> 5] |= 1u << (nb & 31u);
-            stop |= c + 1 < m && nb < L.cand[c + 1];
-          }
+      if (q < 5u) {  // the cells that may still write the cell below it
+        const unsigned p = rank_at(R, ax + (q == 1u) - (q == 2u), y - 1, az + (q == 3u) - (q == 4u));
+        if (p != NOSLOT && !cell_done(L, p)) wait = p + 1u;
+      }
+    }
+  }
+  // room below is final only once nobody writes it: wait first
+  const unsigned hard = __ballot_sync(FULLMASK, fail && q != 1u), soft = __ballot_sync(FULLMASK, fail);
+  const unsigned w = __reduce_max_sync(FULLMASK, wait);
+  return hard ? TEST_FAILED : w ? w : soft ? TEST_FAILED : 0u;
+}
+
+// Between the CTA's rounds, warp 0: the pulls whose turn has come, in order, and the rounds that are
+// too short for the CTA. Ends with a request to the CTA: run the list, open the gate (L.gate changed
+// from `gate`), carry on the search, or the sweep's end. Returns the change in partial entries.
+__device__ __noinline__ int lv_solo(const Region& Rs, LvSmem& L, const int* ring, unsigned n, int gate, int sgn, unsigned long long cap) {
+  const Region R = Rs;
+  const LaneSlot S = lane_slot();
+  int pd = 0;
+  __syncwarp();
+  const unsigned lane = lane_id(), kp = L.kp;
+  HeadState H = L.h;
+  unsigned req, cur = L.cur, cc = L.cc, rounds = L.rounds;
+  const unsigned pb = L.pb;
+  bool finish = L.resume != 0u;
+  unsigned steps = 0;
+  while (true) {
+    if (++steps > 8u * MAX_CELLS_PER_TICK) {  // more than the tick's pulls and rounds: cannot happen
+      if (lane == 0) L.timeout = 1u;
+      req = SR_END;
+      break;
+    }
+    if (!finish && H.head < n) {
+      if (!((vld(&L.pp[H.head >> 5]) >> (H.head & 31u)) & 1u)) {
+        lv_head(R, L, n, H);
+        if (H.gate != gate) {
+          req = SR_GATE;
+          break;
         }
       }
-      L.n_entries += S.entries;
-      L.n_searches += 1u;
-      ++c;
-      if (stop) break;
+      const unsigned dep = (vld(&L.dep[H.head >> 2]) >> ((H.head & 3u) * 8u)) & 0xFFu;
+      if (dep == 0u) {  // its turn has come
+        if (H.blk == 0u || cell_done(L, H.blk - 1u)) H.blk = lv_near(R, L, H.head, sgn);
+        if (H.blk == 0u) {
+          if (search_begin(R, L, ring, H.head, cap)) {
+            search_solo(R, L, ring);
+            if (L.s.status == SS_MORE) {
+              req = SR_SEARCH;
+              break;
+            }
+            // leave the visited set empty
+            for (unsigned t = lane; t <= L.s.qlen; t += 32u) {
+              const unsigned h = L.s.qh[t < L.s.qlen ? t : PRESSURE_SEARCH];
+              L.s.vkey[h] = EMPTY_ID;
+              L.s.vrank[h] = 0xFFFFFFFFu;
+            }
+          }
+          finish = true;
+        }
+      } else if (H.test == 0u || (H.test != TEST_FAILED && cell_done(L, H.test - 1u))) {
+        H.test = lv_prune(R, L, ring, H.head, cap);
+        if (H.test == 0u) {
+          if (lane == 0) L.pp[H.head >> 5] &= ~(1u << (H.head & 31u));
+          __syncwarp();
+          continue;
+        }
+      }
     }
-    L.ncommit = (unsigned)c;
+    if (finish) {
+      finish = false;
+      if (L.s.status == SS_BLOCKED) {
+        H.blk = L.s.blk;
+        if (lane == 0) L.n_again += 1u;
+      } else {
+        pull_end(R, L, ring, S, gate, kp, cur, cc, pb, pd, cap);
+      }
+      continue;
+    }
+    const unsigned cnt = vld(&L.cnt[cc]);
+    if (cnt == 0u || rounds >= cap) {  // with a pull pending a listed cell is always left: a stuck sweep ends as a timeout
+      if (lane == 0) L.timeout = cnt != 0u || H.head < n ? 1u : 0u;
+      req = SR_END;
+      break;
+    }
+    if (cnt > SOLO_CELLS) {
+      req = SR_LIST;
+      break;
+    }
+    const unsigned nc = cc == 2u ? 0u : cc + 1u, zc = nc == 2u ? 0u : nc + 1u;
+    if (lane == 0) L.cnt[zc] = 0u;
+    const unsigned t = lane >> 3;
+    const unsigned i = t < cnt ? list_get(R, L, cur, t) : 0u;
+    lv_cells(R, L, S, t < cnt && !cell_done(L, i), i, false, 0.0f, 0u, gate, kp, cur ^ 1u, nc, pb, pd, cap);
+    cur ^= 1u;
+    cc = nc;
+    ++rounds;
   }
-  __syncthreads();
-  if (team < (int)L.ncommit && L.s[team].status == SS_SUCCESS && tid % TEAM_THREADS < 32u) lv_source(R, L, ring, team, pd, cap);
-  __syncthreads();
+  __syncwarp();
+  if (lane == 0) {
+    L.req = req;
+    L.resume = req == SR_SEARCH ? 1u : 0u;
+    L.h = H;
+    L.cur = cur;
+    L.cc = cc;
+    L.rounds = rounds;
+  }
+  return pd;
 }
 
 }  // namespace vfe
