@@ -494,8 +494,11 @@ int vf_fluid_apply_voxel_edits(vf_fluid* h, const vf_voxel* edits, uint64_t n) {
     q[4 * i + 3] = edits[i].m;
   }
   CK(cudaMemcpyAsync(h->scratch, q.data(), n * 16, cudaMemcpyHostToDevice, h->stream));
-  k_edit<<<1, 32, 0, h->stream>>>(h->R, ED_VOXELS, (const int*)h->scratch, n, 0, 0.0f, nullptr);
-  CK(cudaGetLastError());
+  for (uint64_t o = 0; o < n; o += 1u << 30) {  // (positions in the list are 32-bit)
+    const unsigned m = (unsigned)std::min<uint64_t>(n - o, 1u << 30);
+    k_voxel_edits<<<1, EDIT_THREADS, 0, h->stream>>>(h->R, (const int4*)h->scratch + o, m, h->tune.spin_cap);
+    CK(cudaGetLastError());
+  }
   return sync_ctl(h);
 }
 
@@ -512,6 +515,15 @@ int vf_fluid_wake(vf_fluid* h, int32_t x0, int32_t y0, int32_t z0, int32_t x1, i
   return sync_ctl(h);
 }
 
+// The kernel of an edit over a list in device memory: emitters and carving run in parallel, what may
+// displace water one cell after another.
+static cudaError_t launch_edit(vf_fluid* h, int kind, const int* dev_xyz, uint64_t n, int m, float amount, unsigned long long* dcount) {
+  if (kind == ED_EMIT) k_emit<<<1, EDIT_THREADS, 0, h->stream>>>(h->R, dev_xyz, n, amount, h->tune.spin_cap);
+  else if (kind == ED_BRUSH && m == 0) k_carve<<<1, EDIT_THREADS, 0, h->stream>>>(h->R, dev_xyz, n, dcount, h->tune.spin_cap);
+  else k_edit<<<1, 32, 0, h->stream>>>(h->R, kind, dev_xyz, n, m, amount, dcount);
+  return cudaGetLastError();
+}
+
 static int run_edit(vf_fluid* h, int kind, const int32_t* xyz, uint64_t n, int m, float amount, uint64_t* out_count, size_t ints_per) {
   int rc = check(h);
   if (rc) return rc;
@@ -519,8 +531,7 @@ static int run_edit(vf_fluid* h, int kind, const int32_t* xyz, uint64_t n, int m
   if ((rc = ensure_scratch(h, data + 64))) return rc;
   if (n) CK(cudaMemcpyAsync(h->scratch, xyz, n * ints_per * 4, cudaMemcpyHostToDevice, h->stream));
   unsigned long long* dcount = (unsigned long long*)((char*)h->scratch + data);
-  k_edit<<<1, 32, 0, h->stream>>>(h->R, kind, (const int*)h->scratch, n, m, amount, out_count ? dcount : nullptr);
-  CK(cudaGetLastError());
+  CK(launch_edit(h, kind, (const int*)h->scratch, n, m, amount, out_count ? dcount : nullptr));
   if (out_count) {
     unsigned long long c = 0;
     CK(cudaMemcpyAsync(&c, dcount, 8, cudaMemcpyDeviceToHost, h->stream));
@@ -1263,8 +1274,7 @@ int vf_fluid_emit_device_async(vf_fluid* h, const int32_t* dev_xyz, uint64_t n, 
   int rc = check(h);
   if (rc) return rc;
   DeviceScope scope(h->device);  // the caller's current device is given back on return
-  k_edit<<<1, 32, 0, h->stream>>>(h->R, ED_EMIT, dev_xyz, n, 0, amount, nullptr);
-  CK(cudaGetLastError());
+  CK(launch_edit(h, ED_EMIT, dev_xyz, n, 0, amount, nullptr));
   return VF_OK;
 }
 
@@ -1272,8 +1282,7 @@ int vf_fluid_brush_device_async(vf_fluid* h, const int32_t* dev_xyz, uint64_t n,
   int rc = check(h);
   if (rc) return rc;
   DeviceScope scope(h->device);  // the caller's current device is given back on return
-  k_edit<<<1, 32, 0, h->stream>>>(h->R, ED_BRUSH, dev_xyz, n, m, 0.0f, nullptr);
-  CK(cudaGetLastError());
+  CK(launch_edit(h, ED_BRUSH, dev_xyz, n, m, 0.0f, nullptr));
   return VF_OK;
 }
 
