@@ -1132,19 +1132,159 @@ __device__ __noinline__ void level_finish_cta(const Region& R, TickSmem& sm, WS&
   __syncthreads();
 }
 
+// A small layer's flood fill by one warp, without touching the marks: the cells in the reference's
+// order, and every cell it tested (a set: the marks it would leave). Several run side by side; the
+// layers of one batch are the same or disjoint (their members do not change while it lasts), so the
+// smallest cell id tells them apart.
+constexpr unsigned FILL_CELLS = 64, FILL_SLOTS = 512;
+static_assert(4 * FILL_CELLS + 1 < FILL_SLOTS, "tested cells of a small layer");
+enum FillKind { FK_KEEP = 0, FK_LEVEL = 1, FK_DRAIN = 2, FK_BIG = 3, FK_DUP = 4 };
+struct LevelFill {
+  unsigned id[FILL_CELLS];
+  float vol[FILL_CELLS];
+  unsigned key[FILL_SLOTS];  // tested cells (EMPTY_ID = free)
+  unsigned len, kind, min_id;
+  float avg;
+};
+
+__device__ void level_fill_small(const Region& R, const int* ring, LevelFill& F, unsigned sid) {
+  const unsigned lane = lane_id();
+  const float FULL = full_level();
+  for (unsigned t = lane; t < FILL_SLOTS; t += 32u) F.key[t] = EMPTY_ID;
+  __syncwarp();
+  auto test = [&](unsigned id) {  // true: tested before
+    unsigned h = (id * 2654435761u) >> 23;
+    while (true) {
+      const unsigned old = atomicCAS(&F.key[h], EMPTY_ID, id);
+      if (old == EMPTY_ID) return false;
+      if (old == id) return true;
+      h = (h + 1u) & (FILL_SLOTS - 1u);
+    }
+  };
+  int sx, sy, sz;
+  dom_xyz(R, sid, sx, sy, sz);
+  float v0;
+  level_member(R, ring, sx, sy, sz, &v0);
+  if (lane == 0) {
+    test(sid);
+    F.id[0] = sid;
+    F.vol[0] = v0;
+  }
+  __syncwarp();
+  unsigned len = 1, kind = FK_KEEP, mn = sid;
+  for (unsigned i = 0; i < len; ++i) {
+    int x, y, z;
+    dom_xyz(R, F.id[i], x, y, z);
+    // lanes 0..11: side d = lane / 3, its cell (j = 0), the one below (1) and above (2)
+    const int d = (int)lane / 3, j = (int)lane % 3;
+    int dx = 0, dz = 0;
+    if (lane < 12u) side4(d, dx, dz);
+    const int nx = x + dx, nz = z + dz;
+    const bool skip = lane >= 12u || (R.ring_w == 0 && (nx < 0 || nz < 0));
+    bool seen = true;
+    unsigned nid = EMPTY_ID;
+    if (!skip && j == 0 && in_dom(R, nx, y, nz)) {
+      nid = dom_id(R, nx, y, nz);
+      seen = mark_test(R, nx, y, nz) || test(nid);
+    }
+    CD c = CD{0.0f, NOSLOT, 0u, 0, true};
+    if (!skip) c = load_cell(R, ring, nx, y + (j == 1 ? -1 : (j == 2 ? 1 : 0)), nz);
+    const float v = cd_volume(c);
+    const bool sol = cd_solid(c);
+    const float v1 = __shfl_down_sync(FULLMASK, v, 1), v2 = __shfl_down_sync(FULLMASK, v, 2);
+    const bool s1 = __shfl_down_sync(FULLMASK, (unsigned)sol, 1) != 0u;
+    const bool push = !skip && j == 0 && !seen && !sol && v > 0.0f && (s1 || v1 >= FULL) && v2 <= 0.0f;
+    const unsigned pm = __ballot_sync(FULLMASK, push);
+    if (len + (unsigned)__popc(pm) > FILL_CELLS || len - i > LEVEL_HAND) {  // large: goes to the CTA
+      kind = FK_BIG;
+      break;
+    }
+    if (push) {
+      const unsigned p = len + (unsigned)__popc(pm & lanemask_lt());
+      F.id[p] = nid;
+      F.vol[p] = v;
+    }
+    mn = min(mn, __reduce_min_sync(FULLMASK, push ? nid : EMPTY_ID));
+    len += (unsigned)__popc(pm);
+    __syncwarp();
+  }
+  if (lane == 0) {
+    F.len = len;
+    F.min_id = mn;
+    if (kind != FK_BIG) {  // fluid.rs:430-456: the sum in queue order
+      double a = 0.0;
+      float lo = 2.0f, hi = -1.0f;
+      for (unsigned k = 0; k < len; ++k) {
+        a = __dadd_rn(a, (double)F.vol[k]);
+        lo = fminf(lo, F.vol[k]);
+        hi = fmaxf(hi, F.vol[k]);
+      }
+      if (len >= 2u && __fsub_rn(hi, lo) >= SLEEP) {
+        F.avg = __double2float_rn(__ddiv_rn(a, (double)len));
+        kind = F.avg >= MIN_SPREAD ? FK_LEVEL : FK_DRAIN;
+      }
+    }
+    F.kind = kind;
+  }
+  __syncwarp();
+}
+
+// What a small layer's fill leaves behind, one warp: its marks, and the cells at their average.
+__device__ void level_commit_small(const Region& R, WS& sW, const int* ring, const LevelFill& F, unsigned long long cap, int& pd, unsigned& chg) {
+  const unsigned lane = lane_id();
+  for (unsigned t = lane; t < FILL_SLOTS; t += 32u) {
+    if (F.key[t] == EMPTY_ID) continue;
+    int x, y, z;
+    dom_xyz(R, F.key[t], x, y, z);
+    mark_tas(R, x, y, z);
+  }
+  if (F.kind == FK_LEVEL) {
+    for (unsigned b0 = 0; b0 < F.len; b0 += 32u) {
+      const unsigned k = b0 + lane;
+      int x = 0, y = 0, z = 0;
+      bool wv = false;
+      CD c = CD{0.0f, NOSLOT, 0u, 0, true};
+      if (k < F.len) {
+        dom_xyz(R, F.id[k], x, y, z);
+        c = load_cell_par(R, ring, x, y, z, cap);
+        wv = fabsf(__fsub_rn(cd_volume(c), F.avg)) > 1e-6f;
+      }
+      const bool need = wv && set_volume_needs_slot(c, F.avg);
+      if (__any_sync(FULLMASK, need)) materialize_par(R, need, c.gi, c.slot, cap);
+      if (wv) {
+        const SVPlan p = sv_plan(c.part, c.mat, c.slot != NOSLOT, F.avg);
+        if (c.slot != NOSLOT) sv_apply(R, (size_t)c.slot * 512u + local_index(x, y, z), p);
+        pd += p.dp;
+        if (p.ch) {
+          const unsigned pos = atomicAdd(&sW.nchg, 1u);
+          if (pos < R.ev_chg_cap) R.ev_chg[pos] = F.id[k];
+          else set_status(R, ST_OOM, 9);
+          chg = 1u;
+        }
+      }
+    }
+  }
+  __syncwarp();
+}
+
 // FluidSim::level_surfaces (fluid.rs:489-507) from sW.llc on, over the CTA, in batches of up to one
 // seed per thread (LIFO order = thread order). Every thread walks its seed up to the top water cell
 // (fluid.rs:496-499) and tests the start: a start that is marked, repeats an earlier start of the
 // batch, or is not a layer member needs no flood fill. Levelling a layer to its average changes no
 // cell's solidity, its "vol > 0" or "supported", so these tests stay true while the batch's
 // earlier layers are levelled; a drained layer (which can change them) ends the batch. The
-// remaining starts, the candidates, are levelled in order (warp 0, handing grown layers to the
-// CTA), each marked at its turn as the reference does; the budget (fluid.rs:492) ends the batch
-// after the candidate that spends it. The popped seeds leave the seed set and their starts are
+// remaining starts, the candidates, are levelled in order, each marked at its turn as the reference
+// does; the budget (fluid.rs:492) ends the batch after the candidate that spends it. Where the budget
+// cannot run out in between, one candidate per warp is filled at once (level_fill_small) and those
+// before the first large or drained layer commit together; a large layer starts on warp 0 and is
+// handed to the CTA as it grows. (Rain on the ring world: ~3,000 puddles of ~8 cells a levelling tick,
+// 57 M SM cycles one after another.) The popped seeds leave the seed set and their starts are
 // marked (a start that is not a member is marked, and skipped by every later flood fill, either
 // way). sW.level_round is updated at the end.
 __device__ __noinline__ void level_round_cta(const Region& R, TickSmem& sm, WS& sW, Smem& S, unsigned long long cap) {
-  __shared__ unsigned s_ns, s_stop, s_brk, s_pend, s_qi, s_ql, s_cur;
+  __shared__ unsigned s_ns, s_stop, s_brk, s_pend, s_qi, s_ql, s_cur, s_m, s_group[MAX_WARPS];
+  LevelFill* const fills = reinterpret_cast<LevelFill*>(&sm.u);  // the sweep's shared memory is free now
+  static_assert(sizeof(LevelFill) * MAX_WARPS <= sizeof(LvSmem), "level fills");
   const unsigned tid = threadIdx.x;
   unsigned* b_start = sm.hist;          // the batch's starts (domain ids), by seed
   unsigned* b_cand = sm.hist + NT_;     // candidate seeds in order
@@ -1212,7 +1352,7 @@ __device__ __noinline__ void level_round_cta(const Region& R, TickSmem& sm, WS& 
     // that an earlier layer's flood fill marked is skipped, as its test_and_set would return
     // (entry bits: 31 one cell, 30 marked since the batch began, 0-29 the seed)
     while (true) {
-      if (tid == 0) {
+      if (tid == 0 && !s_brk) {
         unsigned c = s_cur;
         while (c < nc && (b_cand[c] >> 30)) {
           if (b_cand[c] >> 31) {
@@ -1232,6 +1372,52 @@ __device__ __noinline__ void level_round_cta(const Region& R, TickSmem& sm, WS& 
       if (s_brk || s_cur >= nc) break;
       const unsigned cur = s_cur;
       const unsigned j = b_cand[cur];
+      if (tid == 0) {
+        unsigned m = 0;
+        if (sW.llc + nc + FILL_CELLS * NW_ < LEVEL_BUDGET)
+          for (unsigned c = cur; c < nc && m < NW_; ++c)
+            if (!(b_cand[c] >> 30)) s_group[m++] = b_cand[c];
+        s_m = m;
+      }
+      __syncthreads();
+      const unsigned m = s_m;
+      if (m) {
+        const unsigned w = tid >> 5;
+        if (w < m) level_fill_small(R, S.ring, fills[w], b_start[s_group[w]]);
+        __syncthreads();
+        if (tid == 0) {
+          unsigned k = 0, cells = 0;
+          for (; k < m; ++k) {
+            if (fills[k].kind == FK_BIG || fills[k].kind == FK_DRAIN) break;
+            bool dup = false;  // an earlier fill of the group covers it: its start is marked by then
+            for (unsigned o = 0; o < k; ++o) dup |= fills[o].kind != FK_DUP && fills[o].min_id == fills[k].min_id;
+            if (dup) fills[k].kind = FK_DUP;
+            else cells += fills[k].len;
+          }
+          s_m = k;
+          sW.llc += cells;
+          sW.level_cells_total += cells;
+        }
+        __syncthreads();
+        const unsigned done = s_m;
+        int pd = 0;
+        unsigned chg = 0;
+        if (w < done && fills[w].kind != FK_DUP) level_commit_small(R, sW, S.ring, fills[w], cap, pd, chg);
+        if (pd) atomicAdd(reinterpret_cast<unsigned long long*>(&sW.pdelta), (unsigned long long)(long long)pd);
+        if (chg) *(volatile bool*)&sW.changed = true;
+        __syncthreads();
+        if (done) {  // the group's starts, and the later ones its fills marked
+          for (unsigned c = cur + tid; c < nc; c += NT_) {
+            const unsigned e = b_cand[c];
+            if (e >> 30) continue;
+            int cx, cy, cz;
+            dom_xyz(R, b_start[e], cx, cy, cz);
+            if (mark_test(R, cx, cy, cz)) b_cand[c] = e | (1u << 30);
+          }
+          __syncthreads();
+          continue;
+        }
+      }
       if (tid < 32u) {
         WS W = sW;
         W.pdelta = 0;
@@ -1270,8 +1456,7 @@ __device__ __noinline__ void level_round_cta(const Region& R, TickSmem& sm, WS& 
         }
         s_cur += 1u;
       }
-      __syncthreads();
-      if (s_brk) break;
+      __syncthreads();  // (s_brk is looked at after the next barrier only: thread 0 may set it before that)
     }
     // ---- the popped seeds: out of the seed set, starts marked (and the sides a one-cell layer's
     // flood fill tested)
