@@ -40,9 +40,7 @@ struct vf_fluid {
   // download scratch
   void* scratch = nullptr;
   size_t scratch_bytes = 0;
-  // tick launch shape
-  int smem_bytes = 0;
-  Tune tune{TICK_WARPS - 1, PF_RING, 1, 4 | (1 << 8), 1ull << 24};
+  Tune tune{0, 1ull << 24};
   // wake proposal state (allocated on first use)
   int* slot_gi = nullptr;
   SlotAggr* aggr = nullptr;
@@ -52,9 +50,6 @@ struct vf_fluid {
   // ring streaming on a live handle: entries kept for evicted chunks, atlas slots they freed
   std::vector<DetachedPartial> det;
   std::vector<unsigned> free_slots;
-  // engine chosen per launch from the last launches' pressure-search entries per cell-step
-  bool auto_engine = true;
-  uint64_t auto_cells = 0, auto_bfs = 0;
 };
 
 // A set of regions stepped together: one CTA per region in one launch (pattern (2)).
@@ -81,18 +76,13 @@ struct DeviceScope {
   }
 };
 
-// The tick kernel of the handle's engine for `nreg` regions: one CTA per region.
-// The parallel sweep uses only the parallel member of TickSmem's union: its launch asks for that
-// much shared memory, which leaves the rest of the SM's 256 KB to L1.
-constexpr int PAR_SMEM_BYTES = (int)((offsetof(TickSmem, u) + sizeof(LvSmem) + 127) / 128 * 128);
-static_assert(PAR_SMEM_BYTES <= (int)sizeof(TickSmem), "parallel sweep shared memory");
+// The tick kernel for `nreg` regions: one CTA per region.
+constexpr int PAR_SMEM_BYTES = (int)((sizeof(TickSmem) + 127) / 128 * 128);
+static_assert(PAR_SMEM_BYTES + 1024 + 1024 <= 100 * 1024, "the tick fits the 100 KB carve-out, static arrays and the system's 1 KB included");
 
-cudaError_t launch_tick(const Tune& t, Region* regs, int nreg, int n_ticks, int smem, cudaStream_t st) {
-  if (t.engine) {
-    const int warps = (t.gate >> 16) & 0x1F;
-    k_tick_par<<<(unsigned)nreg, warps ? 32 * warps : PAR_THREADS, PAR_SMEM_BYTES, st>>>(regs, nreg, n_ticks, t);
-  }
-  else k_tick<<<(unsigned)nreg, TICK_THREADS, smem, st>>>(regs, nreg, n_ticks, t);
+cudaError_t launch_tick(const Tune& t, Region* regs, int nreg, int n_ticks, cudaStream_t st) {
+  const int warps = (t.gate >> 16) & 0x1F;
+  k_tick_par<<<(unsigned)nreg, warps ? 32 * warps : PAR_THREADS, PAR_SMEM_BYTES, st>>>(regs, nreg, n_ticks, t);
   return cudaGetLastError();
 }
 
@@ -322,14 +312,14 @@ int vf_fluid_create(const vf_fluid_desc* desc, vf_fluid** out) {
   }
   // the tick kernel's image must load (sm_100a only): probe its attributes
   cudaFuncAttributes fa;
-  if (cudaFuncGetAttributes(&fa, k_tick) != cudaSuccess) {
+  if (cudaFuncGetAttributes(&fa, k_tick_par) != cudaSuccess) {
     cudaFreeHost(h->hctl);
     delete h;
     return VF_ERR_NO_DEVICE;
   }
-  h->smem_bytes = (int)sizeof(TickSmem);
-  cudaFuncSetAttribute(k_tick, cudaFuncAttributeMaxDynamicSharedMemorySize, h->smem_bytes);
   cudaFuncSetAttribute(k_tick_par, cudaFuncAttributeMaxDynamicSharedMemorySize, PAR_SMEM_BYTES);
+  // one CTA per SM: all the memory it does not ask for as L1
+  cudaFuncSetAttribute(k_tick_par, cudaFuncAttributePreferredSharedMemoryCarveout, (PAR_SMEM_BYTES + 3072) * 100 / (228 * 1024) + 1);
   *out = h;
   return VF_OK;
 }
@@ -574,8 +564,7 @@ int vf_fluid_tick_async(vf_fluid* h, int32_t n_ticks) {
   h->hzero[0] = 0u;
   CK(cudaMemcpyAsync(&h->R.ctl->changed, h->hzero, sizeof(unsigned), cudaMemcpyHostToDevice, h->stream));
   if (n_ticks > 0) {
-    if (h->auto_engine) h->tune.engine = 1;
-    CK(launch_tick(h->tune, h->dR, 1, n_ticks, h->smem_bytes, h->stream));
+    CK(launch_tick(h->tune, h->dR, 1, n_ticks, h->stream));
   }
   return VF_OK;
 }
@@ -1130,17 +1119,6 @@ int vf_fluid_profile(vf_fluid* h, uint64_t* out16) {
   return VF_OK;
 }
 
-#ifdef VF_FINE_PROFILE
-// Fine-profiling builds only: all 32 counters (the 16 phases and the per-call counters).
-extern "C" int vf_fluid_profile_fine(vf_fluid* h, uint64_t* out32) {
-  int rc = check(h);
-  if (rc) return rc;
-  if ((rc = sync_ctl(h))) return rc;
-  if (out32) std::memcpy(out32, h->hctl->prof, 32 * sizeof(uint64_t));
-  return VF_OK;
-}
-#endif
-
 // ---------------------------------------------------------------- learned wake proposal
 static int proposal_buffers(vf_fluid* h) {
   if (h->slot_gi) return VF_OK;
@@ -1211,10 +1189,9 @@ int vf_fluid_stage_bricks(vf_fluid* h, const float* dev_prob, uint64_t nslots, f
   return VF_OK;
 }
 
+// Knobs of a sweep that earlier versions chose between; accepted as they were, nothing depends on them.
 int vf_fluid_set_tuning(vf_fluid* h, int32_t producers, int32_t depth) {
-  if (!h || producers < 1 || producers > TICK_WARPS - 1 || depth < 1 || depth > PF_RING) return VF_ERR_INVALID;
-  h->tune.producers = producers;
-  h->tune.depth = depth;
+  if (!h || producers < 1 || producers > 7 || depth < 1 || depth > 64) return VF_ERR_INVALID;
   return VF_OK;
 }
 
@@ -1224,9 +1201,7 @@ int vf_fluid_set_sweep(vf_fluid* h, int32_t engine, int32_t gate, uint64_t spin_
       (warps != 0 && (warps < 8 || warps > MAX_WARPS)) || spin_cap == 0)
     return VF_ERR_INVALID;
   if (engine == 1 && h->uploaded && (h->R.PX >= 65536 || h->R.PZ >= 65536 || h->R.PY >= 65536))
-    return fail(h, VF_ERR_RANGE, "the parallel sweep needs domain sides below 65536");
-  h->auto_engine = engine == 2;
-  if (engine != 2) h->tune.engine = engine;
+    return fail(h, VF_ERR_RANGE, "engine 1 needs domain sides below 65536");
   h->tune.gate = gate;
   h->tune.spin_cap = spin_cap;
   return VF_OK;
@@ -1340,7 +1315,7 @@ int vf_batch_tick_async(vf_batch* b, int32_t n_ticks) {
   vf_fluid* h = b->hs[0];
   DeviceScope scope(h->device);
   if (n_ticks) {
-    CK(launch_tick(h->tune, b->dregs, (int)b->hs.size(), n_ticks, h->smem_bytes, b->stream));
+    CK(launch_tick(h->tune, b->dregs, (int)b->hs.size(), n_ticks, b->stream));
   }
   return VF_OK;
 }
@@ -1372,7 +1347,7 @@ int vf_batch_capture(vf_batch* b, int32_t launches, int32_t ticks_per_launch) {
   }
   CK(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
   for (int i = 0; i < launches; ++i)
-    launch_tick(h->tune, b->dregs, (int)b->hs.size(), ticks_per_launch, h->smem_bytes, b->stream);
+    launch_tick(h->tune, b->dregs, (int)b->hs.size(), ticks_per_launch, b->stream);
   cudaError_t e = cudaStreamEndCapture(b->stream, &b->graph);
   if (e != cudaSuccess) return fail(h, VF_ERR_CUDA, std::string("capture: ") + cudaGetErrorString(e));
   CK(cudaGraphInstantiate(&b->exec, b->graph, 0));
@@ -1434,7 +1409,7 @@ int vf_fluid_batch_tick(vf_fluid* const* hs, int32_t n, int32_t n_ticks) {
   CK(cudaMemcpyAsync(h->scratch, regs.data(), sizeof(Region) * n, cudaMemcpyHostToDevice, h->stream));
   for (int i = 0; i < n; ++i) CK(cudaMemsetAsync(&regs[i].ctl->changed, 0, 4, h->stream));
   if (n_ticks) {
-    CK(launch_tick(h->tune, (Region*)h->scratch, n, n_ticks, h->smem_bytes, h->stream));
+    CK(launch_tick(h->tune, (Region*)h->scratch, n, n_ticks, h->stream));
   }
   CK(cudaStreamSynchronize(h->stream));
   for (int i = 0; i < n; ++i) {

@@ -13,11 +13,8 @@ namespace vfe {
 #define NT_ ((unsigned)blockDim.x)
 #define NW_ ((unsigned)(blockDim.x >> 5))
 
-// Launch shapes: the one-warp sweep runs 8 warps per region (the sweep plus prefetchers), the
-// parallel sweep MAX_WARPS (row workers). CTA-wide helpers below use the launched block size;
-// shared arrays are sized for the larger shape.
-constexpr int TICK_THREADS = 256;
-constexpr int TICK_WARPS = TICK_THREADS / 32;
+// Launch shape: MAX_WARPS warps per region. CTA-wide helpers use the launched block size; shared arrays
+// are sized for the full one.
 constexpr int PAR_THREADS = MAX_WARPS * 32;
 
 // ---------------------------------------------------------------- CTA radix sort (LSD, 8 bit)
@@ -129,45 +126,22 @@ __device__ void cta_radix_sort(unsigned* keys, unsigned* tmp, unsigned n, unsign
 }
 
 // ----------------------------------------------------------------------------- the tick
-constexpr int PF_RING = 64;                      // prefetched footprints in flight
-
-// Launch-time knobs of the tick (results do not depend on them): which sweep runs, the one-warp
-// sweep's producer warps and prefetch distance (chosen by the autotuner), the parallel sweep's
-// pull gate radius and the iteration cap of device waits.
+// Launch-time knobs of the tick (results do not depend on them).
 struct Tune {
-  int producers;  // one-warp sweep: 1 .. TICK_WARPS-1 prefetching warps
-  int depth;      // one-warp sweep: 1 .. PF_RING cells ahead
-  int engine;     // 0 one-warp sweep (TICK_THREADS per region), 1 parallel sweep (PAR_THREADS)
-  int gate;       // parallel sweep: bits 0-7 gate radius, 8-15 cone radius (0..GATE_MAX), 16-20 warps (0: MAX_WARPS), 21 global search contexts only
-  unsigned long long spin_cap;  // iterations before a wait gives up (ST_TIMEOUT)
-};
-
-// Shared memory of the one-warp sweep: prefetch ring, store forwarding and search structures.
-struct SeqSmem {
-  int4 pq[PRESS_QCAP];
-  unsigned long long vis[VIS_CAP];
-  unsigned vb[VB_WORDS];        // pressure-search visited bitmap (zero between searches)
-  unsigned vtl[PRESS_QCAP];     // bitmap words touched by the current search
-  CD pf[PF_RING][7];            // prefetched footprints (self, below, up, +x, -x, +z, -z)
-  unsigned pf_ready[PF_RING];   // the cell index whose footprint a slot holds
-  int pxyz[PF_RING][4];         // the cell's coordinates and domain id
-  unsigned pf_c0[PF_RING];      // cells the sweep had finished when the slot's footprint was fetched
-  unsigned pf_quiet[PF_RING];   // classify_quiet of the fetched footprint
-  FwdEntry fwd[FWD_SIZE];       // the sweep's latest writes (store forwarding)
-  unsigned long long gc[GCACHE];  // grid-word cache of the sweep's pressure searches
-  SearchHelp help;              // neighbour loads by idle prefetchers ahead of a search
-  unsigned consumed;            // cells the sweep has finished
-  unsigned abort;               // a wait gave up: every warp leaves the sweep
+  int gate;       // bits 16-20: warps of the region's CTA (0: MAX_WARPS); the other bits are unused
+  unsigned long long spin_cap;  // rounds of the sweep, and iterations of any wait, before the tick gives up (ST_TIMEOUT)
 };
 
 struct TickSmem {
-  unsigned hist[MAX_WARPS * 256];
   unsigned sred[2 * 256 + 64];
   int ring[3 * 16 * 16];
   unsigned scan[MAX_WARPS + 1];
   union {
-    SeqSmem s;  // one-warp sweep
-    LvSmem p;   // parallel sweep
+    LvSmem p;   // the sweep
+    struct {    // before and after the sweep: the sort's histograms, then the levelling's tables
+      unsigned hist[MAX_WARPS * 256];
+      unsigned fills[MAX_WARPS * 1024];  // LevelFill per warp
+    } x;
   } u;
 };
 
@@ -182,45 +156,12 @@ __device__ void load_ws(const Region& R, WS& W) {
   W.level_cells_total = 0;
   W.pdelta = 0;
   W.nseeds = c.nseeds;
-  W.pulls = 0;
   W.llc = c.last_level_cells;
   W.ndrain = 0;
-  W.epoch = 1;
   W.level_round = c.level_round != 0;
   W.changed = false;
   W.deferred = false;
   W.nact = W.nseed = W.nchg = 0;
-  W.fwd = nullptr;
-  W.seq = 0;
-  W.gc = nullptr;
-  W.t_wait = W.t_pull = W.t_act = W.t_write = W.t_top = W.t_pc = W.t_tail = 0;
-#ifdef VF_FINE_PROFILE
-  W.f_pre = W.f_plan = W.f_seed = W.n_pc = W.n_quiet = W.n_rounds = W.f_bload = W.f_bexp = W.f_match = W.f_vis = 0;
-#endif
-}
-
-// Load a cell for the prefetch ring: the grid word is read with a fence after it, pairing with
-// the sweep's fenced publication of freshly materialised bricks.
-__device__ __forceinline__ CD load_cell_acq(const Region& R, const int* ring, int x, int y, int z) {
-  CD c;
-  c.part = 0.0f;
-  c.slot = NOSLOT;
-  c.gi = 0;
-  c.mat = 0;
-  c.out = outside(R, ring, x, y, z);
-  if (c.out) return c;
-  c.gi = grid_index(R, x >> 3, y >> 3, z >> 3);
-  unsigned g = *(volatile const unsigned*)(R.grid + c.gi);
-  __threadfence_block();
-  if (g < 256u) {
-    c.mat = (unsigned char)g;
-    return c;
-  }
-  c.slot = g - 256u;
-  size_t o = (size_t)c.slot * 512u + local_index(x, y, z);
-  c.mat = R.amat[o];
-  c.part = R.avol[o];
-  return c;
 }
 
 // ----------------------------------------------------------------- CTA-wide ordered commits
@@ -393,178 +334,6 @@ __device__ void commit_chgs(const Region& R, unsigned n) {
   __syncthreads();
 }
 
-// ------------------------------------------------------------------------ the sweep
-// Warp 0 walks the sorted cells (the reference's order); warps 1.. prefetch footprints of the
-// cells ahead into a shared-memory ring, each stamped with the number of cells the sweep had
-// finished when it was fetched. Values the sweep wrote after a fetch come from the
-// store-forwarding table (or, when the table cannot tell, from memory).
-__device__ void sweep(const Region& R, TickSmem& sm, WS& sW, const int* ring, unsigned n, bool flip, Tune tune) {
-  const unsigned tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-  if (tid == 0) {
-    sm.u.s.consumed = 0;
-    sm.u.s.abort = 0;
-  }
-  for (unsigned i = tid; i < PF_RING; i += NT_) sm.u.s.pf_ready[i] = 0xFFFFFFFFu;
-  for (unsigned i = tid; i < FWD_SIZE; i += NT_) sm.u.s.fwd[i].meta = 0u;
-  for (unsigned i = tid; i < GCACHE; i += NT_) sm.u.s.gc[i] = ~0ull;
-  __syncthreads();
-  if (warp == 0) {
-    WS W = sW;
-    W.fwd = sm.u.s.fwd;
-    W.gc = sm.u.s.gc;
-    Smem S{sm.u.s.vis, ring, sm.u.s.pq, sm.u.s.vb, sm.u.s.vtl, &sm.u.s.help, &sm.u.s.abort, tune.spin_cap};
-    const unsigned pxy = (unsigned)R.PX * (unsigned)R.PY;
-    // footprint offsets (self, below, up, +x, -x, +z, -z) of this lane, in cells and in ids
-    const int ox = (lane == 3) - (lane == 4), oy = (lane == 2) - (lane == 1), oz = (lane == 5) - (lane == 6);
-    const unsigned oid = (unsigned)ox + (unsigned)oy * (unsigned)R.PX + (unsigned)oz * pxy;
-    for (unsigned r = 0; r < n; ++r) {
-      const unsigned slot = r % PF_RING;
-      // wait (bounded) for the footprint of cell r; every lane reads the same word
-      const long long tw = fine_clock();
-      unsigned long long spins = 0;
-      while (*(volatile unsigned*)&sm.u.s.pf_ready[slot] != r) {
-        if (++spins > tune.spin_cap) break;
-        __nanosleep(20);
-      }
-      if (spins > tune.spin_cap) {
-        if (lane == 0) {
-          set_status(R, ST_TIMEOUT, 20);
-          *(volatile unsigned*)&sm.u.s.abort = 1u;
-        }
-        break;
-      }
-      __threadfence_block();
-      W.t_wait += fine_clock() - tw;
-      const int x = sm.u.s.pxyz[slot][0], y = sm.u.s.pxyz[slot][1], z = sm.u.s.pxyz[slot][2];
-      const unsigned cid = (unsigned)sm.u.s.pxyz[slot][3];
-      const unsigned c0 = sm.u.s.pf_c0[slot];
-      const unsigned quiet = sm.u.s.pf_quiet[slot];
-      // footprint cells the sweep wrote since the fetch: from the forwarding table, or from
-      // memory when another cell's write took the cell's table entry
-      bool touched = false;
-      if (lane < 7) {
-        CD mine = sm.u.s.pf[slot][lane];
-        const int fx = x + ox, fy = y + oy, fz = z + oz;
-        const FwdEntry e = sm.u.s.fwd[fwd_index(fx, fy, fz)];
-        if (!mine.out && (e.meta & 0xFFFFu) > c0) {
-          touched = true;
-          if (e.tag == cid + oid) {
-            mine.mat = (unsigned char)(e.meta >> 16);
-            mine.part = e.part;
-            mine.slot = e.slot;
-          } else {
-            mine = load_cell(R, ring, fx, fy, fz);
-          }
-          sm.u.s.pf[slot][lane] = mine;
-        }
-      }
-      const bool stale = __any_sync(FULLMASK, touched);
-      __syncwarp();
-      const long long t1 = fine_clock();
-      W.t_top += t1 - tw;
-      W.seq = r + 1u;
-      if (!stale && (quiet & QUIET)) {
-        // nothing to write, activate or seed (classified by the prefetcher on this footprint):
-        // only the pull budget counts the attempt
-        if ((quiet & QUIET_PULL) && W.pulls < MAX_PULLS_PER_TICK) {
-          W.pulls += 1;
-          W.pull_attempts += 1;
-        }
-#ifdef VF_FINE_PROFILE
-        W.n_quiet += 1;
-#endif
-      } else {
-        CD fp[7];
-#pragma unroll
-        for (int j = 0; j < 7; ++j) fp[j] = sm.u.s.pf[slot][j];
-        const CD mine = lane < 7 ? sm.u.s.pf[slot][lane] : CD{0.0f, NOSLOT, 0u, 0, true};
-        process_cell(R, W, S, x, y, z, x + ox, y + oy, z + oz, fp, mine);
-      }
-      __syncwarp();
-      const long long t2 = fine_clock();
-      W.t_pc += t2 - t1;
-      __threadfence_block();
-      if (lane == 0) *(volatile unsigned*)&sm.u.s.consumed = r + 1u;
-      W.t_tail += fine_clock() - t2;
-    }
-    W.fwd = nullptr;
-    W.gc = nullptr;
-    long long pd = W.pdelta;  // lane-local partial-count deltas
-    for (int o = 16; o; o >>= 1) pd += __shfl_xor_sync(FULLMASK, pd, o);
-    W.pdelta = pd;
-    if (lane == 0) {
-      sW = W;
-      Ctl& c = *R.ctl;
-      c.prof[3] += W.t_wait;
-      c.prof[4] += W.t_pull;
-      c.prof[5] += W.t_act;
-      c.prof[6] += W.t_write;
-      c.prof[12] += W.t_top;
-      c.prof[13] += W.t_pc;
-      c.prof[14] += W.t_tail;
-      sW.t_wait = sW.t_pull = sW.t_act = sW.t_write = sW.t_top = sW.t_pc = sW.t_tail = 0;
-#ifdef VF_FINE_PROFILE
-      c.prof[16] += W.f_pre;
-      c.prof[17] += W.f_plan;
-      c.prof[18] += W.f_seed;
-      c.prof[19] += W.n_pc;
-      c.prof[20] += W.n_quiet;
-      c.prof[21] += W.n_rounds;
-      c.prof[22] += W.f_bload;
-      c.prof[23] += W.f_bexp;
-      c.prof[24] += W.f_match;
-      c.prof[25] += W.f_vis;
-      sW.f_pre = sW.f_plan = sW.f_seed = sW.n_pc = sW.n_quiet = sW.n_rounds = sW.f_bload = sW.f_bexp = sW.f_match = sW.f_vis = 0;
-#endif
-    }
-    __syncwarp();
-  } else if (warp <= (unsigned)tune.producers) {
-    // producers: warp p prefetches cells p-1, p-1+NP, ...
-    const unsigned NP = (unsigned)tune.producers;
-    const unsigned depth = (unsigned)tune.depth;
-    for (unsigned r = warp - 1; r < n; r += NP) {
-      // wait (bounded) until the ring slot of cell r is free; every lane reads the same words
-      unsigned long long spins = 0;
-      unsigned c0;
-      bool ok = true;
-      while ((c0 = *(volatile unsigned*)&sm.u.s.consumed) + depth <= r) {
-        if (*(volatile unsigned*)&sm.u.s.abort || ++spins > tune.spin_cap) {
-          ok = false;
-          break;
-        }
-        // nothing to prefetch yet: load neighbours for a running pressure search, else yield
-        // issue slots to the sweep warp
-        if (!help_search(R, ring, &sm.u.s.help, sm.u.s.pq)) __nanosleep(200);
-      }
-      if (!ok) break;
-      __threadfence_block();
-      int x, y, z;
-      const unsigned cid = key_to_id(R, R.cells[r], flip);
-      dom_xyz(R, cid, x, y, z);
-      const unsigned s = r % PF_RING;
-      if (lane < 7) {
-        int fx = x + (lane == 3) - (lane == 4), fy = y - (lane == 1) + (lane == 2), fz = z + (lane == 5) - (lane == 6);
-        sm.u.s.pf[s][lane] = load_cell_acq(R, ring, fx, fy, fz);
-      } else if (lane == 7) {
-        sm.u.s.pxyz[s][0] = x;
-        sm.u.s.pxyz[s][1] = y;
-        sm.u.s.pxyz[s][2] = z;
-        sm.u.s.pxyz[s][3] = (int)cid;
-        sm.u.s.pf_c0[s] = c0;
-      }
-      __syncwarp();
-      CD fq[7];
-#pragma unroll
-      for (int j = 0; j < 7; ++j) fq[j] = sm.u.s.pf[s][j];
-      const unsigned q = classify_quiet(fq, x, z);
-      if (lane == 0) sm.u.s.pf_quiet[s] = q;
-      __syncwarp();
-      __threadfence_block();
-      if (lane == 0) *(volatile unsigned*)&sm.u.s.pf_ready[s] = r;
-    }
-  }
-  __syncthreads();
-}
 // ------------------------------------------------------------------- the parallel sweep
 // Sum of a per-thread value over the CTA (all threads call).
 __device__ unsigned long long cta_sum(TickSmem& sm, unsigned long long v) {
@@ -601,10 +370,7 @@ __device__ __noinline__ void sweep_levels(const Region& Rs, TickSmem& sm, WS& sW
   // ---- positions, footprints, and the cells that attempt a pull or may find a start cell
   for (unsigned g = ngrp + tid; g <= NGROUPS; g += NT_) L.att[g] = L.pp[g] = 0u;
   for (unsigned g = tid; g < ngrp; g += NT_) R.pextra[g] = 0u;
-  for (unsigned t = tid; t < VIS_SLOTS; t += NT_) {
-    L.s.vkey[t] = EMPTY_ID;
-    L.s.vrank[t] = 0xFFFFFFFFu;
-  }
+  vis_reset(L.s, tid, NT_);
   if (tid == 0) {
     L.cnt[0] = L.cnt[1] = L.cnt[2] = 0u;
     L.cur = L.cc = L.pb = 0u;
@@ -692,15 +458,15 @@ __device__ __noinline__ void sweep_levels(const Region& Rs, TickSmem& sm, WS& sW
   // ---- the later conflicting cells of every cell, and how many earlier ones each waits for
   const int sgn = flip ? -1 : 1;
   for (unsigned i = tid; i < n; i += NT_) {
-    if (reinterpret_cast<volatile unsigned char*>(L.dep)[i] == DONE) continue;
-    int x, y, z;
-    dom_xyz(R, R.lv[i].cid, x, y, z);
+    if (cell_done(L, i)) continue;
+    const unsigned cid = R.lv[i].cid;
     unsigned s[12];
 #pragma unroll
     for (int q = 0; q < 12; ++q) {
       int dx, dy, dz;
       succ_offset(q, sgn, dx, dy, dz);
-      const unsigned r = (q < 11 || i < kp) ? rank_at(R, x + dx, y + dy, z + dz) : NOSLOT;
+      // (a cell of the world: what lies within two cells of it is inside the padded domain)
+      const unsigned r = (q < 11 || i < kp) ? R.stamp[(int)cid + dx + (dz * R.PY + dy) * R.PX] : NOSLOT;
       s[q] = r == NOSLOT ? NOSUCC : r;
     }
 #pragma unroll
@@ -720,7 +486,7 @@ __device__ __noinline__ void sweep_levels(const Region& Rs, TickSmem& sm, WS& sW
   int gate = L.h.gate;
   // ---- the first round: cells that wait for nobody
   for (unsigned i = tid; i < n; i += NT_) {
-    if (reinterpret_cast<volatile unsigned char*>(L.dep)[i] != 0) continue;
+    if (dep_byte(L, i) != 0u) continue;
     if (R.lv[i].y <= gate) list_put(R, L, 0u, atomicAdd(&L.cnt[0], 1u), i);
     else park_put(R, 0u, atomicAdd(&L.park_n[0], 1u), i);
   }
@@ -1283,11 +1049,11 @@ __device__ void level_commit_small(const Region& R, WS& sW, const int* ring, con
 // way). sW.level_round is updated at the end.
 __device__ __noinline__ void level_round_cta(const Region& R, TickSmem& sm, WS& sW, Smem& S, unsigned long long cap) {
   __shared__ unsigned s_ns, s_stop, s_brk, s_pend, s_qi, s_ql, s_cur, s_m, s_group[MAX_WARPS];
-  LevelFill* const fills = reinterpret_cast<LevelFill*>(&sm.u);  // the sweep's shared memory is free now
-  static_assert(sizeof(LevelFill) * MAX_WARPS <= sizeof(LvSmem), "level fills");
+  LevelFill* const fills = reinterpret_cast<LevelFill*>(sm.u.x.fills);  // the sweep's shared memory is free now
+  static_assert(sizeof(LevelFill) * MAX_WARPS <= sizeof(sm.u.x.fills) && sizeof(sm.u.x) <= sizeof(LvSmem), "level fills");
   const unsigned tid = threadIdx.x;
-  unsigned* b_start = sm.hist;          // the batch's starts (domain ids), by seed
-  unsigned* b_cand = sm.hist + NT_;     // candidate seeds in order
+  unsigned* b_start = sm.u.x.hist;          // the batch's starts (domain ids), by seed
+  unsigned* b_cand = sm.u.x.hist + NT_;     // candidate seeds in order
   while (true) {
     if (tid == 0) s_ns = (sW.llc < LEVEL_BUDGET) ? sW.nseeds : 0u;
     __syncthreads();
@@ -1489,9 +1255,8 @@ __device__ __noinline__ void level_round_cta(const Region& R, TickSmem& sm, WS& 
 }
 
 // FluidSim::tick (fluid.rs:564-657) for region R, n_ticks times. All threads of the CTA enter.
-// Per tick: drain the FIFO head and sort it (CTA), the sweep (warp 0, prefetched by the other
-// warps), the seed log's commit, levelling (warp 0), then the activation and change logs'
-// commits (CTA). The logs keep program order, so the committed FIFO and seed list are exactly
+// Per tick, all by the CTA: drain the FIFO head and sort it, the sweep, the seed log's commit,
+// levelling, then the activation and change logs' commits. The logs keep program order, so the committed FIFO and seed list are exactly
 // the reference's.
 __device__ void run_ticks(const Region& R, TickSmem& sm, int n_ticks, Tune tune) {
   const unsigned tid = threadIdx.x, warp = tid >> 5;
@@ -1499,16 +1264,6 @@ __device__ void run_ticks(const Region& R, TickSmem& sm, int n_ticks, Tune tune)
   if (R.ring_w && R.ring_w <= 16) {
     for (int i = tid; i < 3 * R.ring_w * R.ring_w; i += NT_) sm.ring[i] = R.ring[i];
     ring = sm.ring;
-  }
-  const bool par = tune.engine != 0;
-  if (!par) {
-    for (unsigned i = tid; i < VIS_CAP; i += NT_) sm.u.s.vis[i] = 0ull;
-    for (unsigned i = tid; i < VB_WORDS; i += NT_) sm.u.s.vb[i] = 0u;
-    for (unsigned i = tid; i < HRING; i += NT_) sm.u.s.help.tag[i] = ~0ull;
-    if (tid == 0) {
-      sm.u.s.help.state = 0ull;
-      sm.u.s.help.qlen = sm.u.s.help.done = 0u;
-    }
   }
   __shared__ unsigned s_n, s_flip, s_clear, s_abort, s_nseeds, s_lv;
   __shared__ unsigned long long s_qtail;
@@ -1559,7 +1314,6 @@ __device__ void run_ticks(const Region& R, TickSmem& sm, int n_ticks, Tune tune)
     __syncthreads();
     if (tid == 0) {
       sW.qhead = qh + n;
-      sW.pulls = 0;
       sW.changed = false;
       sW.activations = sW.pull_attempts = sW.pull_success = sW.bfs_visits = sW.level_cells_total = 0;
       sW.pdelta = 0;
@@ -1588,14 +1342,13 @@ __device__ void run_ticks(const Region& R, TickSmem& sm, int n_ticks, Tune tune)
     }
     lap(0);
     // ---- sort (fluid.rs:575-580)
-    cta_radix_sort(R.cells, R.cells_tmp, n, sm.hist, sm.sred);
+    cta_radix_sort(R.cells, R.cells_tmp, n, sm.u.x.hist, sm.sred);
     __syncthreads();
     lap(1);
     // ---- the sweep (fluid.rs:584-651)
-    if (par) sweep_levels(R, sm, sW, ring, n, flip, tune);
-    else sweep(R, sm, sW, ring, n, flip, tune);
+    sweep_levels(R, sm, sW, ring, n, flip, tune);
     lap(2);
-    if (par ? vld((const unsigned*)&R.ctl->status) != 0u : sm.u.s.abort != 0u) {
+    if (vld((const unsigned*)&R.ctl->status) != 0u) {
       if (tid == 0) s_abort = 1;
       __syncthreads();
       break;
@@ -1612,7 +1365,7 @@ __device__ void run_ticks(const Region& R, TickSmem& sm, int n_ticks, Tune tune)
     if (tid == 0) s_lv = (sW.level_round || (R.ctl->tick_no % LEVEL_TICKS) == 0u) ? 1u : 0u;
     __syncthreads();
     if (s_lv) {
-      Smem S{sm.u.s.vis, ring, sm.u.s.pq, sm.u.s.vb, sm.u.s.vtl, nullptr, nullptr, tune.spin_cap};
+      Smem S{ring};
       if (tid == 0) sW.llc = 0;
       __syncthreads();
       level_round_cta(R, sm, sW, S, tune.spin_cap);
@@ -1667,27 +1420,12 @@ __device__ void run_ticks(const Region& R, TickSmem& sm, int n_ticks, Tune tune)
   }
 }
 
-// One CTA per region. k_tick runs the one-warp sweep (TICK_THREADS per CTA), k_tick_par the
-// parallel sweep (PAR_THREADS per CTA).
-__global__ void __launch_bounds__(TICK_THREADS, 1) k_tick(Region* regs, int nreg, int n_ticks, Tune tune) {
-  extern __shared__ __align__(16) unsigned char smraw[];
-  TickSmem& sm = *reinterpret_cast<TickSmem*>(smraw);
-  tune.engine = 0;
-  __shared__ Region s_reg;  // the region's constants, as in k_tick_par
-  for (int r = blockIdx.x; r < nreg; r += gridDim.x) {
-    if (threadIdx.x == 0) s_reg = regs[r];
-    __syncthreads();
-    run_ticks(s_reg, sm, n_ticks, tune);
-    __syncthreads();
-  }
-}
-
+// One CTA of up to PAR_THREADS per region.
 __global__ void __launch_bounds__(PAR_THREADS, 1) k_tick_par(Region* regs, int nreg, int n_ticks, Tune tune) {
   extern __shared__ __align__(16) unsigned char smraw[];
   TickSmem& sm = *reinterpret_cast<TickSmem*>(smraw);
-  tune.engine = 1;
-  // The region's constants (sizes, array bases) are read on every cell of the sweep: a copy in
-  // shared memory keeps them off the L1, which the sweep's records and atlas lines stream through.
+  // The region's constants (sizes, array bases): a copy in shared memory keeps them off the L1, which
+  // the sweep's records and atlas lines stream through.
   __shared__ Region s_reg;
   for (int r = blockIdx.x; r < nreg; r += gridDim.x) {
     if (threadIdx.x == 0) s_reg = regs[r];
@@ -1754,8 +1492,6 @@ __global__ void __launch_bounds__(1024) k_wake_box(Region R, int x0, int y0, int
 
 // A single warp running sequential host edits with the tick's device rules.
 struct EditSmem {
-  unsigned pq[8];
-  unsigned long long vis[8];
   int ring[3 * 16 * 16];
 };
 

@@ -37,14 +37,16 @@ constexpr int MAX_WARPS = 16;                  // warps of a CTA running the swe
 constexpr unsigned SOLO_CELLS = 4;             // a list this short is run by one warp (eight lanes per cell)
 constexpr unsigned SOLO_ENTRIES = 6;           // queue entries one warp examines per search round
 constexpr unsigned SOLO_WAIT = SOLO_ENTRIES;   // a search with more entries waiting goes to all warps
-constexpr unsigned VIS_SLOTS = 2048;           // visited set of a search: <= 6 + 512 + one round's 5 per entry (512)
+constexpr unsigned VIS_SLOTS = 2048;           // visited set, emptied when VIS_FULL cells have been added
 constexpr int VIS_SHIFT = 21;                  // hash bits kept: 32 - log2(VIS_SLOTS)
+constexpr unsigned VIS_FULL = 768;             // one search adds <= 6 + 512 + one round's 5 per entry (480)
+constexpr unsigned VIS_RANKS = 4096;           // ranks of one search: 6 + 5 * 512 at most
 constexpr unsigned NGROUPS = (MAX_CELLS_PER_TICK + 31) / 32;
-constexpr unsigned LIST_CAP = 4096;   // a round's list kept in shared memory; the rest goes to global
+constexpr unsigned LIST_CAP = 2048;   // a round's list kept in shared memory; the rest goes to global
 constexpr unsigned NOSUCC = 0xFFFFu;
 static_assert(MAX_CELLS_PER_TICK < NOSUCC, "sorted positions fit 16 bits");
 constexpr unsigned UNIFORM = 0x80000000u;  // LvCell::slot of a brick that was a uniform grid value
-constexpr unsigned DONE = 0xFFu;           // dependency byte of a finished cell
+constexpr unsigned DONE = 0x80u;           // dependency byte of a finished cell: DONE | the footprint slots it wrote
 constexpr int GATE_MAX = 31;               // range of the gate knob's radii (accepted, unused)
 
 // What a round reads of a drained cell, made in the prepass (one 64-byte line segment per cell).
@@ -60,8 +62,7 @@ static_assert(sizeof(LvCell) == 64, "LvCell");
 
 // The footprint volumes a cell of the gate layer found, for searches of earlier cells.
 struct __align__(16) LvOld {
-  float vol[7];
-  unsigned wmask;  // footprint slots it wrote
+  float vol[8];
 };
 
 // The pressure search under way.
@@ -69,9 +70,12 @@ enum SearchStatus { SS_NONE = 0, SS_SUCCESS = 1, SS_BLOCKED = 2, SS_MORE = 3 };
 struct Search {
   unsigned q[PRESSURE_SEARCH];  // queued cells, relative to the pulling cell (rel_pack)
   float qv[PRESSURE_SEARCH];    // their volume
-  unsigned vkey[VIS_SLOTS];     // visited cells (EMPTY_ID = free); all free between searches
-  unsigned vrank[VIS_SLOTS];    // earliest (entry, direction) that tested the cell
-  unsigned short qh[PRESSURE_SEARCH + 8];  // visited slots of the queued cells, the pulling cell's at [512]
+  // Visited set: a key stays where a search put it; what tells searches apart is the rank, whose
+  // base falls from search to search, so that an older search's rank never wins (a set emptied after
+  // every search cost ~700 cycles of each pull).
+  unsigned vkey[VIS_SLOTS];     // cells tested by this or earlier searches (EMPTY_ID = free)
+  unsigned vrank[VIS_SLOTS];    // rank base + earliest (entry, direction) that tested the cell
+  unsigned rank0, nvis;         // the search's rank base, keys added since the set was last empty
   unsigned m_win[MAX_WARPS], m_side[MAX_WARPS], m_new[MAX_WARPS];
   unsigned blk;                 // 1 + an unfinished earlier cell the search depends on (0: none)
   unsigned pos, status, i, qlen, side;  // the cell, and the search's progress
@@ -93,7 +97,7 @@ struct HeadState {
 constexpr unsigned TEST_FAILED = 0xFFFFFFFFu;
 
 struct LvSmem {
-  unsigned dep[(MAX_CELLS_PER_TICK + 3) / 4];  // a byte per cell: unfinished earlier conflicting cells, DONE
+  unsigned dep[(MAX_CELLS_PER_TICK + 3) / 4];  // a byte per cell: unfinished earlier conflicting cells, or DONE | slots
   unsigned att[NGROUPS + 1];   // bit per cell: not solid and below 1 - 1e-4 at the tick's start
   unsigned pp[NGROUPS + 1];    // bit per unfinished cell that may find a start cell within the budget
   unsigned short gpre[NGROUPS + 1];  // att bits before each group of 32
@@ -310,7 +314,8 @@ __device__ __forceinline__ void park_put(const Region& R, unsigned b, unsigned t
   if (t < MAX_CELLS_PER_TICK) R.lv_park[(size_t)b * MAX_CELLS_PER_TICK + t] = (unsigned short)i;
   else set_status(R, ST_RANGE, 52);
 }
-__device__ __forceinline__ bool cell_done(const LvSmem& L, unsigned i) { return ((vld(&L.dep[i >> 2]) >> ((i & 3u) * 8u)) & 0xFFu) == DONE; }
+__device__ __forceinline__ unsigned dep_byte(const LvSmem& L, unsigned i) { return reinterpret_cast<const volatile unsigned char*>(L.dep)[i]; }
+__device__ __forceinline__ bool cell_done(const LvSmem& L, unsigned i) { return dep_byte(L, i) >= DONE; }
 __device__ __forceinline__ bool bit_of(const unsigned* w, unsigned i) { return (w[i >> 5] >> (i & 31u)) & 1u; }
 // att bits before position i
 __device__ __forceinline__ unsigned attempts_before(const LvSmem& L, unsigned i) {
@@ -439,23 +444,25 @@ __device__ __forceinline__ float lv_cells(const Region& R, LvSmem& L, const Lane
     materialize_par(R, need, gi, s, cap);
     if (need && s != NOSLOT) slot = s;
   }
-  SVPlan p{};
-  if (wr) {
-    const bool hs = !(slot & UNIFORM);
-    p = sv_plan(part, (unsigned char)mat, hs, wv);
-    if (hs) sv_apply(R, (size_t)slot * 512u + at, p);
-    pd += p.dp;
+  // snapped to 0 or full the entry goes; water shows from 0.5 and hides below 0.3 (a snapped volume lies
+  // on the same side of both), and these cells hold air or water only
+  const bool is_water = mat == WATER, mid = wv > 1e-6f && wv < FULL, had = part > 0.0f;
+  const bool wet = wv >= (is_water ? HIDE_BELOW : SHOW_AT), hs = wr && !(slot & UNIFORM), ch = hs && wet != is_water;
+  if (hs) {
+    const size_t o = (size_t)slot * 512u + at;
+    if (mid || had) R.avol[o] = mid ? wv : 0.0f;
+    if (ch) R.amat[o] = wet ? WATER : (unsigned char)0;
+    pd += (mid ? 1 : 0) - (had ? 1 : 0);
   }
   const unsigned wm = __ballot_sync(FULLMASK, wr) >> base;
-  const unsigned cm = __ballot_sync(FULLMASK, wr && p.ch) >> base;
-  const unsigned am = __ballot_sync(FULLMASK, l == 1u ? w_below : ok && f > SLEEP) >> base;
+  const unsigned cm = __ballot_sync(FULLMASK, ch) >> base;
+  // activation slots: 2 below, 3..6 the sides, 7 the cell itself
+  const unsigned am = __ballot_sync(FULLMASK, l == 2u ? w_below : l == 7u ? live && dv > SLEEP : ok && f > SLEEP) >> base;
   if (has) {
-    if (y == gate) reinterpret_cast<unsigned*>(R.lv_old + i)[l] = l == 7u ? wm : __float_as_uint(v);
+    if (y == gate) R.lv_old[i].vol[l] = v;
     if (l == 0u) {
-      // activation slots: 2 below, 3..6 the sides, 7 the cell itself
-      const bool self = live && dv > SLEEP;
-      R.lv_ev[i] = ev | (am & 0x78u) | ((am & 2u) << 1) | (self ? 0x10080u : 0u) | ((cm & 0x7Fu) << 8);
-      reinterpret_cast<volatile unsigned char*>(L.dep)[i] = (unsigned char)DONE;
+      R.lv_ev[i] = ev | (am & 0xFCu) | ((am & 0x80u) << 9) | ((cm & 0x7Fu) << 8);  // bit 16: seeds itself
+      reinterpret_cast<volatile unsigned char*>(L.dep)[i] = (unsigned char)(DONE | (wm & 0x7Fu));
       if (i < kp && bit_of(L.pp, i)) atomicAnd(&L.pp[i >> 5], ~(1u << (i & 31u)));
     }
   }
@@ -473,30 +480,36 @@ __device__ __forceinline__ unsigned vis_slot(Search& C, unsigned key) {
   }
 }
 
+// The set empty and the rank base at its top; by the threads of one warp or of the CTA.
+__device__ __forceinline__ void vis_reset(Search& C, unsigned t0, unsigned nt) {
+  for (unsigned t = t0; t < VIS_SLOTS; t += nt) {
+    C.vkey[t] = EMPTY_ID;
+    C.vrank[t] = 0xFFFFFFFFu;
+  }
+  if (t0 == 0u) {
+    C.rank0 = 0xFFFFFFFFu - VIS_RANKS;
+    C.nvis = 0u;
+  }
+}
+
 // The volume a cell of the pulling layer holds at the turn of the cell at position k, given the volume
 // `v` it holds now and the positions j of its writers (itself, and the cells it is a side of): later
 // ones that already ran and wrote it are looked through (the earliest such write's old value); an
 // unfinished earlier writer is reported in C.blk.
 __device__ __forceinline__ float old_volume(const Region& R, const LvSmem& L, Search& C, unsigned k, const unsigned (&j)[5], float v) {
-  unsigned best = NOSLOT;
+  unsigned best = NOSLOT, blk = 0u, slot = 0u;
 #pragma unroll
   for (int q = 0; q < 5; ++q) {
-    if (j[q] == NOSLOT || j[q] == k) continue;
-    const bool done = cell_done(L, j[q]);
-    if (j[q] < k) {
-      if (!done) atomicMax(&C.blk, j[q] + 1u);
-    } else if (done && j[q] < best) {
-      const LvOld& o = R.lv_old[j[q]];
-      const int fl = q == 0 ? 0 : q + 2;
-      const unsigned wm = o.wmask;
-      const float ov = o.vol[fl];
-      if ((wm >> fl) & 1u) {
-        best = j[q];
-        v = ov;
-      }
+    const unsigned fl = q == 0 ? 0u : q + 2u;
+    const unsigned b = j[q] != NOSLOT ? dep_byte(L, j[q]) : DONE;
+    if (j[q] < k && b < DONE) blk = max(blk, j[q] + 1u);
+    if (j[q] > k && b >= DONE && ((b >> fl) & 1u) && j[q] < best) {
+      best = j[q];
+      slot = fl;
     }
   }
-  return v;
+  if (blk) atomicMax(&C.blk, blk);
+  return best != NOSLOT ? R.lv_old[best].vol[slot] : v;
 }
 
 // What a search round's thread finds: its queue entry's neighbour d.
@@ -509,24 +522,29 @@ __device__ __forceinline__ SearchRead search_read(const Region& R, LvSmem& L, co
   Search& C = L.s;
   SearchRead r{0u, 0.0f, 0.0f, false, false, false};
   if (act) {
-    int a, b, c, dx, dy, dz;
-    rel_unpack(C.q[e], a, b, c);
+    const unsigned k0 = C.q[e];
     r.here = C.qv[e];
-    dir5((int)d, dx, dy, dz);
-    dx += a;
-    dy += b;
-    dz += c;
+    // up, +x, -x, +z, -z as steps of the packed position
+    r.key = k0 + (d == 0u ? 1u << 22 : d == 1u ? 1u : d == 2u ? 0u - 1u : d == 3u ? 1u << 11 : 0u - (1u << 11));
+    int dx, dy, dz;
+    rel_unpack(r.key, dx, dy, dz);
     const int x = C.cx + dx, y = C.cy + dy, z = C.cz + dz;
     // (once the 24 side checks at the start level are spent, what its cells hold no longer matters)
     const bool rd = d == 0u ? y < R.ny : (x >= 0 && z >= 0 && (sides || dy != 0));
     bool top = true;
     if (rd && !outside(R, ring, x, y, z)) {
-      // the grid word and, on the pulling layer, the writers' positions: issued together
+      // the grid word and, on the pulling layer, the writers' positions: issued together (a cell of
+      // the world has its neighbours inside the padded domain)
       const unsigned g = gld(R.grid + grid_index(R, x >> 3, y >> 3, z >> 3));
       unsigned j[5] = {NOSLOT, NOSLOT, NOSLOT, NOSLOT, NOSLOT};
       if (dy == 0) {
-#pragma unroll
-        for (int q = 0; q < 5; ++q) j[q] = rank_at(R, x - (q == 1) + (q == 2), y, z - (q == 3) + (q == 4));
+        const unsigned* st = R.stamp + dom_id(R, x, y, z);
+        const int row = R.PX * R.PY;
+        j[0] = st[0];
+        j[1] = st[-1];
+        j[2] = st[1];
+        j[3] = st[-row];
+        j[4] = st[row];
       }
       const size_t o = g < 256u ? (size_t)0 : (size_t)(g - 256u) * 512u + local_index(x, y, z);
       const float part = R.avol[o];
@@ -538,10 +556,9 @@ __device__ __forceinline__ SearchRead search_read(const Region& R, LvSmem& L, co
       }
     }
     // the surface test of the entry on its up neighbour (fluid.rs:534-535), else an expansion
-    r.win = d == 0u && top && b > 0 && r.here > 0.0f;
+    r.win = d == 0u && top && (k0 >> 22) != 0u && r.here > 0.0f;
     r.cand = rd && !top;
     r.side = r.cand && d != 0u && dy == 0;
-    r.key = rel_pack(dx, dy, dz);
   }
   return r;
 }
@@ -559,21 +576,31 @@ __device__ __forceinline__ void search_won(Search& C, const SearchRead& r, unsig
 }
 
 // FluidSim::pressure_pull (fluid.rs:511-561) of the cell at position k: its start, by one warp. Writes
-// nothing but L.s. Returns whether there is anything to examine.
-__device__ __forceinline__ bool search_begin(const Region& R, LvSmem& L, const int* ring, unsigned k, unsigned long long cap) {
+// nothing but L.s. A search examines at most 24 sides on its own layer, so nearly all it reads there is
+// written by the cells within three rows and columns: `wait` gets 1 + the last unfinished earlier one
+// of them (0: none), one probe per lane instead of a search that finds out. Returns whether there is
+// anything to examine.
+__device__ __forceinline__ bool search_begin(const Region& R, LvSmem& L, const int* ring, unsigned k, int sgn, unsigned& wait, unsigned long long cap) {
   Search& C = L.s;
   const float FULL = full_level();
   const unsigned lane = lane_id();
   const LvCell& rc = R.lv[k];
-  const unsigned flags = rc.flags;
+  const unsigned flags = rc.flags, cid = rc.cid;
   int x, y, z;
-  dom_xyz(R, rc.cid, x, y, z);
+  dom_xyz(R, cid, x, y, z);
+  // lanes 0..20: the three rows before, x - 3 .. x + 3; 21..23: the three cells before in the row
+  const int row = (int)lane / 7, ndx = lane < 21u ? (int)lane - 7 * row - 3 : -sgn * ((int)lane - 20);
+  const int ndz = lane < 21u ? -sgn * (row + 1) : 0;
+  unsigned near = NOSLOT;
+  if (lane < 24u) near = R.stamp[(int)cid + ndx + ndz * R.PX * R.PY];
   float v = 0.0f;
   if (lane < 7u && !((flags >> lane) & 1u)) {
     int ox, oy, oz;
     fp_off((int)lane, ox, oy, oz);
     v = cd_volume(load_cell_par(R, ring, x + ox, y + oy, z + oz, cap));
   }
+  wait = __reduce_max_sync(FULLMASK, near != NOSLOT && !cell_done(L, near) ? near + 1u : 0u);
+  if (wait) return false;
   const float vol = __shfl_sync(FULLMASK, v, 0);
   unsigned starts = (__ballot_sync(FULLMASK, lane >= 2u && lane < 7u && ((flags >> (6u + lane)) & 1u) && v >= FULL) >> 2) & 31u;
   unsigned before = attempts_before(L, k);
@@ -583,6 +610,12 @@ __device__ __forceinline__ bool search_begin(const Region& R, LvSmem& L, const i
     before += __reduce_add_sync(FULLMASK, c);
   }
   if (!(vol < FULL) || before >= MAX_PULLS_PER_TICK) starts = 0u;
+  if (starts && (C.nvis > VIS_FULL || C.rank0 < VIS_RANKS)) {
+    vis_reset(C, lane, 32u);
+    __syncwarp();
+  }
+  const unsigned rank0 = C.rank0 - VIS_RANKS;
+  __syncwarp();
   if (lane == 0) {
     C.pos = k;
     C.status = SS_NONE;
@@ -595,6 +628,10 @@ __device__ __forceinline__ bool search_begin(const Region& R, LvSmem& L, const i
     C.cx = x;
     C.cy = y;
     C.cz = z;
+    if (starts) {
+      C.rank0 = rank0;
+      C.nvis += 6u;
+    }
   }
   if (starts) {
     // the start cells in direction order; visited ranks 0 (the cell itself), 1..5
@@ -603,11 +640,10 @@ __device__ __forceinline__ bool search_begin(const Region& R, LvSmem& L, const i
     if (st || lane == 0u) {
       int dx = 0, dy = 0, dz = 0;
       if (st) dir5((int)d, dx, dy, dz);
-      const unsigned key = rel_pack(dx, dy, dz), h = vis_slot(C, key);
-      C.vrank[h] = st ? d + 1u : 0u;
-      const unsigned p = st ? (unsigned)__popc(starts & ((1u << d) - 1u)) : PRESSURE_SEARCH;
-      C.qh[p] = (unsigned short)h;
+      const unsigned key = rel_pack(dx, dy, dz);
+      C.vrank[vis_slot(C, key)] = rank0 + (st ? d + 1u : 0u);
       if (st) {
+        const unsigned p = (unsigned)__popc(starts & ((1u << d) - 1u));
         C.q[p] = key;
         C.qv[p] = v;
       }
@@ -624,7 +660,8 @@ __device__ __forceinline__ bool search_begin(const Region& R, LvSmem& L, const i
 __device__ __forceinline__ void search_solo(const Region& R, LvSmem& L, const int* ring) {
   Search& C = L.s;
   const unsigned lane = lane_id(), j = lane / 5u, d = lane - 5u * j;
-  unsigned i = C.i, qlen = C.qlen, side = C.side, status = SS_NONE;
+  unsigned i = C.i, qlen = C.qlen, side = C.side, status = SS_NONE, nvis = 0u;
+  const unsigned rank0 = C.rank0 + 6u;
   while (i < qlen) {
     if (qlen - i > SOLO_WAIT || qlen + 5u * SOLO_ENTRIES > PRESSURE_SEARCH) {
       status = SS_MORE;
@@ -642,7 +679,7 @@ __device__ __forceinline__ void search_solo(const Region& R, LvSmem& L, const in
       const unsigned wl = (unsigned)__ffs(wm) - 1u;
       if (lane == wl) {
         search_won(C, r, i + j);
-        C.qlen = qlen;
+        C.nvis += nvis;
       }
       __syncwarp();
       return;
@@ -650,7 +687,7 @@ __device__ __forceinline__ void search_solo(const Region& R, LvSmem& L, const in
     const unsigned sm = __ballot_sync(FULLMASK, r.side);
     const bool cand = r.cand && !(r.side && side + (unsigned)__popc(sm & lanemask_lt()) + 1u > 24u);
     side += (unsigned)__popc(sm);
-    const unsigned rank = 6u + (i + j) * 5u + d;
+    const unsigned rank = rank0 + (i + j) * 5u + d;
     unsigned h = 0;
     if (cand) {
       h = vis_slot(C, r.key);
@@ -663,9 +700,9 @@ __device__ __forceinline__ void search_solo(const Region& R, LvSmem& L, const in
     if (isnew && pos < PRESSURE_SEARCH) {
       C.q[pos] = r.key;
       C.qv[pos] = r.v;
-      C.qh[pos] = (unsigned short)h;
     }
     qlen += (unsigned)__popc(nm);
+    nvis += (unsigned)__popc(nm);
     i += kk;
     __syncwarp();
   }
@@ -674,19 +711,21 @@ __device__ __forceinline__ void search_solo(const Region& R, LvSmem& L, const in
     C.i = i;
     C.qlen = qlen;
     C.side = side;
+    C.nvis += nvis;
   }
   __syncwarp();
 }
 
 // The same rounds by all warps of the CTA, six entries each in queue order, until the search ends.
 // Entries past the 512th are never examined (fluid.rs:530), so appends stop there. All threads; ends
-// with a barrier, the visited set empty.
+// with a barrier.
 __device__ __noinline__ void search_cta(const Region& Rs, LvSmem& L, const int* ring) {
   const Region R = Rs;
   Search& C = L.s;
   const unsigned tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, nw = blockDim.x >> 5;
   const unsigned jl = lane / 5u, d = lane - 5u * jl, j = warp * SOLO_ENTRIES + jl;  // lanes 30, 31 idle
   unsigned i = C.i, qlen = C.qlen, side = C.side;
+  const unsigned rank0 = C.rank0 + 6u;
   while (i < qlen && i < PRESSURE_SEARCH) {
     const unsigned kk = min(SOLO_ENTRIES * nw, min(qlen, PRESSURE_SEARCH) - i);
     const SearchRead r = search_read(R, L, ring, jl < SOLO_ENTRIES && j < kk, i + j, d, side < 24u);
@@ -716,7 +755,7 @@ __device__ __noinline__ void search_cta(const Region& Rs, LvSmem& L, const int* 
       side += __reduce_add_sync(FULLMASK, c);
     }
     if (qlen < PRESSURE_SEARCH) {
-      const unsigned rank = 6u + (i + j) * 5u + d;
+      const unsigned rank = rank0 + (i + j) * 5u + d;
       unsigned h = 0;
       if (cand) {
         h = vis_slot(C, r.key);
@@ -740,13 +779,12 @@ __device__ __noinline__ void search_cta(const Region& Rs, LvSmem& L, const int* 
     __syncthreads();
   }
   __syncthreads();
-  if (tid == 0 && C.status == SS_MORE) {
-    C.status = SS_NONE;
-    C.i = i;
-  }
-  for (unsigned t = tid; t < VIS_SLOTS; t += blockDim.x) {
-    C.vkey[t] = EMPTY_ID;
-    C.vrank[t] = 0xFFFFFFFFu;
+  if (tid == 0) {
+    if (C.status == SS_MORE) {
+      C.status = SS_NONE;
+      C.i = i;
+    }
+    C.nvis += qlen;  // (keys of the last round that found no place in the queue: fewer than VIS_SLOTS - VIS_FULL - 518)
   }
   __syncthreads();
 }
@@ -837,24 +875,6 @@ __device__ __forceinline__ void lv_head(const Region& R, LvSmem& L, unsigned n, 
   }
 }
 
-// 1 + the last unfinished earlier cell of the pulling layer within three rows and columns of the cell
-// at position k (0: none). A search examines at most 24 sides on its own layer, so nearly all it reads
-// there is written by these cells: one probe per lane here instead of a search that finds out.
-__device__ __forceinline__ unsigned lv_near(const Region& R, const LvSmem& L, unsigned k, int sgn) {
-  const unsigned lane = lane_id();
-  int x, y, z;
-  dom_xyz(R, R.lv[k].cid, x, y, z);
-  // lanes 0..20: the three rows before, x - 3 .. x + 3; 21..23: the three cells before in the row
-  const int row = (int)lane / 7, dx = lane < 21u ? (int)lane - 7 * row - 3 : -sgn * ((int)lane - 20);
-  const int dz = lane < 21u ? -sgn * (row + 1) : 0;
-  unsigned w = 0u;
-  if (lane < 24u) {
-    const unsigned p = rank_at(R, x + dx, y, z + dz);
-    if (p != NOSLOT && !cell_done(L, p)) w = p + 1u;
-  }
-  return __reduce_max_sync(FULLMASK, w);
-}
-
 // The first pp cell has yet to have its turn: can it still find a start cell then? A full neighbour
 // stays full unless it runs before the cell does and falls: a side earlier in sorted order, over a
 // cell that no unfinished cell writes and that has room (a full cell makes no attempt, and a fall of
@@ -923,24 +943,17 @@ __device__ __noinline__ int lv_solo(const Region& Rs, LvSmem& L, const int* ring
           break;
         }
       }
-      const unsigned dep = (vld(&L.dep[H.head >> 2]) >> ((H.head & 3u) * 8u)) & 0xFFu;
+      const unsigned dep = dep_byte(L, H.head);
       if (dep == 0u) {  // its turn has come
-        if (H.blk == 0u || cell_done(L, H.blk - 1u)) H.blk = lv_near(R, L, H.head, sgn);
-        if (H.blk == 0u) {
-          if (search_begin(R, L, ring, H.head, cap)) {
+        if (H.blk == 0u || cell_done(L, H.blk - 1u)) {
+          if (search_begin(R, L, ring, H.head, sgn, H.blk, cap)) {
             search_solo(R, L, ring);
             if (L.s.status == SS_MORE) {
               req = SR_SEARCH;
               break;
             }
-            // leave the visited set empty
-            for (unsigned t = lane; t <= L.s.qlen; t += 32u) {
-              const unsigned h = L.s.qh[t < L.s.qlen ? t : PRESSURE_SEARCH];
-              L.s.vkey[h] = EMPTY_ID;
-              L.s.vrank[h] = 0xFFFFFFFFu;
-            }
           }
-          finish = true;
+          finish = H.blk == 0u;
         }
       } else if (H.test == 0u || (H.test != TEST_FAILED && cell_done(L, H.test - 1u))) {
         H.test = lv_prune(R, L, ring, H.head, cap);
