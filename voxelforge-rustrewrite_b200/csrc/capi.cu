@@ -120,6 +120,13 @@ void free_world(vf_fluid* h) {
   h->uploaded = false;
 }
 
+// The dense words in step with the grid and the atlas again.
+int build_dense(vf_fluid* h) {
+  k_dense<<<(unsigned)std::min<uint64_t>(((uint64_t)h->R.ncells + 255) / 256, 148 * 32), 256, 0, h->stream>>>(h->R);
+  CK(cudaGetLastError());
+  return VF_OK;
+}
+
 int ensure_scratch(vf_fluid* h, size_t bytes) {
   if (h->scratch_bytes >= bytes) return VF_OK;
   if (h->scratch) {
@@ -404,6 +411,7 @@ int vf_fluid_upload_world(vf_fluid* h, int32_t nx, int32_t ny, int32_t nz, int32
   if ((rc = dalloc(h, &R.grid, nb, false))) return rc;
   if ((rc = dalloc(h, &R.amat, cap * 512, false))) return rc;
   if ((rc = dalloc(h, &R.avol, cap * 512, false))) return rc;
+  if ((rc = dalloc(h, &R.dense, ncells, false))) return rc;
   CK(cudaMemsetAsync(R.avol, 0, nd * 512 * sizeof(float) + 16, h->stream));
   CK(cudaMemcpyAsync(R.grid, dgrid.data(), nb * 4, cudaMemcpyHostToDevice, h->stream));
   {
@@ -462,8 +470,9 @@ int vf_fluid_upload_world(vf_fluid* h, int32_t nx, int32_t ny, int32_t nz, int32
   CK(cudaMemcpyAsync(R.ctl, h->hctl, sizeof(Ctl), cudaMemcpyHostToDevice, h->stream));
   if ((rc = dalloc(h, &h->dR, 1, false))) return rc;
   CK(cudaMemcpyAsync(h->dR, &R, sizeof(Region), cudaMemcpyHostToDevice, h->stream));
-  CK(cudaStreamSynchronize(h->stream));
   h->R = R;
+  if ((rc = build_dense(h))) return rc;
+  CK(cudaStreamSynchronize(h->stream));
   h->uploaded = true;
   h->acc = 0.0f;
   return VF_OK;
@@ -881,7 +890,10 @@ int vf_fluid_ring_evict(vf_fluid* h, int32_t cx, int32_t cz) {  // sparse_volume
   const int w = h->R.ring_w;
   std::vector<int32_t> ring(3 * w * w);
   CK(cudaMemcpy(ring.data(), h->R.ring, ring.size() * 4, cudaMemcpyDeviceToHost));
-  return ring_evict_slot(h, (cz & (w - 1)) * w + (cx & (w - 1)), ring);
+  if ((rc = ring_evict_slot(h, (cz & (w - 1)) * w + (cx & (w - 1)), ring))) return rc;
+  if ((rc = build_dense(h))) return rc;
+  CK(cudaStreamSynchronize(h->stream));
+  return VF_OK;
 }
 
 int vf_fluid_ring_paste(vf_fluid* h, const uint32_t* chunk_grid, const uint8_t* chunk_bricks, uint64_t chunk_nbricks, int32_t chunk_bricks_y,
@@ -979,6 +991,8 @@ int vf_fluid_ring_paste(vf_fluid* h, const uint32_t* chunk_grid, const uint8_t* 
   if ((rc = detached_bits(h, back, 0))) return rc;
   if ((rc = detached_count(h, -(long long)back.size()))) return rc;
   h->det.swap(keep);
+  if ((rc = build_dense(h))) return rc;
+  CK(cudaStreamSynchronize(h->stream));
   return VF_OK;
 }
 
@@ -1020,6 +1034,7 @@ int vf_fluid_reset(vf_fluid* h) {  // fluid.rs:318-320: the fluid's tables only
   std::memcpy(z.prof, c.prof, sizeof(z.prof));
   CK(cudaMemcpyAsync(R.ctl, &z, sizeof(Ctl), cudaMemcpyHostToDevice, h->stream));
   h->acc = 0.0f;
+  if ((rc = build_dense(h))) return rc;
   return sync_ctl(h);
 }
 

@@ -84,6 +84,7 @@ struct Region {
   unsigned int* grid;        // bx*by*bz
   unsigned char* amat;       // atlas materials [atlas_cap][512]
   float* avol;               // atlas partial volumes [atlas_cap][512]
+  unsigned* dense;           // ncells: every cell of the domain as the rules see it (dense_code), in step with the above
   unsigned int atlas_cap;
   int* ring;                 // ring_w*ring_w triples (cx, cz, loaded)
   // ---- scheduler
@@ -203,7 +204,22 @@ __host__ __device__ inline unsigned grid_index(const Region& R, int ix, int iy, 
   return ((unsigned)iz * (unsigned)R.by + (unsigned)iy) * (unsigned)R.bx + (unsigned)ix;
 }
 
-// One cell as the rules see it.
+// One cell as the rules see it, in a word per cell of the domain: the volume's bits, negative while the
+// material is air (an entry below the show level), 0 empty, 1.0 full water, and a code above for solid
+// cells and cells outside the world (with or without a partial entry of their own). The sweep and its
+// searches read one word at id + offset where bricks take a grid word, a slot, a material and a
+// volume; the atlas stays what the host, the edits and the exports see.
+constexpr unsigned DC_SOLID = 0x40000000u, DC_SOLID_PART = 0x40800000u, DC_FULL = 0x3F800000u, DC_AIR = 0x80000000u;
+__host__ __device__ inline unsigned dense_code(bool out, unsigned mat, unsigned part_bits) {
+  const bool part = (int)part_bits > 0;  // part > 0
+  if (out) return DC_SOLID;
+  if (mat != 0u && mat != WATER) return part ? DC_SOLID_PART : DC_SOLID;
+  if (part) return part_bits | (mat == WATER ? 0u : DC_AIR);
+  return mat == WATER ? DC_FULL : 0u;
+}
+__host__ __device__ inline bool dc_solid(unsigned u) { return (int)u >= (int)DC_SOLID; }
+
+// One cell as the atlas holds it.
 struct __align__(16) CD {
   float part;       // partial volume (0 = none)
   unsigned slot;    // atlas slot of the brick, NOSLOT when the brick is a uniform grid value

@@ -154,18 +154,18 @@ __device__ __forceinline__ void record_change(const Region& R, unsigned id) {
   }
 }
 
-// Material write; the change is recorded at once (host edits) or logged by the caller (ticks,
-// where `deferred` is set and the caller appends the cell to the change log).
-__device__ __forceinline__ void write_mat(const Region& R, CD& c, unsigned l, unsigned id, unsigned char m, bool deferred = false) {
-  if (c.slot == NOSLOT) return;  // materialisation failed (status already set)
-  R.amat[(size_t)c.slot * 512u + l] = m;
-  c.mat = m;
-  if (!deferred) record_change(R, id);
-}
+// The dense word of a cell after its atlas entry was written.
+__device__ __forceinline__ void dense_put(const Region& R, unsigned id, unsigned mat, float part) { R.dense[id] = dense_code(false, mat, __float_as_uint(part)); }
+__device__ __forceinline__ float dc_volume(unsigned u) { return __uint_as_float(u & 0x7FFFFFFFu); }
+// FluidSim::volume as the levelling tests it (> 0, >= 1 - 1e-4): a solid cell's partial entry counts as
+// water there (fluid.rs:251-260 looks at the entry first).
+__device__ __forceinline__ float dc_level(unsigned u) { return u == DC_SOLID ? 0.0f : u == DC_SOLID_PART ? 1.0f : dc_volume(u); }
+__device__ __forceinline__ unsigned dense_at(const Region& R, int x, int y, int z) { return in_dom(R, x, y, z) ? R.dense[dom_id(R, x, y, z)] : DC_SOLID; }
 
-__device__ __forceinline__ void erase_part(const Region& R, CD& c, unsigned l, long long& pdelta) {
+__device__ __forceinline__ void erase_part(const Region& R, CD& c, unsigned l, unsigned id, long long& pdelta) {
   if (c.slot != NOSLOT && c.part > 0.0f) {
     R.avol[(size_t)c.slot * 512u + l] = 0.0f;
+    dense_put(R, id, c.mat, 0.0f);
     c.part = 0.0f;
     pdelta -= 1;
   }
@@ -208,6 +208,7 @@ __device__ __forceinline__ bool set_volume_lane(const Region& R, CD& c, int x, i
   if (wmat) R.amat[(size_t)c.slot * 512u + l] = nmat;
   if (has) c.part = npart;
   if (wmat) c.mat = nmat;
+  if (has) dense_put(R, id, c.mat, npart);
   if (wmat && !deferred) record_change(R, id);
   return ch;
 }
@@ -323,15 +324,12 @@ __device__ __forceinline__ void side4(int d, int& dx, int& dz) {  // SIDES (flui
 
 // FluidSim::level_layer's membership test (fluid.rs:413-415) of (x, y, z): !solid && vol > 0 &&
 // supported && vol(above) <= 0. Returns the cell's volume through *v.
-__device__ __forceinline__ bool level_member(const Region& R, const int* ring, int x, int y, int z, float* v) {
-  const float FULL = full_level();
-  const CD c = load_cell(R, ring, x, y, z);
-  *v = cd_volume(c);
-  if (cd_solid(c) || !(*v > 0.0f)) return false;
-  const CD b = load_cell(R, ring, x, y - 1, z);
-  if (!(cd_solid(b) || cd_volume(b) >= FULL)) return false;
-  const CD a = load_cell(R, ring, x, y + 1, z);
-  return cd_volume(a) <= 0.0f;
+__device__ __forceinline__ bool level_member(const Region& R, int x, int y, int z, float* v) {
+  const unsigned c = dense_at(R, x, y, z);
+  *v = dc_level(c);
+  if (dc_solid(c) || !(*v > 0.0f)) return false;
+  const unsigned b = dense_at(R, x, y - 1, z), a = dense_at(R, x, y + 1, z);  // inside the domain: the cell is in the world
+  return (dc_solid(b) || dc_volume(b) >= full_level()) && !(dc_level(a) > 0.0f);
 }
 
 // The flood fill of FluidSim::level_layer (fluid.rs:425-446) continued by one warp from queue
@@ -359,11 +357,10 @@ __device__ unsigned level_bfs_warp(const Region& R, Smem& S, unsigned& i, unsign
     bool skip = lane >= 12 || (R.ring_w == 0 && (nx < 0 || nz < 0));
     unsigned tas = 0;
     if (!skip && j == 0) tas = mark_tas(R, nx, y, nz);
-    CD c = CD{0.0f, NOSLOT, 0u, 0, true};
-    if (!skip) c = load_cell(R, S.ring, nx, y + (j == 1 ? -1 : (j == 2 ? 1 : 0)), nz);
+    const unsigned c = skip ? DC_SOLID : dense_at(R, nx, y + (j == 1 ? -1 : (j == 2 ? 1 : 0)), nz);
     // gather the three cells of each side at its j==0 lane
-    float v = cd_volume(c);
-    bool sol = cd_solid(c);
+    const bool sol = dc_solid(c);
+    const float v = dc_level(c);
     float v1 = __shfl_down_sync(FULLMASK, v, 1), v2 = __shfl_down_sync(FULLMASK, v, 2);
     bool s1 = __shfl_down_sync(FULLMASK, (unsigned)sol, 1) != 0u;
     bool push = !skip && j == 0 && !tas && !sol && v > 0.0f && (s1 || v1 >= FULL) && v2 <= 0.0f;
@@ -412,7 +409,7 @@ __device__ bool level_layer(const Region& R, WS& W, Smem& S, int sx, int sy, int
   was = __shfl_sync(FULLMASK, was, 0);
   if (was) return false;
   float v0 = 0.0f;
-  const bool member = level_member(R, S.ring, sx, sy, sz, &v0);
+  const bool member = level_member(R, sx, sy, sz, &v0);
   if (!member) return false;
   if (lane == 0) {
     R.lvl_id[0] = dom_id(R, sx, sy, sz);

@@ -386,45 +386,35 @@ __device__ __noinline__ void sweep_levels(const Region& Rs, TickSmem& sm, WS& sW
     bool att = false, pp = false;
     if (i < n) {
       const unsigned cid = key_to_id(R, R.cells[i], flip);
-      int x, y, z;
-      dom_xyz(R, cid, x, y, z);
-      CD c[7];
-#pragma unroll
-      for (int l = 0; l < 7; ++l) {
-        int ox, oy, oz;
-        fp_off(l, ox, oy, oz);
-        c[l] = load_cell(R, ring, x + ox, y + oy, z + oz);
-      }
+      const unsigned u = R.dense[cid];
       R.lv_ev[i] = 0u;
-      if (cd_solid(c[0])) {  // fluid.rs:586-589; nothing reads a solid cell's partial volume
-        if (c[0].slot != NOSLOT && c[0].part > 0.0f) {
-          R.avol[(size_t)c[0].slot * 512u + local_index(x, y, z)] = 0.0f;
+      if (dc_solid(u)) {
+        reinterpret_cast<unsigned char*>(L.dep)[i] = DONE;
+        if (u == DC_SOLID_PART) {  // fluid.rs:586-589; nothing reads a solid cell's partial volume
+          int x, y, z;
+          dom_xyz(R, cid, x, y, z);
+          const CD c = load_cell(R, ring, x, y, z);
+          R.avol[(size_t)c.slot * 512u + local_index(x, y, z)] = 0.0f;
+          R.dense[cid] = DC_SOLID;
           pd -= 1;
         }
-        reinterpret_cast<unsigned char*>(L.dep)[i] = DONE;
       } else {
+        unsigned nu[5];  // up, +x, -x, +z, -z
+#pragma unroll
+        for (int d = 0; d < 5; ++d) nu[d] = R.dense[(int)cid + fp_id(R, 2 + d)];
         reinterpret_cast<unsigned char*>(L.dep)[i] = 0;
         R.stamp[cid] = i;
-        unsigned fl = local_index(x, y, z) << 16;
-        unsigned sl[7];
-        att = cd_volume(c[0]) < FULL;
+        int x, y, z;
+        dom_xyz(R, cid, x, y, z);
+        unsigned ye = (unsigned)y;
+        att = dc_volume(u) < FULL;
 #pragma unroll
-        for (int l = 0; l < 7; ++l) {
-          const bool so = cd_solid(c[l]);
-          sl[l] = c[l].slot != NOSLOT ? c[l].slot : (UNIFORM | c[l].mat);
-          fl |= so ? (1u << l) : 0u;
-          if (l >= 2) {
-            int ox, oy, oz;
-            fp_off(l, ox, oy, oz);
-            const bool st = !so && x + ox >= 0 && z + oz >= 0;
-            fl |= st ? (1u << (6 + l)) : 0u;
-            pp |= att && st && cd_volume(c[l]) >= FULL;
-          }
+        for (int d = 0; d < 5; ++d) {
+          const bool st = x + (d == 1) - (d == 2) >= 0 && z + (d == 3) - (d == 4) >= 0;
+          ye |= st ? 1u << (27 + d) : 0u;
+          pp |= att && st && !dc_solid(nu[d]) && dc_volume(nu[d]) >= FULL;
         }
-        uint4* o = reinterpret_cast<uint4*>(R.lv + i);
-        o[0] = make_uint4(sl[0], sl[1], sl[2], sl[3]);
-        o[1] = make_uint4(sl[4], sl[5], sl[6], cid);
-        reinterpret_cast<uint2*>(o)[7] = make_uint2(fl, (unsigned)y);
+        reinterpret_cast<uint2*>(R.lv + i)[3] = make_uint2(cid, ye);
       }
     }
     const unsigned ab = __ballot_sync(FULLMASK, att), pb = __ballot_sync(FULLMASK, pp);
@@ -473,8 +463,8 @@ __device__ __noinline__ void sweep_levels(const Region& Rs, TickSmem& sm, WS& sW
     for (int q = 0; q < 12; ++q)
       if (s[q] != NOSUCC) atomicAdd(&L.dep[s[q] >> 2], 1u << ((s[q] & 3u) * 8u));
     uint4* o = reinterpret_cast<uint4*>(R.lv + i);
-    o[2] = make_uint4(s[0] | s[1] << 16, s[2] | s[3] << 16, s[4] | s[5] << 16, s[6] | s[7] << 16);
-    reinterpret_cast<uint2*>(o)[6] = make_uint2(s[8] | s[9] << 16, s[10] | s[11] << 16);
+    o[0] = make_uint4(s[0] | s[1] << 16, s[2] | s[3] << 16, s[4] | s[5] << 16, s[6] | s[7] << 16);
+    reinterpret_cast<uint2*>(o)[2] = make_uint2(s[8] | s[9] << 16, s[10] | s[11] << 16);
   }
   __syncthreads();
   if (warp == 0) {
@@ -487,30 +477,30 @@ __device__ __noinline__ void sweep_levels(const Region& Rs, TickSmem& sm, WS& sW
   // ---- the first round: cells that wait for nobody
   for (unsigned i = tid; i < n; i += NT_) {
     if (dep_byte(L, i) != 0u) continue;
-    if (R.lv[i].y <= gate) list_put(R, L, 0u, atomicAdd(&L.cnt[0], 1u), i);
+    if ((int)(R.lv[i].ye & YE_Y) <= gate) list_put(R, L, 0u, atomicAdd(&L.cnt[0], 1u), i);
     else park_put(R, 0u, atomicAdd(&L.park_n[0], 1u), i);
   }
   __syncthreads();
   plap(0);
   // ---- rounds
-  const LaneSlot ls = lane_slot();
+  const LaneSlot ls = lane_slot(R);
   long long t_wide = 0, t_search = 0;
   while (true) {
     // warp 0 alone decides what comes next: nobody else reads the lists' state while it runs
-    if (warp == 0) pd += lv_solo(Rs, L, ring, n, gate, sgn, cap);
+    if (warp == 0) pd += lv_solo(Rs, L, n, gate, sgn, cap);
     __syncthreads();
     const unsigned req = L.req;
     if (req == SR_END) break;
     if (req == SR_SEARCH) {
       const long long c0 = clock64();
-      search_cta(Rs, L, ring);
+      search_cta(Rs, L);
       t_search += clock64() - c0;
     } else if (req == SR_GATE) {
       gate = L.h.gate;
       const unsigned pb = L.pb, np = min(L.park_n[pb], MAX_CELLS_PER_TICK), lb = L.cur, lc = L.cc;
       for (unsigned t = tid; t < np; t += NT_) {
         const unsigned i = R.lv_park[(size_t)pb * MAX_CELLS_PER_TICK + t];
-        if (R.lv[i].y <= gate) list_put(R, L, lb, atomicAdd(&L.cnt[lc], 1u), i);
+        if ((int)(R.lv[i].ye & YE_Y) <= gate) list_put(R, L, lb, atomicAdd(&L.cnt[lc], 1u), i);
         else park_put(R, pb ^ 1u, atomicAdd(&L.park_n[pb ^ 1u], 1u), i);
       }
       __syncthreads();
@@ -530,7 +520,7 @@ __device__ __noinline__ void sweep_levels(const Region& Rs, TickSmem& sm, WS& sW
         for (unsigned t0 = warp * 4u; t0 < fcount; t0 += NW_ * 4u) {
           const unsigned t = t0 + (lane >> 3);
           const unsigned i = t < fcount ? list_get(R, L, cur, t) : 0u;
-          lv_cells(R, L, ls, t < fcount && !cell_done(L, i), i, false, 0.0f, 0u, gate, kp, nb, nc, pb, pd, cap);
+          lv_cells(R, L, ls, t < fcount && !cell_done(L, i), i, false, 0.0f, 0u, gate, kp, nb, nc, pb, pd);
         }
         __syncthreads();
         cur = nb;
@@ -564,6 +554,7 @@ __device__ __noinline__ void sweep_levels(const Region& Rs, TickSmem& sm, WS& sW
     R.ctl->par_rollbacks += L.n_again;
     R.ctl->par_replayed += L.n_searches;
   }
+  sweep_flush(R, L, n, cap);
   // ---- the position map back to idle
   for (unsigned i = tid; i < n; i += NT_) R.stamp[key_to_id(R, R.cells[i], flip)] = 0xFFFFFFFFu;
   // ---- the cells' events in sorted order -> the tick's event logs (program order)
@@ -753,7 +744,7 @@ __device__ __noinline__ unsigned level_bfs_cta(const Region& R, TickSmem& sm, Sm
             R.rb[nid] = 0xFFFFFFFFu;
             unsigned tile;
             const unsigned listed = mark_begin(R, nx, y, nz, tile);  // unmarked: it won the claim
-            f = level_member(R, S.ring, nx, y, nz, &v) ? 1u : 0u;
+            f = level_member(R, nx, y, nz, &v) ? 1u : 0u;
             mark_end(R, tile, listed);
           }
         }
@@ -871,7 +862,7 @@ __device__ __noinline__ void level_finish_cta(const Region& R, TickSmem& sm, WS&
     bool ch = false;
     if (wv) {
       const SVPlan p = sv_plan(c.part, c.mat, c.slot != NOSLOT, avg);
-      if (c.slot != NOSLOT) sv_apply(R, (size_t)c.slot * 512u + local_index(x, y, z), p);
+      if (c.slot != NOSLOT) sv_apply(R, c, id, local_index(x, y, z), p);
       ch = p.ch;
       pd += p.dp;
     }
@@ -913,7 +904,7 @@ struct LevelFill {
   float avg;
 };
 
-__device__ void level_fill_small(const Region& R, const int* ring, LevelFill& F, unsigned sid) {
+__device__ void level_fill_small(const Region& R, LevelFill& F, unsigned sid) {
   const unsigned lane = lane_id();
   const float FULL = full_level();
   for (unsigned t = lane; t < FILL_SLOTS; t += 32u) F.key[t] = EMPTY_ID;
@@ -930,7 +921,7 @@ __device__ void level_fill_small(const Region& R, const int* ring, LevelFill& F,
   int sx, sy, sz;
   dom_xyz(R, sid, sx, sy, sz);
   float v0;
-  level_member(R, ring, sx, sy, sz, &v0);
+  level_member(R, sx, sy, sz, &v0);
   if (lane == 0) {
     test(sid);
     F.id[0] = sid;
@@ -953,10 +944,9 @@ __device__ void level_fill_small(const Region& R, const int* ring, LevelFill& F,
       nid = dom_id(R, nx, y, nz);
       seen = mark_test(R, nx, y, nz) || test(nid);
     }
-    CD c = CD{0.0f, NOSLOT, 0u, 0, true};
-    if (!skip) c = load_cell(R, ring, nx, y + (j == 1 ? -1 : (j == 2 ? 1 : 0)), nz);
-    const float v = cd_volume(c);
-    const bool sol = cd_solid(c);
+    const unsigned c = skip ? DC_SOLID : dense_at(R, nx, y + (j == 1 ? -1 : (j == 2 ? 1 : 0)), nz);
+    const bool sol = dc_solid(c);
+    const float v = dc_level(c);
     const float v1 = __shfl_down_sync(FULLMASK, v, 1), v2 = __shfl_down_sync(FULLMASK, v, 2);
     const bool s1 = __shfl_down_sync(FULLMASK, (unsigned)sol, 1) != 0u;
     const bool push = !skip && j == 0 && !seen && !sol && v > 0.0f && (s1 || v1 >= FULL) && v2 <= 0.0f;
@@ -1019,7 +1009,7 @@ __device__ void level_commit_small(const Region& R, WS& sW, const int* ring, con
       if (__any_sync(FULLMASK, need)) materialize_par(R, need, c.gi, c.slot, cap);
       if (wv) {
         const SVPlan p = sv_plan(c.part, c.mat, c.slot != NOSLOT, F.avg);
-        if (c.slot != NOSLOT) sv_apply(R, (size_t)c.slot * 512u + local_index(x, y, z), p);
+        if (c.slot != NOSLOT) sv_apply(R, c, F.id[k], local_index(x, y, z), p);
         pd += p.dp;
         if (p.ch) {
           const unsigned pos = atomicAdd(&sW.nchg, 1u);
@@ -1072,8 +1062,8 @@ __device__ __noinline__ void level_round_cta(const Region& R, TickSmem& sm, WS& 
           const int yy = y + 1 + q;
           up[q] = false;
           if (yy < R.ny) {
-            const CD c = load_cell(R, S.ring, x, yy, z);
-            up[q] = !cd_solid(c) && cd_volume(c) > 0.0f;
+            const unsigned c = dense_at(R, x, yy, z);
+            up[q] = !dc_solid(c) && dc_volume(c) > 0.0f;
           }
         }
         const int steps = !up[0] ? 0 : !up[1] ? 1 : !up[2] ? 2 : !up[3] ? 3 : 4;
@@ -1091,7 +1081,7 @@ __device__ __noinline__ void level_round_cta(const Region& R, TickSmem& sm, WS& 
     if (first) {
       R.rb[sid] = 0xFFFFFFFFu;
       float v;
-      cand = (!mark_test(R, x, y, z) && level_member(R, S.ring, x, y, z, &v)) ? 1u : 0u;
+      cand = (!mark_test(R, x, y, z) && level_member(R, x, y, z, &v)) ? 1u : 0u;
       // a start none of whose sides is an unmarked member is a layer of one cell: no flood fill
       // (marks only grow and membership holds through the batch, so this stays true)
       if (cand) {
@@ -1101,7 +1091,7 @@ __device__ __noinline__ void level_round_cta(const Region& R, TickSmem& sm, WS& 
           side4(d, dx, dz);
           const int nx = x + dx, nz = z + dz;
           if (R.ring_w == 0 && (nx < 0 || nz < 0)) continue;
-          if (!mark_test(R, nx, y, nz) && level_member(R, S.ring, nx, y, nz, &v)) single = 0u;
+          if (!mark_test(R, nx, y, nz) && level_member(R, nx, y, nz, &v)) single = 0u;
         }
       }
     }
@@ -1149,7 +1139,7 @@ __device__ __noinline__ void level_round_cta(const Region& R, TickSmem& sm, WS& 
       const unsigned m = s_m;
       if (m) {
         const unsigned w = tid >> 5;
-        if (w < m) level_fill_small(R, S.ring, fills[w], b_start[s_group[w]]);
+        if (w < m) level_fill_small(R, fills[w], b_start[s_group[w]]);
         __syncthreads();
         if (tid == 0) {
           unsigned k = 0, cells = 0;
@@ -1573,7 +1563,7 @@ __device__ float give_lanes(const Region& R, WS& W, bool open, CD c, int x, int 
 __device__ void displace_warp(const Region& R, WS& W, const int* ring, int x, int y, int z, CD col) {
   const unsigned lane = lane_id();
   float amount = __shfl_sync(FULLMASK, cd_volume(col), 0);
-  if (lane == 0) erase_part(R, col, local_index(x, y, z), W.pdelta);
+  if (lane == 0 && !col.out) erase_part(R, col, local_index(x, y, z), dom_id(R, x, y, z), W.pdelta);
   __syncwarp();
   wake_box_warp(R, W, x - 1, y - 1, z - 1, x + 1, y + 1, z + 1);
   if (amount <= 0.0f) return;
@@ -1608,7 +1598,9 @@ __device__ unsigned brush_warp(const Region& R, WS& W, const int* ring, int x, i
   const bool differs = lane == 0u && own != m;
   materialize_lanes(R, differs && slot == NOSLOT, col.gi, slot);
   if (differs && slot != NOSLOT) {
-    R.amat[(size_t)slot * 512u + local_index(x, y, z)] = m;
+    const size_t o = (size_t)slot * 512u + local_index(x, y, z);
+    R.amat[o] = m;
+    dense_put(R, dom_id(R, x, y, z), m, R.avol[o]);
     record_change(R, dom_id(R, x, y, z));
   }
   __syncwarp();
@@ -1652,7 +1644,10 @@ __global__ void __launch_bounds__(EDIT_THREADS) k_voxel_edits(Region R, const in
     const unsigned id = dom_id(R, e.x, e.y, e.z);
     if (__ldcg(R.rb + id) != n - 1u - i) continue;  // set by atomics (in L2): read past L1
     const CD c = load_cell_par(R, R.ring, e.x, e.y, e.z, cap);
-    if (c.slot != NOSLOT) R.amat[(size_t)c.slot * 512u + local_index(e.x, e.y, e.z)] = (unsigned char)e.w;
+    if (c.slot != NOSLOT) {
+      R.amat[(size_t)c.slot * 512u + local_index(e.x, e.y, e.z)] = (unsigned char)e.w;
+      dense_put(R, id, (unsigned)e.w & 255u, c.part);
+    }
     R.rb[id] = 0xFFFFFFFFu;
   }
 }
@@ -1712,7 +1707,7 @@ __global__ void __launch_bounds__(EDIT_THREADS) k_emit(Region R, const int* xyz,
       if (__any_sync(FULLMASK, need)) materialize_par(R, need, c.gi, c.slot, cap);
       if (win) {
         const SVPlan p = sv_plan(c.part, c.mat, c.slot != NOSLOT, nv);
-        if (c.slot != NOSLOT) sv_apply(R, (size_t)c.slot * 512u + local_index(x, y, z), p);
+        if (c.slot != NOSLOT) sv_apply(R, c, id, local_index(x, y, z), p);
         if (p.wmat) record_change(R, id);
         if (p.ch) s_ch = 1;
         pd += p.dp;
@@ -1776,6 +1771,7 @@ __global__ void __launch_bounds__(EDIT_THREADS) k_carve(Region R, const int* xyz
     if (win) {
       if (c.slot != NOSLOT) {
         R.amat[(size_t)c.slot * 512u + local_index(x, y, z)] = 0;
+        dense_put(R, id, 0u, c.part);
         record_change(R, id);
       }
       R.rb[id] = 0xFFFFFFFFu;
@@ -1822,6 +1818,7 @@ __global__ void __launch_bounds__(32) k_edit(Region R, int kind, const int* xyz,
         if (lane == 0 && c.slot != NOSLOT) {
           if (!(c.part > 0.0f)) W.pdelta += 1;
           R.avol[(size_t)c.slot * 512u + local_index(x, y, z)] = amount;
+          dense_put(R, dom_id(R, x, y, z), c.mat, amount);
         }
       }
     }
@@ -1829,6 +1826,17 @@ __global__ void __launch_bounds__(32) k_edit(Region R, int kind, const int* xyz,
   if (W.qtail - W.qhead > R.qmask + 1ull) set_status(R, ST_OOM, 7);
   commit_ws(R, W);
   if (lane == 0 && out_count) *out_count = cnt;
+}
+
+// The dense words of the whole domain from the grid and the atlas: after an upload, a reset and ring
+// streaming. Bound by the words' stores (a 576 x 160 x 576 domain: 212 MB).
+__global__ void __launch_bounds__(256) k_dense(Region R) {
+  for (unsigned id = blockIdx.x * blockDim.x + threadIdx.x; id < R.ncells; id += gridDim.x * blockDim.x) {
+    int x, y, z;
+    dom_xyz(R, id, x, y, z);
+    const CD c = load_cell(R, R.ring, x, y, z);
+    R.dense[id] = dense_code(c.out, c.mat, __float_as_uint(c.part));
+  }
 }
 
 // ------------------------------------------------------------------------- inspection

@@ -45,20 +45,19 @@ constexpr unsigned NGROUPS = (MAX_CELLS_PER_TICK + 31) / 32;
 constexpr unsigned LIST_CAP = 2048;   // a round's list kept in shared memory; the rest goes to global
 constexpr unsigned NOSUCC = 0xFFFFu;
 static_assert(MAX_CELLS_PER_TICK < NOSUCC, "sorted positions fit 16 bits");
-constexpr unsigned UNIFORM = 0x80000000u;  // LvCell::slot of a brick that was a uniform grid value
 constexpr unsigned DONE = 0x80u;           // dependency byte of a finished cell: DONE | the footprint slots it wrote
 constexpr int GATE_MAX = 31;               // range of the gate knob's radii (accepted, unused)
 
-// What a round reads of a drained cell, made in the prepass (one 64-byte line segment per cell).
+// What a round reads of a drained cell, made in the prepass: one 32-byte sector, a word per lane of the
+// eight that run the cell.
 struct __align__(16) LvCell {
-  unsigned slot[7];         // atlas slots of the footprint (self, below, up, +x, -x, +z, -z), or UNIFORM
-  unsigned cid;             // domain id
   unsigned short succ[12];  // later conflicting positions (succ_offset's order), NOSUCC = none
-  unsigned flags;           // bits 0-6 solid footprint cells; 8-12 cells a pull may start from (up,
-                            // +x, -x, +z, -z: not solid, x and z >= 0); 16-24 brick voxel index
-  int y;
+  unsigned cid;             // domain id
+  unsigned ye;              // layer | bits 27-31: may a pull start from the cell's up, +x, -x, +z, -z neighbour
+                            // (x and z >= 0, fluid.rs:519)
 };
-static_assert(sizeof(LvCell) == 64, "LvCell");
+static_assert(sizeof(LvCell) == 32, "LvCell");
+constexpr unsigned YE_Y = 0x07FFFFFFu;  // layers: a domain has fewer than 2^31 cells and 65 x 65 columns or more
 
 // The footprint volumes a cell of the gate layer found, for searches of earlier cells.
 struct __align__(16) LvOld {
@@ -80,8 +79,8 @@ struct Search {
   unsigned blk;                 // 1 + an unfinished earlier cell the search depends on (0: none)
   unsigned pos, status, i, qlen, side;  // the cell, and the search's progress
   float vol, got, here;         // its volume, what the pull takes, the source's volume
-  int cx, cy, cz;               // the pulling cell
-  int sx, sy, sz;               // the source
+  unsigned cid, skey;           // the pulling cell, the source relative to it
+  int cx, cz;
 };
 
 // What warp 0 asks of the CTA between rounds.
@@ -265,9 +264,11 @@ __device__ __forceinline__ SVPlan sv_plan(float part, unsigned char mat, bool ha
   p.dp = ((mid && has && !had) ? 1 : 0) - ((!mid && had) ? 1 : 0);
   return p;
 }
-__device__ __forceinline__ void sv_apply(const Region& R, size_t o, const SVPlan& p) {
+__device__ __forceinline__ void sv_apply(const Region& R, const CD& c, unsigned id, unsigned local, const SVPlan& p) {
+  const size_t o = (size_t)c.slot * 512u + local;
   if (p.wpart) R.avol[o] = p.npart;
   if (p.wmat) R.amat[o] = p.nmat;
+  dense_put(R, id, p.nmat, p.npart);
 }
 
 // Footprint slot offsets: 0 self, 1 below, 2 up, 3 +x, 4 -x, 5 +z, 6 -z.
@@ -325,16 +326,18 @@ __device__ __forceinline__ unsigned attempts_before(const LvSmem& L, unsigned i)
 // -------------------------------------------------------------------------------- the cells
 // Lane constants of the eight lanes that run a cell: lane l < 7 holds footprint slot l.
 struct LaneSlot {
-  int ox, oy, oz;        // the slot's offset
-  unsigned lm, la;       // brick voxel index of the slot: the axis' bits, and what is added to them
+  int off;               // the slot's offset in domain ids
   unsigned open1, open2; // the lane's two successors: one layer up (bit per successor), two layers up
 };
-__device__ __forceinline__ LaneSlot lane_slot() {
+__device__ __forceinline__ int fp_id(const Region& R, int l) {
+  int ox, oy, oz;
+  fp_off(l, ox, oy, oz);
+  return ox + (oz * R.PY + oy) * R.PX;
+}
+__device__ __forceinline__ LaneSlot lane_slot(const Region& R) {
   const int l = (int)(threadIdx.x & 7u);
   LaneSlot s;
-  fp_off(l, s.ox, s.oy, s.oz);
-  s.lm = l == 7 || l == 0 ? 0u : l <= 2 ? 0x38u : l <= 4 ? 7u : 0x1C0u;
-  s.la = (unsigned)(s.ox + 8 * s.oy + 64 * s.oz);
+  s.off = l < 7 ? fp_id(R, l) : 0;
   s.open1 = l == 3 || l == 4 ? 3u : l == 5 ? 1u : 0u;  // successors 6..10
   s.open2 = l == 5 ? 2u : 0u;                          // successor 11
   return s;
@@ -346,43 +349,24 @@ __device__ __forceinline__ LaneSlot lane_slot() {
 // successors join and its counter; pb: the parked list. Returns the cell's volume afterwards.
 //
 // Eight lanes rather than one thread per cell: a round is a latency chain (a few dozen to a few
-// hundred cells on 16 warps), and a lane that holds one slot issues one address, one pair of loads,
-// one set_volume and two successor counts where a thread issues seven, seven, six and twelve. A
-// cell that is sure to run counts its successors down while its volumes are on their way: nobody
-// reads the next list before the round has ended.
+// hundred cells on 16 warps), and a lane that holds one slot issues one load, one set_volume and two
+// successor counts where a thread issues seven, six and twelve. A cell that is sure to run counts its
+// successors down while its volumes are on their way: nobody reads the next list before the round
+// has ended. The sweep writes the dense words only; sweep_flush brings the atlas in step.
 __device__ __forceinline__ float lv_cells(const Region& R, LvSmem& L, const LaneSlot& S, bool has, unsigned i, bool pulled, float got, unsigned ev,
-                                         int gate, unsigned kp, unsigned nb, unsigned nc, unsigned pb, int& pd, unsigned long long cap) {
+                                         int gate, unsigned kp, unsigned nb, unsigned nc, unsigned pb, int& pd) {
   const float FULL = full_level();
   const unsigned lane = lane_id(), l = lane & 7u, base = lane & 24u;
-  unsigned w1 = UNIFORM, w2 = 0xFFFFFFFFu;
-  if (has) {
-    const unsigned* p = reinterpret_cast<const unsigned*>(R.lv + i) + l;
-    w1 = p[0];
-    w2 = p[8];
-  }
-  const unsigned flags = __shfl_sync(FULLMASK, w2, 6, 8);
-  const int y = (int)__shfl_sync(FULLMASK, w2, 7, 8);
-  const bool cell = has && l < 7u && !((flags >> l) & 1u);  // the lane holds a cell that is not solid
-  const unsigned loc = flags >> 16, at = (loc & ~S.lm) | ((loc + S.la) & S.lm);
-  unsigned slot = cell ? w1 : UNIFORM, gi = 0;
-  if (cell && (slot & UNIFORM)) {  // uniform at the tick's start: the value, or the slot the brick has now
-    int x, yy, z;
-    dom_xyz(R, R.lv[i].cid, x, yy, z);
-    gi = grid_index(R, (x + S.ox) >> 3, (yy + S.oy) >> 3, (z + S.oz) >> 3);
-    const unsigned g = grid_word(R, gi, cap);
-    slot = g < 256u ? (UNIFORM | g) : g - 256u;
-  }
-  float part = 0.0f;
-  unsigned mat = slot & 255u;
-  if (!(slot & UNIFORM)) {
-    const size_t o = (size_t)slot * 512u + at;
-    part = R.avol[o];
-    mat = R.amat[o];
-  }
+  unsigned w = 0xFFFFFFFFu;
+  if (has) w = reinterpret_cast<const unsigned*>(R.lv + i)[l];
+  const unsigned cid = __shfl_sync(FULLMASK, w, 6, 8), ye = __shfl_sync(FULLMASK, w, 7, 8);
+  const int y = (int)(ye & YE_Y);
+  unsigned u = DC_SOLID;
+  if (has && l < 7u) u = R.dense[(int)cid + S.off];
   // ---- a cell that attempts a pull and has a start cell waits for the pull
   if (__any_sync(FULLMASK, has && !pulled && i < kp && bit_of(L.pp, i))) {
-    const float v = part > 0.0f ? part : (cell && mat == WATER ? 1.0f : 0.0f);
-    const unsigned starts = (__ballot_sync(FULLMASK, cell && l >= 2u && ((flags >> (6u + l)) & 1u) && v >= FULL) >> base) & 0xFFu;
+    const float v = dc_volume(u);
+    const unsigned starts = (__ballot_sync(FULLMASK, l >= 2u && l < 7u && ((ye >> (25u + l)) & 1u) && !dc_solid(u) && v >= FULL) >> base) & 0xFFu;
     const float self = __shfl_sync(FULLMASK, v, 0, 8);
     if (!pulled && i < kp && self < FULL && starts) has = false;
   }
@@ -390,7 +374,7 @@ __device__ __forceinline__ float lv_cells(const Region& R, LvSmem& L, const Lane
   {
     bool r0 = false, r1 = false;
     if (has && l < 6u) {
-      const unsigned a = w2 & 0xFFFFu, b = w2 >> 16;
+      const unsigned a = w & 0xFFFFu, b = w >> 16;
       unsigned oa = 0, ob = 0;
       if (a != NOSUCC) oa = atomicSub(&L.dep[a >> 2], 1u << ((a & 3u) * 8u)) >> ((a & 3u) * 8u);
       if (b != NOSUCC) ob = atomicSub(&L.dep[b >> 2], 1u << ((b & 3u) * 8u)) >> ((b & 3u) * 8u);
@@ -404,23 +388,24 @@ __device__ __forceinline__ float lv_cells(const Region& R, LvSmem& L, const Lane
       unsigned t = 0;
       if (lane == 0u) t = atomicAdd(&L.cnt[nc], (unsigned)(__popc(g0) + __popc(g1)));
       t = __shfl_sync(FULLMASK, t, 0);
-      if (p0) list_put(R, L, nb, t + (unsigned)__popc(g0 & lanemask_lt()), w2 & 0xFFFFu);
-      if (p1) list_put(R, L, nb, t + (unsigned)(__popc(g0) + __popc(g1 & lanemask_lt())), w2 >> 16);
+      if (p0) list_put(R, L, nb, t + (unsigned)__popc(g0 & lanemask_lt()), w & 0xFFFFu);
+      if (p1) list_put(R, L, nb, t + (unsigned)(__popc(g0) + __popc(g1 & lanemask_lt())), w >> 16);
     }
     if ((r0 && !p0) || (r1 && !p1)) {
       unsigned t = atomicAdd(&L.park_n[pb], (r0 && !p0 ? 1u : 0u) + (r1 && !p1 ? 1u : 0u));
-      if (r0 && !p0) park_put(R, pb, t++, w2 & 0xFFFFu);
-      if (r1 && !p1) park_put(R, pb, t, w2 >> 16);
+      if (r0 && !p0) park_put(R, pb, t++, w & 0xFFFFu);
+      if (r1 && !p1) park_put(R, pb, t, w >> 16);
     }
   }
   // ---- 1. fall into the free capacity below, 2. share with lower sides when supported, 3. evaporate
   // crumbs (fluid.rs:606-650). Every side's flow depends on the volume after the fall and its own
   // volume only; the running volume subtracts the flows in side order (a side without one: 0).
-  const float v = part > 0.0f ? part : (cell && mat == WATER ? 1.0f : 0.0f);
+  const bool solid = dc_solid(u);
+  const float v = solid ? 0.0f : dc_volume(u);
   const float v0 = __shfl_sync(FULLMASK, v, 0, 8), bv = __shfl_sync(FULLMASK, v, 1, 8);
+  const bool below_solid = (__ballot_sync(FULLMASK, solid) >> (base + 1u)) & 1u;
   float vol = pulled && got > 0.0f ? __fadd_rn(v0, got) : v0;
   const bool live = has && vol > 0.0f;  // fluid.rs:602-604
-  const bool below_solid = (flags >> 1) & 1u;
   const float ff = fminf(vol, __fsub_rn(1.0f, bv));
   const bool w_below = live && !below_solid && ff > 1e-6f;
   const float below_new = __fadd_rn(bv, ff);
@@ -428,46 +413,81 @@ __device__ __forceinline__ float lv_cells(const Region& R, LvSmem& L, const Lane
   const float below_after = w_below ? (below_new >= FULL ? 1.0f : below_new) : bv;
   const bool spread = live && vol > MIN_SPREAD && (below_solid || below_after >= FULL);
   const float f = __fmul_rn(__fsub_rn(vol, v), 0.2f);
-  const bool ok = spread && l >= 3u && cell && !(v >= vol) && !(f < MIN_FLOW) && !(__fsub_rn(vol, f) < MIN_SPREAD * 0.5f);
+  const bool ok = spread && l >= 3u && !solid && !(v >= vol) && !(f < MIN_FLOW) && !(__fsub_rn(vol, f) < MIN_SPREAD * 0.5f);
   const float fs = ok ? f : 0.0f;
   const float f3 = __shfl_sync(FULLMASK, fs, 3, 8), f4 = __shfl_sync(FULLMASK, fs, 4, 8);
   const float f5 = __shfl_sync(FULLMASK, fs, 5, 8), f6 = __shfl_sync(FULLMASK, fs, 6, 8);
   vol = __fsub_rn(__fsub_rn(__fsub_rn(__fsub_rn(vol, f3), f4), f5), f6);
   vol = vol < EVAPORATE ? 0.0f : vol;
   const float dv = fabsf(__fsub_rn(vol, v0));
+  // ---- set_volume of the lane's cell (fluid.rs:327-355): snapped to 0 or full the entry goes; water
+  // shows from 0.5 and hides below 0.3 (a snapped volume lies on the same side of both)
   const bool wr = l == 0u ? (live && dv > 1e-7f) : l == 1u ? w_below : ok;
   const float wv = l == 0u ? vol : l == 1u ? below_new : __fadd_rn(v, f);
-  // ---- set_volume of the lane's cell (fluid.rs:327-355)
-  const bool need = wr && (slot & UNIFORM) && (wv <= 1e-6f ? mat == WATER : wv >= FULL ? mat != WATER : true);
-  if (__any_sync(FULLMASK, need)) {
-    unsigned s = NOSLOT;
-    materialize_par(R, need, gi, s, cap);
-    if (need && s != NOSLOT) slot = s;
-  }
-  // snapped to 0 or full the entry goes; water shows from 0.5 and hides below 0.3 (a snapped volume lies
-  // on the same side of both), and these cells hold air or water only
-  const bool is_water = mat == WATER, mid = wv > 1e-6f && wv < FULL, had = part > 0.0f;
-  const bool wet = wv >= (is_water ? HIDE_BELOW : SHOW_AT), hs = wr && !(slot & UNIFORM), ch = hs && wet != is_water;
-  if (hs) {
-    const size_t o = (size_t)slot * 512u + at;
-    if (mid || had) R.avol[o] = mid ? wv : 0.0f;
-    if (ch) R.amat[o] = wet ? WATER : (unsigned char)0;
+  const bool is_water = (int)u > 0, mid = wv > 1e-6f && wv < FULL, had = v > 0.0f && v < 1.0f;
+  const bool wet = wv >= (is_water ? HIDE_BELOW : SHOW_AT);
+  const unsigned nu = mid ? (__float_as_uint(wv) | (wet ? 0u : DC_AIR)) : (wet ? DC_FULL : 0u);
+  const bool put = wr && nu != u;
+  if (put) {
+    R.dense[(int)cid + S.off] = nu;
     pd += (mid ? 1 : 0) - (had ? 1 : 0);
   }
-  const unsigned wm = __ballot_sync(FULLMASK, wr) >> base;
-  const unsigned cm = __ballot_sync(FULLMASK, ch) >> base;
+  const unsigned pm = __ballot_sync(FULLMASK, put) >> base;
+  const unsigned cm = __ballot_sync(FULLMASK, put && wet != is_water) >> base;
   // activation slots: 2 below, 3..6 the sides, 7 the cell itself
   const unsigned am = __ballot_sync(FULLMASK, l == 2u ? w_below : l == 7u ? live && dv > SLEEP : ok && f > SLEEP) >> base;
   if (has) {
     if (y == gate) R.lv_old[i].vol[l] = v;
     if (l == 0u) {
       R.lv_ev[i] = ev | (am & 0xFCu) | ((am & 0x80u) << 9) | ((cm & 0x7Fu) << 8);  // bit 16: seeds itself
-      reinterpret_cast<volatile unsigned char*>(L.dep)[i] = (unsigned char)(DONE | (wm & 0x7Fu));
+      reinterpret_cast<volatile unsigned char*>(L.dep)[i] = (unsigned char)(DONE | (pm & 0x7Fu));
       if (i < kp && bit_of(L.pp, i)) atomicAnd(&L.pp[i >> 5], ~(1u << (i & 31u)));
     }
   }
   __syncwarp();
   return vol;
+}
+
+// The atlas entry of a cell the sweep wrote, warp-collective: its brick gets a slot (sparse_volume.rs:
+// 250-266) and the dense word's material and volume.
+__device__ __forceinline__ void flush_cell(const Region& R, bool w, unsigned id, unsigned long long cap) {
+  int x = 0, y = 0, z = 0;
+  unsigned slot = NOSLOT, gi = 0, u = 0;
+  if (w) {
+    dom_xyz(R, id, x, y, z);
+    u = R.dense[id];
+    gi = grid_index(R, x >> 3, y >> 3, z >> 3);
+    const unsigned g = grid_word(R, gi, cap);
+    if (g >= 256u) slot = g - 256u;
+  }
+  if (__any_sync(FULLMASK, w && slot == NOSLOT)) materialize_par(R, w && slot == NOSLOT, gi, slot, cap);
+  if (w && slot != NOSLOT) {
+    const size_t o = (size_t)slot * 512u + local_index(x, y, z);
+    const float v = dc_volume(u);
+    R.avol[o] = v < 1.0f ? v : 0.0f;
+    R.amat[o] = (int)u > 0 ? WATER : (unsigned char)0;
+  }
+}
+
+// After the sweep: every cell it wrote (the slots in the dependency bytes, the pulls' sources) to the
+// atlas, all at once. All threads.
+__device__ __forceinline__ void sweep_flush(const Region& R, const LvSmem& L, unsigned n, unsigned long long cap) {
+  for (unsigned base = threadIdx.x & ~31u; base < n; base += blockDim.x) {
+    const unsigned i = base + lane_id();
+    unsigned m = 0, cid = 0, src = NOSLOT;
+    if (i < n) {
+      m = dep_byte(L, i) & 0x7Fu;
+      if (R.lv_ev[i] & 1u) src = R.lv_src[i];
+      if (m) cid = R.lv[i].cid;
+    }
+#pragma unroll
+    for (int l = 0; l < 7; ++l) {
+      if (l == 2) continue;
+      const bool w = (m >> l) & 1u;
+      if (__any_sync(FULLMASK, w)) flush_cell(R, w, (unsigned)((int)cid + fp_id(R, l)), cap);
+    }
+    if (__any_sync(FULLMASK, src != NOSLOT)) flush_cell(R, src != NOSLOT, src, cap);
+  }
 }
 
 // --------------------------------------------------------------------------- pressure search
@@ -518,7 +538,7 @@ struct SearchRead {
   float here, v;
   bool win, cand, side;
 };
-__device__ __forceinline__ SearchRead search_read(const Region& R, LvSmem& L, const int* ring, bool act, unsigned e, unsigned d, bool sides) {
+__device__ __forceinline__ SearchRead search_read(const Region& R, LvSmem& L, bool act, unsigned e, unsigned d, bool sides) {
   Search& C = L.s;
   SearchRead r{0u, 0.0f, 0.0f, false, false, false};
   if (act) {
@@ -528,30 +548,26 @@ __device__ __forceinline__ SearchRead search_read(const Region& R, LvSmem& L, co
     r.key = k0 + (d == 0u ? 1u << 22 : d == 1u ? 1u : d == 2u ? 0u - 1u : d == 3u ? 1u << 11 : 0u - (1u << 11));
     int dx, dy, dz;
     rel_unpack(r.key, dx, dy, dz);
-    const int x = C.cx + dx, y = C.cy + dy, z = C.cz + dz;
-    // (once the 24 side checks at the start level are spent, what its cells hold no longer matters)
-    const bool rd = d == 0u ? y < R.ny : (x >= 0 && z >= 0 && (sides || dy != 0));
+    // Once the 24 side checks at the start level are spent, what its cells hold no longer matters.
+    // Negative coordinates are passed over (fluid.rs:542); a bounded world has none, its padding is solid.
+    bool rd = d == 0u || sides || dy != 0;
+    if (R.ring_w && d != 0u) rd = rd && C.cx + dx >= 0 && C.cz + dz >= 0;
     bool top = true;
-    if (rd && !outside(R, ring, x, y, z)) {
-      // the grid word and, on the pulling layer, the writers' positions: issued together (a cell of
-      // the world has its neighbours inside the padded domain)
-      const unsigned g = gld(R.grid + grid_index(R, x >> 3, y >> 3, z >> 3));
-      unsigned j[5] = {NOSLOT, NOSLOT, NOSLOT, NOSLOT, NOSLOT};
+    if (rd) {
+      // the cell and, on the pulling layer, the writers' positions: issued together (the neighbours of
+      // a cell of the world lie inside the padded domain)
+      const int id = (int)C.cid + dx + (dz * R.PY + dy) * R.PX;
+      const unsigned u = R.dense[id];
       if (dy == 0) {
-        const unsigned* st = R.stamp + dom_id(R, x, y, z);
+        const unsigned* st = R.stamp + id;
         const int row = R.PX * R.PY;
-        j[0] = st[0];
-        j[1] = st[-1];
-        j[2] = st[1];
-        j[3] = st[-row];
-        j[4] = st[row];
-      }
-      const size_t o = g < 256u ? (size_t)0 : (size_t)(g - 256u) * 512u + local_index(x, y, z);
-      const float part = R.avol[o];
-      const unsigned am = R.amat[o], m = g < 256u ? g : am;
-      if (m == 0u || m == WATER) {
-        r.v = g >= 256u && part > 0.0f ? part : (m == WATER ? 1.0f : 0.0f);
-        if (dy == 0) r.v = old_volume(R, L, C, C.pos, j, r.v);
+        const unsigned j[5] = {st[0], st[-1], st[1], st[-row], st[row]};
+        if (!dc_solid(u)) {
+          r.v = old_volume(R, L, C, C.pos, j, dc_volume(u));
+          top = r.v <= 0.0f;
+        }
+      } else if (!dc_solid(u)) {
+        r.v = dc_volume(u);
         top = r.v <= 0.0f;
       }
     }
@@ -564,11 +580,7 @@ __device__ __forceinline__ SearchRead search_read(const Region& R, LvSmem& L, co
 }
 
 __device__ __forceinline__ void search_won(Search& C, const SearchRead& r, unsigned e) {
-  int a, b, c;
-  rel_unpack(C.q[e], a, b, c);
-  C.sx = C.cx + a;
-  C.sy = C.cy + b;
-  C.sz = C.cz + c;
+  C.skey = C.q[e];
   C.here = r.here;
   C.got = fminf(__fsub_rn(1.0f, C.vol), r.here);
   C.status = SS_SUCCESS;
@@ -580,29 +592,22 @@ __device__ __forceinline__ void search_won(Search& C, const SearchRead& r, unsig
 // written by the cells within three rows and columns: `wait` gets 1 + the last unfinished earlier one
 // of them (0: none), one probe per lane instead of a search that finds out. Returns whether there is
 // anything to examine.
-__device__ __forceinline__ bool search_begin(const Region& R, LvSmem& L, const int* ring, unsigned k, int sgn, unsigned& wait, unsigned long long cap) {
+__device__ __forceinline__ bool search_begin(const Region& R, LvSmem& L, const LaneSlot& S, unsigned k, int sgn, unsigned& wait) {
   Search& C = L.s;
   const float FULL = full_level();
   const unsigned lane = lane_id();
-  const LvCell& rc = R.lv[k];
-  const unsigned flags = rc.flags, cid = rc.cid;
-  int x, y, z;
-  dom_xyz(R, cid, x, y, z);
+  const unsigned cid = R.lv[k].cid, ye = R.lv[k].ye;
   // lanes 0..20: the three rows before, x - 3 .. x + 3; 21..23: the three cells before in the row
   const int row = (int)lane / 7, ndx = lane < 21u ? (int)lane - 7 * row - 3 : -sgn * ((int)lane - 20);
   const int ndz = lane < 21u ? -sgn * (row + 1) : 0;
-  unsigned near = NOSLOT;
+  unsigned near = NOSLOT, u = DC_SOLID;
   if (lane < 24u) near = R.stamp[(int)cid + ndx + ndz * R.PX * R.PY];
-  float v = 0.0f;
-  if (lane < 7u && !((flags >> lane) & 1u)) {
-    int ox, oy, oz;
-    fp_off((int)lane, ox, oy, oz);
-    v = cd_volume(load_cell_par(R, ring, x + ox, y + oy, z + oz, cap));
-  }
+  if (lane < 7u) u = R.dense[(int)cid + S.off];
+  const float v = dc_solid(u) ? 0.0f : dc_volume(u);
   wait = __reduce_max_sync(FULLMASK, near != NOSLOT && !cell_done(L, near) ? near + 1u : 0u);
   if (wait) return false;
   const float vol = __shfl_sync(FULLMASK, v, 0);
-  unsigned starts = (__ballot_sync(FULLMASK, lane >= 2u && lane < 7u && ((flags >> (6u + lane)) & 1u) && v >= FULL) >> 2) & 31u;
+  unsigned starts = (__ballot_sync(FULLMASK, lane >= 2u && lane < 7u && ((ye >> (25u + lane)) & 1u) && v >= FULL) >> 2) & 31u;
   unsigned before = attempts_before(L, k);
   if (before + L.nx >= MAX_PULLS_PER_TICK) {  // near the budget: the cells before this one that pulls took below full
     unsigned c = 0;
@@ -625,9 +630,11 @@ __device__ __forceinline__ bool search_begin(const Region& R, LvSmem& L, const i
     C.qlen = (unsigned)__popc(starts);
     C.vol = vol;
     C.got = 0.0f;
-    C.cx = x;
-    C.cy = y;
-    C.cz = z;
+    C.cid = cid;
+    if (R.ring_w) {
+      int y;
+      dom_xyz(R, cid, C.cx, y, C.cz);
+    }
     if (starts) {
       C.rank0 = rank0;
       C.nvis += 6u;
@@ -657,7 +664,7 @@ __device__ __forceinline__ bool search_begin(const Region& R, LvSmem& L, const i
 // queue order kept exactly: the first surface entry in queue order wins; the 24 side checks at the
 // start level are counted in (entry, direction) order; a cell several lanes find belongs to the
 // earliest. Ends with C.status, or SS_MORE when many entries wait (all warps take over).
-__device__ __forceinline__ void search_solo(const Region& R, LvSmem& L, const int* ring) {
+__device__ __forceinline__ void search_solo(const Region& R, LvSmem& L) {
   Search& C = L.s;
   const unsigned lane = lane_id(), j = lane / 5u, d = lane - 5u * j;
   unsigned i = C.i, qlen = C.qlen, side = C.side, status = SS_NONE, nvis = 0u;
@@ -668,7 +675,7 @@ __device__ __forceinline__ void search_solo(const Region& R, LvSmem& L, const in
       break;
     }
     const unsigned kk = min(SOLO_ENTRIES, qlen - i);
-    const SearchRead r = search_read(R, L, ring, j < kk, i + j, d, side < 24u);
+    const SearchRead r = search_read(R, L, j < kk, i + j, d, side < 24u);
     __syncwarp();
     if (vld(&C.blk)) {  // an earlier cell has yet to write what the search read: run it again later
       status = SS_BLOCKED;
@@ -719,7 +726,7 @@ __device__ __forceinline__ void search_solo(const Region& R, LvSmem& L, const in
 // The same rounds by all warps of the CTA, six entries each in queue order, until the search ends.
 // Entries past the 512th are never examined (fluid.rs:530), so appends stop there. All threads; ends
 // with a barrier.
-__device__ __noinline__ void search_cta(const Region& Rs, LvSmem& L, const int* ring) {
+__device__ __noinline__ void search_cta(const Region& Rs, LvSmem& L) {
   const Region R = Rs;
   Search& C = L.s;
   const unsigned tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, nw = blockDim.x >> 5;
@@ -728,7 +735,7 @@ __device__ __noinline__ void search_cta(const Region& Rs, LvSmem& L, const int* 
   const unsigned rank0 = C.rank0 + 6u;
   while (i < qlen && i < PRESSURE_SEARCH) {
     const unsigned kk = min(SOLO_ENTRIES * nw, min(qlen, PRESSURE_SEARCH) - i);
-    const SearchRead r = search_read(R, L, ring, jl < SOLO_ENTRIES && j < kk, i + j, d, side < 24u);
+    const SearchRead r = search_read(R, L, jl < SOLO_ENTRIES && j < kk, i + j, d, side < 24u);
     const unsigned wm = __ballot_sync(FULLMASK, r.win), smk = __ballot_sync(FULLMASK, r.side);
     // no more than 24 side checks at the start level (fluid.rs:546-549): their order over the warps
     // matters only in the round that passes the limit
@@ -790,26 +797,24 @@ __device__ __noinline__ void search_cta(const Region& Rs, LvSmem& L, const int* 
 }
 
 // The end of a pull, one warp: the source's write (fluid.rs:536-540), then the cell itself.
-__device__ __forceinline__ void pull_end(const Region& R, LvSmem& L, const int* ring, const LaneSlot& S, int gate, unsigned kp, unsigned cur, unsigned cc,
-                                         unsigned pb, int& pd, unsigned long long cap) {
+__device__ __forceinline__ void pull_end(const Region& R, LvSmem& L, const LaneSlot& S, int gate, unsigned kp, unsigned cur, unsigned cc, unsigned pb,
+                                         int& pd) {
   Search& C = L.s;
   const unsigned lane = lane_id(), k = C.pos;
   unsigned ev = 0u;
   if (C.status == SS_SUCCESS) {
-    const float nv = __fsub_rn(C.here, C.got);
-    CD c = CD{0.0f, NOSLOT, 0u, 0, true};
-    if (lane == 0) c = load_cell_par(R, ring, C.sx, C.sy, C.sz, cap);
-    const bool need = lane == 0 && c.slot == NOSLOT && set_volume_needs_slot(c, nv);
-    if (__any_sync(FULLMASK, need)) materialize_par(R, need, c.gi, c.slot, cap);
     if (lane == 0) {
-      const unsigned sid = dom_id(R, C.sx, C.sy, C.sz);
-      const unsigned j = R.stamp[sid];
-      const SVPlan p = sv_plan(c.part, c.mat, c.slot != NOSLOT, nv);
-      if (c.slot != NOSLOT) sv_apply(R, (size_t)c.slot * 512u + local_index(C.sx, C.sy, C.sz), p);
-      pd += p.dp;
+      int dx, dy, dz;
+      rel_unpack(C.skey, dx, dy, dz);
+      const unsigned sid = (unsigned)((int)C.cid + dx + (dz * R.PY + dy) * R.PX);
+      const unsigned u = R.dense[sid], j = R.stamp[sid];
+      const float nv = __fsub_rn(C.here, C.got), v = dc_volume(u);
+      const bool is_water = (int)u > 0, mid = nv > 1e-6f && nv < full_level(), wet = nv >= (is_water ? HIDE_BELOW : SHOW_AT);
+      R.dense[sid] = mid ? (__float_as_uint(nv) | (wet ? 0u : DC_AIR)) : (wet ? DC_FULL : 0u);
+      pd += (mid ? 1 : 0) - (v < 1.0f ? 1 : 0);  // (a source holds water)
       R.lv_src[k] = sid;
       // activation slots 0 (the source) and 1 (around the cell); bit 17 seeds the source
-      ev = 3u | (p.ch ? 0x8000u : 0u) | (2u << 16);
+      ev = 3u | (wet != is_water ? 0x8000u : 0u) | (2u << 16);
       // a drained source that was full attempts a pull of its own when its turn comes
       if (j != NOSLOT && nv < full_level() && !bit_of(L.att, j) && !((R.pextra[j >> 5] >> (j & 31u)) & 1u)) {
         R.pextra[j >> 5] |= 1u << (j & 31u);
@@ -826,7 +831,7 @@ __device__ __forceinline__ void pull_end(const Region& R, LvSmem& L, const int* 
     L.n_searches += 1u;
   }
   __syncwarp();
-  const float vol = lv_cells(R, L, S, lane < 8u, k, true, C.got, ev, gate, kp, cur, cc, pb, pd, cap);
+  const float vol = lv_cells(R, L, S, lane < 8u, k, true, C.got, ev, gate, kp, cur, cc, pb, pd);
   if (lane == 0u && ev && vol >= full_level()) {
     // a pull that leaves its own cell full gives its later neighbours on the layer a start cell
     const LvCell& rc = R.lv[k];
@@ -860,7 +865,7 @@ __device__ __forceinline__ void lv_head(const Region& R, LvSmem& L, unsigned n, 
   H.word = w + (unsigned)fl;
   H.head = H.word * 32u + (unsigned)__ffs(__shfl_sync(FULLMASK, P, fl)) - 1u;
   if (H.head >= H.lend) {  // a new gate layer: its first position after the layer, by a 32-way search
-    H.gate = R.lv[H.head].y;
+    H.gate = (int)(R.lv[H.head].ye & YE_Y);
     const unsigned lim = (unsigned)(H.gate + 1) * (unsigned)R.PZ * (unsigned)R.PX;
     unsigned lo = H.head, hi = n;  // cells[lo] is on the layer; the answer lies in (lo, hi]
     while (hi - lo > 1u) {
@@ -881,32 +886,26 @@ __device__ __forceinline__ void lv_head(const Region& R, LvSmem& L, unsigned n, 
 // 2e-4 leaves it below 1 - 1e-4). A cell whose full neighbours all do that will not pull and leaves
 // pp: later pulls need not wait for it. Returns 0 = it will not pull, 1 + a cell to wait for before
 // the test can tell, or TEST_FAILED.
-__device__ __forceinline__ unsigned lv_prune(const Region& R, LvSmem& L, const int* ring, unsigned k, unsigned long long cap) {
+__device__ __forceinline__ unsigned lv_prune(const Region& R, LvSmem& L, unsigned k) {
   const unsigned lane = lane_id();
-  const LvCell& rc = R.lv[k];
-  const unsigned flags = rc.flags;
-  int x, y, z;
-  dom_xyz(R, rc.cid, x, y, z);
+  const unsigned cid = R.lv[k].cid, ye = R.lv[k].ye;
   const float FULL = full_level();
   // lanes 8m .. 8m + 7 (m = 0..3) look at side m; lane 0 at the cell above too
   const unsigned m = lane >> 3, q = lane & 7u;
-  const int ax = x + (m == 0u) - (m == 1u), az = z + (m == 2u) - (m == 3u);
-  bool fail = false;
+  const int row = R.PX * R.PY, at = (int)cid + (m == 0u ? 1 : m == 1u ? -1 : m == 2u ? row : -row);
+  const int w5 = at - R.PX + (q == 1u ? 1 : q == 2u ? -1 : q == 3u ? row : q == 4u ? -row : 0);  // who may write the cell below it
+  const unsigned us = R.dense[at], ub = q == 1u ? R.dense[at - R.PX] : DC_SOLID, ps = q == 0u ? R.stamp[at] : NOSLOT;
+  const unsigned uu = lane == 0u ? R.dense[(int)cid + R.PX] : DC_SOLID;
+  // (a side that is solid has no start cell, and what lies around it may be outside the domain)
+  const bool full = ((ye >> (28u + m)) & 1u) && !dc_solid(us) && dc_volume(us) >= FULL;
+  bool fail = lane == 0u && ((ye >> 27) & 1u) && !dc_solid(uu) && dc_volume(uu) >= FULL;
   unsigned wait = 0u;
-  if (lane == 0u && ((flags >> 8) & 1u)) fail = cd_volume(load_cell_par(R, ring, x, y + 1, z, cap)) >= FULL;
-  if ((flags >> (9u + m)) & 1u) {
-    if (cd_volume(load_cell_par(R, ring, ax, y, az, cap)) >= FULL) {
-      if (q == 0u) {  // the side itself: earlier and unfinished
-        const unsigned p = rank_at(R, ax, y, az);
-        fail |= p == NOSLOT || p > k || cell_done(L, p);
-      } else if (q == 1u) {  // room below it
-        const CD b = load_cell_par(R, ring, ax, y - 1, az, cap);
-        fail |= cd_solid(b) || !(__fsub_rn(1.0f, cd_volume(b)) >= 2e-4f);
-      }
-      if (q < 5u) {  // the cells that may still write the cell below it
-        const unsigned p = rank_at(R, ax + (q == 1u) - (q == 2u), y - 1, az + (q == 3u) - (q == 4u));
-        if (p != NOSLOT && !cell_done(L, p)) wait = p + 1u;
-      }
+  if (full) {
+    if (q == 0u) fail |= ps == NOSLOT || ps > k || cell_done(L, ps);  // the side itself: earlier and unfinished
+    if (q == 1u) fail |= dc_solid(ub) || !(__fsub_rn(1.0f, dc_volume(ub)) >= 2e-4f);  // room below it
+    if (q < 5u) {
+      const unsigned p = R.stamp[w5];
+      if (p != NOSLOT && !cell_done(L, p)) wait = p + 1u;
     }
   }
   // room below is final only once nobody writes it: wait first
@@ -918,9 +917,9 @@ __device__ __forceinline__ unsigned lv_prune(const Region& R, LvSmem& L, const i
 // Between the CTA's rounds, warp 0: the pulls whose turn has come, in order, and the rounds that are
 // too short for the CTA. Ends with a request to the CTA: run the list, open the gate (L.gate changed
 // from `gate`), carry on the search, or the sweep's end. Returns the change in partial entries.
-__device__ __noinline__ int lv_solo(const Region& Rs, LvSmem& L, const int* ring, unsigned n, int gate, int sgn, unsigned long long cap) {
+__device__ __noinline__ int lv_solo(const Region& Rs, LvSmem& L, unsigned n, int gate, int sgn, unsigned long long cap) {
   const Region R = Rs;
-  const LaneSlot S = lane_slot();
+  const LaneSlot S = lane_slot(R);
   int pd = 0;
   __syncwarp();
   const unsigned lane = lane_id(), kp = L.kp;
@@ -946,8 +945,8 @@ __device__ __noinline__ int lv_solo(const Region& Rs, LvSmem& L, const int* ring
       const unsigned dep = dep_byte(L, H.head);
       if (dep == 0u) {  // its turn has come
         if (H.blk == 0u || cell_done(L, H.blk - 1u)) {
-          if (search_begin(R, L, ring, H.head, sgn, H.blk, cap)) {
-            search_solo(R, L, ring);
+          if (search_begin(R, L, S, H.head, sgn, H.blk)) {
+            search_solo(R, L);
             if (L.s.status == SS_MORE) {
               req = SR_SEARCH;
               break;
@@ -956,7 +955,7 @@ __device__ __noinline__ int lv_solo(const Region& Rs, LvSmem& L, const int* ring
           finish = H.blk == 0u;
         }
       } else if (H.test == 0u || (H.test != TEST_FAILED && cell_done(L, H.test - 1u))) {
-        H.test = lv_prune(R, L, ring, H.head, cap);
+        H.test = lv_prune(R, L, H.head);
         if (H.test == 0u) {
           if (lane == 0) L.pp[H.head >> 5] &= ~(1u << (H.head & 31u));
           __syncwarp();
@@ -970,7 +969,7 @@ __device__ __noinline__ int lv_solo(const Region& Rs, LvSmem& L, const int* ring
         H.blk = L.s.blk;
         if (lane == 0) L.n_again += 1u;
       } else {
-        pull_end(R, L, ring, S, gate, kp, cur, cc, pb, pd, cap);
+        pull_end(R, L, S, gate, kp, cur, cc, pb, pd);
       }
       continue;
     }
@@ -988,7 +987,7 @@ __device__ __noinline__ int lv_solo(const Region& Rs, LvSmem& L, const int* ring
     if (lane == 0) L.cnt[zc] = 0u;
     const unsigned t = lane >> 3;
     const unsigned i = t < cnt ? list_get(R, L, cur, t) : 0u;
-    lv_cells(R, L, S, t < cnt && !cell_done(L, i), i, false, 0.0f, 0u, gate, kp, cur ^ 1u, nc, pb, pd, cap);
+    lv_cells(R, L, S, t < cnt && !cell_done(L, i), i, false, 0.0f, 0u, gate, kp, cur ^ 1u, nc, pb, pd);
     cur ^= 1u;
     cc = nc;
     ++rounds;
