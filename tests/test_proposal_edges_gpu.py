@@ -1,0 +1,44 @@
+"""The gradient kernel at the edges of its row tiles (16 rows a warp, 64 a CTA) and where a CTA takes several
+tiles, called twice (the second call finds the gradients empty), against a restatement in 64 bits that
+rounds to halves where the kernel does."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _half(a):
+    return a.astype(np.float16).astype(np.float64)
+
+
+def _gradients(p, x, y):
+    p, x, y = p.astype(np.float64), x.astype(np.float64), y.astype(np.float64)
+    w1, b1, w2, b2, w3, b3 = _half(p[:2048]).reshape(32, 64), p[2048:2112], _half(p[2112:6208]).reshape(64, 64), p[6208:6272], p[6272:6336], p[6336]
+    h1 = np.maximum(x @ w1 + b1, 0)
+    h2 = np.maximum(_half(h1) @ w2 + b2, 0)
+    dz = (1 / (1 + np.exp(-(h2 @ w3 + b3))) - y) / len(y)
+    d2 = np.outer(dz, w3) * (h2 > 0)
+    d1 = (_half(d2) @ w2.T) * (h1 > 0)
+    return np.concatenate([(x.T @ _half(d1)).ravel(), d1.sum(0), (_half(h1).T @ _half(d2)).ravel(), d2.sum(0), h2.T @ dz, [dz.sum()]])
+
+
+@pytest.mark.parametrize("n", [1, 15, 16, 17, 63, 64, 65, 129, 2 * 148 * 64 + 1])
+def test_gradients_at_tile_edges(vf, n):
+    import torch
+
+    from vfwater import proposal
+
+    mlp = proposal.MLP(seed=4)
+    rng = np.random.default_rng(n)
+    x = (rng.random((n, 32)) * (rng.random((n, 32)) < 0.5)).astype(np.float16)
+    # labels of one row in 64 only, so that the gradients of many rows do not cancel; halves of 1/n keep
+    # their precision down to n = 2^14 / 2^-14 (below 6e-5 their step is 2^-24)
+    y = (rng.random(n) < 1 / 64).astype(np.float32)
+    ref = _gradients(mlp.params(), x, y)
+    xd, yd = torch.from_numpy(x).cuda(), torch.from_numpy(y).cuda()
+    # the sums differ in the order of fp32 additions, and an operand next to a rounding boundary by a half's
+    # step: 2^-10 of its value, or 2^-24 of each of the n rows' products with values up to 4
+    tol = 2.0**-10 * np.abs(ref).max() + 4 * n * 2.0**-24 * 2.0**-5
+    for _ in range(2):
+        assert np.abs(mlp.grads(xd, yd) - ref).max() <= tol
+    mlp.close()

@@ -8,6 +8,7 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
 #include <cstring>
@@ -33,6 +34,7 @@ struct Dev {
   __half* w2t;    // [H][H]   output-major: B operand of H1.W2
   __half* w2n;    // [H][H]   input-major: B operand of dH2.W2^T
   float* loss;    // scratch scalar
+  unsigned* ticket;  // CTAs that have added their gradients
 };
 
 __device__ __forceinline__ void mma16816(float* c, const unsigned* a, const unsigned* b) {
@@ -144,177 +146,190 @@ __global__ void k_forward(Dev d, const __half* X, int n, float* prob) {
   }
 }
 
-// Backward of mean BCE-with-logits; gradients accumulate into d.g (fp32). Each warp: 16 rows.
-__global__ void k_backward(Dev d, const __half* X, const float* y, int n, float inv_n) {
-  __shared__ __half sh_h1[WARPS][16][H];   // H1 tile (row-major) for dW2
-  __shared__ __half sh_d2[WARPS][16][H];   // dZ2 tile for dW2, then dZ1 for dW1
-  __shared__ float sg[NPARAM];
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  for (int i = threadIdx.x; i < NPARAM; i += blockDim.x) sg[i] = 0.f;
-  __syncthreads();
-  const int tile = blockIdx.x * WARPS + w;
-  const int row0 = tile * 16;
-  if (row0 < n) {
-    Fwd f;
-    forward_tile(d, X, row0, n, f);
-    const int r0 = row0 + g, r1 = row0 + g + 8;
-    const float dz0 = r0 < n ? (sigmoidf_(f.z[0]) - y[r0]) * inv_n : 0.f;
-    const float dz1 = r1 < n ? (sigmoidf_(f.z[1]) - y[r1]) * inv_n : 0.f;
-    if (t == 0) atomicAdd(&sg[OFF_B3], dz0 + dz1);
-    // dw3, dZ2 = dz w3 (relu')
-    float d2[8][4];
+// Four 8x8 blocks of a row-major half matrix in shared memory, transposed: lane 8m + r gives the address
+// of row r of block m, and each lane gets elements (2t, g), (2t + 1, g) of every block.
+__device__ __forceinline__ void ldsm_t(unsigned (&r)[4], const __half* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"((unsigned)__cvta_generic_to_shared(p)));
+}
+
+// Sums of v[8j'..] over the eight row groups g: on return lane (g, t) holds those of v[2g], v[2g + 1], that
+// is of columns 8g + 2t, 8g + 2t + 1 (each step hands half of the values to the other half of the groups:
+// 14 shuffles instead of 48).
+__device__ __forceinline__ void column_sums(float (&v)[16], int lane) {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int c0 = 8 * j + 2 * t;
-      const float w0 = d.p[OFF_W3 + c0], w1 = d.p[OFF_W3 + c0 + 1];
-      float gw0 = f.h2[j][0] * dz0 + f.h2[j][2] * dz1;
-      float gw1 = f.h2[j][1] * dz0 + f.h2[j][3] * dz1;
-      // sum over the 8 row groups (lanes with equal t)
+  for (int h = 8; h >= 2; h >>= 1) {
+    const int o = 2 * h;  // lanes 16, 8, 4 apart
+    const bool hi = lane & o;
 #pragma unroll
-      for (int o = 4; o < 32; o <<= 1) {
-        gw0 += __shfl_xor_sync(0xFFFFFFFFu, gw0, o);
-        gw1 += __shfl_xor_sync(0xFFFFFFFFu, gw1, o);
-      }
-      if (g == 0) {
-        atomicAdd(&sg[OFF_W3 + c0], gw0);
-        atomicAdd(&sg[OFF_W3 + c0 + 1], gw1);
-      }
-      d2[j][0] = f.h2[j][0] > 0.f ? dz0 * w0 : 0.f;
-      d2[j][1] = f.h2[j][1] > 0.f ? dz0 * w1 : 0.f;
-      d2[j][2] = f.h2[j][2] > 0.f ? dz1 * w0 : 0.f;
-      d2[j][3] = f.h2[j][3] > 0.f ? dz1 * w1 : 0.f;
-      // db2
-      float s0 = d2[j][0] + d2[j][2], s1 = d2[j][1] + d2[j][3];
-#pragma unroll
-      for (int o = 4; o < 32; o <<= 1) {
-        s0 += __shfl_xor_sync(0xFFFFFFFFu, s0, o);
-        s1 += __shfl_xor_sync(0xFFFFFFFFu, s1, o);
-      }
-      if (g == 0) {
-        atomicAdd(&sg[OFF_B2 + c0], s0);
-        atomicAdd(&sg[OFF_B2 + c0 + 1], s1);
-      }
-      sh_h1[w][g][c0] = __float2half_rn(f.h1[j][0]);
-      sh_h1[w][g][c0 + 1] = __float2half_rn(f.h1[j][1]);
-      sh_h1[w][g + 8][c0] = __float2half_rn(f.h1[j][2]);
-      sh_h1[w][g + 8][c0 + 1] = __float2half_rn(f.h1[j][3]);
-      sh_d2[w][g][c0] = __float2half_rn(d2[j][0]);
-      sh_d2[w][g][c0 + 1] = __float2half_rn(d2[j][1]);
-      sh_d2[w][g + 8][c0] = __float2half_rn(d2[j][2]);
-      sh_d2[w][g + 8][c0 + 1] = __float2half_rn(d2[j][3]);
-    }
-    __syncwarp();
-    // dW2[i][j] = sum_r H1[r][i] dZ2[r][j]: M = 64 (i), N = 64 (j), K = 16 (r)
-#pragma unroll
-    for (int mi = 0; mi < 4; ++mi) {
-      unsigned a[4];  // A[i][r] = H1[r][i]
-      const int i0 = 16 * mi + g;
-      auto h = [&](int r, int i) { return sh_h1[w][r][i]; };
-      __half2 p;
-      p = __halves2half2(h(2 * t, i0), h(2 * t + 1, i0));
-      a[0] = *reinterpret_cast<unsigned*>(&p);
-      p = __halves2half2(h(2 * t, i0 + 8), h(2 * t + 1, i0 + 8));
-      a[1] = *reinterpret_cast<unsigned*>(&p);
-      p = __halves2half2(h(2 * t + 8, i0), h(2 * t + 9, i0));
-      a[2] = *reinterpret_cast<unsigned*>(&p);
-      p = __halves2half2(h(2 * t + 8, i0 + 8), h(2 * t + 9, i0 + 8));
-      a[3] = *reinterpret_cast<unsigned*>(&p);
-#pragma unroll
-      for (int nj = 0; nj < 8; ++nj) {
-        unsigned b[2];  // B[r][j] = dZ2[r][j], column j = 8nj + g
-        const int jc = 8 * nj + g;
-        __half2 q = __halves2half2(sh_d2[w][2 * t][jc], sh_d2[w][2 * t + 1][jc]);
-        b[0] = *reinterpret_cast<unsigned*>(&q);
-        q = __halves2half2(sh_d2[w][2 * t + 8][jc], sh_d2[w][2 * t + 9][jc]);
-        b[1] = *reinterpret_cast<unsigned*>(&q);
-        float c[4] = {0.f, 0.f, 0.f, 0.f};
-        mma16816(c, a, b);
-        const int ci = 16 * mi + g, cj = 8 * nj + 2 * t;
-        atomicAdd(&sg[OFF_W2 + ci * H + cj], c[0]);
-        atomicAdd(&sg[OFF_W2 + ci * H + cj + 1], c[1]);
-        atomicAdd(&sg[OFF_W2 + (ci + 8) * H + cj], c[2]);
-        atomicAdd(&sg[OFF_W2 + (ci + 8) * H + cj + 1], c[3]);
-      }
-    }
-    __syncwarp();  // the dZ2 tile is reused for dZ1 below
-    // dH1 = dZ2 W2^T (relu'): M = 16, N = 64 (i), K = 64 (j); A from the dZ2 accumulators
-    unsigned ad[4][4];
-#pragma unroll
-    for (int kk = 0; kk < 4; ++kk) {
-      ad[kk][0] = pack2(d2[2 * kk][0], d2[2 * kk][1]);
-      ad[kk][1] = pack2(d2[2 * kk][2], d2[2 * kk][3]);
-      ad[kk][2] = pack2(d2[2 * kk + 1][0], d2[2 * kk + 1][1]);
-      ad[kk][3] = pack2(d2[2 * kk + 1][2], d2[2 * kk + 1][3]);
-    }
-    float d1[8][4];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      float c[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-      for (int kk = 0; kk < 4; ++kk) {
-        unsigned b[2];  // B[k=j'][n=i] = W2[i][j'] (input-major copy), column i = 8j + g
-        const __half* col = d.w2n + (size_t)(8 * j + g) * H + kk * 16 + 2 * t;
-        b[0] = ld2(col);
-        b[1] = ld2(col + 8);
-        mma16816(c, ad[kk], b);
-      }
-      const int c0 = 8 * j + 2 * t;
-      d1[j][0] = f.h1[j][0] > 0.f ? c[0] : 0.f;
-      d1[j][1] = f.h1[j][1] > 0.f ? c[1] : 0.f;
-      d1[j][2] = f.h1[j][2] > 0.f ? c[2] : 0.f;
-      d1[j][3] = f.h1[j][3] > 0.f ? c[3] : 0.f;
-      float s0 = d1[j][0] + d1[j][2], s1 = d1[j][1] + d1[j][3];
-#pragma unroll
-      for (int o = 4; o < 32; o <<= 1) {
-        s0 += __shfl_xor_sync(0xFFFFFFFFu, s0, o);
-        s1 += __shfl_xor_sync(0xFFFFFFFFu, s1, o);
-      }
-      if (g == 0) {
-        atomicAdd(&sg[OFF_B1 + c0], s0);
-        atomicAdd(&sg[OFF_B1 + c0 + 1], s1);
-      }
-      sh_d2[w][g][c0] = __float2half_rn(d1[j][0]);
-      sh_d2[w][g][c0 + 1] = __float2half_rn(d1[j][1]);
-      sh_d2[w][g + 8][c0] = __float2half_rn(d1[j][2]);
-      sh_d2[w][g + 8][c0 + 1] = __float2half_rn(d1[j][3]);
-    }
-    __syncwarp();
-    // dW1[i][j] = sum_r X[r][i] dZ1[r][j]: M = 32 (i), N = 64 (j), K = 16 (r)
-#pragma unroll
-    for (int mi = 0; mi < 2; ++mi) {
-      unsigned a[4];  // A[i][r] = X[r][i]
-      const int i0 = 16 * mi + g;
-      auto xv = [&](int r, int i) { return (row0 + r < n) ? X[(size_t)(row0 + r) * IN + i] : __float2half_rn(0.f); };
-      __half2 p;
-      p = __halves2half2(xv(2 * t, i0), xv(2 * t + 1, i0));
-      a[0] = *reinterpret_cast<unsigned*>(&p);
-      p = __halves2half2(xv(2 * t, i0 + 8), xv(2 * t + 1, i0 + 8));
-      a[1] = *reinterpret_cast<unsigned*>(&p);
-      p = __halves2half2(xv(2 * t + 8, i0), xv(2 * t + 9, i0));
-      a[2] = *reinterpret_cast<unsigned*>(&p);
-      p = __halves2half2(xv(2 * t + 8, i0 + 8), xv(2 * t + 9, i0 + 8));
-      a[3] = *reinterpret_cast<unsigned*>(&p);
-#pragma unroll
-      for (int nj = 0; nj < 8; ++nj) {
-        unsigned b[2];
-        const int jc = 8 * nj + g;
-        __half2 q = __halves2half2(sh_d2[w][2 * t][jc], sh_d2[w][2 * t + 1][jc]);
-        b[0] = *reinterpret_cast<unsigned*>(&q);
-        q = __halves2half2(sh_d2[w][2 * t + 8][jc], sh_d2[w][2 * t + 9][jc]);
-        b[1] = *reinterpret_cast<unsigned*>(&q);
-        float c[4] = {0.f, 0.f, 0.f, 0.f};
-        mma16816(c, a, b);
-        const int ci = 16 * mi + g, cj = 8 * nj + 2 * t;
-        atomicAdd(&sg[OFF_W1 + ci * H + cj], c[0]);
-        atomicAdd(&sg[OFF_W1 + ci * H + cj + 1], c[1]);
-        atomicAdd(&sg[OFF_W1 + (ci + 8) * H + cj], c[2]);
-        atomicAdd(&sg[OFF_W1 + (ci + 8) * H + cj + 1], c[3]);
-      }
+    for (int q = 0; q < h; ++q) {
+      const float keep = hi ? v[q + h] : v[q], give = hi ? v[q] : v[q + h];
+      v[q] = keep + __shfl_xor_sync(0xFFFFFFFFu, give, o);
     }
   }
+}
+
+// Backward of mean BCE-with-logits over n rows; gradients accumulate into d.g (fp32). With `host` (mapped
+// host memory) the last CTA to finish moves the sums there and leaves d.g empty.
+//
+// What bounds it: latency; a training batch of 4096 rows is 64 CTAs and 0.2 GFLOP. A CTA takes 64 rows a
+// time. Each warp runs the chain of 16 rows forward and back in registers and leaves H1, dZ2, dZ1 and X
+// in shared memory; then the warps share out the two weight gradients, which are contractions over the
+// 64 rows, so that every sum has one owner and stays in its accumulators until the CTA's rows are done: no
+// atomics in shared memory (6,144 per warp when each warp made the products of its own 16 rows), and
+// half as many to global memory (pairs).
+constexpr int LDX = IN + 8, LDH = H + 8;  // row strides in halves: eight rows fall into different banks
+__global__ void __launch_bounds__(32 * WARPS) k_backward(Dev d, const __half* X, const float* y, int n, float inv_n, float* host) {
+  constexpr int ROWS = 16 * WARPS, NT = 32 * WARPS, NSUM = 3 * H + 1;
+  static_assert(WARPS == 4, "the weight gradients are shared out over four warps");
+  __shared__ __align__(16) __half sh_x[ROWS][LDX], sh_h1[ROWS][LDH], sh_d2[ROWS][LDH], sh_d1[ROWS][LDH];
+  __shared__ __align__(8) float sh_sum[WARPS][NSUM + 1];  // column sums of a warp's rows: dw3, db2, db1, db3
+  __shared__ bool s_last;
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  float a2[8][4] = {}, a1[4][4] = {}, as[2] = {0.f, 0.f};  // rows 16w of dW2; 16(w & 1) x 32(w >> 1) of dW1; sums
+  for (int tile = blockIdx.x; tile * ROWS < n; tile += gridDim.x) {
+    const int row0 = tile * ROWS + 16 * w;
+    // X rows of the warp, 16 bytes a lane twice (rows past the end: zero)
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int r = 8 * k + (lane >> 2), c = 8 * (lane & 3);
+      uint4 v = make_uint4(0u, 0u, 0u, 0u);
+      if (row0 + r < n) {
+        const unsigned* src = reinterpret_cast<const unsigned*>(X + (size_t)(row0 + r) * IN + c);
+        v = make_uint4(src[0], src[1], src[2], src[3]);  // (rows need be no more than 4-byte aligned)
+      }
+      *reinterpret_cast<uint4*>(&sh_x[16 * w + r][c]) = v;
+    }
+    {
+      Fwd f;
+      forward_tile(d, X, row0, n, f);
+      const int r0 = row0 + g, r1 = row0 + g + 8;
+      const float dz0 = r0 < n ? (sigmoidf_(f.z[0]) - y[r0]) * inv_n : 0.f;
+      const float dz1 = r1 < n ? (sigmoidf_(f.z[1]) - y[r1]) * inv_n : 0.f;
+      float sz = dz0 + dz1;
+#pragma unroll
+      for (int o = 4; o < 32; o <<= 1) sz += __shfl_xor_sync(0xFFFFFFFFu, sz, o);
+      if (lane == 0) sh_sum[w][3 * H] = sz;
+      // dw3, dZ2 = dz w3 (relu')
+      float d2[8][4], v[16];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int c0 = 8 * j + 2 * t;
+        const float w0 = d.p[OFF_W3 + c0], w1 = d.p[OFF_W3 + c0 + 1];
+        v[2 * j] = f.h2[j][0] * dz0 + f.h2[j][2] * dz1;
+        v[2 * j + 1] = f.h2[j][1] * dz0 + f.h2[j][3] * dz1;
+        d2[j][0] = f.h2[j][0] > 0.f ? dz0 * w0 : 0.f;
+        d2[j][1] = f.h2[j][1] > 0.f ? dz0 * w1 : 0.f;
+        d2[j][2] = f.h2[j][2] > 0.f ? dz1 * w0 : 0.f;
+        d2[j][3] = f.h2[j][3] > 0.f ? dz1 * w1 : 0.f;
+        *reinterpret_cast<unsigned*>(&sh_h1[16 * w + g][c0]) = pack2(f.h1[j][0], f.h1[j][1]);
+        *reinterpret_cast<unsigned*>(&sh_h1[16 * w + g + 8][c0]) = pack2(f.h1[j][2], f.h1[j][3]);
+        *reinterpret_cast<unsigned*>(&sh_d2[16 * w + g][c0]) = pack2(d2[j][0], d2[j][1]);
+        *reinterpret_cast<unsigned*>(&sh_d2[16 * w + g + 8][c0]) = pack2(d2[j][2], d2[j][3]);
+      }
+      column_sums(v, lane);
+      *reinterpret_cast<float2*>(&sh_sum[w][8 * g + 2 * t]) = make_float2(v[0], v[1]);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        v[2 * j] = d2[j][0] + d2[j][2];
+        v[2 * j + 1] = d2[j][1] + d2[j][3];
+      }
+      column_sums(v, lane);
+      *reinterpret_cast<float2*>(&sh_sum[w][H + 8 * g + 2 * t]) = make_float2(v[0], v[1]);
+      // dH1 = dZ2 W2^T (relu'): M = 16, N = 64 (i), K = 64 (j); A from the dZ2 accumulators
+      unsigned ad[4][4];
+#pragma unroll
+      for (int kk = 0; kk < 4; ++kk) {
+        ad[kk][0] = pack2(d2[2 * kk][0], d2[2 * kk][1]);
+        ad[kk][1] = pack2(d2[2 * kk][2], d2[2 * kk][3]);
+        ad[kk][2] = pack2(d2[2 * kk + 1][0], d2[2 * kk + 1][1]);
+        ad[kk][3] = pack2(d2[2 * kk + 1][2], d2[2 * kk + 1][3]);
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        float c[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk) {
+          unsigned b[2];  // B[k=j'][n=i] = W2[i][j'] (input-major copy), column i = 8j + g
+          const __half* col = d.w2n + (size_t)(8 * j + g) * H + kk * 16 + 2 * t;
+          b[0] = ld2(col);
+          b[1] = ld2(col + 8);
+          mma16816(c, ad[kk], b);
+        }
+        const int c0 = 8 * j + 2 * t;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) c[q] = f.h1[j][q] > 0.f ? c[q] : 0.f;
+        v[2 * j] = c[0] + c[2];
+        v[2 * j + 1] = c[1] + c[3];
+        *reinterpret_cast<unsigned*>(&sh_d1[16 * w + g][c0]) = pack2(c[0], c[1]);
+        *reinterpret_cast<unsigned*>(&sh_d1[16 * w + g + 8][c0]) = pack2(c[2], c[3]);
+      }
+      column_sums(v, lane);
+      *reinterpret_cast<float2*>(&sh_sum[w][2 * H + 8 * g + 2 * t]) = make_float2(v[0], v[1]);
+    }
+    __syncthreads();
+    // dW2[i][j] = sum_r H1[r][i] dZ2[r][j], dW1[i][j] = sum_r X[r][i] dZ1[r][j]; K = 64 (r)
+    const int m = lane >> 3, l8 = lane & 7;
+#pragma unroll
+    for (int ks = 0; ks < WARPS; ++ks) {
+      const int ra = 16 * ks + 8 * (m >> 1) + l8, rb = 16 * ks + 8 * (m & 1) + l8;
+      unsigned a[4], b[4];
+      ldsm_t(a, &sh_h1[ra][16 * w + 8 * (m & 1)]);
+#pragma unroll
+      for (int np = 0; np < 4; ++np) {
+        ldsm_t(b, &sh_d2[rb][16 * np + 8 * (m >> 1)]);
+        mma16816(a2[2 * np], a, b);
+        mma16816(a2[2 * np + 1], a, b + 2);
+      }
+      ldsm_t(a, &sh_x[ra][16 * (w & 1) + 8 * (m & 1)]);
+#pragma unroll
+      for (int np = 0; np < 2; ++np) {
+        ldsm_t(b, &sh_d1[rb][32 * (w >> 1) + 16 * np + 8 * (m >> 1)]);
+        mma16816(a1[2 * np], a, b);
+        mma16816(a1[2 * np + 1], a, b + 2);
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int c = (int)threadIdx.x + k * NT;
+      if (c < NSUM) as[k] += (sh_sum[0][c] + sh_sum[1][c]) + (sh_sum[2][c] + sh_sum[3][c]);
+    }
+    __syncthreads();
+  }
+  // ---- the CTA's sums to d.g
+  auto add2 = [&](int at, float x, float z) { atomicAdd(reinterpret_cast<float2*>(d.g + at), make_float2(x, z)); };
+#pragma unroll
+  for (int nj = 0; nj < 8; ++nj) {
+    const int at = OFF_W2 + (16 * w + g) * H + 8 * nj + 2 * t;
+    add2(at, a2[nj][0], a2[nj][1]);
+    add2(at + 8 * H, a2[nj][2], a2[nj][3]);
+  }
+#pragma unroll
+  for (int nj = 0; nj < 4; ++nj) {
+    const int at = OFF_W1 + (16 * (w & 1) + g) * H + 32 * (w >> 1) + 8 * nj + 2 * t;
+    add2(at, a1[nj][0], a1[nj][1]);
+    add2(at + 8 * H, a1[nj][2], a1[nj][3]);
+  }
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const int c = (int)threadIdx.x + k * NT;
+    const int at = c < H ? OFF_W3 + c : c < 2 * H ? OFF_B2 + c - H : c < 3 * H ? OFF_B1 + c - 2 * H : OFF_B3;
+    if (c < NSUM) atomicAdd(d.g + at, as[k]);
+  }
+  if (!host) return;
+  // ---- the last CTA hands the sums over
+  __threadfence();
   __syncthreads();
-  for (int i = threadIdx.x; i < NPARAM; i += blockDim.x)
-    if (sg[i] != 0.f) atomicAdd(&d.g[i], sg[i]);
+  if (threadIdx.x == 0) s_last = atomicAdd(d.ticket, 1u) == gridDim.x - 1u;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  for (int i = threadIdx.x; i < NPARAM; i += NT) {
+    host[i] = __ldcg(d.g + i);
+    d.g[i] = 0.f;
+  }
+  if (threadIdx.x == 0) *d.ticket = 0u;
 }
 
 // mean BCE-with-logits over n rows (for monitoring)
@@ -373,6 +388,9 @@ struct vf_mlp {
   int device = 0;
   Dev d{};
   int step = 0;
+  int ctas = 1;           // resident CTAs of k_backward
+  float* hgrad = nullptr; // mapped host memory the gradients come back in
+  float* dgrad = nullptr; // its device address
   std::vector<void*> allocs;
 };
 
@@ -383,6 +401,11 @@ bool alloc(vf_mlp* h, T** p, size_t n) {
   h->allocs.push_back(*p);
   cudaMemset(*p, 0, sizeof(T) * n);
   return true;
+}
+void release(vf_mlp* h) {
+  for (void* p : h->allocs) cudaFree(p);
+  if (h->hgrad) cudaFreeHost(h->hgrad);
+  delete h;
 }
 unsigned blocks_for(uint64_t n) { return (unsigned)((n + 16 * WARPS - 1) / (16 * WARPS)); }
 }  // namespace
@@ -395,11 +418,15 @@ int vf_mlp_create(int32_t device, uint64_t seed, vf_mlp** out) {
   auto* h = new vf_mlp();
   h->device = device;
   if (!alloc(h, &h->d.p, NPARAM) || !alloc(h, &h->d.g, NPARAM) || !alloc(h, &h->d.m, NPARAM) || !alloc(h, &h->d.v, NPARAM) ||
-      !alloc(h, &h->d.w1t, H * IN) || !alloc(h, &h->d.w2t, H * H) || !alloc(h, &h->d.w2n, H * H) || !alloc(h, &h->d.loss, 1)) {
-    for (void* p : h->allocs) cudaFree(p);
-    delete h;
+      !alloc(h, &h->d.w1t, H * IN) || !alloc(h, &h->d.w2t, H * H) || !alloc(h, &h->d.w2n, H * H) || !alloc(h, &h->d.loss, 1) || !alloc(h, &h->d.ticket, 1) ||
+      cudaHostAlloc((void**)&h->hgrad, NPARAM * 4, cudaHostAllocMapped) != cudaSuccess ||
+      cudaHostGetDevicePointer((void**)&h->dgrad, h->hgrad, 0) != cudaSuccess) {
+    release(h);
     return VF_ERR_OOM;
   }
+  int sms = 1;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+  h->ctas = 2 * sms;
   // He-uniform init from a splitmix64 stream (host), biases 0
   std::vector<float> p(NPARAM, 0.f);
   uint64_t s = seed * 0x9E3779B97F4A7C15ULL + 1;
@@ -417,8 +444,7 @@ int vf_mlp_create(int32_t device, uint64_t seed, vf_mlp** out) {
   cudaMemcpy(h->d.p, p.data(), NPARAM * 4, cudaMemcpyHostToDevice);
   k_refresh<<<32, 256>>>(h->d);
   if (cudaDeviceSynchronize() != cudaSuccess) {
-    for (void* q : h->allocs) cudaFree(q);
-    delete h;
+    release(h);
     return VF_ERR_CUDA;
   }
   *out = h;
@@ -427,8 +453,7 @@ int vf_mlp_create(int32_t device, uint64_t seed, vf_mlp** out) {
 
 void vf_mlp_destroy(vf_mlp* h) {
   if (!h) return;
-  for (void* p : h->allocs) cudaFree(p);
-  delete h;
+  release(h);
 }
 
 int vf_mlp_nparams(void) { return NPARAM; }
@@ -457,12 +482,11 @@ int vf_mlp_forward(vf_mlp* h, const void* dev_x, uint64_t n, float* dev_prob, vo
 int vf_mlp_grads(vf_mlp* h, const void* dev_x, const float* dev_y, uint64_t n, float* grads, void* stream) {
   if (!h || !dev_x || !dev_y || !n || !grads) return VF_ERR_INVALID;
   cudaStream_t st = (cudaStream_t)stream;
-  cudaMemsetAsync(h->d.g, 0, NPARAM * 4, st);
-  k_backward<<<blocks_for(n), 32 * WARPS, 0, st>>>(h->d, (const __half*)dev_x, dev_y, (int)n, 1.0f / (float)n);
-  if (cudaMemcpyAsync(grads, h->d.g, NPARAM * 4, cudaMemcpyDeviceToHost, st) != cudaSuccess) return VF_ERR_CUDA;
-  if (cudaStreamSynchronize(st) != cudaSuccess) return VF_ERR_CUDA;
-  cudaMemsetAsync(h->d.g, 0, NPARAM * 4, st);
-  return cudaStreamSynchronize(st) == cudaSuccess ? VF_OK : VF_ERR_CUDA;
+  // (d.g is empty between calls: its reader empties it)
+  k_backward<<<std::min(blocks_for(n), (unsigned)h->ctas), 32 * WARPS, 0, st>>>(h->d, (const __half*)dev_x, dev_y, (int)n, 1.0f / (float)n, h->dgrad);
+  if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(st) != cudaSuccess) return VF_ERR_CUDA;
+  std::memcpy(grads, h->hgrad, NPARAM * 4);
+  return VF_OK;
 }
 
 // one Adam step on a minibatch (device arrays); *loss (host, optional) = the batch's mean BCE
@@ -474,7 +498,7 @@ int vf_mlp_train_step(vf_mlp* h, const void* dev_x, const float* dev_y, uint64_t
     cudaMemsetAsync(h->d.loss, 0, 4, st);
     k_loss<<<blocks_for(n), 32 * WARPS, 0, st>>>(h->d, (const __half*)dev_x, dev_y, (int)n, 1.0f / (float)n);
   }
-  k_backward<<<blocks_for(n), 32 * WARPS, 0, st>>>(h->d, (const __half*)dev_x, dev_y, (int)n, 1.0f / (float)n);
+  k_backward<<<std::min(blocks_for(n), (unsigned)h->ctas), 32 * WARPS, 0, st>>>(h->d, (const __half*)dev_x, dev_y, (int)n, 1.0f / (float)n, nullptr);
   h->step += 1;
   const float b1 = 0.9f, b2 = 0.999f;
   const float c1 = 1.f - std::pow(b1, (float)h->step), c2 = 1.f - std::pow(b2, (float)h->step);
