@@ -50,6 +50,47 @@ __device__ __forceinline__ unsigned pack2(float lo, float hi) {
 }
 __device__ __forceinline__ unsigned ld2(const __half* p) { return *reinterpret_cast<const unsigned*>(p); }
 
+// Four 8x8 blocks of a row-major half matrix in shared memory: lane 8m + r gives the address of row r of
+// block m; lane (g, t) gets elements (g, 2t), (g, 2t + 1) of every block, of its transpose with ldsm_t.
+__device__ __forceinline__ void ldsm(unsigned (&r)[4], const __half* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"((unsigned)__cvta_generic_to_shared(p)));
+}
+__device__ __forceinline__ void ldsm_t(unsigned (&r)[4], const __half* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"((unsigned)__cvta_generic_to_shared(p)));
+}
+
+// The network in shared memory, all of it fetched at once: a kernel here is one chain of latencies, and
+// the 96 fragment loads of a 16-row tile from L2 were most of it.
+constexpr int LDX = IN + 8, LDH = H + 8;  // row strides in halves: eight rows fall into different banks
+struct __align__(16) Net {
+  __half w1t[H][LDX], w2t[H][LDH];
+  float b1[H], b2[H], w3[H], b3;
+};
+template <int COLS, int LD, int NT>
+__device__ __forceinline__ void load_matrix(__half (*dst)[LD], const __half* src) {
+#pragma unroll
+  for (int k = 0; k < H * COLS / 8 / NT; ++k) {
+    const int e = (threadIdx.x + k * NT) * 8;
+    *reinterpret_cast<uint4*>(&dst[e / COLS][e % COLS]) = *reinterpret_cast<const uint4*>(src + e);
+  }
+}
+template <int NT>
+__device__ __forceinline__ void load_net(const Dev& d, Net& s) {
+  static_assert(H * IN / 8 % NT == 0, "whole 16-byte pieces for every thread");
+  load_matrix<IN, LDX, NT>(s.w1t, d.w1t);
+  load_matrix<H, LDH, NT>(s.w2t, d.w2t);
+  if (threadIdx.x < H) {
+    s.b1[threadIdx.x] = d.p[OFF_B1 + threadIdx.x];
+    s.b2[threadIdx.x] = d.p[OFF_B2 + threadIdx.x];
+    s.w3[threadIdx.x] = d.p[OFF_W3 + threadIdx.x];
+    if (threadIdx.x == 0) s.b3 = d.p[OFF_B3];
+  }
+}
+
 // Per-warp forward of 16 rows. Fragment conventions of m16n8k16: g = lane/4, t = lane%4; an A
 // fragment holds (row g | g+8) x (cols 2t,2t+1 | 2t+8,2t+9) of a 16x16 tile; an accumulator tile
 // (16x8) holds rows g, g+8 x cols 2t, 2t+1; a B fragment holds k = 2t,2t+1 (+8) of column g.
@@ -59,11 +100,10 @@ struct Fwd {
   float z[2];      // logits of rows g and g+8
 };
 
-__device__ void forward_tile(const Dev& d, const __half* X, int row0, int n, Fwd& f) {
+// The A fragments of a warp's 16 rows of X (16 x 32: two k-steps), rows past the end zero.
+__device__ __forceinline__ void load_rows(const __half* X, int row0, int n, unsigned (&a)[2][4]) {
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int r0 = row0 + g, r1 = row0 + g + 8;
-  // A fragments of X (16 x 32): two k-steps
-  unsigned a[2][4];
 #pragma unroll
   for (int kk = 0; kk < 2; ++kk) {
     const int c = kk * 16 + 2 * t;
@@ -72,18 +112,18 @@ __device__ void forward_tile(const Dev& d, const __half* X, int row0, int n, Fwd
     a[kk][2] = r0 < n ? ld2(X + (size_t)r0 * IN + c + 8) : 0u;
     a[kk][3] = r1 < n ? ld2(X + (size_t)r1 * IN + c + 8) : 0u;
   }
+}
+
+__device__ __forceinline__ void forward_tile(const Net& s, const unsigned (&a)[2][4], Fwd& f) {
+  const int lane = threadIdx.x & 31, t = lane & 3, m = lane >> 3, l8 = lane & 7;
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
     float c[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-    for (int kk = 0; kk < 2; ++kk) {
-      unsigned b[2];
-      const __half* col = d.w1t + (size_t)(8 * j + g) * IN + kk * 16 + 2 * t;
-      b[0] = ld2(col);
-      b[1] = ld2(col + 8);
-      mma16816(c, a[kk], b);
-    }
-    const float bb0 = d.p[OFF_B1 + 8 * j + 2 * t], bb1 = d.p[OFF_B1 + 8 * j + 2 * t + 1];
+    unsigned b[4];  // k = 0..31 of columns 8j..8j+7
+    ldsm(b, &s.w1t[8 * j + l8][8 * m]);
+    mma16816(c, a[0], b);
+    mma16816(c, a[1], b + 2);
+    const float bb0 = s.b1[8 * j + 2 * t], bb1 = s.b1[8 * j + 2 * t + 1];
     f.h1[j][0] = fmaxf(c[0] + bb0, 0.f);
     f.h1[j][1] = fmaxf(c[1] + bb1, 0.f);
     f.h1[j][2] = fmaxf(c[2] + bb0, 0.f);
@@ -102,14 +142,13 @@ __device__ void forward_tile(const Dev& d, const __half* X, int row0, int n, Fwd
   for (int j = 0; j < 8; ++j) {
     float c[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-    for (int kk = 0; kk < 4; ++kk) {
-      unsigned b[2];
-      const __half* col = d.w2t + (size_t)(8 * j + g) * H + kk * 16 + 2 * t;
-      b[0] = ld2(col);
-      b[1] = ld2(col + 8);
-      mma16816(c, a2[kk], b);
+    for (int kk = 0; kk < 2; ++kk) {
+      unsigned b[4];
+      ldsm(b, &s.w2t[8 * j + l8][32 * kk + 8 * m]);
+      mma16816(c, a2[2 * kk], b);
+      mma16816(c, a2[2 * kk + 1], b + 2);
     }
-    const float bb0 = d.p[OFF_B2 + 8 * j + 2 * t], bb1 = d.p[OFF_B2 + 8 * j + 2 * t + 1];
+    const float bb0 = s.b2[8 * j + 2 * t], bb1 = s.b2[8 * j + 2 * t + 1];
     f.h2[j][0] = fmaxf(c[0] + bb0, 0.f);
     f.h2[j][1] = fmaxf(c[1] + bb1, 0.f);
     f.h2[j][2] = fmaxf(c[2] + bb0, 0.f);
@@ -119,7 +158,7 @@ __device__ void forward_tile(const Dev& d, const __half* X, int row0, int n, Fwd
   float z0 = 0.f, z1 = 0.f;
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
-    const float w0 = d.p[OFF_W3 + 8 * j + 2 * t], w1 = d.p[OFF_W3 + 8 * j + 2 * t + 1];
+    const float w0 = s.w3[8 * j + 2 * t], w1 = s.w3[8 * j + 2 * t + 1];
     z0 += f.h2[j][0] * w0 + f.h2[j][1] * w1;
     z1 += f.h2[j][2] * w0 + f.h2[j][3] * w1;
   }
@@ -127,31 +166,29 @@ __device__ void forward_tile(const Dev& d, const __half* X, int row0, int n, Fwd
   z0 += __shfl_xor_sync(0xFFFFFFFFu, z0, 2);
   z1 += __shfl_xor_sync(0xFFFFFFFFu, z1, 1);
   z1 += __shfl_xor_sync(0xFFFFFFFFu, z1, 2);
-  f.z[0] = z0 + d.p[OFF_B3];
-  f.z[1] = z1 + d.p[OFF_B3];
+  f.z[0] = z0 + s.b3;
+  f.z[1] = z1 + s.b3;
 }
 
 __device__ __forceinline__ float sigmoidf_(float z) { return 1.0f / (1.0f + expf(-z)); }
 
-__global__ void k_forward(Dev d, const __half* X, int n, float* prob) {
-  const int tile = blockIdx.x * WARPS + (threadIdx.x >> 5);
-  const int row0 = tile * 16;
+// Probabilities of n rows, 16 a warp. 23,137 rows: 5.0 us, 7.8 with the weights read from L2 (their bytes
+// and products take 0.3 us; the rest is launch and one round of latencies).
+__global__ void __launch_bounds__(32 * WARPS) k_forward(Dev d, const __half* X, int n, float* prob) {
+  __shared__ Net s;
+  const int row0 = (blockIdx.x * WARPS + (threadIdx.x >> 5)) * 16;
+  unsigned a[2][4];
+  load_rows(X, row0, n, a);
+  load_net<32 * WARPS>(d, s);
+  __syncthreads();
   if (row0 >= n) return;
   Fwd f;
-  forward_tile(d, X, row0, n, f);
+  forward_tile(s, a, f);
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   if (t == 0) {
     if (row0 + g < n) prob[row0 + g] = sigmoidf_(f.z[0]);
     if (row0 + g + 8 < n) prob[row0 + g + 8] = sigmoidf_(f.z[1]);
   }
-}
-
-// Four 8x8 blocks of a row-major half matrix in shared memory, transposed: lane 8m + r gives the address
-// of row r of block m, and each lane gets elements (2t, g), (2t + 1, g) of every block.
-__device__ __forceinline__ void ldsm_t(unsigned (&r)[4], const __half* p) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-               : "r"((unsigned)__cvta_generic_to_shared(p)));
 }
 
 // Sums of v[8j'..] over the eight row groups g: on return lane (g, t) holds those of v[2g], v[2g + 1], that
@@ -173,70 +210,78 @@ __device__ __forceinline__ void column_sums(float (&v)[16], int lane) {
 // Backward of mean BCE-with-logits over n rows; gradients accumulate into d.g (fp32). With `host` (mapped
 // host memory) the last CTA to finish moves the sums there and leaves d.g empty.
 //
-// What bounds it: latency; a training batch of 4096 rows is 64 CTAs and 0.2 GFLOP. A CTA takes 64 rows a
-// time. Each warp runs the chain of 16 rows forward and back in registers and leaves H1, dZ2, dZ1 and X
+// What bounds it: latency; a training batch of 4096 rows is 64 CTAs and 0.2 GFLOP. A call took 77 us with a
+// kernel per 16 rows a warp, two memsets, a copy and two waits; 40 us in this form with the weights read
+// from L2 fragment by fragment (kernel 24 us); 26 us with them in shared memory (kernel 11.5 us, of which
+// about 3 are the last CTA's). A CTA takes 64 rows a time. Each warp runs the chain of 16 rows forward and back in registers and leaves H1, dZ2, dZ1 and X
 // in shared memory; then the warps share out the two weight gradients, which are contractions over the
 // 64 rows, so that every sum has one owner and stays in its accumulators until the CTA's rows are done: no
 // atomics in shared memory (6,144 per warp when each warp made the products of its own 16 rows), and
 // half as many to global memory (pairs).
-constexpr int LDX = IN + 8, LDH = H + 8;  // row strides in halves: eight rows fall into different banks
+struct __align__(16) BackSmem {
+  static constexpr int ROWS = 16 * WARPS, NSUM = 3 * H + 1;
+  Net net;
+  __half w2n[H][LDH];
+  __half x[ROWS][LDX], h1[ROWS][LDH], d2[ROWS][LDH], d1[ROWS][LDH];
+  float sum[WARPS][NSUM + 1];  // column sums of a warp's rows: dw3, db2, db1, db3
+  bool last;
+};
 __global__ void __launch_bounds__(32 * WARPS) k_backward(Dev d, const __half* X, const float* y, int n, float inv_n, float* host) {
-  constexpr int ROWS = 16 * WARPS, NT = 32 * WARPS, NSUM = 3 * H + 1;
+  constexpr int ROWS = BackSmem::ROWS, NT = 32 * WARPS, NSUM = BackSmem::NSUM;
   static_assert(WARPS == 4, "the weight gradients are shared out over four warps");
-  __shared__ __align__(16) __half sh_x[ROWS][LDX], sh_h1[ROWS][LDH], sh_d2[ROWS][LDH], sh_d1[ROWS][LDH];
-  __shared__ __align__(8) float sh_sum[WARPS][NSUM + 1];  // column sums of a warp's rows: dw3, db2, db1, db3
-  __shared__ bool s_last;
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  extern __shared__ __align__(16) unsigned char smem[];
+  BackSmem& S = *reinterpret_cast<BackSmem*>(smem);
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, m = lane >> 3, l8 = lane & 7;
   float a2[8][4] = {}, a1[4][4] = {}, as[2] = {0.f, 0.f};  // rows 16w of dW2; 16(w & 1) x 32(w >> 1) of dW1; sums
   for (int tile = blockIdx.x; tile * ROWS < n; tile += gridDim.x) {
     const int row0 = tile * ROWS + 16 * w;
-    // X rows of the warp, 16 bytes a lane twice (rows past the end: zero)
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const int r = 8 * k + (lane >> 2), c = 8 * (lane & 3);
-      uint4 v = make_uint4(0u, 0u, 0u, 0u);
-      if (row0 + r < n) {
-        const unsigned* src = reinterpret_cast<const unsigned*>(X + (size_t)(row0 + r) * IN + c);
-        v = make_uint4(src[0], src[1], src[2], src[3]);  // (rows need be no more than 4-byte aligned)
-      }
-      *reinterpret_cast<uint4*>(&sh_x[16 * w + r][c]) = v;
+    unsigned ax[2][4];
+    load_rows(X, row0, n, ax);
+    if (tile == (int)blockIdx.x) {
+      load_net<NT>(d, S.net);
+      load_matrix<H, LDH, NT>(S.w2n, d.w2n);
+      __syncthreads();
     }
+#pragma unroll
+    for (int kk = 0; kk < 2; ++kk)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) *reinterpret_cast<unsigned*>(&S.x[16 * w + g + 8 * (q & 1)][16 * kk + 2 * t + 8 * (q >> 1)]) = ax[kk][q];
     {
       Fwd f;
-      forward_tile(d, X, row0, n, f);
+      forward_tile(S.net, ax, f);
       const int r0 = row0 + g, r1 = row0 + g + 8;
       const float dz0 = r0 < n ? (sigmoidf_(f.z[0]) - y[r0]) * inv_n : 0.f;
       const float dz1 = r1 < n ? (sigmoidf_(f.z[1]) - y[r1]) * inv_n : 0.f;
       float sz = dz0 + dz1;
 #pragma unroll
       for (int o = 4; o < 32; o <<= 1) sz += __shfl_xor_sync(0xFFFFFFFFu, sz, o);
-      if (lane == 0) sh_sum[w][3 * H] = sz;
+      if (lane == 0) S.sum[w][3 * H] = sz;
       // dw3, dZ2 = dz w3 (relu')
       float d2[8][4], v[16];
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         const int c0 = 8 * j + 2 * t;
-        const float w0 = d.p[OFF_W3 + c0], w1 = d.p[OFF_W3 + c0 + 1];
+        const float w0 = S.net.w3[c0], w1 = S.net.w3[c0 + 1];
         v[2 * j] = f.h2[j][0] * dz0 + f.h2[j][2] * dz1;
         v[2 * j + 1] = f.h2[j][1] * dz0 + f.h2[j][3] * dz1;
         d2[j][0] = f.h2[j][0] > 0.f ? dz0 * w0 : 0.f;
         d2[j][1] = f.h2[j][1] > 0.f ? dz0 * w1 : 0.f;
         d2[j][2] = f.h2[j][2] > 0.f ? dz1 * w0 : 0.f;
         d2[j][3] = f.h2[j][3] > 0.f ? dz1 * w1 : 0.f;
-        *reinterpret_cast<unsigned*>(&sh_h1[16 * w + g][c0]) = pack2(f.h1[j][0], f.h1[j][1]);
-        *reinterpret_cast<unsigned*>(&sh_h1[16 * w + g + 8][c0]) = pack2(f.h1[j][2], f.h1[j][3]);
-        *reinterpret_cast<unsigned*>(&sh_d2[16 * w + g][c0]) = pack2(d2[j][0], d2[j][1]);
-        *reinterpret_cast<unsigned*>(&sh_d2[16 * w + g + 8][c0]) = pack2(d2[j][2], d2[j][3]);
+        *reinterpret_cast<unsigned*>(&S.h1[16 * w + g][c0]) = pack2(f.h1[j][0], f.h1[j][1]);
+        *reinterpret_cast<unsigned*>(&S.h1[16 * w + g + 8][c0]) = pack2(f.h1[j][2], f.h1[j][3]);
+        *reinterpret_cast<unsigned*>(&S.d2[16 * w + g][c0]) = pack2(d2[j][0], d2[j][1]);
+        *reinterpret_cast<unsigned*>(&S.d2[16 * w + g + 8][c0]) = pack2(d2[j][2], d2[j][3]);
       }
       column_sums(v, lane);
-      *reinterpret_cast<float2*>(&sh_sum[w][8 * g + 2 * t]) = make_float2(v[0], v[1]);
+      *reinterpret_cast<float2*>(&S.sum[w][8 * g + 2 * t]) = make_float2(v[0], v[1]);
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         v[2 * j] = d2[j][0] + d2[j][2];
         v[2 * j + 1] = d2[j][1] + d2[j][3];
       }
       column_sums(v, lane);
-      *reinterpret_cast<float2*>(&sh_sum[w][H + 8 * g + 2 * t]) = make_float2(v[0], v[1]);
+      *reinterpret_cast<float2*>(&S.sum[w][H + 8 * g + 2 * t]) = make_float2(v[0], v[1]);
       // dH1 = dZ2 W2^T (relu'): M = 16, N = 64 (i), K = 64 (j); A from the dZ2 accumulators
       unsigned ad[4][4];
 #pragma unroll
@@ -250,42 +295,40 @@ __global__ void __launch_bounds__(32 * WARPS) k_backward(Dev d, const __half* X,
       for (int j = 0; j < 8; ++j) {
         float c[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-        for (int kk = 0; kk < 4; ++kk) {
-          unsigned b[2];  // B[k=j'][n=i] = W2[i][j'] (input-major copy), column i = 8j + g
-          const __half* col = d.w2n + (size_t)(8 * j + g) * H + kk * 16 + 2 * t;
-          b[0] = ld2(col);
-          b[1] = ld2(col + 8);
-          mma16816(c, ad[kk], b);
+        for (int kk = 0; kk < 2; ++kk) {
+          unsigned b[4];  // B[k=j'][n=i] = W2[i][j'] (input-major copy), columns i = 8j..8j+7
+          ldsm(b, &S.w2n[8 * j + l8][32 * kk + 8 * m]);
+          mma16816(c, ad[2 * kk], b);
+          mma16816(c, ad[2 * kk + 1], b + 2);
         }
         const int c0 = 8 * j + 2 * t;
 #pragma unroll
         for (int q = 0; q < 4; ++q) c[q] = f.h1[j][q] > 0.f ? c[q] : 0.f;
         v[2 * j] = c[0] + c[2];
         v[2 * j + 1] = c[1] + c[3];
-        *reinterpret_cast<unsigned*>(&sh_d1[16 * w + g][c0]) = pack2(c[0], c[1]);
-        *reinterpret_cast<unsigned*>(&sh_d1[16 * w + g + 8][c0]) = pack2(c[2], c[3]);
+        *reinterpret_cast<unsigned*>(&S.d1[16 * w + g][c0]) = pack2(c[0], c[1]);
+        *reinterpret_cast<unsigned*>(&S.d1[16 * w + g + 8][c0]) = pack2(c[2], c[3]);
       }
       column_sums(v, lane);
-      *reinterpret_cast<float2*>(&sh_sum[w][2 * H + 8 * g + 2 * t]) = make_float2(v[0], v[1]);
+      *reinterpret_cast<float2*>(&S.sum[w][2 * H + 8 * g + 2 * t]) = make_float2(v[0], v[1]);
     }
     __syncthreads();
     // dW2[i][j] = sum_r H1[r][i] dZ2[r][j], dW1[i][j] = sum_r X[r][i] dZ1[r][j]; K = 64 (r)
-    const int m = lane >> 3, l8 = lane & 7;
 #pragma unroll
     for (int ks = 0; ks < WARPS; ++ks) {
       const int ra = 16 * ks + 8 * (m >> 1) + l8, rb = 16 * ks + 8 * (m & 1) + l8;
       unsigned a[4], b[4];
-      ldsm_t(a, &sh_h1[ra][16 * w + 8 * (m & 1)]);
+      ldsm_t(a, &S.h1[ra][16 * w + 8 * (m & 1)]);
 #pragma unroll
       for (int np = 0; np < 4; ++np) {
-        ldsm_t(b, &sh_d2[rb][16 * np + 8 * (m >> 1)]);
+        ldsm_t(b, &S.d2[rb][16 * np + 8 * (m >> 1)]);
         mma16816(a2[2 * np], a, b);
         mma16816(a2[2 * np + 1], a, b + 2);
       }
-      ldsm_t(a, &sh_x[ra][16 * (w & 1) + 8 * (m & 1)]);
+      ldsm_t(a, &S.x[ra][16 * (w & 1) + 8 * (m & 1)]);
 #pragma unroll
       for (int np = 0; np < 2; ++np) {
-        ldsm_t(b, &sh_d1[rb][32 * (w >> 1) + 16 * np + 8 * (m >> 1)]);
+        ldsm_t(b, &S.d1[rb][32 * (w >> 1) + 16 * np + 8 * (m >> 1)]);
         mma16816(a1[2 * np], a, b);
         mma16816(a1[2 * np + 1], a, b + 2);
       }
@@ -293,7 +336,7 @@ __global__ void __launch_bounds__(32 * WARPS) k_backward(Dev d, const __half* X,
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
       const int c = (int)threadIdx.x + k * NT;
-      if (c < NSUM) as[k] += (sh_sum[0][c] + sh_sum[1][c]) + (sh_sum[2][c] + sh_sum[3][c]);
+      if (c < NSUM) as[k] += (S.sum[0][c] + S.sum[1][c]) + (S.sum[2][c] + S.sum[3][c]);
     }
     __syncthreads();
   }
@@ -321,24 +364,42 @@ __global__ void __launch_bounds__(32 * WARPS) k_backward(Dev d, const __half* X,
   // ---- the last CTA hands the sums over
   __threadfence();
   __syncthreads();
-  if (threadIdx.x == 0) s_last = atomicAdd(d.ticket, 1u) == gridDim.x - 1u;
+  if (threadIdx.x == 0) S.last = atomicAdd(d.ticket, 1u) == gridDim.x - 1u;
   __syncthreads();
-  if (!s_last) return;
+  if (!S.last) return;
   __threadfence();
-  for (int i = threadIdx.x; i < NPARAM; i += NT) {
-    host[i] = __ldcg(d.g + i);
-    d.g[i] = 0.f;
+  constexpr int QUADS = NPARAM / 4;
+  float4* g4 = reinterpret_cast<float4*>(d.g);
+  float4* h4 = reinterpret_cast<float4*>(host);
+  float4 q[(QUADS + NT - 1) / NT];  // all under way at once
+#pragma unroll
+  for (int k = 0; k < (QUADS + NT - 1) / NT; ++k) q[k] = __ldcg(g4 + min((int)threadIdx.x + k * NT, QUADS - 1));
+  static_assert(NPARAM == 4 * QUADS + 1, "one parameter past the quads");
+  if (threadIdx.x == 0) {
+    host[NPARAM - 1] = __ldcg(d.g + NPARAM - 1);
+    d.g[NPARAM - 1] = 0.f;
+    *d.ticket = 0u;
   }
-  if (threadIdx.x == 0) *d.ticket = 0u;
+#pragma unroll
+  for (int k = 0; k < (QUADS + NT - 1) / NT; ++k) {
+    const int i = (int)threadIdx.x + k * NT;
+    if (i >= QUADS) continue;
+    h4[i] = q[k];
+    g4[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  }
 }
 
 // mean BCE-with-logits over n rows (for monitoring)
-__global__ void k_loss(Dev d, const __half* X, const float* y, int n, float inv_n) {
-  const int tile = blockIdx.x * WARPS + (threadIdx.x >> 5);
-  const int row0 = tile * 16;
+__global__ void __launch_bounds__(32 * WARPS) k_loss(Dev d, const __half* X, const float* y, int n, float inv_n) {
+  __shared__ Net s;
+  const int row0 = (blockIdx.x * WARPS + (threadIdx.x >> 5)) * 16;
+  unsigned a[2][4];
+  load_rows(X, row0, n, a);
+  load_net<32 * WARPS>(d, s);
+  __syncthreads();
   if (row0 >= n) return;
   Fwd f;
-  forward_tile(d, X, row0, n, f);
+  forward_tile(s, a, f);
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   float l = 0.f;
   if (t == 0) {
@@ -424,6 +485,10 @@ int vf_mlp_create(int32_t device, uint64_t seed, vf_mlp** out) {
     release(h);
     return VF_ERR_OOM;
   }
+  if (cudaFuncSetAttribute(k_backward, cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(BackSmem)) != cudaSuccess) {
+    release(h);
+    return VF_ERR_CUDA;
+  }
   int sms = 1;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
   h->ctas = 2 * sms;
@@ -483,7 +548,7 @@ int vf_mlp_grads(vf_mlp* h, const void* dev_x, const float* dev_y, uint64_t n, f
   if (!h || !dev_x || !dev_y || !n || !grads) return VF_ERR_INVALID;
   cudaStream_t st = (cudaStream_t)stream;
   // (d.g is empty between calls: its reader empties it)
-  k_backward<<<std::min(blocks_for(n), (unsigned)h->ctas), 32 * WARPS, 0, st>>>(h->d, (const __half*)dev_x, dev_y, (int)n, 1.0f / (float)n, h->dgrad);
+  k_backward<<<std::min(blocks_for(n), (unsigned)h->ctas), 32 * WARPS, sizeof(BackSmem), st>>>(h->d, (const __half*)dev_x, dev_y, (int)n, 1.0f / (float)n, h->dgrad);
   if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(st) != cudaSuccess) return VF_ERR_CUDA;
   std::memcpy(grads, h->hgrad, NPARAM * 4);
   return VF_OK;
@@ -498,7 +563,7 @@ int vf_mlp_train_step(vf_mlp* h, const void* dev_x, const float* dev_y, uint64_t
     cudaMemsetAsync(h->d.loss, 0, 4, st);
     k_loss<<<blocks_for(n), 32 * WARPS, 0, st>>>(h->d, (const __half*)dev_x, dev_y, (int)n, 1.0f / (float)n);
   }
-  k_backward<<<std::min(blocks_for(n), (unsigned)h->ctas), 32 * WARPS, 0, st>>>(h->d, (const __half*)dev_x, dev_y, (int)n, 1.0f / (float)n, nullptr);
+  k_backward<<<std::min(blocks_for(n), (unsigned)h->ctas), 32 * WARPS, sizeof(BackSmem), st>>>(h->d, (const __half*)dev_x, dev_y, (int)n, 1.0f / (float)n, nullptr);
   h->step += 1;
   const float b1 = 0.9f, b2 = 0.999f;
   const float c1 = 1.f - std::pow(b1, (float)h->step), c2 = 1.f - std::pow(b2, (float)h->step);
