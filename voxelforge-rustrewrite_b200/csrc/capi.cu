@@ -495,7 +495,7 @@ int vf_fluid_apply_voxel_edits(vf_fluid* h, const vf_voxel* edits, uint64_t n) {
   CK(cudaMemcpyAsync(h->scratch, q.data(), n * 16, cudaMemcpyHostToDevice, h->stream));
   for (uint64_t o = 0; o < n; o += 1u << 30) {  // (positions in the list are 32-bit)
     const unsigned m = (unsigned)std::min<uint64_t>(n - o, 1u << 30);
-    k_voxel_edits<<<1, EDIT_THREADS, 0, h->stream>>>(h->R, (const int4*)h->scratch + o, m, h->tune.spin_cap);
+    k_voxel_edits<<<1, EDIT_THREADS, 0, h->stream>>>(h->R, (const int4*)h->scratch + o, m);
     CK(cudaGetLastError());
   }
   return sync_ctl(h);
@@ -517,8 +517,8 @@ int vf_fluid_wake(vf_fluid* h, int32_t x0, int32_t y0, int32_t z0, int32_t x1, i
 // The kernel of an edit over a list in device memory: emitters and carving run in parallel, what may
 // displace water one cell after another.
 static cudaError_t launch_edit(vf_fluid* h, int kind, const int* dev_xyz, uint64_t n, int m, float amount, unsigned long long* dcount) {
-  if (kind == ED_EMIT) k_emit<<<1, EDIT_THREADS, 0, h->stream>>>(h->R, dev_xyz, n, amount, h->tune.spin_cap);
-  else if (kind == ED_BRUSH && m == 0) k_carve<<<1, EDIT_THREADS, 0, h->stream>>>(h->R, dev_xyz, n, dcount, h->tune.spin_cap);
+  if (kind == ED_EMIT) k_emit<<<1, EDIT_THREADS, 0, h->stream>>>(h->R, dev_xyz, n, amount);
+  else if (kind == ED_BRUSH && m == 0) k_carve<<<1, EDIT_THREADS, 0, h->stream>>>(h->R, dev_xyz, n, dcount);
   else k_edit<<<1, 32, 0, h->stream>>>(h->R, kind, dev_xyz, n, m, amount, dcount);
   return cudaGetLastError();
 }

@@ -129,7 +129,7 @@ __device__ void cta_radix_sort(unsigned* keys, unsigned* tmp, unsigned n, unsign
 // Launch-time knobs of the tick (results do not depend on them).
 struct Tune {
   int gate;       // bits 16-20: warps of the region's CTA (0: MAX_WARPS); the other bits are unused
-  unsigned long long spin_cap;  // rounds of the sweep, and iterations of any wait, before the tick gives up (ST_TIMEOUT)
+  unsigned long long spin_cap;  // rounds of the sweep before the tick gives up (ST_TIMEOUT)
 };
 
 struct TickSmem {
@@ -554,7 +554,7 @@ __device__ __noinline__ void sweep_levels(const Region& Rs, TickSmem& sm, WS& sW
     R.ctl->par_rollbacks += L.n_again;
     R.ctl->par_replayed += L.n_searches;
   }
-  sweep_flush(R, L, n, cap);
+  sweep_flush(R, L, n);
   // ---- the position map back to idle
   for (unsigned i = tid; i < n; i += NT_) R.stamp[key_to_id(R, R.cells[i], flip)] = 0xFFFFFFFFu;
   // ---- the cells' events in sorted order -> the tick's event logs (program order)
@@ -788,6 +788,42 @@ __device__ void cta_minmax(float& lo, float& hi) {
   __syncthreads();
 }
 
+// Cells of levelled layers, one per thread in order: each takes its layer's average (fluid.rs:457-470).
+// Returns the thread's change in partial entries. All threads.
+__device__ __forceinline__ int level_write(const Region& R, TickSmem& sm, WS& sW, const int* ring, bool has, unsigned id, float avg) {
+  int x = 0, y = 0, z = 0;
+  bool wv = false;
+  CD c = CD{0.0f, NOSLOT, 0u, 0, true};
+  if (has) {
+    dom_xyz(R, id, x, y, z);
+    c = load_cell_par(R, ring, x, y, z);
+    wv = fabsf(__fsub_rn(cd_volume(c), avg)) > 1e-6f;
+  }
+  materialize_cta(R, wv && set_volume_needs_slot(c, avg), c.gi, c.slot);
+  bool ch = false;
+  int pd = 0;
+  if (wv) {
+    const SVPlan p = sv_plan(c.part, c.mat, c.slot != NOSLOT, avg);
+    if (c.slot != NOSLOT) sv_apply(R, c, id, local_index(x, y, z), p);
+    ch = p.ch;
+    pd = p.dp;
+  }
+  unsigned tot;
+  const unsigned off = cta_scan(sm, ch, &tot);
+  if (ch) {
+    const unsigned pos = sW.nchg + off;
+    if (pos < R.ev_chg_cap) R.ev_chg[pos] = id;
+    else set_status(R, ST_OOM, 9);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    sW.nchg += tot;
+    if (tot) sW.changed = true;
+  }
+  __syncthreads();
+  return pd;
+}
+
 // What FluidSim::level_layer does with a gathered layer of len cells (fluid.rs:430-485), over the
 // CTA. The f64 sum in queue order is formed exactly whenever every partial sum is representable:
 // all volumes are multiples of 2^L (L from the smallest, lo) and every partial sum is below
@@ -796,7 +832,7 @@ __device__ void cta_minmax(float& lo, float& hi) {
 // average writes each cell once, in parallel, the change log in cell order; the drain branch
 // (`left` runs through the cells in order) and layers left as they are go to warp 0's
 // level_finish.
-__device__ __noinline__ void level_finish_cta(const Region& R, TickSmem& sm, WS& sW, Smem& S, unsigned len, unsigned long long cap) {
+__device__ __noinline__ void level_finish_cta(const Region& R, TickSmem& sm, WS& sW, Smem& S, unsigned len) {
   __shared__ double s_sum;
   const unsigned tid = threadIdx.x;
   float lo = 2.0f, hi = -1.0f;
@@ -847,38 +883,7 @@ __device__ __noinline__ void level_finish_cta(const Region& R, TickSmem& sm, WS&
   long long pd = 0;
   for (unsigned base = 0; base < len; base += NT_) {
     const unsigned k = base + tid;
-    bool wv = false;
-    int x = 0, y = 0, z = 0;
-    unsigned id = 0;
-    CD c = CD{0.0f, NOSLOT, 0u, 0, true};
-    if (k < len) {
-      id = R.lvl_id[k];
-      dom_xyz(R, id, x, y, z);
-      c = load_cell_par(R, S.ring, x, y, z, cap);
-      wv = fabsf(__fsub_rn(cd_volume(c), avg)) > 1e-6f;
-    }
-    const bool need = wv && set_volume_needs_slot(c, avg);
-    if (__any_sync(FULLMASK, need)) materialize_par(R, need, c.gi, c.slot, cap);
-    bool ch = false;
-    if (wv) {
-      const SVPlan p = sv_plan(c.part, c.mat, c.slot != NOSLOT, avg);
-      if (c.slot != NOSLOT) sv_apply(R, c, id, local_index(x, y, z), p);
-      ch = p.ch;
-      pd += p.dp;
-    }
-    unsigned tot;
-    const unsigned off = cta_scan(sm, ch, &tot);
-    if (ch) {
-      const unsigned pos = sW.nchg + off;
-      if (pos < R.ev_chg_cap) R.ev_chg[pos] = id;
-      else set_status(R, ST_OOM, 9);
-    }
-    __syncthreads();
-    if (tid == 0) {
-      sW.nchg += tot;
-      if (tot) sW.changed = true;
-    }
-    __syncthreads();
+    pd += level_write(R, sm, sW, S.ring, k < len, k < len ? R.lvl_id[k] : 0u, avg);
   }
   const long long dp = (long long)cta_sum(sm, (unsigned long long)pd);
   if (tid == 0) {
@@ -985,8 +990,8 @@ __device__ void level_fill_small(const Region& R, LevelFill& F, unsigned sid) {
   __syncwarp();
 }
 
-// What a small layer's fill leaves behind, one warp: its marks, and the cells at their average.
-__device__ void level_commit_small(const Region& R, WS& sW, const int* ring, const LevelFill& F, unsigned long long cap, int& pd, unsigned& chg) {
+// The marks a small layer's fill leaves behind, one warp.
+__device__ __forceinline__ void level_mark_small(const Region& R, const LevelFill& F) {
   const unsigned lane = lane_id();
   for (unsigned t = lane; t < FILL_SLOTS; t += 32u) {
     if (F.key[t] == EMPTY_ID) continue;
@@ -994,33 +999,6 @@ __device__ void level_commit_small(const Region& R, WS& sW, const int* ring, con
     dom_xyz(R, F.key[t], x, y, z);
     mark_tas(R, x, y, z);
   }
-  if (F.kind == FK_LEVEL) {
-    for (unsigned b0 = 0; b0 < F.len; b0 += 32u) {
-      const unsigned k = b0 + lane;
-      int x = 0, y = 0, z = 0;
-      bool wv = false;
-      CD c = CD{0.0f, NOSLOT, 0u, 0, true};
-      if (k < F.len) {
-        dom_xyz(R, F.id[k], x, y, z);
-        c = load_cell_par(R, ring, x, y, z, cap);
-        wv = fabsf(__fsub_rn(cd_volume(c), F.avg)) > 1e-6f;
-      }
-      const bool need = wv && set_volume_needs_slot(c, F.avg);
-      if (__any_sync(FULLMASK, need)) materialize_par(R, need, c.gi, c.slot, cap);
-      if (wv) {
-        const SVPlan p = sv_plan(c.part, c.mat, c.slot != NOSLOT, F.avg);
-        if (c.slot != NOSLOT) sv_apply(R, c, F.id[k], local_index(x, y, z), p);
-        pd += p.dp;
-        if (p.ch) {
-          const unsigned pos = atomicAdd(&sW.nchg, 1u);
-          if (pos < R.ev_chg_cap) R.ev_chg[pos] = F.id[k];
-          else set_status(R, ST_OOM, 9);
-          chg = 1u;
-        }
-      }
-    }
-  }
-  __syncwarp();
 }
 
 // FluidSim::level_surfaces (fluid.rs:489-507) from sW.llc on, over the CTA, in batches of up to one
@@ -1037,7 +1015,7 @@ __device__ void level_commit_small(const Region& R, WS& sW, const int* ring, con
 // 57 M SM cycles one after another.) The popped seeds leave the seed set and their starts are
 // marked (a start that is not a member is marked, and skipped by every later flood fill, either
 // way). sW.level_round is updated at the end.
-__device__ __noinline__ void level_round_cta(const Region& R, TickSmem& sm, WS& sW, Smem& S, unsigned long long cap) {
+__device__ __noinline__ void level_round_cta(const Region& R, TickSmem& sm, WS& sW, Smem& S) {
   __shared__ unsigned s_ns, s_stop, s_brk, s_pend, s_qi, s_ql, s_cur, s_m, s_group[MAX_WARPS];
   LevelFill* const fills = reinterpret_cast<LevelFill*>(sm.u.x.fills);  // the sweep's shared memory is free now
   static_assert(sizeof(LevelFill) * MAX_WARPS <= sizeof(sm.u.x.fills) && sizeof(sm.u.x) <= sizeof(LvSmem), "level fills");
@@ -1156,11 +1134,22 @@ __device__ __noinline__ void level_round_cta(const Region& R, TickSmem& sm, WS& 
         }
         __syncthreads();
         const unsigned done = s_m;
+        if (w < done && fills[w].kind != FK_DUP) level_mark_small(R, fills[w]);
+        // the cells of the layers that are levelled, in order, one per thread
         int pd = 0;
-        unsigned chg = 0;
-        if (w < done && fills[w].kind != FK_DUP) level_commit_small(R, sW, S.ring, fills[w], cap, pd, chg);
+        for (unsigned base = 0;; base += NT_) {
+          unsigned k = base + tid, f = 0, total = 0;
+          for (unsigned o = 0; o < done; ++o) {
+            const unsigned l = fills[o].kind == FK_LEVEL ? fills[o].len : 0u;
+            total += l;
+            if (k >= total) f = o + 1u;
+            else if (f == o) k -= total - l;
+          }
+          if (base >= total) break;
+          const bool has = base + tid < total;
+          pd += level_write(R, sm, sW, S.ring, has, has ? fills[f].id[k] : 0u, has ? fills[f].avg : 0.0f);
+        }
         if (pd) atomicAdd(reinterpret_cast<unsigned long long*>(&sW.pdelta), (unsigned long long)(long long)pd);
-        if (chg) *(volatile bool*)&sW.changed = true;
         __syncthreads();
         if (done) {  // the group's starts, and the later ones its fills marked
           for (unsigned c = cur + tid; c < nc; c += NT_) {
@@ -1195,7 +1184,7 @@ __device__ __noinline__ void level_round_cta(const Region& R, TickSmem& sm, WS& 
       __syncthreads();
       if (s_pend) {
         const unsigned len = level_bfs_cta(R, sm, S, s_qi, s_ql);
-        level_finish_cta(R, sm, sW, S, len, cap);
+        level_finish_cta(R, sm, sW, S, len);
       }
       // the later candidates this layer's flood fill marked
       for (unsigned c = cur + 1u + tid; c < nc; c += NT_) {
@@ -1358,7 +1347,7 @@ __device__ void run_ticks(const Region& R, TickSmem& sm, int n_ticks, Tune tune)
       Smem S{ring};
       if (tid == 0) sW.llc = 0;
       __syncthreads();
-      level_round_cta(R, sm, sW, S, tune.spin_cap);
+      level_round_cta(R, sm, sW, S);
       if (tid == 0) s_clear = sW.level_round ? 0u : 1u;
     }
     __syncthreads();
@@ -1614,7 +1603,7 @@ __device__ unsigned brush_warp(const Region& R, WS& W, const int* ring, int x, i
 // brick a slot, and the winners store. A warp going through the list one write after another spent
 // ~1.5 us on each (16,000 writes 24 ms; here 0.1 ms).
 constexpr int EDIT_THREADS = 1024;
-__global__ void __launch_bounds__(EDIT_THREADS) k_voxel_edits(Region R, const int4* edits, unsigned n, unsigned long long cap) {
+__global__ void __launch_bounds__(EDIT_THREADS) k_voxel_edits(Region R, const int4* edits, unsigned n) {
   const unsigned nt = blockDim.x;
   for (unsigned base = 0; base < n; base += nt) {
     const unsigned i = base + threadIdx.x;
@@ -1628,11 +1617,11 @@ __global__ void __launch_bounds__(EDIT_THREADS) k_voxel_edits(Region R, const in
     CD c = CD{0.0f, NOSLOT, 0u, 0, true};
     if (i < n) {
       e = edits[i];
-      c = load_cell_par(R, R.ring, e.x, e.y, e.z, cap);
+      c = load_cell_par(R, R.ring, e.x, e.y, e.z);
     }
     const bool differs = !c.out && c.mat != (unsigned char)e.w;
     unsigned slot = c.slot;
-    materialize_par(R, differs && slot == NOSLOT, c.gi, slot, cap);
+    materialize_cta(R, differs && slot == NOSLOT, c.gi, slot);
     if (differs && slot != NOSLOT) record_change(R, dom_id(R, e.x, e.y, e.z));
   }
   __syncthreads();
@@ -1643,7 +1632,7 @@ __global__ void __launch_bounds__(EDIT_THREADS) k_voxel_edits(Region R, const in
     if (outside(R, R.ring, e.x, e.y, e.z)) continue;
     const unsigned id = dom_id(R, e.x, e.y, e.z);
     if (__ldcg(R.rb + id) != n - 1u - i) continue;  // set by atomics (in L2): read past L1
-    const CD c = load_cell_par(R, R.ring, e.x, e.y, e.z, cap);
+    const CD c = load_cell_par(R, R.ring, e.x, e.y, e.z);
     if (c.slot != NOSLOT) {
       R.amat[(size_t)c.slot * 512u + local_index(e.x, e.y, e.z)] = (unsigned char)e.w;
       dense_put(R, id, (unsigned)e.w & 255u, c.part);
@@ -1670,7 +1659,7 @@ __device__ __forceinline__ unsigned edit_scan(unsigned* cnt, bool f, unsigned* t
 // activate it), one CTA. Cells of the list that differ do not touch each other, so a chunk of 1024
 // runs at once; a cell listed again in the chunk waits for its earlier entry (claims in rb) and the
 // activations join the FIFO in list order by a scan. One warp in order spent ~1.6 us per emitter.
-__global__ void __launch_bounds__(EDIT_THREADS) k_emit(Region R, const int* xyz, unsigned long long n, float amount, unsigned long long cap) {
+__global__ void __launch_bounds__(EDIT_THREADS) k_emit(Region R, const int* xyz, unsigned long long n, float amount) {
   __shared__ unsigned cnt[32];
   __shared__ int s_pd, s_ch;
   const unsigned tid = threadIdx.x;
@@ -1687,7 +1676,7 @@ __global__ void __launch_bounds__(EDIT_THREADS) k_emit(Region R, const int* xyz,
       x = xyz[3 * i];
       y = xyz[3 * i + 1];
       z = xyz[3 * i + 2];
-      pend = !cd_solid(load_cell_par(R, R.ring, x, y, z, cap));  // a cell's solidity does not change here
+      pend = !cd_solid(load_cell_par(R, R.ring, x, y, z));  // a cell's solidity does not change here
       if (pend) id = dom_id(R, x, y, z);
     }
     bool act = false;
@@ -1700,11 +1689,11 @@ __global__ void __launch_bounds__(EDIT_THREADS) k_emit(Region R, const int* xyz,
       CD c = CD{0.0f, NOSLOT, 0u, 0, true};
       float nv = 0.0f;
       if (win) {
-        c = load_cell_par(R, R.ring, x, y, z, cap);
+        c = load_cell_par(R, R.ring, x, y, z);
         nv = fminf(1.0f, __fadd_rn(cd_volume(c), amount));
       }
       const bool need = win && set_volume_needs_slot(c, nv);
-      if (__any_sync(FULLMASK, need)) materialize_par(R, need, c.gi, c.slot, cap);
+      materialize_cta(R, need, c.gi, c.slot);
       if (win) {
         const SVPlan p = sv_plan(c.part, c.mat, c.slot != NOSLOT, nv);
         if (c.slot != NOSLOT) sv_apply(R, c, id, local_index(x, y, z), p);
@@ -1741,7 +1730,7 @@ __global__ void __launch_bounds__(EDIT_THREADS) k_emit(Region R, const int* xyz,
 // apply_brush with an empty material (src/edit/brush.rs:93-111), one CTA: every listed solid voxel
 // becomes air, once. Nothing is displaced or woken, so the list has no order to keep; the voxels are
 // claimed (rb) so that one listed twice counts once.
-__global__ void __launch_bounds__(EDIT_THREADS) k_carve(Region R, const int* xyz, unsigned long long n, unsigned long long* out_count, unsigned long long cap) {
+__global__ void __launch_bounds__(EDIT_THREADS) k_carve(Region R, const int* xyz, unsigned long long n, unsigned long long* out_count) {
   __shared__ unsigned s_n;
   const unsigned tid = threadIdx.x;
   if (tid == 0) s_n = 0u;
@@ -1756,7 +1745,7 @@ __global__ void __launch_bounds__(EDIT_THREADS) k_carve(Region R, const int* xyz
       x = xyz[3 * i];
       y = xyz[3 * i + 1];
       z = xyz[3 * i + 2];
-      c = load_cell_par(R, R.ring, x, y, z, cap);
+      c = load_cell_par(R, R.ring, x, y, z);
       hit = !c.out && c.mat != 0 && c.mat != WATER;
     }
     if (hit) {
@@ -1767,7 +1756,7 @@ __global__ void __launch_bounds__(EDIT_THREADS) k_carve(Region R, const int* xyz
     const bool win = hit && __ldcg(R.rb + id) == tid;  // set by atomics (in L2): read past L1
     __syncthreads();
     const bool need = win && c.slot == NOSLOT;
-    if (__any_sync(FULLMASK, need)) materialize_par(R, need, c.gi, c.slot, cap);
+    materialize_cta(R, need, c.gi, c.slot);
     if (win) {
       if (c.slot != NOSLOT) {
         R.amat[(size_t)c.slot * 512u + local_index(x, y, z)] = 0;

@@ -32,7 +32,7 @@
 
 namespace vfe {
 
-constexpr unsigned GRID_LOCKED = 0xFFFFFFFFu;  // grid word while a warp materialises the brick
+constexpr unsigned GRID_CLAIM = 0x80000000u;   // grid word while a CTA gives out slots: | writer's key << 8 | uniform value
 constexpr int MAX_WARPS = 16;                  // warps of a CTA running the sweep
 constexpr unsigned SOLO_CELLS = 4;             // a list this short is run by one warp (eight lanes per cell)
 constexpr unsigned SOLO_ENTRIES = 6;           // queue entries one warp examines per search round
@@ -122,29 +122,7 @@ __device__ __forceinline__ unsigned gld(const unsigned* p) {
   return v;
 }
 
-// Back-off of a polling loop after n polls: a few polls at full rate, then sleeps of up to 1 us.
-__device__ __forceinline__ void backoff(unsigned long long n) {
-  if (n > 4) __nanosleep(min(32u << (unsigned)min((n - 4) >> 2, 5ull), 1024u));
-}
-
-// The grid word of a brick, past a lock another warp holds while it materialises it (a lock's holder
-// waits for nobody, so the wait is short; it is bounded all the same).
-__device__ __forceinline__ unsigned grid_word(const Region& R, unsigned gi, unsigned long long cap) {
-  unsigned g = gld(R.grid + gi);
-  unsigned long long spins = 0;
-  while (g == GRID_LOCKED) {
-    if (++spins > cap) {
-      set_status(R, ST_TIMEOUT, 30);
-      return 0u;
-    }
-    backoff(spins);
-    g = gld(R.grid + gi);
-  }
-  __threadfence_block();
-  return g;
-}
-
-__device__ __forceinline__ CD load_cell_par(const Region& R, const int* ring, int x, int y, int z, unsigned long long cap) {
+__device__ __forceinline__ CD load_cell_par(const Region& R, const int* ring, int x, int y, int z) {
   CD c;
   c.part = 0.0f;
   c.slot = NOSLOT;
@@ -153,7 +131,7 @@ __device__ __forceinline__ CD load_cell_par(const Region& R, const int* ring, in
   c.out = outside(R, ring, x, y, z);
   if (c.out) return c;
   c.gi = grid_index(R, x >> 3, y >> 3, z >> 3);
-  const unsigned g = grid_word(R, c.gi, cap);
+  const unsigned g = gld(R.grid + c.gi);
   if (g < 256u) {
     c.mat = (unsigned char)g;
     return c;
@@ -165,10 +143,11 @@ __device__ __forceinline__ CD load_cell_par(const Region& R, const int* ring, in
   return c;
 }
 
-// Atlas slots for the bricks lanes with `need` are about to write (sparse_volume.rs:250-266), warp-
-// collective. The first warp to take a brick's grid word (CAS to GRID_LOCKED) allocates and fills the
-// slot and publishes it; the others read the published slot. A warp publishes every brick it has
-// locked before it waits for one, so two warps never wait for each other.
+// Atlas slots for the bricks a CTA's threads are about to write first (sparse_volume.rs:250-266): bit q of
+// `mask` names brick gi[q]. Slots are given out in the order of the writes (thread, then q), which is
+// the program's order where the callers pass cells in it: whatever follows the slots' order (the rows
+// of the proposal's features) is the same in every run. A brick goes to its first writer, found by an
+// atomic minimum in the grid word itself. All threads; callers skip it when nothing is needed.
 // (By value: a Region behind a reference would keep the caller's copy out of registers.)
 struct AtlasRef {
   unsigned* grid;
@@ -177,65 +156,80 @@ struct AtlasRef {
   Ctl* ctl;
   unsigned atlas_cap;
 };
-__device__ __noinline__ unsigned materialize_warp(AtlasRef R, bool need, unsigned gi, unsigned slot, unsigned long long cap) {
-  const unsigned lane = lane_id();
-  const unsigned key = need ? gi : (0xFFFFFFFFu - lane);
-  const unsigned peers = __match_any_sync(FULLMASK, key);
-  bool open = need && !(peers & lanemask_lt());
-  unsigned s = NOSLOT;
-  unsigned long long spins = 0;
-  while (__any_sync(FULLMASK, open)) {
-    unsigned g = 0;
-    bool fill = false;
-    if (open) {
-      g = gld(R.grid + gi);
-      if (g < 256u) {
-        if (atomicCAS(R.grid + gi, g, GRID_LOCKED) == g) {
-          s = atomicAdd(&R.ctl->atlas_used, 1u);
-          if (s >= R.atlas_cap) {
-            if (atomicCAS(&R.ctl->status, 0, ST_OOM) == 0) R.ctl->err_info = 1;
-            atomicExch(R.grid + gi, g);
-            s = NOSLOT;
-            open = false;
-          } else {
-            fill = true;
-          }
-        }
-      } else if (g != GRID_LOCKED) {
-        s = g - 256u;
-        open = false;
-      } else if (++spins > cap) {
-        if (atomicCAS(&R.ctl->status, 0, ST_TIMEOUT) == 0) R.ctl->err_info = 31;
-        open = false;
-      } else {
-        backoff(spins);
-      }
+template <int K>
+__device__ __noinline__ void give_slots(AtlasRef R, unsigned mask, const unsigned (&gi)[K]) {
+  __shared__ unsigned s_cnt[32], s_base;
+  const unsigned tid = threadIdx.x, lane = lane_id(), warp = tid >> 5, nw = blockDim.x >> 5;
+  static_assert(1024 * K <= 1 << 23, "keys fit the grid word");
+  __syncthreads();  // nobody reads the grid any more
+#pragma unroll
+  for (int q = 0; q < K; ++q) {
+    if (!((mask >> q) & 1u)) continue;
+    unsigned* gp = R.grid + gi[q];
+    unsigned g = __ldcg(gp);
+    while (g < 256u || g >= GRID_CLAIM) {
+      const unsigned mine = GRID_CLAIM | (tid * K + q) << 8 | (g & 255u);
+      if (g >= GRID_CLAIM && g <= mine) break;
+      const unsigned old = atomicCAS(gp, g, mine);
+      if (old == g) break;
+      g = old;
     }
-    for (unsigned m = __ballot_sync(FULLMASK, fill); m; m &= m - 1) {
+  }
+  __syncthreads();
+  unsigned win = 0, fill[K];
+#pragma unroll
+  for (int q = 0; q < K; ++q) {
+    fill[q] = 0;
+    if (!((mask >> q) & 1u)) continue;
+    const unsigned g = __ldcg(R.grid + gi[q]);
+    if (g < GRID_CLAIM || (g & ~GRID_CLAIM) >> 8 != tid * K + q) continue;
+    win |= 1u << q;
+    fill[q] = g & 255u;
+  }
+  const unsigned k = (unsigned)__popc(win);
+  unsigned pre = k;
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned v = __shfl_up_sync(FULLMASK, pre, o);
+    if (lane >= (unsigned)o) pre += v;
+  }
+  if (lane == 31u) s_cnt[warp] = pre;
+  __syncthreads();
+  const unsigned c = lane < nw ? s_cnt[lane] : 0u;
+  const unsigned before = __reduce_add_sync(FULLMASK, lane < warp ? c : 0u), total = __reduce_add_sync(FULLMASK, c);
+  if (tid == 0) s_base = atomicAdd(&R.ctl->atlas_used, total);
+  __syncthreads();
+  unsigned next = s_base + before + pre - k;
+#pragma unroll
+  for (int q = 0; q < K; ++q) {
+    const bool w = (win >> q) & 1u;
+    const unsigned s = w ? next++ : NOSLOT;
+    const bool ok = w && s < R.atlas_cap;
+    if (w && !ok) {
+      if (atomicCAS(&R.ctl->status, 0, ST_OOM) == 0) R.ctl->err_info = 1;
+      atomicExch(R.grid + gi[q], fill[q]);
+    }
+    for (unsigned m = __ballot_sync(FULLMASK, ok); m; m &= m - 1) {
       const int l = __ffs(m) - 1;
       const unsigned sl = __shfl_sync(FULLMASK, s, l);
-      unsigned fv = __shfl_sync(FULLMASK, g, l) & 255u;
-      fv |= fv << 8;
-      fv |= fv << 16;
+      const unsigned fv = __shfl_sync(FULLMASK, fill[q], l) * 0x01010101u;
       reinterpret_cast<uint4*>(R.amat + (size_t)sl * 512u)[lane] = make_uint4(fv, fv, fv, fv);
       uint4* vv = reinterpret_cast<uint4*>(R.avol + (size_t)sl * 512u);
 #pragma unroll
-      for (int k = 0; k < 4; ++k) vv[lane + 32 * k] = make_uint4(0, 0, 0, 0);
+      for (int p = 0; p < 4; ++p) vv[lane + 32 * p] = make_uint4(0, 0, 0, 0);
     }
-    __syncwarp();
-    __threadfence_block();
-    if (fill) {
-      atomicExch(R.grid + gi, 256u + s);
-      open = false;
-    }
+    if (ok) atomicExch(R.grid + gi[q], 256u + s);
   }
-  const int src = need ? (__ffs(peers) - 1) : (int)lane;
-  const unsigned s2 = __shfl_sync(FULLMASK, s, src);
-  __syncwarp();
-  return need ? s2 : slot;
+  __syncthreads();
 }
-__device__ __forceinline__ void materialize_par(const Region& R, bool need, unsigned gi, unsigned& slot, unsigned long long cap) {
-  slot = materialize_warp(AtlasRef{R.grid, R.amat, R.avol, R.ctl, R.atlas_cap}, need, gi, slot, cap);
+// The same for one brick a thread, and the slot it got. All threads.
+__device__ __forceinline__ void materialize_cta(const Region& R, bool need, unsigned gi, unsigned& slot) {
+  if (!__syncthreads_or(need)) return;
+  const unsigned a[1] = {gi};
+  give_slots<1>(AtlasRef{R.grid, R.amat, R.avol, R.ctl, R.atlas_cap}, need ? 1u : 0u, a);
+  if (need) {
+    const unsigned g = __ldcg(R.grid + gi);
+    slot = g >= 256u ? g - 256u : NOSLOT;
+  }
 }
 
 // FluidSim::set_volume (fluid.rs:327-355) split into the decision and the stores.
@@ -448,45 +442,64 @@ __device__ __forceinline__ float lv_cells(const Region& R, LvSmem& L, const Lane
   return vol;
 }
 
-// The atlas entry of a cell the sweep wrote, warp-collective: its brick gets a slot (sparse_volume.rs:
-// 250-266) and the dense word's material and volume.
-__device__ __forceinline__ void flush_cell(const Region& R, bool w, unsigned id, unsigned long long cap) {
-  int x = 0, y = 0, z = 0;
-  unsigned slot = NOSLOT, gi = 0, u = 0;
-  if (w) {
-    dom_xyz(R, id, x, y, z);
-    u = R.dense[id];
-    gi = grid_index(R, x >> 3, y >> 3, z >> 3);
-    const unsigned g = grid_word(R, gi, cap);
-    if (g >= 256u) slot = g - 256u;
-  }
-  if (__any_sync(FULLMASK, w && slot == NOSLOT)) materialize_par(R, w && slot == NOSLOT, gi, slot, cap);
-  if (w && slot != NOSLOT) {
-    const size_t o = (size_t)slot * 512u + local_index(x, y, z);
-    const float v = dc_volume(u);
-    R.avol[o] = v < 1.0f ? v : 0.0f;
-    R.amat[o] = (int)u > 0 ? WATER : (unsigned char)0;
-  }
-}
-
 // After the sweep: every cell it wrote (the slots in the dependency bytes, the pulls' sources) to the
-// atlas, all at once. All threads.
-__device__ __forceinline__ void sweep_flush(const Region& R, const LvSmem& L, unsigned n, unsigned long long cap) {
-  for (unsigned base = threadIdx.x & ~31u; base < n; base += blockDim.x) {
-    const unsigned i = base + lane_id();
-    unsigned m = 0, cid = 0, src = NOSLOT;
+// atlas, all at once, in batches of one drained cell per thread in sorted order. Bricks written for
+// the first time get their slots in the program's order (a pull's source before its cell). All threads.
+__device__ __forceinline__ void sweep_flush(const Region& R, const LvSmem& L, unsigned n) {
+  for (unsigned base = 0; base < n; base += blockDim.x) {
+    const unsigned i = base + threadIdx.x;
+    unsigned w = 0, need = 0;  // entry 0: the source, 1 + l: slot l (never 2, the cell above)
+    unsigned gi[8], g[8], u[8], at[8];  // brick, its grid word, the dense word, the cell in its brick
     if (i < n) {
-      m = dep_byte(L, i) & 0x7Fu;
-      if (R.lv_ev[i] & 1u) src = R.lv_src[i];
-      if (m) cid = R.lv[i].cid;
+      w = (dep_byte(L, i) & 0x7Fu) << 1 | (R.lv_ev[i] & 1u);
+      if (w) {
+        const unsigned cid = R.lv[i].cid, sid = (w & 1u) ? R.lv_src[i] : cid;
+        int x, y, z;
+        dom_xyz(R, cid, x, y, z);
+        const unsigned gc = grid_index(R, x >> 3, y >> 3, z >> 3), gw = gld(R.grid + gc);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          if (q == 3 || !((w >> q) & 1u)) continue;
+          int ax, ay, az;
+          unsigned id = sid;
+          if (q == 0) {
+            dom_xyz(R, sid, ax, ay, az);
+          } else {
+            fp_off(q - 1, ax, ay, az);
+            id = (unsigned)((int)cid + fp_id(R, q - 1));
+            ax += x;
+            ay += y;
+            az += z;
+          }
+          u[q] = R.dense[id];
+          gi[q] = gc;
+          g[q] = gw;
+          if (((ax ^ x) | (ay ^ y) | (az ^ z)) & ~7) {  // another brick
+            gi[q] = grid_index(R, ax >> 3, ay >> 3, az >> 3);
+            g[q] = gld(R.grid + gi[q]);
+          }
+          at[q] = local_index(ax, ay, az);
+          need |= g[q] < 256u ? 1u << q : 0u;
+        }
+      }
+    }
+    if (__syncthreads_or(need != 0u)) {
+      unsigned a[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) a[q] = gi[q];
+      give_slots<8>(AtlasRef{R.grid, R.amat, R.avol, R.ctl, R.atlas_cap}, need, a);
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        if ((need >> q) & 1u) g[q] = __ldcg(R.grid + gi[q]);
     }
 #pragma unroll
-    for (int l = 0; l < 7; ++l) {
-      if (l == 2) continue;
-      const bool w = (m >> l) & 1u;
-      if (__any_sync(FULLMASK, w)) flush_cell(R, w, (unsigned)((int)cid + fp_id(R, l)), cap);
+    for (int q = 0; q < 8; ++q) {
+      if (q == 3 || !((w >> q) & 1u) || g[q] < 256u) continue;  // (no slot left: the status says so)
+      const size_t o = (size_t)(g[q] - 256u) * 512u + at[q];
+      const float v = dc_volume(u[q]);
+      R.avol[o] = v < 1.0f ? v : 0.0f;
+      R.amat[o] = (int)u[q] > 0 ? WATER : (unsigned char)0;
     }
-    if (__any_sync(FULLMASK, src != NOSLOT)) flush_cell(R, src != NOSLOT, src, cap);
   }
 }
 
