@@ -274,13 +274,6 @@ __device__ __forceinline__ void activate_round(const Region& R, WS& W, bool vali
 // Activation-log word: the cell id, bit 31 set for a wake_around centre (7 cells).
 constexpr unsigned ACT_AROUND = 0x80000000u;
 
-// D of pressure_pull (fluid.rs:512): up, +x, -x, +z, -z.
-__device__ __forceinline__ void dir5(int d, int& dx, int& dy, int& dz) {
-  dx = (d == 1) - (d == 2);
-  dy = (d == 0);
-  dz = (d == 3) - (d == 4);
-}
-
 // ------------------------------------------------------------------------ level fill
 // LayerMarks::test_and_set (fluid.rs:194-200): one bit per cell in 64x64 tiles per layer; the
 // tiles touched during a levelling round are listed so the round's end clears only those.

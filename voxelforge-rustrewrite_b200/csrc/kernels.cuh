@@ -484,6 +484,7 @@ __device__ __noinline__ void sweep_levels(const Region& Rs, TickSmem& sm, WS& sW
   plap(0);
   // ---- rounds
   const LaneSlot ls = lane_slot(R);
+  unsigned unused = 0;
   long long t_wide = 0, t_search = 0;
   while (true) {
     // warp 0 alone decides what comes next: nobody else reads the lists' state while it runs
@@ -520,7 +521,7 @@ __device__ __noinline__ void sweep_levels(const Region& Rs, TickSmem& sm, WS& sW
         for (unsigned t0 = warp * 4u; t0 < fcount; t0 += NW_ * 4u) {
           const unsigned t = t0 + (lane >> 3);
           const unsigned i = t < fcount ? list_get(R, L, cur, t) : 0u;
-          lv_cells(R, L, ls, t < fcount && !cell_done(L, i), i, false, 0.0f, 0u, gate, kp, nb, nc, pb, pd);
+          lv_cells<false>(R, L, ls, t < fcount && !cell_done(L, i), i, false, 0.0f, 0u, gate, kp, nb, nc, unused, pb, unused, pd);
         }
         __syncthreads();
         cur = nb;

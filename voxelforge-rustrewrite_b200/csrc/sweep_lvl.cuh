@@ -44,6 +44,7 @@ constexpr unsigned VIS_RANKS = 4096;           // ranks of one search: 6 + 5 * 5
 constexpr unsigned NGROUPS = (MAX_CELLS_PER_TICK + 31) / 32;
 constexpr unsigned LIST_CAP = 2048;   // a round's list kept in shared memory; the rest goes to global
 constexpr unsigned NOSUCC = 0xFFFFu;
+static_assert(SOLO_CELLS <= LIST_CAP, "a short list is in shared memory");
 static_assert(MAX_CELLS_PER_TICK < NOSUCC, "sorted positions fit 16 bits");
 constexpr unsigned DONE = 0x80u;           // dependency byte of a finished cell: DONE | the footprint slots it wrote
 constexpr int GATE_MAX = 31;               // range of the gate knob's radii (accepted, unused)
@@ -67,8 +68,7 @@ struct __align__(16) LvOld {
 // The pressure search under way.
 enum SearchStatus { SS_NONE = 0, SS_SUCCESS = 1, SS_BLOCKED = 2, SS_MORE = 3 };
 struct Search {
-  unsigned q[PRESSURE_SEARCH];  // queued cells, relative to the pulling cell (rel_pack)
-  float qv[PRESSURE_SEARCH];    // their volume
+  uint2 q[PRESSURE_SEARCH];  // queued cells: domain id | ABOVE where it lies above the pulling layer, volume
   // Visited set: a key stays where a search put it; what tells searches apart is the rank, whose
   // base falls from search to search, so that an older search's rank never wins (a set emptied after
   // every search cost ~700 cycles of each pull).
@@ -79,9 +79,9 @@ struct Search {
   unsigned blk;                 // 1 + an unfinished earlier cell the search depends on (0: none)
   unsigned pos, status, i, qlen, side;  // the cell, and the search's progress
   float vol, got, here;         // its volume, what the pull takes, the source's volume
-  unsigned cid, skey;           // the pulling cell, the source relative to it
-  int cx, cz;
+  unsigned cid, skey;           // the pulling cell, the source's queue key
 };
+constexpr unsigned ABOVE = 0x80000000u;
 
 // What warp 0 asks of the CTA between rounds.
 enum SoloRequest { SR_LIST = 0, SR_GATE = 1, SR_SEARCH = 2, SR_END = 3 };
@@ -284,16 +284,6 @@ __device__ __forceinline__ unsigned rank_at(const Region& R, int x, int y, int z
   return R.stamp[dom_id(R, x, y, z)];
 }
 
-// Cells relative to a pulling cell: a search examines 512 entries, so it stays within 513 steps.
-__device__ __forceinline__ unsigned rel_pack(int dx, int dy, int dz) {
-  return (unsigned)(dx + 1024) | (unsigned)(dz + 1024) << 11 | (unsigned)dy << 22;
-}
-__device__ __forceinline__ void rel_unpack(unsigned k, int& dx, int& dy, int& dz) {
-  dx = (int)(k & 2047u) - 1024;
-  dz = (int)((k >> 11) & 2047u) - 1024;
-  dy = (int)(k >> 22);
-}
-
 // ------------------------------------------------------------------------------- the lists
 // A cell enters a list once and the parked list once, so neither outgrows the tick's cells; the bounds
 // are checked all the same where an entry goes to global memory.
@@ -339,58 +329,45 @@ __device__ __forceinline__ LaneSlot lane_slot(const Region& R) {
 
 // Four cells at sorted positions i (fluid.rs:584-651), eight lanes each, warp-collective (groups
 // without a cell: `has` false). `pulled`: the cell's pull has run and took `got` (event bits `ev`);
-// otherwise a cell with a start cell is left for its pull (lv_solo). nb / nc: the list that ready
-// successors join and its counter; pb: the parked list. Returns the cell's volume afterwards.
+// otherwise a cell with a start cell is left for its pull (lv_solo). Ready successors join list nb or, above
+// the gate, parked list pb; their counts are the caller's registers (SOLO: no other warp runs) or
+// L.cnt[nc] and L.park_n[pb]. Returns the cell's volume afterwards.
 //
 // Eight lanes rather than one thread per cell: a round is a latency chain (a few dozen to a few
 // hundred cells on 16 warps), and a lane that holds one slot issues one load, one set_volume and two
-// successor counts where a thread issues seven, six and twelve. A cell that is sure to run counts its
-// successors down while its volumes are on their way: nobody reads the next list before the round
-// has ended. The sweep writes the dense words only; sweep_flush brings the atlas in step.
+// successor counts where a thread issues seven, six and twelve. A lone warp takes ~8 cycles for every
+// dependent instruction, so what counts is their number and that the counts and the volumes travel
+// together: the code is one straight line, and successors are counted down before the volumes are
+// looked at (nobody reads the next list before the round has ended). The sweep writes the dense words only;
+// sweep_flush brings the atlas in step.
+template <bool SOLO>
 __device__ __forceinline__ float lv_cells(const Region& R, LvSmem& L, const LaneSlot& S, bool has, unsigned i, bool pulled, float got, unsigned ev,
-                                         int gate, unsigned kp, unsigned nb, unsigned nc, unsigned pb, int& pd) {
+                                         int gate, unsigned kp, unsigned nb, unsigned nc, unsigned& cnt, unsigned pb, unsigned& park, int& pd) {
   const float FULL = full_level();
   const unsigned lane = lane_id(), l = lane & 7u, base = lane & 24u;
   unsigned w = 0xFFFFFFFFu;
-  if (has) w = reinterpret_cast<const unsigned*>(R.lv + i)[l];
-  const unsigned cid = __shfl_sync(FULLMASK, w, 6, 8), ye = __shfl_sync(FULLMASK, w, 7, 8);
-  const int y = (int)(ye & YE_Y);
+  uint2 ce = make_uint2(0u, 0u);
+  if (has) {
+    w = reinterpret_cast<const unsigned*>(R.lv + i)[l];
+    ce = reinterpret_cast<const uint2*>(R.lv + i)[3];
+  }
+  const bool pp = has && i < kp && bit_of(L.pp, i);
+  const int y = (int)(ce.y & YE_Y), at = (int)ce.x + S.off;
   unsigned u = DC_SOLID;
-  if (has && l < 7u) u = R.dense[(int)cid + S.off];
+  if (has && l < 7u) u = R.dense[at];
   // ---- a cell that attempts a pull and has a start cell waits for the pull
-  if (__any_sync(FULLMASK, has && !pulled && i < kp && bit_of(L.pp, i))) {
+  if (__any_sync(FULLMASK, pp && !pulled)) {
     const float v = dc_volume(u);
-    const unsigned starts = (__ballot_sync(FULLMASK, l >= 2u && l < 7u && ((ye >> (25u + l)) & 1u) && !dc_solid(u) && v >= FULL) >> base) & 0xFFu;
+    const unsigned starts = (__ballot_sync(FULLMASK, l >= 2u && l < 7u && ((ce.y >> (25u + l)) & 1u) && !dc_solid(u) && v >= FULL) >> base) & 0xFFu;
     const float self = __shfl_sync(FULLMASK, v, 0, 8);
-    if (!pulled && i < kp && self < FULL && starts) has = false;
+    if (!pulled && pp && self < FULL && starts) has = false;
   }
-  // ---- successors whose last earlier cell this was: to the next list, or parked above the gate
-  {
-    bool r0 = false, r1 = false;
-    if (has && l < 6u) {
-      const unsigned a = w & 0xFFFFu, b = w >> 16;
-      unsigned oa = 0, ob = 0;
-      if (a != NOSUCC) oa = atomicSub(&L.dep[a >> 2], 1u << ((a & 3u) * 8u)) >> ((a & 3u) * 8u);
-      if (b != NOSUCC) ob = atomicSub(&L.dep[b >> 2], 1u << ((b & 3u) * 8u)) >> ((b & 3u) * 8u);
-      r0 = (oa & 0xFFu) == 1u;
-      r1 = (ob & 0xFFu) == 1u;
-    }
-    const unsigned shut = (y + 1 > gate ? S.open1 : 0u) | (y + 2 > gate ? S.open2 : 0u);
-    const bool p0 = r0 && !(shut & 1u), p1 = r1 && !(shut & 2u);
-    const unsigned g0 = __ballot_sync(FULLMASK, p0), g1 = __ballot_sync(FULLMASK, p1);
-    if (g0 | g1) {
-      unsigned t = 0;
-      if (lane == 0u) t = atomicAdd(&L.cnt[nc], (unsigned)(__popc(g0) + __popc(g1)));
-      t = __shfl_sync(FULLMASK, t, 0);
-      if (p0) list_put(R, L, nb, t + (unsigned)__popc(g0 & lanemask_lt()), w & 0xFFFFu);
-      if (p1) list_put(R, L, nb, t + (unsigned)(__popc(g0) + __popc(g1 & lanemask_lt())), w >> 16);
-    }
-    if ((r0 && !p0) || (r1 && !p1)) {
-      unsigned t = atomicAdd(&L.park_n[pb], (r0 && !p0 ? 1u : 0u) + (r1 && !p1 ? 1u : 0u));
-      if (r0 && !p0) park_put(R, pb, t++, w & 0xFFFFu);
-      if (r1 && !p1) park_put(R, pb, t, w >> 16);
-    }
-  }
+  // ---- successors whose last earlier cell this was
+  const unsigned a = w & 0xFFFFu, b = w >> 16, sa = (a & 3u) * 8u, sb = (b & 3u) * 8u;
+  const bool cnts = has && l < 6u;
+  unsigned oa = 0, ob = 0;
+  if (cnts && a != NOSUCC) oa = atomicSub(&L.dep[a >> 2], 1u << sa);
+  if (cnts && b != NOSUCC) ob = atomicSub(&L.dep[b >> 2], 1u << sb);
   // ---- 1. fall into the free capacity below, 2. share with lower sides when supported, 3. evaporate
   // crumbs (fluid.rs:606-650). Every side's flow depends on the volume after the fall and its own
   // volume only; the running volume subtracts the flows in side order (a side without one: 0).
@@ -422,21 +399,53 @@ __device__ __forceinline__ float lv_cells(const Region& R, LvSmem& L, const Lane
   const bool wet = wv >= (is_water ? HIDE_BELOW : SHOW_AT);
   const unsigned nu = mid ? (__float_as_uint(wv) | (wet ? 0u : DC_AIR)) : (wet ? DC_FULL : 0u);
   const bool put = wr && nu != u;
-  if (put) {
-    R.dense[(int)cid + S.off] = nu;
-    pd += (mid ? 1 : 0) - (had ? 1 : 0);
-  }
+  if (put) R.dense[at] = nu;
+  pd += put ? (mid ? 1 : 0) - (had ? 1 : 0) : 0;
+  if (has && y == gate) R.lv_old[i].vol[l] = v;
   const unsigned pm = __ballot_sync(FULLMASK, put) >> base;
   const unsigned cm = __ballot_sync(FULLMASK, put && wet != is_water) >> base;
   // activation slots: 2 below, 3..6 the sides, 7 the cell itself
   const unsigned am = __ballot_sync(FULLMASK, l == 2u ? w_below : l == 7u ? live && dv > SLEEP : ok && f > SLEEP) >> base;
-  if (has) {
-    if (y == gate) R.lv_old[i].vol[l] = v;
-    if (l == 0u) {
-      R.lv_ev[i] = ev | (am & 0xFCu) | ((am & 0x80u) << 9) | ((cm & 0x7Fu) << 8);  // bit 16: seeds itself
-      reinterpret_cast<volatile unsigned char*>(L.dep)[i] = (unsigned char)(DONE | (pm & 0x7Fu));
-      if (i < kp && bit_of(L.pp, i)) atomicAnd(&L.pp[i >> 5], ~(1u << (i & 31u)));
+  // ---- the ready ones to the next list, or parked above the gate
+  const bool r0 = ((oa >> sa) & 0xFFu) == 1u, r1 = ((ob >> sb) & 0xFFu) == 1u;
+  const unsigned shut = (y + 1 > gate ? S.open1 : 0u) | (y + 2 > gate ? S.open2 : 0u);
+  const bool p0 = r0 && !(shut & 1u), p1 = r1 && !(shut & 2u);
+  const unsigned g0 = __ballot_sync(FULLMASK, p0), g1 = __ballot_sync(FULLMASK, p1);
+  const unsigned h0 = __ballot_sync(FULLMASK, r0 && !p0), h1 = __ballot_sync(FULLMASK, r1 && !p1);
+  if (g0 | g1) {
+    const unsigned k = (unsigned)(__popc(g0) + __popc(g1));
+    unsigned t = cnt;
+    if (SOLO) {
+      cnt += k;
+    } else {
+      if (lane == 0u) t = atomicAdd(&L.cnt[nc], k);
+      t = __shfl_sync(FULLMASK, t, 0);
     }
+    const unsigned t0 = t + (unsigned)__popc(g0 & lanemask_lt()), t1 = t + (unsigned)(__popc(g0) + __popc(g1 & lanemask_lt()));
+    if (t + k <= LIST_CAP) {
+      if (p0) L.list[nb][t0] = (unsigned short)a;
+      if (p1) L.list[nb][t1] = (unsigned short)b;
+    } else {
+      if (p0) list_put(R, L, nb, t0, a);
+      if (p1) list_put(R, L, nb, t1, b);
+    }
+  }
+  if (h0 | h1) {
+    const unsigned k = (unsigned)(__popc(h0) + __popc(h1));
+    unsigned t = park;
+    if (SOLO) {
+      park += k;
+    } else {
+      if (lane == 0u) t = atomicAdd(&L.park_n[pb], k);
+      t = __shfl_sync(FULLMASK, t, 0);
+    }
+    if (r0 && !p0) park_put(R, pb, t + (unsigned)__popc(h0 & lanemask_lt()), a);
+    if (r1 && !p1) park_put(R, pb, t + (unsigned)(__popc(h0) + __popc(h1 & lanemask_lt())), b);
+  }
+  if (has && l == 0u) {
+    R.lv_ev[i] = ev | (am & 0xFCu) | ((am & 0x80u) << 9) | ((cm & 0x7Fu) << 8);  // bit 16: seeds itself
+    reinterpret_cast<volatile unsigned char*>(L.dep)[i] = (unsigned char)(DONE | (pm & 0x7Fu));
+    if (pp) atomicAnd(&L.pp[i >> 5], ~(1u << (i & 31u)));
   }
   __syncwarp();
   return vol;
@@ -528,9 +537,9 @@ __device__ __forceinline__ void vis_reset(Search& C, unsigned t0, unsigned nt) {
 // The volume a cell of the pulling layer holds at the turn of the cell at position k, given the volume
 // `v` it holds now and the positions j of its writers (itself, and the cells it is a side of): later
 // ones that already ran and wrote it are looked through (the earliest such write's old value); an
-// unfinished earlier writer is reported in C.blk.
-__device__ __forceinline__ float old_volume(const Region& R, const LvSmem& L, Search& C, unsigned k, const unsigned (&j)[5], float v) {
-  unsigned best = NOSLOT, blk = 0u, slot = 0u;
+// unfinished earlier writer is reported in blk.
+__device__ __forceinline__ float old_volume(const Region& R, const LvSmem& L, unsigned k, const unsigned (&j)[5], float v, unsigned& blk) {
+  unsigned best = NOSLOT, slot = 0u;
 #pragma unroll
   for (int q = 0; q < 5; ++q) {
     const unsigned fl = q == 0 ? 0u : q + 2u;
@@ -541,59 +550,62 @@ __device__ __forceinline__ float old_volume(const Region& R, const LvSmem& L, Se
       slot = fl;
     }
   }
-  if (blk) atomicMax(&C.blk, blk);
   return best != NOSLOT ? R.lv_old[best].vol[slot] : v;
 }
 
-// What a search round's thread finds: its queue entry's neighbour d.
+// The direction d of a search round's lane: up, +x, -x, +z, -z (none for lanes 30 and 31).
+struct SearchLane {
+  int off;        // its step in domain ids
+  bool up, neg;   // d = 0; negative coordinates have to be looked for (fluid.rs:542): a ring world's only
+};
+__device__ __forceinline__ SearchLane search_lane(const Region& R, unsigned d) {
+  const int row = R.PX * R.PY;
+  return SearchLane{d == 0u ? R.PX : d == 1u ? 1 : d == 2u ? -1 : d == 3u ? row : -row, d == 0u, R.ring_w && (R.px0 < 0 || R.pz0 < 0)};
+}
+// What a search round's thread finds: its queue entry's neighbour. blk: 1 + an unfinished earlier cell
+// that what it read depends on (0: none).
 struct SearchRead {
-  unsigned key;  // the neighbour, packed
+  unsigned key;  // the neighbour's queue key
   float here, v;
   bool win, cand, side;
+  unsigned blk;
 };
-__device__ __forceinline__ SearchRead search_read(const Region& R, LvSmem& L, bool act, unsigned e, unsigned d, bool sides) {
-  Search& C = L.s;
-  SearchRead r{0u, 0.0f, 0.0f, false, false, false};
-  if (act) {
-    const unsigned k0 = C.q[e];
-    r.here = C.qv[e];
-    // up, +x, -x, +z, -z as steps of the packed position
-    r.key = k0 + (d == 0u ? 1u << 22 : d == 1u ? 1u : d == 2u ? 0u - 1u : d == 3u ? 1u << 11 : 0u - (1u << 11));
-    int dx, dy, dz;
-    rel_unpack(r.key, dx, dy, dz);
-    // Once the 24 side checks at the start level are spent, what its cells hold no longer matters.
-    // Negative coordinates are passed over (fluid.rs:542); a bounded world has none, its padding is solid.
-    bool rd = d == 0u || sides || dy != 0;
-    if (R.ring_w && d != 0u) rd = rd && C.cx + dx >= 0 && C.cz + dz >= 0;
-    bool top = true;
-    if (rd) {
-      // the cell and, on the pulling layer, the writers' positions: issued together (the neighbours of
-      // a cell of the world lie inside the padded domain)
-      const int id = (int)C.cid + dx + (dz * R.PY + dy) * R.PX;
-      const unsigned u = R.dense[id];
-      if (dy == 0) {
-        const unsigned* st = R.stamp + id;
-        const int row = R.PX * R.PY;
-        const unsigned j[5] = {st[0], st[-1], st[1], st[-row], st[row]};
-        if (!dc_solid(u)) {
-          r.v = old_volume(R, L, C, C.pos, j, dc_volume(u));
-          top = r.v <= 0.0f;
-        }
-      } else if (!dc_solid(u)) {
-        r.v = dc_volume(u);
-        top = r.v <= 0.0f;
-      }
-    }
-    // the surface test of the entry on its up neighbour (fluid.rs:534-535), else an expansion
-    r.win = d == 0u && top && (k0 >> 22) != 0u && r.here > 0.0f;
-    r.cand = rd && !top;
-    r.side = r.cand && d != 0u && dy == 0;
+__device__ __forceinline__ SearchRead search_read(const Region& R, const LvSmem& L, const SearchLane& D, bool act, unsigned e, bool sides) {
+  const Search& C = L.s;
+  const uint2 q = C.q[act ? e : 0u];  // (a lane without an entry looks at the first one's neighbour for nothing)
+  SearchRead r;
+  const int id = (int)(q.x & ~ABOVE) + D.off;  // the neighbours of a cell of the world lie inside the padded domain
+  const bool above0 = q.x >= ABOVE, above = above0 || D.up;
+  r.key = (unsigned)id | (above ? ABOVE : 0u);
+  r.here = __uint_as_float(q.y);
+  r.blk = 0u;
+  // Once the 24 side checks at the start level are spent, what its cells hold no longer matters.
+  bool rd = act && (sides || above);
+  const unsigned u = R.dense[id];
+  r.v = dc_volume(u);
+  if (D.neg) {
+    int x, y, z;
+    dom_xyz(R, (unsigned)id, x, y, z);
+    rd = rd && (D.up || (x >= 0 && z >= 0));
   }
+  const bool level = rd && !above && !dc_solid(u);
+  if (__any_sync(FULLMASK, level)) {
+    if (level) {
+      const unsigned* st = R.stamp + id;
+      const int row = R.PX * R.PY;
+      const unsigned j[5] = {st[0], st[-1], st[1], st[-row], st[row]};
+      r.v = old_volume(R, L, C.pos, j, r.v, r.blk);
+    }
+  }
+  // the surface test of the entry on its up neighbour (fluid.rs:534-535), else an expansion
+  r.cand = rd && !dc_solid(u) && r.v > 0.0f;
+  r.win = act && D.up && !r.cand && above0 && r.here > 0.0f;
+  r.side = r.cand && !above;
   return r;
 }
 
 __device__ __forceinline__ void search_won(Search& C, const SearchRead& r, unsigned e) {
-  C.skey = C.q[e];
+  C.skey = C.q[e].x;
   C.here = r.here;
   C.got = fminf(__fsub_rn(1.0f, C.vol), r.here);
   C.status = SS_SUCCESS;
@@ -644,10 +656,6 @@ __device__ __forceinline__ bool search_begin(const Region& R, LvSmem& L, const L
     C.vol = vol;
     C.got = 0.0f;
     C.cid = cid;
-    if (R.ring_w) {
-      int y;
-      dom_xyz(R, cid, C.cx, y, C.cz);
-    }
     if (starts) {
       C.rank0 = rank0;
       C.nvis += 6u;
@@ -658,14 +666,11 @@ __device__ __forceinline__ bool search_begin(const Region& R, LvSmem& L, const L
     const unsigned d = lane - 2u;
     const bool st = lane >= 2u && lane < 7u && ((starts >> d) & 1u);
     if (st || lane == 0u) {
-      int dx = 0, dy = 0, dz = 0;
-      if (st) dir5((int)d, dx, dy, dz);
-      const unsigned key = rel_pack(dx, dy, dz);
+      const unsigned key = (unsigned)((int)cid + S.off) | (lane == 2u ? ABOVE : 0u);  // (slot 0: the cell)
       C.vrank[vis_slot(C, key)] = rank0 + (st ? d + 1u : 0u);
       if (st) {
         const unsigned p = (unsigned)__popc(starts & ((1u << d) - 1u));
-        C.q[p] = key;
-        C.qv[p] = v;
+        C.q[p] = make_uint2(key, __float_as_uint(v));
       }
     }
   }
@@ -680,6 +685,7 @@ __device__ __forceinline__ bool search_begin(const Region& R, LvSmem& L, const L
 __device__ __forceinline__ void search_solo(const Region& R, LvSmem& L) {
   Search& C = L.s;
   const unsigned lane = lane_id(), j = lane / 5u, d = lane - 5u * j;
+  const SearchLane D = search_lane(R, d);
   unsigned i = C.i, qlen = C.qlen, side = C.side, status = SS_NONE, nvis = 0u;
   const unsigned rank0 = C.rank0 + 6u;
   while (i < qlen) {
@@ -688,9 +694,10 @@ __device__ __forceinline__ void search_solo(const Region& R, LvSmem& L) {
       break;
     }
     const unsigned kk = min(SOLO_ENTRIES, qlen - i);
-    const SearchRead r = search_read(R, L, j < kk, i + j, d, side < 24u);
-    __syncwarp();
-    if (vld(&C.blk)) {  // an earlier cell has yet to write what the search read: run it again later
+    const SearchRead r = search_read(R, L, D, j < kk, i + j, side < 24u);
+    if (__any_sync(FULLMASK, r.blk != 0u)) {  // an earlier cell has yet to write what the search read: run it again later
+      const unsigned blk = __reduce_max_sync(FULLMASK, r.blk);
+      if (lane == 0) C.blk = blk;
       status = SS_BLOCKED;
       break;
     }
@@ -717,10 +724,7 @@ __device__ __forceinline__ void search_solo(const Region& R, LvSmem& L) {
     const bool isnew = cand && vld(&C.vrank[h]) == rank;
     const unsigned nm = __ballot_sync(FULLMASK, isnew);
     const unsigned pos = qlen + (unsigned)__popc(nm & lanemask_lt());
-    if (isnew && pos < PRESSURE_SEARCH) {
-      C.q[pos] = r.key;
-      C.qv[pos] = r.v;
-    }
+    if (isnew && pos < PRESSURE_SEARCH) C.q[pos] = make_uint2(r.key, __float_as_uint(r.v));
     qlen += (unsigned)__popc(nm);
     nvis += (unsigned)__popc(nm);
     i += kk;
@@ -744,11 +748,13 @@ __device__ __noinline__ void search_cta(const Region& Rs, LvSmem& L) {
   Search& C = L.s;
   const unsigned tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, nw = blockDim.x >> 5;
   const unsigned jl = lane / 5u, d = lane - 5u * jl, j = warp * SOLO_ENTRIES + jl;  // lanes 30, 31 idle
+  const SearchLane D = search_lane(R, d);
   unsigned i = C.i, qlen = C.qlen, side = C.side;
   const unsigned rank0 = C.rank0 + 6u;
   while (i < qlen && i < PRESSURE_SEARCH) {
     const unsigned kk = min(SOLO_ENTRIES * nw, min(qlen, PRESSURE_SEARCH) - i);
-    const SearchRead r = search_read(R, L, jl < SOLO_ENTRIES && j < kk, i + j, d, side < 24u);
+    const SearchRead r = search_read(R, L, D, jl < SOLO_ENTRIES && j < kk, i + j, side < 24u);
+    if (r.blk) atomicMax(&C.blk, r.blk);
     const unsigned wm = __ballot_sync(FULLMASK, r.win), smk = __ballot_sync(FULLMASK, r.side);
     // no more than 24 side checks at the start level (fluid.rs:546-549): their order over the warps
     // matters only in the round that passes the limit
@@ -789,10 +795,7 @@ __device__ __noinline__ void search_cta(const Region& Rs, LvSmem& L) {
       const unsigned c = lane < nw ? C.m_new[lane] : 0u;
       const unsigned before = __reduce_add_sync(FULLMASK, lane < warp ? c : 0u), all = __reduce_add_sync(FULLMASK, c);
       const unsigned pos = qlen + before + (unsigned)__popc(nm & lanemask_lt());
-      if (isnew && pos < PRESSURE_SEARCH) {
-        C.q[pos] = r.key;
-        C.qv[pos] = r.v;
-      }
+      if (isnew && pos < PRESSURE_SEARCH) C.q[pos] = make_uint2(r.key, __float_as_uint(r.v));
       qlen += all;
     }
     i += kk;
@@ -810,16 +813,14 @@ __device__ __noinline__ void search_cta(const Region& Rs, LvSmem& L) {
 }
 
 // The end of a pull, one warp: the source's write (fluid.rs:536-540), then the cell itself.
-__device__ __forceinline__ void pull_end(const Region& R, LvSmem& L, const LaneSlot& S, int gate, unsigned kp, unsigned cur, unsigned cc, unsigned pb,
-                                         int& pd) {
+__device__ __forceinline__ void pull_end(const Region& R, LvSmem& L, const LaneSlot& S, int gate, unsigned kp, unsigned cur, unsigned& cnt, unsigned pb,
+                                         unsigned& park, int& pd) {
   Search& C = L.s;
   const unsigned lane = lane_id(), k = C.pos;
   unsigned ev = 0u;
   if (C.status == SS_SUCCESS) {
     if (lane == 0) {
-      int dx, dy, dz;
-      rel_unpack(C.skey, dx, dy, dz);
-      const unsigned sid = (unsigned)((int)C.cid + dx + (dz * R.PY + dy) * R.PX);
+      const unsigned sid = C.skey & ~ABOVE;
       const unsigned u = R.dense[sid], j = R.stamp[sid];
       const float nv = __fsub_rn(C.here, C.got), v = dc_volume(u);
       const bool is_water = (int)u > 0, mid = nv > 1e-6f && nv < full_level(), wet = nv >= (is_water ? HIDE_BELOW : SHOW_AT);
@@ -844,7 +845,7 @@ __device__ __forceinline__ void pull_end(const Region& R, LvSmem& L, const LaneS
     L.n_searches += 1u;
   }
   __syncwarp();
-  const float vol = lv_cells(R, L, S, lane < 8u, k, true, C.got, ev, gate, kp, cur, cc, pb, pd);
+  const float vol = lv_cells<true>(R, L, S, lane < 8u, k, true, C.got, ev, gate, kp, cur, 0u, cnt, pb, park, pd);
   if (lane == 0u && ev && vol >= full_level()) {
     // a pull that leaves its own cell full gives its later neighbours on the layer a start cell
     const LvCell& rc = R.lv[k];
@@ -937,8 +938,8 @@ __device__ __noinline__ int lv_solo(const Region& Rs, LvSmem& L, unsigned n, int
   __syncwarp();
   const unsigned lane = lane_id(), kp = L.kp;
   HeadState H = L.h;
-  unsigned req, cur = L.cur, cc = L.cc, rounds = L.rounds;
-  const unsigned pb = L.pb;
+  const unsigned pb = L.pb, cc = L.cc;
+  unsigned req, cur = L.cur, cnt = L.cnt[cc], park = L.park_n[pb], rounds = L.rounds;  // (nobody else adds to the lists now)
   bool finish = L.resume != 0u;
   unsigned steps = 0;
   while (true) {
@@ -982,11 +983,10 @@ __device__ __noinline__ int lv_solo(const Region& Rs, LvSmem& L, unsigned n, int
         H.blk = L.s.blk;
         if (lane == 0) L.n_again += 1u;
       } else {
-        pull_end(R, L, S, gate, kp, cur, cc, pb, pd);
+        pull_end(R, L, S, gate, kp, cur, cnt, pb, park, pd);
       }
       continue;
     }
-    const unsigned cnt = vld(&L.cnt[cc]);
     if (cnt == 0u || rounds >= cap) {  // with a pull pending a listed cell is always left: a stuck sweep ends as a timeout
       if (lane == 0) L.timeout = cnt != 0u || H.head < n ? 1u : 0u;
       req = SR_END;
@@ -996,13 +996,12 @@ __device__ __noinline__ int lv_solo(const Region& Rs, LvSmem& L, unsigned n, int
       req = SR_LIST;
       break;
     }
-    const unsigned nc = cc == 2u ? 0u : cc + 1u, zc = nc == 2u ? 0u : nc + 1u;
-    if (lane == 0) L.cnt[zc] = 0u;
     const unsigned t = lane >> 3;
-    const unsigned i = t < cnt ? list_get(R, L, cur, t) : 0u;
-    lv_cells(R, L, S, t < cnt && !cell_done(L, i), i, false, 0.0f, 0u, gate, kp, cur ^ 1u, nc, pb, pd);
+    const unsigned i = t < cnt ? L.list[cur][t] : 0u;
+    const bool run = t < cnt && !cell_done(L, i);
+    cnt = 0u;
+    lv_cells<true>(R, L, S, run, i, false, 0.0f, 0u, gate, kp, cur ^ 1u, 0u, cnt, pb, park, pd);
     cur ^= 1u;
-    cc = nc;
     ++rounds;
   }
   __syncwarp();
@@ -1011,7 +1010,9 @@ __device__ __noinline__ int lv_solo(const Region& Rs, LvSmem& L, unsigned n, int
     L.resume = req == SR_SEARCH ? 1u : 0u;
     L.h = H;
     L.cur = cur;
-    L.cc = cc;
+    L.cnt[0] = L.cnt[1] = L.cnt[2] = 0u;
+    L.cnt[cc] = cnt;
+    L.park_n[pb] = park;
     L.rounds = rounds;
   }
   return pd;
