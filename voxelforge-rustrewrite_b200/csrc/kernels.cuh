@@ -483,8 +483,6 @@ __device__ __noinline__ void sweep_levels(const Region& Rs, TickSmem& sm, WS& sW
   __syncthreads();
   plap(0);
   // ---- rounds
-  const LaneSlot ls = lane_slot(R);
-  unsigned unused = 0;
   long long t_wide = 0, t_search = 0;
   while (true) {
     // warp 0 alone decides what comes next: nobody else reads the lists' state while it runs
@@ -512,29 +510,7 @@ __device__ __noinline__ void sweep_levels(const Region& Rs, TickSmem& sm, WS& sW
       __syncthreads();
     } else {
       const long long c0 = clock64();
-      const bool alive = L.h.head < n;  // pulls are still possible: warp 0 looks after every round
-      unsigned cur = L.cur, cc = L.cc, rounds = L.rounds, fcount = min(L.cnt[cc], MAX_CELLS_PER_TICK);
-      const unsigned pb = L.pb;
-      do {
-        const unsigned nb = cur ^ 1u, nc = cc == 2u ? 0u : cc + 1u, zc = nc == 2u ? 0u : nc + 1u;
-        if (tid == 0) L.cnt[zc] = 0u;
-        for (unsigned t0 = warp * 4u; t0 < fcount; t0 += NW_ * 4u) {
-          const unsigned t = t0 + (lane >> 3);
-          const unsigned i = t < fcount ? list_get(R, L, cur, t) : 0u;
-          lv_cells<false>(R, L, ls, t < fcount && !cell_done(L, i), i, false, 0.0f, 0u, gate, kp, nb, nc, unused, pb, unused, pd);
-        }
-        __syncthreads();
-        cur = nb;
-        cc = nc;
-        ++rounds;
-        fcount = min(L.cnt[cc], MAX_CELLS_PER_TICK);
-      } while (!alive && fcount > SOLO_CELLS && rounds < cap);
-      __syncthreads();  // everybody has read the count
-      if (tid == 0) {
-        L.cur = cur;
-        L.cc = cc;
-        L.rounds = rounds;
-      }
+      pd += lv_wide(Rs, L, n, gate, cap);
       t_wide += clock64() - c0;
     }
   }
