@@ -347,6 +347,13 @@ __device__ __forceinline__ void cell_slot(const Region& R, const LaneSlot& S, La
   if (c.has && (threadIdx.x & 7u) < 7u) c.u = R.dense[(int)c.ce.x + S.off];
 }
 
+// A lone warp touches its cells' successors' records, some of which it runs next: they come from L2 (~850
+// cycles) while it works (the prefetch instruction to L1 does nothing here). What was read is looked at
+// in the next call, when it has long arrived.
+struct Touch {
+  unsigned a = 0, b = 0, seen = 0;  // domain ids: below 2^31
+};
+
 // Four cells at sorted positions i (fluid.rs:584-651), eight lanes each, warp-collective (groups
 // without a cell: `has` false). `pulled`: the cell's pull has run and took `got` (event bits `ev`);
 // otherwise a cell with a start cell is left for its pull (lv_solo). Ready successors join list nb or, above
@@ -362,7 +369,7 @@ __device__ __forceinline__ void cell_slot(const Region& R, const LaneSlot& S, La
 // sweep_flush brings the atlas in step.
 template <bool SOLO>
 __device__ __forceinline__ float lv_cells(const Region& R, LvSmem& L, const LaneSlot& S, const LaneCell& c, bool pulled, float got, unsigned ev, int gate,
-                                          unsigned kp, unsigned nb, unsigned nc, unsigned& cnt, unsigned pb, unsigned& park, int& pd) {
+                                          unsigned kp, unsigned nb, unsigned nc, unsigned& cnt, unsigned pb, unsigned& park, Touch& T, int& pd) {
   const float FULL = full_level();
   const unsigned lane = lane_id(), l = lane & 7u, base = lane & 24u;
   const unsigned i = c.i, w = c.w, u = c.u;
@@ -383,6 +390,11 @@ __device__ __forceinline__ float lv_cells(const Region& R, LvSmem& L, const Lane
   unsigned oa = 0, ob = 0;
   if (cnts && a != NOSUCC) oa = atomicSub(&L.dep[a >> 2], 1u << sa);
   if (cnts && b != NOSUCC) ob = atomicSub(&L.dep[b >> 2], 1u << sb);
+  {
+    T.seen |= T.a | T.b;
+    if (cnts && a != NOSUCC) T.a = R.lv[a].cid;
+    if (cnts && b != NOSUCC) T.b = R.lv[b].cid;
+  }
   // ---- 1. fall into the free capacity below, 2. share with lower sides when supported, 3. evaporate
   // crumbs (fluid.rs:606-650). Every side's flow depends on the volume after the fall and its own
   // volume only; the running volume subtracts the flows in side order (a side without one: 0).
@@ -829,7 +841,7 @@ __device__ __noinline__ void search_cta(const Region& Rs, LvSmem& L) {
 
 // The end of a pull, one warp: the source's write (fluid.rs:536-540), then the cell itself.
 __device__ __forceinline__ void pull_end(const Region& R, LvSmem& L, const LaneSlot& S, int gate, unsigned kp, unsigned cur, unsigned& cnt, unsigned pb,
-                                         unsigned& park, int& pd) {
+                                         unsigned& park, Touch& T, int& pd) {
   Search& C = L.s;
   const unsigned lane = lane_id(), k = C.pos;
   unsigned ev = 0u;
@@ -862,7 +874,7 @@ __device__ __forceinline__ void pull_end(const Region& R, LvSmem& L, const LaneS
   __syncwarp();
   LaneCell c = cell_record(R, lane < 8u, k);
   cell_slot(R, S, c);
-  const float vol = lv_cells<true>(R, L, S, c, true, C.got, ev, gate, kp, cur, 0u, cnt, pb, park, pd);
+  const float vol = lv_cells<true>(R, L, S, c, true, C.got, ev, gate, kp, cur, 0u, cnt, pb, park, T, pd);
   if (lane == 0u && ev && vol >= full_level()) {
     // a pull that leaves its own cell full gives its later neighbours on the layer a start cell
     const LvCell& rc = R.lv[k];
@@ -959,6 +971,7 @@ __device__ __noinline__ int lv_solo(const Region& Rs, LvSmem& L, unsigned n, int
   unsigned req, cur = L.cur, cnt = L.cnt[cc], park = L.park_n[pb], rounds = L.rounds;  // (nobody else adds to the lists now)
   bool finish = L.resume != 0u;
   unsigned steps = 0;
+  Touch T;
   while (true) {
     if (++steps > 8u * MAX_CELLS_PER_TICK) {  // more than the tick's pulls and rounds: cannot happen
       if (lane == 0) L.timeout = 1u;
@@ -1000,7 +1013,7 @@ __device__ __noinline__ int lv_solo(const Region& Rs, LvSmem& L, unsigned n, int
         H.blk = L.s.blk;
         if (lane == 0) L.n_again += 1u;
       } else {
-        pull_end(R, L, S, gate, kp, cur, cnt, pb, park, pd);
+        pull_end(R, L, S, gate, kp, cur, cnt, pb, park, T, pd);
       }
       continue;
     }
@@ -1019,10 +1032,11 @@ __device__ __noinline__ int lv_solo(const Region& Rs, LvSmem& L, unsigned n, int
     cnt = 0u;
     LaneCell c = cell_record(R, run, i);
     cell_slot(R, S, c);
-    lv_cells<true>(R, L, S, c, false, 0.0f, 0u, gate, kp, cur ^ 1u, 0u, cnt, pb, park, pd);
+    lv_cells<true>(R, L, S, c, false, 0.0f, 0u, gate, kp, cur ^ 1u, 0u, cnt, pb, park, T, pd);
     cur ^= 1u;
     ++rounds;
   }
+  if ((T.seen | T.a | T.b) >> 31) set_status(R, ST_RANGE, 53);
   __syncwarp();
   if (lane == 0) {
     L.req = req;
@@ -1049,6 +1063,7 @@ __device__ __noinline__ int lv_wide(const Region& Rs, LvSmem& L, unsigned n, int
   const bool alive = L.h.head < n;
   const unsigned pb = L.pb, kp = L.kp;
   unsigned cur = L.cur, cc = L.cc, rounds = L.rounds, fcount = min(L.cnt[cc], MAX_CELLS_PER_TICK), unused = 0;
+  Touch T;
   int pd = 0;
   do {
     const unsigned nb = cur ^ 1u, nc = cc == 2u ? 0u : cc + 1u, zc = nc == 2u ? 0u : nc + 1u;
@@ -1061,7 +1076,7 @@ __device__ __noinline__ int lv_wide(const Region& Rs, LvSmem& L, unsigned n, int
       if (t0 < fcount) {
         LaneCell c = record(t0);
         cell_slot(R, S, c);
-        lv_cells<false>(R, L, S, c, false, 0.0f, 0u, gate, kp, nb, nc, unused, pb, unused, pd);
+        lv_cells<false>(R, L, S, c, false, 0.0f, 0u, gate, kp, nb, nc, unused, pb, unused, T, pd);
       }
     } else if (t0 < fcount) {
       LaneCell c = record(t0), d = record(t0 + step);
@@ -1069,7 +1084,7 @@ __device__ __noinline__ int lv_wide(const Region& Rs, LvSmem& L, unsigned n, int
       for (unsigned at = t0; at < fcount; at += step) {
         const LaneCell e = record(at + 2u * step);
         cell_slot(R, S, d);
-        lv_cells<false>(R, L, S, c, false, 0.0f, 0u, gate, kp, nb, nc, unused, pb, unused, pd);
+        lv_cells<false>(R, L, S, c, false, 0.0f, 0u, gate, kp, nb, nc, unused, pb, unused, T, pd);
         c = d;
         d = e;
       }
@@ -1080,6 +1095,7 @@ __device__ __noinline__ int lv_wide(const Region& Rs, LvSmem& L, unsigned n, int
     ++rounds;
     fcount = min(L.cnt[cc], MAX_CELLS_PER_TICK);
   } while (!alive && fcount > SOLO_CELLS && rounds < cap);
+  if ((T.seen | T.a | T.b) >> 31) set_status(R, ST_RANGE, 53);
   __syncthreads();  // everybody has read the count
   if (tid == 0) {
     L.cur = cur;
