@@ -78,7 +78,7 @@ struct DeviceScope {
 
 // The tick kernel for `nreg` regions: one CTA per region.
 constexpr int PAR_SMEM_BYTES = (int)((sizeof(TickSmem) + 127) / 128 * 128);
-static_assert(PAR_SMEM_BYTES + 1024 + 1024 <= 100 * 1024, "the tick fits the 100 KB carve-out, static arrays and the system's 1 KB included");
+static_assert(PAR_SMEM_BYTES + 2048 + 1024 <= 132 * 1024, "the tick fits the 132 KB carve-out, static arrays and the system's 1 KB included");
 
 cudaError_t launch_tick(const Tune& t, Region* regs, int nreg, int n_ticks, cudaStream_t st) {
   const int warps = (t.gate >> 16) & 0x1F;

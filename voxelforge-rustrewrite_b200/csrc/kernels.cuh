@@ -380,6 +380,7 @@ __device__ __noinline__ void sweep_levels(const Region& Rs, TickSmem& sm, WS& sW
     L.rounds = L.resume = L.timeout = 0u;
     L.n_succ = L.n_searches = L.n_again = 0u;
     L.n_entries = 0ull;
+    L.hard = 0u;
   }
   for (unsigned g = warp; g < ngrp; g += NW_) {
     const unsigned i = g * 32u + lane;
