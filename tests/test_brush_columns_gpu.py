@@ -1,0 +1,81 @@
+"""Strokes of a solid material through water, whose columns run side by side, against the oracle's cell after
+cell: spheres around every limit of that path (list length, chunk of 4096, columns that fit, water that has to
+go to the sides, films of hidden water, lists that go down a column or name a voxel twice)."""
+import numpy as np
+import pytest
+
+from conftest import assert_same_digest, oracle_for
+
+pytestmark = pytest.mark.gpu
+STONE, WATER = 3, 5
+
+
+def pool(vf, orc, ny=64, top=40, lid=None):
+    w = vf.World(48, ny, 48)
+    w.fill_box(0, 0, 0, 47, 3, 47, STONE)
+    for b in ((0, 0, 47, 1), (0, 46, 47, 47), (0, 0, 1, 47), (46, 0, 47, 47)):
+        w.fill_box(b[0], 4, b[1], b[2], ny - 1, b[3], STONE)
+    w.fill_box(2, 4, 2, 45, top, 45, WATER)
+    if lid is not None:
+        w.fill_box(20, lid, 20, 27, lid, 27, STONE)
+    return vf.FluidSim(w, device=0), oracle_for(orc, w)
+
+
+def sphere(c, r):
+    a = np.arange(-r, r + 1)
+    z, y, x = np.meshgrid(a, a, a, indexing="ij")
+    keep = x * x + y * y + z * z <= r * r
+    return np.stack([x[keep] + c[0], y[keep] + c[1], z[keep] + c[2]], 1).astype(np.int32)
+
+
+def same(sim, o, ticks=0):
+    assert_same_digest(sim, o)
+    assert sim.partial_count() == o.partial_count()
+    if ticks:
+        sim.tick(ticks)
+        o.tick(ticks)
+        assert_same_digest(sim, o)
+
+
+@pytest.mark.parametrize("r", [1, 2, 3, 6, 10])  # 7, 33, 123, 925 and 4169 cells
+@pytest.mark.parametrize("at", [(24, 16, 24), (24, 38, 24), (3, 30, 5), (24, 60, 24)])  # deep, at the surface, in a wall, past the top
+def test_spheres(vf, orc, r, at):
+    sim, o = pool(vf, orc)
+    cells = sphere(at, r)
+    assert sim.apply_brush(cells, STONE) == o.apply_brush(cells, STONE)
+    same(sim, o)
+    cells = sphere((at[0] + r, at[1] + 1, at[2]), r)  # a second stroke beside it: partly stone, raised surface
+    assert sim.apply_brush(cells, STONE) == o.apply_brush(cells, STONE)
+    same(sim, o, 3)
+    cells = sphere((at[0] - 1, at[1] + 2, at[2] + r), r)  # in water that has moved: partial and hidden volumes
+    assert sim.apply_brush(cells, STONE) == o.apply_brush(cells, STONE)
+    same(sim, o, 2)
+    sim.close()
+
+
+@pytest.mark.parametrize("lid", [19, 24, 41])  # in the stroke, just above it, on the surface: water goes to the sides
+def test_water_that_does_not_fit_its_column(vf, orc, lid):
+    sim, o = pool(vf, orc, lid=lid)
+    cells = sphere((24, 16, 24), 6)
+    assert sim.apply_brush(cells, STONE) == o.apply_brush(cells, STONE)
+    same(sim, o, 2)
+    sim.close()
+
+
+@pytest.mark.parametrize("ny,top", [(64, 40), (160, 150)])  # the tall one: more than 128 cells of column above
+@pytest.mark.parametrize("order", ["down", "twice", "shuffled", "outside"])
+def test_lists(vf, orc, ny, top, order):
+    sim, o = pool(vf, orc, ny, top)
+    cells = sphere((24, 16, 24), 4)
+    if order == "down":
+        cells = cells[::-1]
+    elif order == "twice":
+        cells = np.concatenate([cells, cells[:40]])
+    elif order == "shuffled":
+        cells = np.random.default_rng(3).permutation(cells)
+    else:
+        cells = np.concatenate([cells, np.array([[-5, 16, 24], [24, -1, 24], [24, ny, 24], [500, 16, 24]], np.int32)])
+    cells = np.ascontiguousarray(cells)
+    assert sim.apply_brush(cells, STONE) == o.apply_brush(cells, STONE)
+    same(sim, o, 2)
+    sim.close()

@@ -514,11 +514,12 @@ int vf_fluid_wake(vf_fluid* h, int32_t x0, int32_t y0, int32_t z0, int32_t x1, i
   return sync_ctl(h);
 }
 
-// The kernel of an edit over a list in device memory: emitters and carving run in parallel, what may
-// displace water one cell after another.
+// The kernel of an edit over a list in device memory: emitters, carving and longer lists of a solid material run in
+// parallel, short ones and water one cell after another (BRUSH_MIN cells take the same time either way).
 static cudaError_t launch_edit(vf_fluid* h, int kind, const int* dev_xyz, uint64_t n, int m, float amount, unsigned long long* dcount) {
   if (kind == ED_EMIT) k_emit<<<1, EDIT_THREADS, 0, h->stream>>>(h->R, dev_xyz, n, amount);
   else if (kind == ED_BRUSH && m == 0) k_carve<<<1, EDIT_THREADS, 0, h->stream>>>(h->R, dev_xyz, n, dcount);
+  else if (kind == ED_BRUSH && m != WATER && n >= BRUSH_MIN) k_brush<<<1, BRUSH_THREADS, 0, h->stream>>>(h->R, dev_xyz, n, m, dcount);
   else k_edit<<<1, 32, 0, h->stream>>>(h->R, kind, dev_xyz, n, m, amount, dcount);
   return cudaGetLastError();
 }

@@ -1749,6 +1749,295 @@ __global__ void __launch_bounds__(EDIT_THREADS) k_carve(Region R, const int* xyz
   if (tid == 0 && out_count) *out_count = s_n;
 }
 
+// apply_brush with a solid material (src/edit/brush.rs:93-111) over a long list, one CTA. A listed water
+// cell's water goes up its own column (FluidSim::displace, fluid.rs:370-408), so the columns of a stroke
+// are independent as long as every column's cells are listed upwards and its water finds room above: a
+// warp then takes a column, in registers. In chunks of the list: the voxels and columns are claimed (rb, stamp); every
+// column is tried without writing, up to its first cell that does not fit (water that has to go to the sides, a
+// cell listed below or twice, a film of air that keeps its entry, a column of more than 128 cells, water that
+// goes to more than three cells). What the list holds before the first of those commits to the dense words and logs what
+// each listed cell did, and the log is followed in list order: slots, the atlas, and the
+// activations (27 around a displaced cell, then those that took its water), 16 cells at a time, each cell
+// activated by its first mention. That first cell then takes its turn as brush_warp does (twice as many cells each
+// time the next chunk stops early), and the rest is the next chunk. One warp in list order spent 3.2 us
+// on each displaced cell.
+constexpr int BRUSH_THREADS = 512;
+constexpr unsigned BRUSH_CHUNK = 4096, BRUSH_MIN = 24;
+constexpr int BRUSH_ROWS = 4, BRUSH_TARGETS = 3;
+static_assert(BRUSH_CHUNK * sizeof(uint4) <= MAX_CELLS_PER_TICK * sizeof(LvCell), "the log lies where a tick keeps its records");
+// A log entry: .x = cells that took water | 4 placed | 8 it was water | 16 << t: cell t's voxel changed; .y, .z, .w
+// those cells.
+
+// The listed cells of a column before entry `limit`, from its first (the lowest) up, by one warp. Returns the
+// first entry that does not fit, or `limit` (nothing is written unless `commit`).
+__device__ __forceinline__ unsigned brush_column(const Region& R, const int* xyz, unsigned lead, unsigned limit, bool commit, uint4* log, int& pd,
+                                                 unsigned& placed) {
+  const unsigned lane = lane_id();
+  const int x = xyz[3 * lead], y = xyz[3 * lead + 1], z = xyz[3 * lead + 2];
+  const unsigned id0 = dom_id(R, x, y, z);
+  unsigned u[BRUSH_ROWS], at[BRUSH_ROWS], dirty = 0;
+#pragma unroll
+  for (int k = 0; k < BRUSH_ROWS; ++k) {
+    const int up = 32 * k + (int)lane;
+    const bool in = y + up < R.ny;
+    u[k] = in ? R.dense[id0 + (unsigned)(up * R.PX)] : DC_SOLID;
+    at[k] = in ? __ldcg(R.rb + id0 + (unsigned)(up * R.PX)) : NOSLOT;
+  }
+  bool ok = true;
+  unsigned prev = lead;
+#pragma unroll
+  for (int k = 0; k < BRUSH_ROWS; ++k) {
+    for (unsigned listed = __ballot_sync(FULLMASK, at[k] != NOSLOT); listed && ok; listed &= listed - 1u) {
+      const unsigned b = (unsigned)__ffs(listed) - 1u;
+      const unsigned i = __shfl_sync(FULLMASK, at[k], b), own = __shfl_sync(FULLMASK, u[k], b);
+      if (i >= limit) {  // (the column's cells before it in the list lie below it)
+        ok = false;
+        continue;
+      }
+      if (i < prev) {
+        ok = false;
+        limit = i;
+        continue;
+      }
+      prev = i;
+      if (dc_solid(own)) continue;
+      unsigned nt = 0, t[BRUSH_TARGETS] = {0, 0, 0}, flags = 4u;
+      if ((int)own > 0) {
+        flags |= 8u;
+        float amount = dc_volume(own);
+        if (lane == 0u && amount < 1.0f) pd -= 1;  // its entry goes
+        bool shut = false;
+#pragma unroll
+        for (int kk = 0; kk < BRUSH_ROWS; ++kk) {
+          if (kk < k || shut || amount <= 1e-6f) continue;
+          const unsigned over = kk > k ? 0xFFFFFFFFu : ~((2u << b) - 1u);
+          const unsigned solid = __ballot_sync(FULLMASK, dc_solid(u[kk])) & over;
+          const unsigned below = solid ? (solid & (0u - solid)) - 1u : 0xFFFFFFFFu;
+          const float cur = dc_volume(u[kk]);
+          unsigned room = __ballot_sync(FULLMASK, !dc_solid(u[kk]) && __fsub_rn(1.0f, cur) > 0.0f) & over & below;
+          for (; room && amount > 1e-6f; room &= room - 1u) {
+            const unsigned q = (unsigned)__ffs(room) - 1u;
+            const float cq = __shfl_sync(FULLMASK, cur, q);
+            const unsigned uq = __shfl_sync(FULLMASK, u[kk], q);
+            const float take = fminf(amount, __fsub_rn(1.0f, cq));
+            if (!(take > 0.0f)) continue;
+            const float nv = __fadd_rn(cq, take);
+            amount = __fsub_rn(amount, take);
+            const bool is_water = (int)uq > 0, mid = nv > 1e-6f && nv < full_level(), had = cq > 0.0f && cq < 1.0f;
+            const bool wet = nv >= (is_water ? HIDE_BELOW : SHOW_AT);
+            if (lane == q) {
+              u[kk] = mid ? (__float_as_uint(nv) | (wet ? 0u : DC_AIR)) : (wet ? DC_FULL : 0u);
+              dirty |= 1u << kk;
+            }
+            if (lane == 0u) pd += (mid ? 1 : 0) - (had ? 1 : 0);
+            if (wet != is_water) flags |= 16u << nt;
+            const unsigned tid_ = id0 + (unsigned)((32 * kk + (int)q) * R.PX);
+            if (nt == 0u) t[0] = tid_;
+            if (nt == 1u) t[1] = tid_;
+            if (nt == 2u) t[2] = tid_;
+            ++nt;
+            if (nt > BRUSH_TARGETS) {
+              ok = false;
+              amount = 0.0f;
+            }
+          }
+          shut = solid != 0u;
+        }
+        ok = ok && !(amount > 1e-6f);
+      } else if (own != 0u) {
+        ok = false;
+      }
+      if (lane == b) {
+        u[k] = DC_SOLID;
+        dirty |= 1u << k;
+      }
+      placed += 1u;
+      if (!ok) limit = i;
+      if (commit && lane == 0u) log[i] = make_uint4(flags | nt, t[0], t[1], t[2]);
+    }
+  }
+  if (commit) {
+#pragma unroll
+    for (int k = 0; k < BRUSH_ROWS; ++k)
+      if ((dirty >> k) & 1u) R.dense[id0 + (unsigned)((32 * k + (int)lane) * R.PX)] = u[k];
+  }
+  return limit;
+}
+
+__global__ void __launch_bounds__(BRUSH_THREADS) k_brush(Region R, const int* list, unsigned long long n, int m, unsigned long long* out_count) {
+  __shared__ EditSmem es;
+  __shared__ unsigned cnt[32], s_placed, s_ch, s_limit;
+  __shared__ int s_pd;
+  const unsigned tid = threadIdx.x, lane = lane_id(), warp = tid >> 5;
+  const int* ring = edit_ring(R, es.ring);
+  uint4* log = reinterpret_cast<uint4*>(R.lv);
+  if (tid == 0) {
+    s_placed = s_ch = 0u;
+    s_pd = 0;
+  }
+  unsigned long long serial = 0;
+  unsigned turns = 1;  // cells that take their turn by themselves when a chunk stops early
+  for (unsigned long long base = 0; base < n;) {
+    const int* xyz = list + 3 * base;
+    const unsigned all = (unsigned)min((unsigned long long)BRUSH_CHUNK, n - base);
+    if (tid == 0) s_limit = all;
+    __syncthreads();
+    // ---- claims: a voxel's first entry, a column's first entry
+    for (unsigned i = tid; i < all; i += BRUSH_THREADS) {
+      const int x = xyz[3 * i], y = xyz[3 * i + 1], z = xyz[3 * i + 2];
+      log[i] = make_uint4(0u, 0u, 0u, 0u);
+      if (outside(R, ring, x, y, z)) continue;
+      atomicMin(R.rb + dom_id(R, x, y, z), i);
+      atomicMin(R.stamp + dom_id(R, x, 0, z), i);
+    }
+    __syncthreads();
+    for (unsigned i = tid; i < all; i += BRUSH_THREADS) {
+      const int x = xyz[3 * i], y = xyz[3 * i + 1], z = xyz[3 * i + 2];
+      if (outside(R, ring, x, y, z)) continue;
+      const unsigned lead = __ldcg(R.stamp + dom_id(R, x, 0, z));
+      const int yl = xyz[3 * lead + 1];
+      if (__ldcg(R.rb + dom_id(R, x, y, z)) != i || y < yl || y - yl >= 32 * BRUSH_ROWS) atomicMin(&s_limit, i);
+    }
+    __syncthreads();
+    // ---- the columns: tried, then committed
+    int pd = 0;
+    unsigned placed = 0, len = 0;
+    for (int commit = 0; commit < 2; ++commit) {
+      len = s_limit;
+      pd = 0;
+      placed = 0;
+      __syncthreads();
+      for (unsigned b0 = warp * 32u; b0 < len; b0 += BRUSH_THREADS) {
+        const unsigned i = b0 + lane;
+        bool lead = false;
+        if (i < len) {
+          const int x = xyz[3 * i], y = xyz[3 * i + 1], z = xyz[3 * i + 2];
+          lead = !outside(R, ring, x, y, z) && __ldcg(R.stamp + dom_id(R, x, 0, z)) == i;
+        }
+        for (unsigned mask = __ballot_sync(FULLMASK, lead); mask; mask &= mask - 1u) {
+          const unsigned fit = brush_column(R, xyz, b0 + (unsigned)__ffs(mask) - 1u, len, commit != 0, log, pd, placed);
+          if (lane == 0u && fit < len) atomicMin(&s_limit, fit);
+        }
+      }
+      __syncthreads();
+    }
+    for (unsigned i = tid; i < all; i += BRUSH_THREADS) {
+      const int x = xyz[3 * i], y = xyz[3 * i + 1], z = xyz[3 * i + 2];
+      if (outside(R, ring, x, y, z)) continue;
+      R.rb[dom_id(R, x, y, z)] = 0xFFFFFFFFu;
+      R.stamp[dom_id(R, x, 0, z)] = 0xFFFFFFFFu;
+    }
+    __syncthreads();
+    if (pd) atomicAdd(&s_pd, pd);
+    if (lane == 0u && placed) atomicAdd(&s_placed, placed);
+    // ---- the atlas, in list order: the cells that took a cell's water, then the cell
+    for (unsigned b0 = 0; b0 < len; b0 += BRUSH_THREADS) {
+      const unsigned i = b0 + tid;
+      uint4 e = make_uint4(0u, 0u, 0u, 0u);
+      if (i < len) e = log[i];
+      const unsigned nt = e.x & 3u;
+      unsigned w = (e.x & 4u) ? (1u << nt) - 1u | 8u : 0u, need = 0, id[4] = {e.y, e.z, e.w, 0u}, gi[4], g[4], at[4];
+      if (w) id[3] = dom_id(R, xyz[3 * i], xyz[3 * i + 1], xyz[3 * i + 2]);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        gi[q] = g[q] = at[q] = 0u;
+        if (!((w >> q) & 1u)) continue;
+        int x, y, z;
+        dom_xyz(R, id[q], x, y, z);
+        gi[q] = grid_index(R, x >> 3, y >> 3, z >> 3);
+        at[q] = local_index(x, y, z);
+        g[q] = __ldcg(R.grid + gi[q]);
+        need |= g[q] < 256u ? 1u << q : 0u;
+      }
+      if (__syncthreads_or(need != 0u)) {
+        give_slots<4>(AtlasRef{R.grid, R.amat, R.avol, R.ctl, R.atlas_cap}, need, gi);
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          if ((need >> q) & 1u) g[q] = __ldcg(R.grid + gi[q]);
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        if (!((w >> q) & 1u)) continue;
+        if (q == 3 || ((e.x >> (4 + q)) & 1u)) {
+          record_change(R, id[q]);
+          if (q < 3) s_ch = 1u;
+        }
+        if (g[q] < 256u) continue;  // (no slot left: the status says so)
+        const size_t o = (size_t)(g[q] - 256u) * 512u + at[q];
+        const unsigned u = R.dense[id[q]];
+        const float v = dc_solid(u) ? 1.0f : dc_volume(u);
+        R.avol[o] = v < 1.0f ? v : 0.0f;
+        R.amat[o] = dc_solid(u) ? (unsigned char)m : (int)u > 0 ? WATER : (unsigned char)0;
+      }
+    }
+    __syncthreads();
+    // ---- the activations, in list order, a displaced cell per warp
+    unsigned long long tail = R.ctl->qtail;
+    const unsigned long long tail0 = tail;
+    for (unsigned b0 = 0; b0 < len; b0 += BRUSH_THREADS / 32) {
+      const unsigned i = b0 + warp;
+      bool act = false;
+      unsigned id = 0;
+      if (i < len) {
+        const uint4 e = log[i];
+        if (e.x & 8u) {
+          if (lane < 27u) {
+            const int x = xyz[3 * i] - 1 + (int)lane % 3, y = xyz[3 * i + 1] - 1 + (int)lane / 3 % 3, z = xyz[3 * i + 2] - 1 + (int)lane / 9;
+            act = y >= 0;
+            if (act && !in_dom(R, x, y, z)) {
+              set_status(R, ST_RANGE, 3);
+              act = false;
+            }
+            if (act) id = dom_id(R, x, y, z);
+          } else if (lane - 27u < (e.x & 3u)) {
+            act = true;
+            id = lane == 27u ? e.y : lane == 28u ? e.z : e.w;
+          }
+        }
+      }
+      if (!__syncthreads_or(act)) continue;
+      if (act) atomicMin(R.rb + id, tid);
+      __syncthreads();
+      const bool first = act && __ldcg(R.rb + id) == tid;
+      const bool isnew = first && !((__ldcg(&R.active[id >> 5]) >> (id & 31u)) & 1u);
+      unsigned total;
+      const unsigned off = edit_scan(cnt, isnew, &total);
+      if (isnew) {
+        R.queue[(tail + off) & R.qmask] = id;
+        atomicOr(&R.active[id >> 5], 1u << (id & 31u));
+      }
+      if (first) R.rb[id] = 0xFFFFFFFFu;
+      tail += total;
+    }
+    __syncthreads();
+    if (tid == 0) {
+      R.ctl->qtail = tail;
+      R.ctl->activations += tail - tail0;
+      if (tail - R.ctl->qhead > R.qmask + 1ull) set_status(R, ST_OOM, 7);
+    }
+    __syncthreads();
+    base += len;
+    if (len == all) continue;
+    // ---- the cell that did not fit
+    const unsigned k = (unsigned)min((unsigned long long)turns, n - base);
+    if (warp == 0) {
+      WS W;
+      load_ws(R, W);
+      for (unsigned i = len; i < len + k; ++i) serial += brush_warp(R, W, ring, xyz[3 * i], xyz[3 * i + 1], xyz[3 * i + 2], (unsigned char)m);
+      if (W.qtail - W.qhead > R.qmask + 1ull) set_status(R, ST_OOM, 7);
+      commit_ws(R, W);
+    }
+    __syncthreads();
+    base += k;
+    turns = len >= 64u ? 1u : min(2u * turns, BRUSH_CHUNK);
+  }
+  if (tid == 0) {
+    R.ctl->partial_count += s_pd;
+    if (s_ch) R.ctl->changed = 1u;
+    if (out_count) *out_count = serial + s_placed;
+  }
+}
+
 enum EditKind { ED_DISPLACE = 1, ED_BRUSH = 2, ED_EMIT = 3, ED_SET_PARTIAL = 4 };
 
 // kind/args: ED_DISPLACE: xyz[0..3]; ED_BRUSH: n cells, m; ED_SET_PARTIAL: xyz[0..3], amount.
