@@ -1753,20 +1753,20 @@ __global__ void __launch_bounds__(EDIT_THREADS) k_carve(Region R, const int* xyz
 // cell's water goes up its own column (FluidSim::displace, fluid.rs:370-408), so the columns of a stroke
 // are independent as long as every column's cells are listed upwards and its water finds room above: a
 // warp then takes a column, in registers. In chunks of the list: the voxels and columns are claimed (rb, stamp); every
-// column is tried without writing, up to its first cell that does not fit (water that has to go to the sides, a
-// cell listed below or twice, a film of air that keeps its entry, a column of more than 128 cells, water that
+// column is tried without writing, up to its first cell that does not fit (water that goes to the sides, a
+// cell listed below or twice, a column of more than 128 cells, water that
 // goes to more than three cells). What the list holds before the first of those commits to the dense words and logs what
 // each listed cell did, and the log is followed in list order: slots, the atlas, and the
 // activations (27 around a displaced cell, then those that took its water), 16 cells at a time, each cell
-// activated by its first mention. That first cell then takes its turn as brush_warp does (twice as many cells each
-// time the next chunk stops early), and the rest is the next chunk. One warp in list order spent 3.2 us
+// activated by its first mention. That first cell then takes its turn as brush_warp does (up to 64 cells when
+// the next chunks stop early too), and the rest is the next chunk. One warp in list order spent 3.2 us
 // on each displaced cell.
 constexpr int BRUSH_THREADS = 512;
-constexpr unsigned BRUSH_CHUNK = 4096, BRUSH_MIN = 24;
+constexpr unsigned BRUSH_CHUNK = 4096, BRUSH_MIN = 12;
 constexpr int BRUSH_ROWS = 4, BRUSH_TARGETS = 3;
 static_assert(BRUSH_CHUNK * sizeof(uint4) <= MAX_CELLS_PER_TICK * sizeof(LvCell), "the log lies where a tick keeps its records");
-// A log entry: .x = cells that took water | 4 placed | 8 it was water | 16 << t: cell t's voxel changed; .y, .z, .w
-// those cells.
+// A log entry: .x = cells that took water | 4 placed | 8 it was water | 16 << t: cell t's voxel changed |
+// 128 it keeps an entry; .y, .z, .w those cells, or the entry's volume.
 
 // The listed cells of a column before entry `limit`, from its first (the lowest) up, by one warp. Returns the
 // first entry that does not fit, or `limit` (nothing is written unless `commit`).
@@ -1843,12 +1843,20 @@ __device__ __forceinline__ unsigned brush_column(const Region& R, const int* xyz
           }
           shut = solid != 0u;
         }
-        ok = ok && !(amount > 1e-6f);
-      } else if (own != 0u) {
-        ok = false;
+        if (ok && amount > 1e-6f) {
+          // to the sides, if one of them has room: during a stroke a cell only fills or turns solid, so one without
+          // room stays so; where none has any, the water is gone (fluid.rs:396-408)
+          const int row = R.PX * R.PY;
+          const int off = lane == 0u ? 1 : lane == 1u ? -1 : lane == 2u ? row : -row;
+          const unsigned us = lane < 4u ? R.dense[(int)(id0 + (32u * k + b) * (unsigned)R.PX) + off] : DC_SOLID;
+          ok = shut && !__any_sync(FULLMASK, !dc_solid(us) && __fsub_rn(1.0f, dc_volume(us)) > 0.0f);
+        }
+      } else if (own != 0u) {  // a film of hidden water: its entry stays in the solid cell
+        flags |= 128u;
+        t[0] = __float_as_uint(dc_volume(own));
       }
       if (lane == b) {
-        u[k] = DC_SOLID;
+        u[k] = (flags & 128u) ? DC_SOLID_PART : DC_SOLID;
         dirty |= 1u << k;
       }
       placed += 1u;
@@ -1876,10 +1884,10 @@ __global__ void __launch_bounds__(BRUSH_THREADS) k_brush(Region R, const int* li
     s_pd = 0;
   }
   unsigned long long serial = 0;
-  unsigned turns = 1;  // cells that take their turn by themselves when a chunk stops early
+  unsigned turns = 1, size = BRUSH_CHUNK;  // cells that take their turn by themselves when a chunk stops early; the next chunk
   for (unsigned long long base = 0; base < n;) {
     const int* xyz = list + 3 * base;
-    const unsigned all = (unsigned)min((unsigned long long)BRUSH_CHUNK, n - base);
+    const unsigned all = (unsigned)min((unsigned long long)size, n - base);
     if (tid == 0) s_limit = all;
     __syncthreads();
     // ---- claims: a voxel's first entry, a column's first entry
@@ -1964,10 +1972,16 @@ __global__ void __launch_bounds__(BRUSH_THREADS) k_brush(Region R, const int* li
         }
         if (g[q] < 256u) continue;  // (no slot left: the status says so)
         const size_t o = (size_t)(g[q] - 256u) * 512u + at[q];
+        if (q == 3) {
+          R.avol[o] = (e.x & 128u) ? __uint_as_float(e.y) : 0.0f;
+          R.amat[o] = (unsigned char)m;
+          continue;
+        }
         const unsigned u = R.dense[id[q]];
-        const float v = dc_solid(u) ? 1.0f : dc_volume(u);
+        if (dc_solid(u)) continue;  // placed later in the list
+        const float v = dc_volume(u);
         R.avol[o] = v < 1.0f ? v : 0.0f;
-        R.amat[o] = dc_solid(u) ? (unsigned char)m : (int)u > 0 ? WATER : (unsigned char)0;
+        R.amat[o] = (int)u > 0 ? WATER : (unsigned char)0;
       }
     }
     __syncthreads();
@@ -2017,7 +2031,10 @@ __global__ void __launch_bounds__(BRUSH_THREADS) k_brush(Region R, const int* li
     }
     __syncthreads();
     base += len;
-    if (len == all) continue;
+    if (len == all) {
+      size = min(4u * size, BRUSH_CHUNK);
+      continue;
+    }
     // ---- the cell that did not fit
     const unsigned k = (unsigned)min((unsigned long long)turns, n - base);
     if (warp == 0) {
@@ -2029,7 +2046,8 @@ __global__ void __launch_bounds__(BRUSH_THREADS) k_brush(Region R, const int* li
     }
     __syncthreads();
     base += k;
-    turns = len >= 64u ? 1u : min(2u * turns, BRUSH_CHUNK);
+    turns = len >= 64u ? 1u : min(2u * turns, 64u);
+    size = min(max(128u, 2u * len), BRUSH_CHUNK);  // (what lies behind the next such cell is tried for nothing)
   }
   if (tid == 0) {
     R.ctl->partial_count += s_pd;
