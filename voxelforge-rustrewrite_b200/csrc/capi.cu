@@ -785,20 +785,16 @@ int vf_fluid_export_partials(vf_fluid* h, int32_t* xyz, float* vol, uint64_t cap
   if (rc) return rc;
   DeviceScope scope(h->device);  // the caller's current device is given back on return
   if ((rc = sync_ctl(h))) return rc;
-  unsigned nslots = std::min(h->hctl->atlas_used, h->R.atlas_cap);
-  const size_t o_count = align16((size_t)nslots * 4), o_xyz = o_count + 64, o_vol = o_xyz + align16(cap * 12);
+  const unsigned spans = (h->R.ncells + PART_SPAN - 1) / PART_SPAN;
+  cap = std::min<uint64_t>(cap, (uint64_t)h->R.ncells + h->det.size());  // there are no more
+  const size_t o_count = align16((size_t)spans * 4), o_xyz = o_count + 64, o_vol = o_xyz + align16(cap * 12);
   if ((rc = ensure_scratch(h, o_vol + align16(cap * 4) + 16))) return rc;
-  int* slot_brick = (int*)h->scratch;
+  unsigned* counts = (unsigned*)h->scratch;
   unsigned long long* dcount = (unsigned long long*)((char*)h->scratch + o_count);
   int* dxyz = (int*)((char*)h->scratch + o_xyz);
   float* dvol = (float*)((char*)h->scratch + o_vol);
-  CK(cudaMemsetAsync(slot_brick, 0xFF, (size_t)nslots * 4 + 8, h->stream));
-  CK(cudaMemsetAsync(dcount, 0, 8, h->stream));
-  uint64_t nb = (uint64_t)h->R.bx * h->R.by * h->R.bz;
-  k_slot_map<<<(unsigned)std::min<uint64_t>((nb + 255) / 256, 8192), 256, 0, h->stream>>>(h->R, slot_brick, nslots);
-  if (nslots)
-    k_export_partials<<<(unsigned)std::min<uint64_t>(((uint64_t)nslots * 512 + 255) / 256, 16384), 256, 0, h->stream>>>(h->R, nslots, dxyz, dvol,
-                                                                                                                         cap, dcount, slot_brick);
+  k_part_count<<<spans, 256, 0, h->stream>>>(h->R, counts);
+  k_part_write<<<spans, 256, 0, h->stream>>>(h->R, counts, dxyz, dvol, cap, dcount);
   CK(cudaGetLastError());
   unsigned long long cnt = 0;
   CK(cudaMemcpyAsync(&cnt, dcount, 8, cudaMemcpyDeviceToHost, h->stream));
@@ -823,8 +819,8 @@ int vf_fluid_export_partials(vf_fluid* h, int32_t* xyz, float* vol, uint64_t cap
     ++cnt;
   }
   if (n) *n = cnt;
-  // canonical order: by (x, y, z) ascending? keep (slot, voxel) order but make it deterministic
-  if (take && xyz && vol) {
+  // the device's entries come by (z, y, x); kept ones join them
+  if (take && xyz && vol && !h->det.empty()) {
     std::vector<uint64_t> idx(take);
     for (uint64_t i = 0; i < take; ++i) idx[i] = i;
     std::sort(idx.begin(), idx.end(), [&](uint64_t a, uint64_t b) {

@@ -2239,29 +2239,76 @@ __global__ void k_gather_changes(Region R, unsigned long long n, Voxel* out) {
   }
 }
 
-// Partial entries of every atlas slot, compacted (ascending slot, voxel index order).
-__global__ void k_export_partials(Region R, unsigned nslots, int* xyz, float* vol, unsigned long long cap, unsigned long long* count,
-                                  const int* slot_brick /* slot -> grid index */) {
-  for (unsigned long long t = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; t < (unsigned long long)nslots * 512ull;
-       t += (unsigned long long)gridDim.x * blockDim.x) {
-    unsigned s = (unsigned)(t >> 9), l = (unsigned)(t & 511u);
-    float p = R.avol[t];
-    if (!(p > 0.0f)) continue;
-    int gi = slot_brick[s];
-    if (gi < 0) continue;
-    int bx = gi % R.bx, by = (gi / R.bx) % R.by, bz = gi / (R.bx * R.by);
-    int ax = bx, az = bz;
-    if (R.ring_w) {
-      const int* rs = R.ring + 3 * ((bz / 16) * R.ring_w + (bx / 16));
-      ax = rs[0] * 16 + bx % 16;
-      az = rs[1] * 16 + bz % 16;
+// Partial entries in (z, y, x) order, which is the order of domain ids: a count per span of PART_SPAN dense
+// words, then every span writes behind the ones before it. Bound by reading the dense words twice (a
+// 320 x 160 x 320 domain: 66 MB, 12 us each); entries gathered by atlas slot had to be sorted on the host (9,656
+// of them: 0.4 ms).
+constexpr unsigned PART_SPAN = 8192;
+__device__ __forceinline__ bool dc_has_part(unsigned u) { return dc_solid(u) ? u == DC_SOLID_PART : dc_volume(u) > 0.0f && dc_volume(u) < 1.0f; }
+__device__ __forceinline__ uint4 dense_quad(const Region& R, unsigned id) {
+  if (id + 4u <= R.ncells) return *reinterpret_cast<const uint4*>(R.dense + id);
+  uint4 u = make_uint4(0u, 0u, 0u, 0u);
+  if (id < R.ncells) u.x = R.dense[id];
+  if (id + 1u < R.ncells) u.y = R.dense[id + 1u];
+  if (id + 2u < R.ncells) u.z = R.dense[id + 2u];
+  return u;
+}
+__device__ __forceinline__ unsigned block_sum(unsigned v) {
+  __shared__ unsigned s[32];
+  v = __reduce_add_sync(FULLMASK, v);
+  __syncthreads();
+  if ((threadIdx.x & 31u) == 0u) s[threadIdx.x >> 5] = v;
+  __syncthreads();
+  return __reduce_add_sync(FULLMASK, (threadIdx.x & 31u) < (blockDim.x >> 5) ? s[threadIdx.x & 31u] : 0u);
+}
+__global__ void __launch_bounds__(256) k_part_count(Region R, unsigned* counts) {
+  unsigned c = 0;
+#pragma unroll
+  for (unsigned r = 0; r < PART_SPAN / 1024u; ++r) {
+    const uint4 u = dense_quad(R, blockIdx.x * PART_SPAN + r * 1024u + threadIdx.x * 4u);
+    c += (dc_has_part(u.x) ? 1u : 0u) + (dc_has_part(u.y) ? 1u : 0u) + (dc_has_part(u.z) ? 1u : 0u) + (dc_has_part(u.w) ? 1u : 0u);
+  }
+  c = block_sum(c);
+  if (threadIdx.x == 0) counts[blockIdx.x] = c;
+}
+__global__ void __launch_bounds__(256) k_part_write(Region R, const unsigned* counts, int* xyz, float* vol, unsigned long long cap, unsigned long long* count) {
+  const unsigned tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+  __shared__ unsigned s[8];
+  if (counts[blockIdx.x] == 0u && blockIdx.x != gridDim.x - 1u) return;
+  unsigned before = 0;
+  for (unsigned b = tid; b < blockIdx.x; b += 256u) before += counts[b];
+  before = block_sum(before);
+  if (blockIdx.x == gridDim.x - 1u && tid == 0u) *count = before + counts[blockIdx.x];
+  for (unsigned r = 0; r < PART_SPAN / 1024u; ++r) {
+    const unsigned id = blockIdx.x * PART_SPAN + r * 1024u + tid * 4u;
+    const uint4 q = dense_quad(R, id);
+    const unsigned u[4] = {q.x, q.y, q.z, q.w};
+    unsigned c = 0;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) c += dc_has_part(u[e]) ? 1u : 0u;
+    unsigned pre = c;
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned v = __shfl_up_sync(FULLMASK, pre, o);
+      if (lane >= (unsigned)o) pre += v;
     }
-    unsigned long long k = atomicAdd(count, 1ull);
-    if (k < cap) {
-      xyz[3 * k] = ax * 8 + (int)(l & 7u);
-      xyz[3 * k + 1] = by * 8 + (int)((l >> 3) & 7u);
-      xyz[3 * k + 2] = az * 8 + (int)(l >> 6);
-      vol[k] = p;
+    __syncthreads();
+    if (lane == 31u) s[warp] = pre;
+    __syncthreads();
+    const unsigned w = lane < 8u ? s[lane] : 0u;
+    unsigned long long k = before + __reduce_add_sync(FULLMASK, lane < warp ? w : 0u) + pre - c;
+    before += __reduce_add_sync(FULLMASK, w);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      if (!dc_has_part(u[e])) continue;
+      if (k < cap) {
+        int x, y, z;
+        dom_xyz(R, id + e, x, y, z);
+        xyz[3 * k] = x;
+        xyz[3 * k + 1] = y;
+        xyz[3 * k + 2] = z;
+        vol[k] = dc_solid(u[e]) ? load_cell(R, R.ring, x, y, z).part : dc_volume(u[e]);
+      }
+      ++k;
     }
   }
 }
