@@ -206,14 +206,10 @@ __device__ unsigned cta_scan_count(TickSmem& sm, unsigned c, unsigned* total) {
   }
   if (lane == 31) sm.scan[warp] = incl;
   __syncthreads();
-  unsigned before = 0, all = 0;
-  for (int w = 0; w < NW_; ++w) {
-    unsigned s = sm.scan[w];
-    if ((unsigned)w < warp) before += s;
-    all += s;
-  }
+  const unsigned s = lane < NW_ ? sm.scan[lane] : 0u;
+  const unsigned before = __reduce_add_sync(FULLMASK, lane < warp ? s : 0u);
+  *total = __reduce_add_sync(FULLMASK, s);
   __syncthreads();
-  *total = all;
   return before + incl - c;
 }
 
@@ -533,39 +529,36 @@ __device__ __noinline__ void sweep_levels(const Region& Rs, TickSmem& sm, WS& sW
     R.ctl->par_replayed += L.n_searches;
   }
   sweep_flush(R, L, n);
-  // ---- the position map back to idle
-  for (unsigned i = tid; i < n; i += NT_) R.stamp[key_to_id(R, R.cells[i], flip)] = 0xFFFFFFFFu;
-  // ---- the cells' events in sorted order -> the tick's event logs (program order)
-  __shared__ unsigned s_na, s_ns, s_nc;
-  if (tid == 0) {
-    s_na = 0;
-    s_ns = 0;
-    s_nc = 0;
-  }
-  __syncthreads();
+  // ---- the cells' events in sorted order -> the tick's event logs (program order), and the position map
+  // back to idle. A batch's events are on their way while the one before is logged.
   const unsigned pxy = (unsigned)R.PX * (unsigned)R.PY;
   const bool lr = sW.level_round;
-  unsigned any_chg = 0;
+  unsigned any_chg = 0, s_na = 0, s_ns = 0, s_nc = 0;  // (the same in every thread)
+  unsigned ev_next = tid < n ? R.lv_ev[tid] : 0u, key_next = tid < n ? R.cells[tid] : 0u;
   for (unsigned base = 0; base < n; base += NT_) {
-    const unsigned i = base + tid;
+    const unsigned i = base + tid, ev = ev_next, key = key_next;
+    if (i + NT_ < n) {
+      ev_next = R.lv_ev[i + NT_];
+      key_next = R.cells[i + NT_];
+    }
     unsigned am = 0, fl = 0, cm = 0, src = 0, cid = 0;
     if (i < n) {
-      const unsigned e = R.lv_ev[i];
-      am = e & 0xFFu;
-      cm = (e >> 8) & 0xFFu;
-      fl = e >> 16;
-      cid = key_to_id(R, R.cells[i], flip);
+      am = ev & 0xFFu;
+      cm = (ev >> 8) & 0xFFu;
+      fl = ev >> 16;
+      cid = key_to_id(R, key, flip);
+      R.stamp[cid] = 0xFFFFFFFFu;
       if (am & 1u) src = R.lv_src[i];
       any_chg |= cm;
     }
     const unsigned ns = lr ? 0u : (unsigned)__popc(fl & 3u);
-    unsigned ta, ts, tc;
-    const unsigned oa = cta_scan_count(sm, (unsigned)__popc(am), &ta);
-    const unsigned os = cta_scan_count(sm, ns, &ts);
-    const unsigned oc = cta_scan_count(sm, (unsigned)__popc(cm), &tc);
+    unsigned ta, ts = 0u, os = 0u;  // activations and changes in one scan: at most 8 a cell
+    static_assert(8 * PAR_THREADS < 1 << 16, "two counts in a word");
+    const unsigned oa = cta_scan_count(sm, (unsigned)__popc(am) | (unsigned)__popc(cm) << 16, &ta);
+    if (!lr) os = cta_scan_count(sm, ns, &ts);
     if (i < n) {
       // activations: slot 0 the source (one cell), slots 1..7 wake_around centres
-      unsigned pa = s_na + oa;
+      unsigned pa = s_na + (oa & 0xFFFFu);
       for (int g = 0; g < 8; ++g) {
         if (!((am >> g) & 1u)) continue;
         unsigned w;
@@ -594,7 +587,7 @@ __device__ __noinline__ void sweep_levels(const Region& Rs, TickSmem& sm, WS& sW
           else set_status(R, ST_OOM, 41);
         }
       }
-      unsigned pc = s_nc + oc;
+      unsigned pc = s_nc + (oa >> 16);
       for (int l = 0; l < 8; ++l) {
         if (!((cm >> l) & 1u)) continue;
         unsigned id;
@@ -612,13 +605,9 @@ __device__ __noinline__ void sweep_levels(const Region& Rs, TickSmem& sm, WS& sW
         ++pc;
       }
     }
-    __syncthreads();
-    if (tid == 0) {
-      s_na += ta;
-      s_ns += ts;
-      s_nc += tc;
-    }
-    __syncthreads();
+    s_na += ta & 0xFFFFu;
+    s_ns += ts;
+    s_nc += ta >> 16;
   }
   const unsigned long long c_pd = cta_sum(sm, (unsigned long long)(long long)pd);
   any_chg = __syncthreads_or((int)any_chg);
