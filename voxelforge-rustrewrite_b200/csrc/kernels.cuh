@@ -61,7 +61,14 @@ __device__ void cta_radix_sort(unsigned* keys, unsigned* tmp, unsigned n, unsign
     const int sh = 8 * p;
     for (unsigned i = tid; i < NW_ * 256; i += NT_) hist[i] = 0;
     __syncthreads();
-    for (unsigned i = b0 + lane; i < b1; i += 32) atomicAdd(&hist[warp * 256 + (((src[i] - kmin) >> sh) & 255u)], 1u);
+    for (unsigned i = b0 + lane; i < b1; i += 128) {  // four loads under way at a time
+      unsigned k[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) k[q] = i + 32u * q < b1 ? src[i + 32u * q] : 0u;
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (i + 32u * q < b1) atomicAdd(&hist[warp * 256 + (((k[q] - kmin) >> sh) & 255u)], 1u);
+    }
     __syncthreads();
     // offsets: digit-major, warp-minor
     if (tid < 256) {
@@ -98,10 +105,16 @@ __device__ void cta_radix_sort(unsigned* keys, unsigned* tmp, unsigned n, unsign
       }
     }
     __syncthreads();
+    unsigned ahead[3];  // the next three keys are on their way
+#pragma unroll
+    for (int q = 0; q < 3; ++q) ahead[q] = b0 + 32u * q + lane < b1 ? src[b0 + 32u * q + lane] : 0u;
     for (unsigned base = b0; base < b1; base += 32) {
       unsigned i = base + lane;
       bool valid = i < b1;
-      unsigned k = valid ? src[i] : 0u;
+      const unsigned k = ahead[0];
+      ahead[0] = ahead[1];
+      ahead[1] = ahead[2];
+      ahead[2] = i + 96u < b1 ? src[i + 96u] : 0u;
       unsigned d = valid ? (((k - kmin) >> sh) & 255u) : (256u + lane);
       unsigned peers = __match_any_sync(FULLMASK, d);
       unsigned rank = __popc(peers & lanemask_lt());
