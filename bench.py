@@ -48,7 +48,7 @@ def parse():
     ap.add_argument("--impl", default="ours", choices=["ours", "reference"])
     ap.add_argument("--workload", type=int, default=2)
     ap.add_argument("--scale", type=float, default=1.0)
-    ap.add_argument("--engine", type=int, default=1, help="0: one-warp sweep, 1: parallel sweep")
+    ap.add_argument("--engine", type=int, default=1, help="accepted by the library, without effect")
     ap.add_argument("--gate", type=int, default=4 | (1 << 8), help="same-layer gate | lower-layer cone << 8")
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--no-variants", action="store_true")
@@ -403,7 +403,7 @@ def ours(args):
         "data": "synthetic",
         "config": config(args),
         "engine": {"engine": args.engine, "gate": args.gate,
-                   "sweep": "parallel exact sweep, rows on 16 warps of one CTA" if args.engine else "one-warp exact sweep + 7 prefetching warps"},
+                   "sweep": "exact sweep in rounds over the cells' dependencies, 16 warps of one CTA"},
         "e2e": {"value": e2e, "unit": UNIT, "h2d_bytes_per_step": h2d // max(args.steps, 1), "d2h_bytes_per_step": d2h // max(args.steps, 1),
                 "steps": args.steps, "timer": "host wall clock", "same_ticks_as_value": True, "same_end_state": bool(e2e_same)},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak, "traffic": STEP_DRAM_BYTES,

@@ -210,34 +210,21 @@ int vf_mlp_forward(vf_mlp* m, const void* dev_x_f16, uint64_t n, float* dev_prob
 int vf_mlp_grads(vf_mlp* m, const void* dev_x_f16, const float* dev_y, uint64_t n, float* host_grads, void* stream);
 int vf_mlp_train_step(vf_mlp* m, const void* dev_x_f16, const float* dev_y, uint64_t n, float lr, float* host_loss, void* stream);
 
-/* Launch knobs of the one-warp sweep (the autotuner's search space; results never depend on them):
- * warps prefetching footprints (1..7) and how many cells ahead of the sweep they run (1..64). */
+/* Launch knobs that earlier sweeps had (prefetching warps, 1..7, and their distance, 1..64): checked and
+ * without effect. */
 int vf_fluid_set_tuning(vf_fluid* h, int32_t producers, int32_t depth);
 
-/* Which sweep runs FluidSim::tick's cell loop (src/fluid.rs:584-651); results never depend on it.
- * engine 2 (default): chosen per tick call from the last calls' pressure-search entries per drained
- * cell (above 1.5: engine 0, else engine 1; a batch launch uses its first handle's last choice).
- * engine 0: one warp walks the sorted cells (8 warps per region: the sweep and prefetchers).
- * engine 1: all 16 warps of the region's CTA walk rows of the sorted order at once, each
- * cell waiting for the earlier cells it conflicts with; pressure searches read cells as of their own
- * position; a segment whose order the schedule cannot keep is undone and replayed by one warp.
- * gate: bits 0-7 (0..31, default 4) before a pressure search, wait for the earlier cells of its layer
- * within this Chebyshev distance; bits 8-15 (0..31, 0 = the same value, default 1) a cell of a segment with
- * pulls starts only when rows in work on lower layers within that many rows have passed its x plus
- * that distance (fewer replays, less overlap); bits 16-20 (0 = 16, else 8..16) the warps of the
- * region's CTA (for measuring the speed-up against warps); bit 21: pressure searches leave the four
- * search contexts in shared memory unused and run on each warp's context in global memory (the path
- * a search takes when the shared ones are all in use; for tests). spin_cap (> 0, default 2^24): iterations of any device
- * wait (both engines, and the levelling's brick materialisation) before the tick gives up with
- * VF_ERR_TIMEOUT; the kernel then returns and the handle can only be destroyed.
+/* Knobs of FluidSim::tick's cell loop (src/fluid.rs:584-651); results never depend on them. One sweep runs
+ * whatever `engine` says (0, 1 or 2, the default; 1 is refused for domain sides of 65536 and more).
+ * gate: bits 0-7 and 8-15 (0..31 each) and bit 21 are accepted and without effect; bits 16-20 (0 = 16, else
+ * 8..16) the warps of the region's CTA. spin_cap (> 0, default 2^24): rounds of the sweep before the
+ * tick gives up with VF_ERR_TIMEOUT; the kernel then returns and the handle can only be destroyed.
  * No reference counterpart: a device scheduling knob of this library. */
 int vf_fluid_set_sweep(vf_fluid* h, int32_t engine, int32_t gate, uint64_t spin_cap);
 
-/* Parallel-sweep counters summed over ticks: budget segments run, segments undone and replayed in
- * sorted order, cells replayed, and (conflicts3, 3 entries, optional) the conflicts that caused the
- * replays: a later reader of a pull's source had started, a later pull had read the source, more
- * cells of a segment attempted a pull than the tick's budget had left (cells that earlier pulls
- * took below full). No reference counterpart (diagnostics). */
+/* Sweep counters summed over ticks: rounds (in segments), pressure searches that were run again because an
+ * earlier cell had yet to write what they read (in rollbacks), pressure searches (in replayed); conflicts3
+ * (3 entries, optional) zeros: nothing is undone. No reference counterpart (diagnostics). */
 int vf_fluid_sweep_stats(vf_fluid* h, uint64_t* segments, uint64_t* rollbacks, uint64_t* replayed, uint64_t* conflicts3);
 
 /* Lower the per-tick event-log capacities (activations, level seeds, voxel changes; each 1 .. its
@@ -246,11 +233,9 @@ int vf_fluid_sweep_stats(vf_fluid* h, uint64_t* segments, uint64_t* rollbacks, u
  * lower values serve tests of the overflow path. No reference counterpart. */
 int vf_fluid_set_log_caps(vf_fluid* h, uint32_t act, uint32_t seed, uint32_t chg);
 
-/* Parallel-sweep SM cycle counters summed over ticks (18 entries): prepass, segments, rollbacks,
- * event logs; then summed over warps: dependency waits, blocked starts, footprint loads, pulls,
- * writes, cells run, row fetches, worker total, lower-layer (cone) waits, gate waits, pressure
- * searches run, search rounds, cycles in search reads, cycles in source writes. No reference
- * counterpart (diagnostics). */
+/* Sweep SM cycle counters summed over ticks (18 entries): 0 prepass, 1 rounds and pulls, 3 the atlas and the
+ * event logs, 7 searches by all warps, 8 wide rounds; 9 drained cells, 14 pressure searches, 15 rounds; the others
+ * zero. No reference counterpart (diagnostics). */
 int vf_fluid_sweep_profile(vf_fluid* h, uint64_t* out18);
 
 /* Non-blocking host edits whose cell lists already live in device memory (x,y,z int32 triples),

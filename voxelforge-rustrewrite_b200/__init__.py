@@ -387,12 +387,12 @@ class FluidSim:
         return bool(ch.value)
 
     def set_tuning(self, producers: int, depth: int):
-        """Launch knobs of the one-warp sweep (prefetch warps, prefetch distance); results never depend on them."""
+        """Launch knobs that earlier sweeps had (prefetch warps 1..7, distance 1..64): checked, without effect."""
         self._check(lib().vf_fluid_set_tuning(self.h, producers, depth), "set_tuning")
 
     def set_sweep(self, engine: int = 2, gate: int = 4 | (1 << 8), spin_cap: int = 1 << 24):
-        """Which sweep runs (0 one warp, 1 all warps of the region's CTA, 2 chosen per call), the parallel sweep's pull
-        gate radius and the iteration cap of device waits; results never depend on them."""
+        """Knobs of the sweep: `engine` is checked and without effect, bits 16-20 of `gate` are the warps of the region's
+        CTA (0: 16), spin_cap the rounds after which a tick gives up; results never depend on them."""
         self._check(lib().vf_fluid_set_sweep(self.h, engine, gate, spin_cap), "set_sweep")
 
     def set_log_caps(self, act: int, seed: int, chg: int):
@@ -404,13 +404,13 @@ class FluidSim:
                      "source_writes")
 
     def sweep_profile(self) -> dict:
-        """Parallel-sweep SM cycle counters summed over ticks (the per-cell ones also over warps)."""
+        """Sweep counters summed over ticks (vf_fluid_sweep_profile: SM cycles, and counts of cells, searches, rounds)."""
         a = (C.c_uint64 * 18)()
         self._check(lib().vf_fluid_sweep_profile(self.h, a), "sweep_profile")
         return dict(zip(self.SWEEP_PROFILE, map(int, a)))
 
     def sweep_stats(self) -> dict:
-        """Parallel-sweep counters over all ticks: segments, segments replayed in order, cells replayed."""
+        """Sweep counters over all ticks: rounds (segments), searches run again (rollbacks), searches (replayed)."""
         a, b, c = C.c_uint64(), C.c_uint64(), C.c_uint64()
         k = (C.c_uint64 * 3)()
         self._check(lib().vf_fluid_sweep_stats(self.h, C.byref(a), C.byref(b), C.byref(c), k), "sweep_stats")

@@ -1,11 +1,8 @@
 """Autotuner for the tick's launch knobs.
 
 The knobs change how fast a tick runs, never what it computes (every setting is bit-exact):
-  * engine    - 0: the one-warp sweep with prefetching warps (256 threads per region);
-                1: the parallel sweep, rows of the sorted order on 16 warps (512 threads per region)
-  * gate      - engine 1: the pull gate / lower-layer cone radius in cells (the schedule's shape)
-  * producers - engine 0: warps that prefetch upcoming cells' footprints into the shared-memory ring
-  * depth     - engine 0: how many cells ahead of the sweep they may run (1..64)
+  * engine, producers, depth - knobs of earlier sweeps: accepted, without effect
+  * gate      - bits 16-20: warps of the region's CTA (8..16, 0 = 16); the other bits without effect
   * ticks_per_launch - ticks one persistent launch runs before returning to the host
 
 A candidate is timed on fresh copies of the workload's regions: `warmup` ticks with the default
@@ -19,7 +16,7 @@ import os
 from pathlib import Path
 
 DEFAULT = {"engine": 1, "gate": 4 | (1 << 8), "producers": 7, "depth": 64, "ticks_per_launch": 10}
-CANDIDATES = [dict(DEFAULT, engine=0, producers=p, depth=d) for p in (2, 7) for d in (16, 64)] + [dict(DEFAULT, gate=g) for g in (2, 4, 4 | (1 << 8), 8)]
+CANDIDATES = [dict(DEFAULT, gate=DEFAULT["gate"] | w << 16) for w in (0, 8, 12)]
 
 
 def apply(sim, knobs: dict):

@@ -442,7 +442,7 @@ int vf_fluid_upload_world(vf_fluid* h, int32_t nx, int32_t ny, int32_t nz, int32
   if ((rc = dalloc(h, &R.stamp, ncells, false))) return rc;
   if ((rc = dalloc(h, &R.last_woken, cap))) return rc;
   CK(cudaMemsetAsync(R.stamp, 0xFF, ncells * 4, h->stream));
-  // parallel sweep: per-cell records, events, lists
+  // the sweep's per-cell records, events, lists
   if ((rc = dalloc(h, &R.lv, MAX_CELLS_PER_TICK, false))) return rc;
   if ((rc = dalloc(h, &R.lv_old, MAX_CELLS_PER_TICK, false))) return rc;
   if ((rc = dalloc(h, &R.lv_ev, MAX_CELLS_PER_TICK, false))) return rc;
@@ -1022,7 +1022,6 @@ int vf_fluid_reset(vf_fluid* h) {  // fluid.rs:318-320: the fluid's tables only
   z.bfs_visits = c.bfs_visits;
   z.level_cells_total = c.level_cells_total;
   z.activations = c.activations;
-  z.seg_epoch = c.seg_epoch;
   z.par_segments = c.par_segments;
   z.par_rollbacks = c.par_rollbacks;
   z.par_replayed = c.par_replayed;

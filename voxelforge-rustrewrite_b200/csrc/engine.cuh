@@ -47,25 +47,15 @@ struct Ctl {
   unsigned int last_cells, last_level_cells, changed, mark_ntiles;
   int status;
   unsigned int err_info;
-  unsigned int seg_epoch;           // parallel sweep: segments begun so far (tags versions and reads)
-  unsigned int ptn;                 // parallel sweep: cells listed in Region::ptlist this tick
-  unsigned int pxn;                 // parallel sweep: positions listed in Region::pxlist this tick
-  unsigned int att_ratio;           // parallel sweep: pull attempts per possible attempter of the
-                                    // last tick's completed segments, x 65536 (0: none yet)
   unsigned int ndetached;           // ring worlds: partial entries kept for evicted chunks (detbits set)
-  // parallel sweep diagnostics, summed over ticks: budget segments run, segments rolled back and
-  // replayed in order by one warp, cells replayed
+  // sweep diagnostics, summed over ticks: rounds, searches run again, searches; par_conflicts: zero
   unsigned long long par_segments, par_rollbacks, par_replayed;
-  // conflicts by kind: a later reader of a pull's source had started, a later pull had read the
-  // source, more cells of a segment attempted a pull than the budget had left
   unsigned long long par_conflicts[4];
-  // parallel sweep cycle counters: 0 prepass, 1 segments (workers), 2 rollbacks, 3 event logs;
-  // summed over warps: 4 dependency waits, 5 start (blocked), 6 footprint loads, 7 pulls (gate and
-  // search), 8 writes, 9 cells run, 10 between cells (row fetch), 11 worker total
-  unsigned long long pprof[18];  // + 12 cone waits, 13 gate waits, 14 searches, 15 rounds, 16 reads, 17 source writes
+  // sweep cycle counters: 0 prepass, 1 rounds and pulls, 3 atlas and event logs, 7 searches by all warps, 8 wide rounds;
+  // counts: 9 drained cells, 14 searches, 15 rounds
+  unsigned long long pprof[18];
   // SM cycles spent per tick phase, summed over ticks (clock64 on the SM running the region):
-  // 0 drain, 1 sort, 2 sweep, 3 sweep waits for prefetch, 4 pressure pulls, 5 activation logs,
-  // 6 writes, 7 seed commit, 8 levelling, 9 activation commit, 10 change commit, 11 mark clear
+  // 0 drain, 1 sort, 2 sweep, 7 seed commit, 8 levelling, 9 activation commit, 10 change commit, 11 mark clear
   unsigned long long prof[16];
 };
 constexpr int NPROF = 16;
@@ -110,7 +100,7 @@ struct Region {
   unsigned int ev_act_cap, ev_seed_cap, ev_chg_cap;
   unsigned int* stamp;       // ncells: first event index per cell during a commit (0xFFFFFFFF idle)
   unsigned int* last_woken;  // atlas_cap: last tick a cell of the slot's brick was drained (0 = never)
-  // ---- parallel sweep (per tick; `stamp` doubles as the cell -> sorted position map), all of
+  // ---- sweep (per tick; `stamp` doubles as the cell -> sorted position map), all of
   // MAX_CELLS_PER_TICK entries (two of the lists)
   LvCell* lv;              // what a round reads of each drained cell
   LvOld* lv_old;           // the volumes a cell of the gate layer replaced
@@ -122,7 +112,7 @@ struct Region {
   unsigned short* lv_park; // ready cells above the gate layer (two)
   unsigned* pextra;        // bits: full cells a pull took below 1 - 1e-4
   unsigned* pxlist;        // their positions
-  unsigned* rb;            // ncells: claims of the levelling's flood fill (0xFFFFFFFF idle)
+  unsigned* rb;            // ncells: claims of the levelling's flood fill and of the edits (0xFFFFFFFF idle)
   unsigned* detbits;       // ring worlds: ncells bits, the cell's partial entry is kept for an evicted chunk
   Ctl* ctl;
 };

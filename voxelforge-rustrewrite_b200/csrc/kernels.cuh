@@ -343,7 +343,7 @@ __device__ void commit_chgs(const Region& R, unsigned n) {
   __syncthreads();
 }
 
-// ------------------------------------------------------------------- the parallel sweep
+// ------------------------------------------------------------------- the sweep
 // Sum of a per-thread value over the CTA (all threads call).
 __device__ unsigned long long cta_sum(TickSmem& sm, unsigned long long v) {
   for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(FULLMASK, v, o);
