@@ -877,7 +877,8 @@ __device__ __noinline__ void level_finish_cta(const Region& R, TickSmem& sm, WS&
 // A small layer's flood fill by one warp, without touching the marks: the cells in the reference's
 // order, and every cell it tested (a set: the marks it would leave). Several run side by side; the
 // layers of one batch are the same or disjoint (their members do not change while it lasts), so the
-// smallest cell id tells them apart.
+// smallest cell id tells them apart. Bound by the longest layer of a group, ~1,200 cycles for each
+// one or two of its entries (ring rain: 14.4 M cycles of levelling with one a step, 11.4 with two).
 constexpr unsigned FILL_CELLS = 64, FILL_SLOTS = 512;
 static_assert(4 * FILL_CELLS + 1 < FILL_SLOTS, "tested cells of a small layer");
 enum FillKind { FK_KEEP = 0, FK_LEVEL = 1, FK_DRAIN = 2, FK_BIG = 3, FK_DUP = 4 };
@@ -914,21 +915,25 @@ __device__ void level_fill_small(const Region& R, LevelFill& F, unsigned sid) {
   }
   __syncwarp();
   unsigned len = 1, kind = FK_KEEP, mn = sid;
-  for (unsigned i = 0; i < len; ++i) {
+  // two queue entries a step where two wait: lanes 0..11 the first, 12..23 the second; of an entry's lanes, side
+  // d = lane / 3, its cell (j = 0), the one below (1) and above (2)
+  const unsigned half = lane >= 12u ? 1u : 0u, r = lane - 12u * half;
+  const int d = (int)r / 3, j = (int)r % 3;
+  int dx = 0, dz = 0;
+  if (lane < 24u) side4(d, dx, dz);
+  for (unsigned i = 0, step; i < len; i += step) {
+    step = min(len - i, 2u);
     int x, y, z;
-    dom_xyz(R, F.id[i], x, y, z);
-    // lanes 0..11: side d = lane / 3, its cell (j = 0), the one below (1) and above (2)
-    const int d = (int)lane / 3, j = (int)lane % 3;
-    int dx = 0, dz = 0;
-    if (lane < 12u) side4(d, dx, dz);
+    dom_xyz(R, F.id[i + (half < step ? half : 0u)], x, y, z);
     const int nx = x + dx, nz = z + dz;
-    const bool skip = lane >= 12u || (R.ring_w == 0 && (nx < 0 || nz < 0));
+    const bool skip = lane >= 24u || half >= step || (R.ring_w == 0 && (nx < 0 || nz < 0));
+    const bool look = !skip && j == 0 && in_dom(R, nx, y, nz);
+    const unsigned nid = look ? dom_id(R, nx, y, nz) : EMPTY_ID;
     bool seen = true;
-    unsigned nid = EMPTY_ID;
-    if (!skip && j == 0 && in_dom(R, nx, y, nz)) {
-      nid = dom_id(R, nx, y, nz);
-      seen = mark_test(R, nx, y, nz) || test(nid);
-    }
+    if (look) seen = mark_test(R, nx, y, nz);
+    // a cell both entries test is the first one's
+    const unsigned peers = __match_any_sync(FULLMASK, nid);
+    if (look && !seen) seen = (peers & lanemask_lt()) != 0u || test(nid);
     const unsigned c = skip ? DC_SOLID : dense_at(R, nx, y + (j == 1 ? -1 : (j == 2 ? 1 : 0)), nz);
     const bool sol = dc_solid(c);
     const float v = dc_level(c);
