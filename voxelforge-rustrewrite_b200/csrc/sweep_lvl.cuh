@@ -40,9 +40,9 @@ constexpr int MAX_WARPS = 16;                  // warps of a CTA running the swe
 constexpr unsigned SOLO_CELLS = 4;             // a list this short is run by one warp (eight lanes per cell)
 constexpr unsigned SOLO_ENTRIES = 6;           // queue entries one warp examines per search round
 constexpr unsigned SOLO_WAIT = SOLO_ENTRIES;   // a search with more entries waiting goes to all warps
-constexpr unsigned VIS_SLOTS = 2048;           // visited set, emptied when VIS_FULL cells have been added
-constexpr int VIS_SHIFT = 21;                  // hash bits kept: 32 - log2(VIS_SLOTS)
-constexpr unsigned VIS_FULL = 768;             // one search adds <= 6 + 512 + one round's 5 per entry (480)
+constexpr unsigned VIS_SLOTS = 4096;           // visited set, emptied when VIS_FULL cells have been added
+constexpr int VIS_SHIFT = 20;                  // hash bits kept: 32 - log2(VIS_SLOTS)
+constexpr unsigned VIS_FULL = 1536;            // one search adds <= 6 + 512 + one round's 5 per entry (480)
 constexpr unsigned VIS_RANKS = 4096;           // ranks of one search: 6 + 5 * 512 at most
 constexpr unsigned NGROUPS = (MAX_CELLS_PER_TICK + 31) / 32;
 constexpr unsigned LIST_CAP = 2048;   // a round's list kept in shared memory; the rest goes to global
