@@ -478,7 +478,7 @@ __device__ __noinline__ void sweep_levels(const Region& Rs, TickSmem& sm, WS& sW
   }
   __syncthreads();
   if (warp == 0) {
-    HeadState H{n, 0u, 0u, 0u, -1, 0u};
+    HeadState H{n, 0u, 0u, 0u, -1};
     lv_head(R, L, n, H);
     if (lane == 0) L.h = H;
   }

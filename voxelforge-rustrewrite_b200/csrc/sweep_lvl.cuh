@@ -94,7 +94,6 @@ struct HeadState {
   unsigned blk;         // 1 + the cell its search waits for (0: none)
   unsigned test;        // lv_prune: 0 to be tested, 1 + the cell the test waits for, or TEST_FAILED
   int gate;             // its layer: cells above it wait
-  unsigned lend;        // first position after that layer
 };
 constexpr unsigned TEST_FAILED = 0xFFFFFFFFu;
 
@@ -1010,20 +1009,7 @@ __device__ __forceinline__ void lv_head(const Region& R, LvSmem& L, unsigned n, 
   const int fl = __ffs(any) - 1;
   H.word = w + (unsigned)fl;
   H.head = H.word * 32u + (unsigned)__ffs(__shfl_sync(FULLMASK, P, fl)) - 1u;
-  if (H.head >= H.lend) {  // a new gate layer: its first position after the layer, by a 32-way search
-    H.gate = (int)(R.lv[H.head].ye & YE_Y);
-    const unsigned lim = (unsigned)(H.gate + 1) * (unsigned)R.PZ * (unsigned)R.PX;
-    unsigned lo = H.head, hi = n;  // cells[lo] is on the layer; the answer lies in (lo, hi]
-    while (hi - lo > 1u) {
-      const unsigned st = (hi - lo + 31u) / 32u, p = lo + (lane + 1u) * st;
-      const unsigned b = __ballot_sync(FULLMASK, p < hi && R.cells[p] < lim);
-      const unsigned k = (unsigned)__popc(b);  // keys ascend: the first k probes are on the layer
-      const unsigned nlo = lo + k * st, nhi = min(hi, lo + (k + 1u) * st);
-      lo = nlo;
-      hi = nhi;
-    }
-    H.lend = hi;
-  }
+  H.gate = (int)(R.lv[H.head].ye & YE_Y);  // (its search or its test reads the record next)
 }
 
 // The first pp cell has yet to have its turn: can it still find a start cell then? A full neighbour
