@@ -520,7 +520,7 @@ __device__ __noinline__ void sweep_levels(const Region& Rs, TickSmem& sm, WS& sW
       __syncthreads();
     } else {
       const long long c0 = clock64();
-      pd += lv_wide(Rs, L, n, gate, cap);
+      pd += L.cnt[L.cc] >= THREAD_CELLS ? lv_long(Rs, L, n, gate, cap) : lv_wide(Rs, L, n, gate, cap);
       t_wide += clock64() - c0;
     }
   }

@@ -483,6 +483,126 @@ __device__ __forceinline__ float lv_cells(const Region& R, LvSmem& L, const Lane
   return vol;
 }
 
+// The same for a long list, one thread per cell, warp-collective: a warp's instructions then serve 32
+// cells instead of four, and it is the number of instructions that bounds a round of hundreds of cells
+// (the chain of one thread, twelve counts and seven cells, is longer: rounds of fewer than THREAD_CELLS take
+// eight lanes).
+constexpr unsigned THREAD_CELLS = 192;  // lake: 5.1 M cycles of rounds from 192 on, 6.0 from 256 on, 5.9 without; ring rain 7.9 against 14.4
+__device__ __forceinline__ void lv_cell_thread(const Region& R, LvSmem& L, bool has, unsigned i, int gate, unsigned kp, unsigned nb, unsigned nc, unsigned pb,
+                                               int& pd) {
+  const float FULL = full_level();
+  const unsigned lane = lane_id();
+  uint4 ra = make_uint4(~0u, ~0u, ~0u, ~0u), rb = make_uint4(~0u, ~0u, 0u, 0u);
+  if (has) {
+    ra = reinterpret_cast<const uint4*>(R.lv + i)[0];
+    rb = reinterpret_cast<const uint4*>(R.lv + i)[1];
+  }
+  const unsigned w[6] = {ra.x, ra.y, ra.z, ra.w, rb.x, rb.y}, ye = rb.w;
+  const int cid = (int)rb.z, y = (int)(ye & YE_Y);
+  const bool pp = has && i < kp && bit_of(L.pp, i);
+  unsigned u[7];
+#pragma unroll
+  for (int l = 0; l < 7; ++l) {
+    u[l] = DC_SOLID;
+    if (l == 2 ? pp : has) u[l] = R.dense[cid + fp_id(R, l)];
+  }
+  if (pp && dc_volume(u[0]) < FULL) {  // a cell that attempts a pull and has a start cell waits for the pull
+    bool start = false;
+#pragma unroll
+    for (int l = 2; l < 7; ++l) start |= ((ye >> (25 + l)) & 1u) && !dc_solid(u[l]) && dc_volume(u[l]) >= FULL;
+    if (start) has = false;
+  }
+  // ---- successors whose last earlier cell this was (succ_offset's order: 6..10 one layer up, 11 two)
+  unsigned ready = 0;
+#pragma unroll
+  for (int q = 0; q < 12; ++q) {
+    const unsigned a = (q & 1) ? w[q >> 1] >> 16 : w[q >> 1] & 0xFFFFu, sh = (a & 3u) * 8u;
+    unsigned o = 0;
+    if (has && a != NOSUCC) o = atomicSub(&L.dep[a >> 2], 1u << sh);
+    ready |= ((o >> sh) & 0xFFu) == 1u ? 1u << q : 0u;
+  }
+  // ---- the rules, as in lv_cells
+  const float v0 = dc_volume(u[0]);
+  const bool below_solid = dc_solid(u[1]);
+  const float bv = below_solid ? 0.0f : dc_volume(u[1]);
+  float vol = v0;
+  const bool live = has && vol > 0.0f;
+  const float ff = fminf(vol, __fsub_rn(1.0f, bv));
+  const bool w_below = live && !below_solid && ff > 1e-6f;
+  const float below_new = __fadd_rn(bv, ff);
+  vol = w_below ? __fsub_rn(vol, ff) : vol;
+  const float below_after = w_below ? (below_new >= FULL ? 1.0f : below_new) : bv;
+  const bool spread = live && vol > MIN_SPREAD && (below_solid || below_after >= FULL);
+  float wv[7], v[7], run = vol;
+  bool wr[7];
+  unsigned am = w_below ? 4u : 0u;
+#pragma unroll
+  for (int l = 3; l < 7; ++l) {
+    const bool solid = dc_solid(u[l]);
+    v[l] = solid ? 0.0f : dc_volume(u[l]);
+    const float f = __fmul_rn(__fsub_rn(vol, v[l]), 0.2f);
+    wr[l] = spread && !solid && !(v[l] >= vol) && !(f < MIN_FLOW) && !(__fsub_rn(vol, f) < MIN_SPREAD * 0.5f);
+    wv[l] = __fadd_rn(v[l], f);
+    run = __fsub_rn(run, wr[l] ? f : 0.0f);
+    am |= wr[l] && f > SLEEP ? 1u << l : 0u;
+  }
+  run = run < EVAPORATE ? 0.0f : run;
+  const float dv = fabsf(__fsub_rn(run, v0));
+  am |= live && dv > SLEEP ? 0x80u : 0u;
+  v[0] = v0;
+  v[1] = bv;
+  wr[0] = live && dv > 1e-7f;
+  wv[0] = run;
+  wr[1] = w_below;
+  wv[1] = below_new;
+  unsigned pm = 0, cm = 0;
+#pragma unroll
+  for (int l = 0; l < 7; ++l) {
+    if (l == 2) continue;
+    const bool is_water = (int)u[l] > 0, mid = wv[l] > 1e-6f && wv[l] < FULL, had = v[l] > 0.0f && v[l] < 1.0f;
+    const bool wet = wv[l] >= (is_water ? HIDE_BELOW : SHOW_AT);
+    const unsigned nu = mid ? (__float_as_uint(wv[l]) | (wet ? 0u : DC_AIR)) : (wet ? DC_FULL : 0u);
+    if (wr[l] && nu != u[l]) {
+      R.dense[cid + fp_id(R, l)] = nu;
+      pd += (mid ? 1 : 0) - (had ? 1 : 0);
+      pm |= 1u << l;
+      cm |= wet != is_water ? 1u << l : 0u;
+    }
+  }
+  if (has && y == gate) {  // (a search asks for slots 0 and 3..6)
+    float4* o = reinterpret_cast<float4*>(R.lv_old + i);
+    o[0] = make_float4(v[0], v[1], 0.0f, v[3]);
+    o[1] = make_float4(v[4], v[5], v[6], 0.0f);
+  }
+  if (has) {
+    R.lv_ev[i] = (am & 0xFCu) | ((am & 0x80u) << 9) | cm << 8;
+    reinterpret_cast<volatile unsigned char*>(L.dep)[i] = (unsigned char)(DONE | pm);
+    if (pp) atomicAnd(&L.pp[i >> 5], ~(1u << (i & 31u)));
+  }
+  // ---- the ready ones to the next list, or parked above the gate: places by a scan over the warp
+  const unsigned shut = (y + 1 > gate ? 0x7C0u : 0u) | (y + 2 > gate ? 0x800u : 0u), go = ready & ~shut, stay = ready & shut;
+  const unsigned both = (unsigned)__popc(go) | (unsigned)__popc(stay) << 16;
+  unsigned pre = both;
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned x = __shfl_up_sync(FULLMASK, pre, o);
+    if (lane >= (unsigned)o) pre += x;
+  }
+  unsigned t = 0, p = 0;
+  if (lane == 31u) {
+    if (pre & 0xFFFFu) t = atomicAdd(&L.cnt[nc], pre & 0xFFFFu);
+    if (pre >> 16) p = atomicAdd(&L.park_n[pb], pre >> 16);
+  }
+  t = __shfl_sync(FULLMASK, t, 31) + ((pre - both) & 0xFFFFu);
+  p = __shfl_sync(FULLMASK, p, 31) + ((pre - both) >> 16);
+#pragma unroll
+  for (int q = 0; q < 12; ++q) {
+    const unsigned a = (q & 1) ? w[q >> 1] >> 16 : w[q >> 1] & 0xFFFFu;
+    if ((go >> q) & 1u) list_put(R, L, nb, t++, a);
+    if (q >= 6 && ((stay >> q) & 1u)) park_put(R, pb, p++, a);
+  }
+  __syncwarp();
+}
+
 // After the sweep: every cell it wrote (the slots in the dependency bytes, the pulls' sources) to the
 // atlas, all at once, in batches of one drained cell per thread in sorted order. Bricks written for
 // the first time get their slots in the program's order (a pull's source before its cell). All threads.
@@ -1145,8 +1265,41 @@ __device__ __noinline__ int lv_solo(const Region& Rs, LvSmem& L, unsigned n, int
   return pd;
 }
 
+// Rounds of THREAD_CELLS cells and more, by the whole CTA, one thread per cell: one while pulls are still possible
+// (warp 0 looks after every round), else as long as the lists are that long. All threads; ends with a barrier.
+// Returns the thread's change in partial entries. (The long rounds, those of four cells a warp and warp 0's work
+// are functions of their own for the registers: one holding two of them slowed the shorter one by 6-15%.)
+__device__ __noinline__ int lv_long(const Region& Rs, LvSmem& L, unsigned n, int gate, unsigned long long cap) {
+  const Region R = Rs;
+  const unsigned tid = threadIdx.x;
+  const bool alive = L.h.head < n;
+  const unsigned pb = L.pb, kp = L.kp;
+  unsigned cur = L.cur, cc = L.cc, rounds = L.rounds, fcount = min(L.cnt[cc], MAX_CELLS_PER_TICK);
+  int pd = 0;
+  do {
+    const unsigned nc = cc == 2u ? 0u : cc + 1u, zc = nc == 2u ? 0u : nc + 1u;
+    if (tid == 0) L.cnt[zc] = 0u;
+    for (unsigned at = tid & ~31u; at < fcount; at += blockDim.x) {
+      const unsigned t = at + lane_id(), i = t < fcount ? list_get(R, L, cur, t) : 0u;
+      lv_cell_thread(R, L, t < fcount && !cell_done(L, i), i, gate, kp, cur ^ 1u, nc, pb, pd);
+    }
+    __syncthreads();
+    cur ^= 1u;
+    cc = nc;
+    ++rounds;
+    fcount = min(L.cnt[cc], MAX_CELLS_PER_TICK);
+  } while (!alive && fcount >= THREAD_CELLS && rounds < cap);
+  __syncthreads();  // everybody has read the count
+  if (tid == 0) {
+    L.cur = cur;
+    L.cc = cc;
+    L.rounds = rounds;
+  }
+  return pd;
+}
+
 // Rounds by the whole CTA, four cells a warp at a time: one while pulls are still possible (warp 0 looks
-// after every round), else until the list is short. All threads; ends with a barrier. A long list's
+// after every round), else until the list is short or long. All threads; ends with a barrier. A long list's
 // records are fetched two steps ahead and its volumes one (a function of its own for the registers
 // that takes): ring rain 18.6 -> 13.8 M cycles of its rounds, lake 7.6 -> 6.3 M. Returns the thread's change in
 // partial entries.
@@ -1188,7 +1341,7 @@ __device__ __noinline__ int lv_wide(const Region& Rs, LvSmem& L, unsigned n, int
     cc = nc;
     ++rounds;
     fcount = min(L.cnt[cc], MAX_CELLS_PER_TICK);
-  } while (!alive && fcount > SOLO_CELLS && rounds < cap);
+  } while (!alive && fcount > SOLO_CELLS && fcount < THREAD_CELLS && rounds < cap);
   if ((T.seen | T.a | T.b) >> 31) set_status(R, ST_RANGE, 53);
   __syncthreads();  // everybody has read the count
   if (tid == 0) {
