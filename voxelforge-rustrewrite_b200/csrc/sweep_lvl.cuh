@@ -1,5 +1,5 @@
 // Exact sweep: the body of FluidSim::tick (src/fluid.rs:584-651) over the region's CTA, eight lanes per
-// cell, with results bit-identical to the reference's sequential loop.
+// cell (one thread in long rounds), with results bit-identical to the reference's sequential loop.
 //
 // The order of the sequential loop matters only between cells that touch a common cell, so the
 // sweep runs in rounds over the dependency graph of the drained cells:
@@ -29,7 +29,7 @@
 // cells -> plan -> stores -> successor counts -> barrier), on one SM per region, and between the rounds warp 0's
 // chain of pulls: a lone warp takes ~8 cycles for each dependent instruction (a cell 1,700, a search round
 // 1,600, a search's start 1,200 cycles). Dam break, first 16 ticks: 817 M SM cycles when every cell waited
-// for its conflicts in rows of the sorted order and conflicting pulls were undone, 206 M here.
+// for its conflicts in rows of the sorted order and conflicting pulls were undone, 204 M here.
 #pragma once
 #include "engine_dev.cuh"
 
