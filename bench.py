@@ -407,7 +407,7 @@ def ours(args):
         "e2e": {"value": e2e, "unit": UNIT, "h2d_bytes_per_step": h2d // max(args.steps, 1), "d2h_bytes_per_step": d2h // max(args.steps, 1),
                 "steps": args.steps, "timer": "host wall clock", "same_ticks_as_value": True, "same_end_state": bool(e2e_same)},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak, "traffic": STEP_DRAM_BYTES,
-                     "traffic_source": "one-off ncu capture of one step's k_tick_par launch (dram__bytes read + write)",
+                     "traffic_source": "one-off ncu capture of one step's k_tick_par launch (dram__bytes read + write), taken with the sweep in rows",
                      "peak_kind": peak_kind, "kernel": "k_tick_par" if args.engine else "k_tick", "alg_bytes_per_step": alg_bytes / args.steps},
         "gpu_launches": args.steps,
         "clocks": clk.summary(),
