@@ -116,3 +116,17 @@ def test_slots_do_not_change_from_run_to_run(vf):
         return h.hexdigest()
 
     assert features() == features()
+
+
+# cells side by side: one word of counts holds cells that finish and cells that are counted down
+@pytest.mark.parametrize("width", [1, 2, 3, 4, 5, 7, 9])
+def test_words_shared_by_finishing_and_waiting_cells(vf, orc, width):
+    w = vf.World(96, 32, 96)
+    w.fill_box(0, 0, 0, 95, 3, 95, STONE)
+    for x in range(4, 90 - width, width + 3):
+        w.fill_box(x, 10, 4, x + width - 1, 13, 80, WATER)
+    sim, o = vf.FluidSim(w, device=0), oracle_for(orc, w)
+    for s in (sim, o):
+        s.wake(0, 8, 0, 95, 14, 95)
+    run(sim, o, 4)
+    sim.close()

@@ -304,9 +304,14 @@ __device__ __forceinline__ void park_put(const Region& R, unsigned b, unsigned t
   if (t < MAX_CELLS_PER_TICK) R.lv_park[(size_t)b * MAX_CELLS_PER_TICK + t] = (unsigned short)i;
   else set_status(R, ST_RANGE, 52);
 }
-__device__ __forceinline__ unsigned dep_byte(const LvSmem& L, unsigned i) { return reinterpret_cast<const volatile unsigned char*>(L.dep)[i]; }
+// Four cells' bytes share a word, and in a round one warp finishes a cell while others count down its
+// neighbours: during the rounds every access is to the whole word, and every change an atomic one.
+__device__ __forceinline__ unsigned dep_byte(const LvSmem& L, unsigned i) { return (vld(&L.dep[i >> 2]) >> ((i & 3u) * 8u)) & 0xFFu; }
+__device__ __forceinline__ void cell_finish(LvSmem& L, unsigned i, unsigned slots) {  // (the byte of a cell that runs is 0)
+  atomicOr(&L.dep[i >> 2], (DONE | slots) << ((i & 3u) * 8u));
+}
 __device__ __forceinline__ bool cell_done(const LvSmem& L, unsigned i) { return dep_byte(L, i) >= DONE; }
-__device__ __forceinline__ bool bit_of(const unsigned* w, unsigned i) { return (w[i >> 5] >> (i & 31u)) & 1u; }
+__device__ __forceinline__ bool bit_of(const unsigned* w, unsigned i) { return (vld(w + (i >> 5)) >> (i & 31u)) & 1u; }  // (a round's other warps clear pp bits)
 // att bits before position i
 __device__ __forceinline__ unsigned attempts_before(const LvSmem& L, unsigned i) {
   return (unsigned)L.gpre[i >> 5] + (unsigned)__popc(L.att[i >> 5] & ((1u << (i & 31u)) - 1u));
@@ -476,7 +481,7 @@ __device__ __forceinline__ float lv_cells(const Region& R, LvSmem& L, const Lane
   }
   if (has && l == 0u) {
     R.lv_ev[i] = ev | (am & 0xFCu) | ((am & 0x80u) << 9) | ((cm & 0x7Fu) << 8);  // bit 16: seeds itself
-    reinterpret_cast<volatile unsigned char*>(L.dep)[i] = (unsigned char)(DONE | (pm & 0x7Fu));
+    cell_finish(L, i, pm & 0x7Fu);
     if (pp) atomicAnd(&L.pp[i >> 5], ~(1u << (i & 31u)));
   }
   __syncwarp();
@@ -576,7 +581,7 @@ __device__ __forceinline__ void lv_cell_thread(const Region& R, LvSmem& L, bool 
   }
   if (has) {
     R.lv_ev[i] = (am & 0xFCu) | ((am & 0x80u) << 9) | cm << 8;
-    reinterpret_cast<volatile unsigned char*>(L.dep)[i] = (unsigned char)(DONE | pm);
+    cell_finish(L, i, pm);
     if (pp) atomicAnd(&L.pp[i >> 5], ~(1u << (i & 31u)));
   }
   // ---- the ready ones to the next list, or parked above the gate: places by a scan over the warp
@@ -1171,10 +1176,10 @@ __device__ __forceinline__ unsigned lv_prune(const Region& R, LvSmem& L, unsigne
 // from `gate`), carry on the search, or the sweep's end. Returns the change in partial entries.
 __device__ __noinline__ int lv_solo(const Region& Rs, LvSmem& L, unsigned n, int gate, int sgn, unsigned long long cap) {
   const Region R = Rs;
-  const LaneSlot S = lane_slot(R);
   int pd = 0;
   __syncwarp();
   const unsigned lane = lane_id(), kp = L.kp;
+  const LaneSlot S = lane_slot(R);
   HeadState H = L.h;
   const unsigned pb = L.pb, cc = L.cc;
   unsigned req, cur = L.cur, cnt = L.cnt[cc], park = L.park_n[pb], rounds = L.rounds;  // (nobody else adds to the lists now)
@@ -1305,10 +1310,10 @@ __device__ __noinline__ int lv_long(const Region& Rs, LvSmem& L, unsigned n, int
 // partial entries.
 __device__ __noinline__ int lv_wide(const Region& Rs, LvSmem& L, unsigned n, int gate, unsigned long long cap) {
   const Region R = Rs;
-  const LaneSlot S = lane_slot(R);
   const unsigned tid = threadIdx.x, lane = tid & 31u, step = (blockDim.x >> 5) * 4u, t0 = (tid >> 5) * 4u;
   const bool alive = L.h.head < n;
   const unsigned pb = L.pb, kp = L.kp;
+  const LaneSlot S = lane_slot(R);
   unsigned cur = L.cur, cc = L.cc, rounds = L.rounds, fcount = min(L.cnt[cc], MAX_CELLS_PER_TICK), unused = 0;
   Touch T;
   int pd = 0;
