@@ -130,3 +130,17 @@ def test_words_shared_by_finishing_and_waiting_cells(vf, orc, width):
         s.wake(0, 8, 0, 95, 14, 95)
     run(sim, o, 4)
     sim.close()
+
+
+# more cells below full than the budget has attempts: past it a cell does not wait for the cell two above it
+def test_partial_block_past_the_attempt_budget(vf, orc):
+    w = vf.World(90, 40, 90)
+    w.fill_box(0, 0, 0, 89, 3, 89, STONE)
+    sim, o = vf.FluidSim(w, device=0), oracle_for(orc, w)
+    y, z, x = np.meshgrid(np.arange(12, 18), np.arange(8, 80), np.arange(8, 80), indexing="ij")
+    cells = np.stack([x.ravel(), y.ravel(), z.ravel()], 1).astype(np.int32)
+    for s in (sim, o):
+        s.emit(cells, 0.9)
+    run(sim, o, 4)
+    assert sim.stats().pull_attempts >= 4096
+    sim.close()

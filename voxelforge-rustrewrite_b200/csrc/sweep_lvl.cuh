@@ -321,6 +321,8 @@ __device__ __forceinline__ unsigned attempts_before(const LvSmem& L, unsigned i)
 // Lane constants of the eight lanes that run a cell: lane l < 7 holds footprint slot l.
 struct LaneSlot {
   int off;               // the slot's offset in domain ids
+  unsigned end;          // cells from this position on leave the lane's slot unread: 0 for lane 7, and kp for the
+                         // cell above, which only a cell that may pull looks at (another of the round may write it)
   unsigned open1, open2; // the lane's two successors: one layer up (bit per successor), two layers up
 };
 __device__ __forceinline__ int fp_id(const Region& R, int l) {
@@ -328,10 +330,11 @@ __device__ __forceinline__ int fp_id(const Region& R, int l) {
   fp_off(l, ox, oy, oz);
   return ox + (oz * R.PY + oy) * R.PX;
 }
-__device__ __forceinline__ LaneSlot lane_slot(const Region& R) {
+__device__ __forceinline__ LaneSlot lane_slot(const Region& R, unsigned kp) {
   const int l = (int)(threadIdx.x & 7u);
   LaneSlot s;
   s.off = l < 7 ? fp_id(R, l) : 0;
+  s.end = l == 7 ? 0u : l == 2 ? kp : MAX_CELLS_PER_TICK;
   s.open1 = l == 3 || l == 4 ? 3u : l == 5 ? 1u : 0u;  // successors 6..10
   s.open2 = l == 5 ? 2u : 0u;                          // successor 11
   return s;
@@ -354,7 +357,7 @@ __device__ __forceinline__ LaneCell cell_record(const Region& R, bool has, unsig
   return c;
 }
 __device__ __forceinline__ void cell_slot(const Region& R, const LaneSlot& S, LaneCell& c) {
-  if (c.has && (threadIdx.x & 7u) < 7u) c.u = R.dense[(int)c.ce.x + S.off];
+  if (c.has && c.i < S.end) c.u = R.dense[(int)c.ce.x + S.off];
 }
 
 // A lone warp touches its cells' successors' records, some of which it runs next: they come from L2 (~850
@@ -1179,7 +1182,7 @@ __device__ __noinline__ int lv_solo(const Region& Rs, LvSmem& L, unsigned n, int
   int pd = 0;
   __syncwarp();
   const unsigned lane = lane_id(), kp = L.kp;
-  const LaneSlot S = lane_slot(R);
+  const LaneSlot S = lane_slot(R, kp);
   HeadState H = L.h;
   const unsigned pb = L.pb, cc = L.cc;
   unsigned req, cur = L.cur, cnt = L.cnt[cc], park = L.park_n[pb], rounds = L.rounds;  // (nobody else adds to the lists now)
@@ -1313,7 +1316,7 @@ __device__ __noinline__ int lv_wide(const Region& Rs, LvSmem& L, unsigned n, int
   const unsigned tid = threadIdx.x, lane = tid & 31u, step = (blockDim.x >> 5) * 4u, t0 = (tid >> 5) * 4u;
   const bool alive = L.h.head < n;
   const unsigned pb = L.pb, kp = L.kp;
-  const LaneSlot S = lane_slot(R);
+  const LaneSlot S = lane_slot(R, kp);
   unsigned cur = L.cur, cc = L.cc, rounds = L.rounds, fcount = min(L.cnt[cc], MAX_CELLS_PER_TICK), unused = 0;
   Touch T;
   int pd = 0;
