@@ -79,3 +79,18 @@ def test_lists(vf, orc, ny, top, order):
     assert sim.apply_brush(cells, STONE) == o.apply_brush(cells, STONE)
     same(sim, o, 2)
     sim.close()
+
+
+def test_water_with_nowhere_to_go(vf, orc):
+    """A closed tank full of water: a displaced cell's water finds no room above or beside it and is gone, in
+    columns that touch each other."""
+    w = vf.World(40, 40, 40)
+    w.fill_box(0, 0, 0, 39, 39, 39, STONE)
+    w.fill_box(4, 4, 4, 35, 35, 35, WATER)
+    sim, o = vf.FluidSim(w, device=0), oracle_for(orc, w)
+    for c, r in (((20, 20, 20), 6), ((24, 22, 20), 5), ((6, 30, 6), 9)):
+        cells = sphere(c, r)
+        assert sim.apply_brush(cells, STONE) == o.apply_brush(cells, STONE)
+        same(sim, o)
+    same(sim, o, 2)
+    sim.close()

@@ -1850,9 +1850,10 @@ __device__ __forceinline__ unsigned brush_column(const Region& R, const int* xyz
           }
           shut = solid != 0u;
         }
-        if (ok && amount > 1e-6f) {
+        if (!commit && ok && amount > 1e-6f) {
           // to the sides, if one of them has room: during a stroke a cell only fills or turns solid, so one without
-          // room stays so; where none has any, the water is gone (fluid.rs:396-408)
+          // room stays so; where none has any, the water is gone (fluid.rs:396-408). Asked while nothing is written
+          // (a commit goes no further than its try did): the side columns may be other warps'.
           const int row = R.PX * R.PY;
           const int off = lane == 0u ? 1 : lane == 1u ? -1 : lane == 2u ? row : -row;
           const unsigned us = lane < 4u ? R.dense[(int)(id0 + (32u * k + b) * (unsigned)R.PX) + off] : DC_SOLID;
