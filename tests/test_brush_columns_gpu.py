@@ -94,3 +94,24 @@ def test_water_with_nowhere_to_go(vf, orc):
         same(sim, o)
     same(sim, o, 2)
     sim.close()
+
+
+# lists in no order: what a chunk leaves for later may lie between cells of its column that it takes
+@pytest.mark.parametrize("order", [0, 1, 2, 4, 5, "low high twice middle", "stairs", "zigzag", "far up"])
+def test_lists_in_no_order(vf, orc, order):
+    sim, o = pool(vf, orc, *((160, 150) if order == "far up" else ()))
+    cells = sphere((24, 16, 24), 4)
+    if isinstance(order, int):
+        cells = np.random.default_rng(order).permutation(cells)
+    elif order == "low high twice middle":
+        cells = np.array([[5, 5, 5], [5, 7, 5], [5, 5, 5], [5, 6, 5]] + [[10 + i, 6, 9] for i in range(12)], np.int32)
+    elif order == "stairs":  # every column: the lowest cell, the highest, then the ones between downwards
+        cells = np.array([[x, y, 20] for x in range(10, 20) for y in (5, 12, 11, 10, 9, 8, 7, 6)], np.int32)
+    elif order == "zigzag":  # layers in turn over all columns, each column up and down
+        cells = np.array([[x, y, 20] for y in (5, 9, 7, 12, 6, 8, 20, 10, 11) for x in range(10, 20)], np.int32)
+    else:  # a column's second cell lies more than 128 cells up: it ends the chunk, the rest of the column does not
+        cells = np.array([[x, y, 20] for x in range(10, 20) for y in (5, 140, 6, 100, 7)], np.int32)
+    cells = np.ascontiguousarray(cells)
+    assert sim.apply_brush(cells, STONE) == o.apply_brush(cells, STONE)
+    same(sim, o, 2)
+    sim.close()

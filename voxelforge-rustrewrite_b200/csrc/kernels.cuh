@@ -1761,7 +1761,7 @@ __global__ void __launch_bounds__(EDIT_THREADS) k_carve(Region R, const int* xyz
 // are independent as long as every column's cells are listed upwards and its water finds room above: a
 // warp then takes a column, in registers. In chunks of the list: the voxels and columns are claimed (rb, stamp); every
 // column is tried without writing, up to its first cell that does not fit (water that goes to the sides, a
-// cell listed below or twice, a column of more than 128 cells, water that
+// cell listed after one above it or twice, a column of more than 128 cells, water that
 // goes to more than three cells). What the list holds before the first of those commits to the dense words and logs what
 // each listed cell did, and the log is followed in list order: slots, the atlas, and the
 // activations (27 around a displaced cell, then those that took its water), 16 cells at a time, each cell
@@ -1790,24 +1790,32 @@ __device__ __forceinline__ unsigned brush_column(const Region& R, const int* xyz
     u[k] = in ? R.dense[id0 + (unsigned)(up * R.PX)] : DC_SOLID;
     at[k] = in ? __ldcg(R.rb + id0 + (unsigned)(up * R.PX)) : NOSLOT;
   }
+  // Up to `limit` the column is listed upwards: it ends before the first entry with an earlier one above it. A later
+  // end then only takes the column's last cells away, so the commit finds what the try found.
+  if (!commit) {
+    unsigned above = NOSLOT, bad = NOSLOT;  // the earliest entry of the rows above
+#pragma unroll
+    for (int k = BRUSH_ROWS - 1; k >= 0; --k) {
+      if (!__any_sync(FULLMASK, at[k] != NOSLOT)) continue;
+      unsigned first = at[k];  // the earliest entry of the lane's cell and those above it
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned v = __shfl_down_sync(FULLMASK, first, o);
+        first = min(first, lane + (unsigned)o < 32u ? v : above);
+      }
+      const unsigned over = __shfl_down_sync(FULLMASK, first, 1);
+      if (at[k] != NOSLOT && at[k] > (lane < 31u ? over : above)) bad = at[k] < bad ? at[k] : bad;
+      above = __shfl_sync(FULLMASK, first, 0);
+    }
+    limit = min(limit, __reduce_min_sync(FULLMASK, bad));
+  }
   bool ok = true;
-  unsigned prev = lead;
 #pragma unroll
   for (int k = 0; k < BRUSH_ROWS; ++k) {
     for (unsigned listed = __ballot_sync(FULLMASK, at[k] != NOSLOT); listed && ok; listed &= listed - 1u) {
       const unsigned b = (unsigned)__ffs(listed) - 1u;
       const unsigned i = __shfl_sync(FULLMASK, at[k], b), own = __shfl_sync(FULLMASK, u[k], b);
-      if (i >= limit) {  // (the column's cells before it in the list lie below it)
-        ok = false;
-        continue;
-      }
-      if (i < prev) {
-        ok = false;
-        limit = i;
-        continue;
-      }
-      prev = i;
-      if (dc_solid(own)) continue;
+      if (i >= limit || dc_solid(own)) continue;  // (left for the next chunk, cells above it may come before it in the list)
       unsigned nt = 0, t[BRUSH_TARGETS] = {0, 0, 0}, flags = 4u;
       if ((int)own > 0) {
         flags |= 8u;
