@@ -206,7 +206,8 @@ int detached_count(vf_fluid* h, long long delta) {
 
 // SparseVolume::ring_evict (sparse_volume.rs:513-537) of ring slot `si` on the device: the slot's
 // bricks become empty and their atlas slots free; the partial volumes they held are kept per cell,
-// as the reference's PartialField keeps them. `ring` is the device ring table, updated here.
+// as the reference's PartialField keeps them. `ring` is the device ring table, updated here, and the
+// dense words follow: a paste may be refused after its slot was emptied.
 int ring_evict_slot(vf_fluid* h, int si, std::vector<int32_t>& ring) {
   const Region& R = h->R;
   if (!ring[3 * si + 2]) return VF_OK;
@@ -260,7 +261,7 @@ int ring_evict_slot(vf_fluid* h, int si, std::vector<int32_t>& ring) {
   CK(cudaMemcpy(R.grid, grid.data(), nb * 4, cudaMemcpyHostToDevice));
   ring[3 * si + 2] = 0;
   CK(cudaMemcpy(R.ring, ring.data(), ring.size() * 4, cudaMemcpyHostToDevice));
-  return VF_OK;
+  return build_dense(h);
 }
 
 uint64_t next_pow2(uint64_t v) {
@@ -888,7 +889,6 @@ int vf_fluid_ring_evict(vf_fluid* h, int32_t cx, int32_t cz) {  // sparse_volume
   std::vector<int32_t> ring(3 * w * w);
   CK(cudaMemcpy(ring.data(), h->R.ring, ring.size() * 4, cudaMemcpyDeviceToHost));
   if ((rc = ring_evict_slot(h, (cz & (w - 1)) * w + (cx & (w - 1)), ring))) return rc;
-  if ((rc = build_dense(h))) return rc;
   CK(cudaStreamSynchronize(h->stream));
   return VF_OK;
 }
