@@ -200,7 +200,7 @@ int detached_count(vf_fluid* h, long long delta) {
   if ((h->hctl->ndetached + delta) > 0xFFFFFFFFll) return fail(h, VF_ERR_OOM, "too many kept partial entries");
   const unsigned v = (unsigned)((long long)h->hctl->ndetached + delta);
   h->hctl->ndetached = v;
-  CK(cudaMemcpy(&h->R.ctl->ndetached, &v, 4, cudaMemcpyHostToDevice));
+  CK(cudaMemcpyAsync(&h->R.ctl->ndetached, &h->hctl->ndetached, 4, cudaMemcpyHostToDevice, h->stream));
   return VF_OK;
 }
 
@@ -258,10 +258,13 @@ int ring_evict_slot(vf_fluid* h, int si, std::vector<int32_t>& ring) {
     if ((rc = detached_bits(h, ids, 1))) return rc;
     if ((rc = detached_count(h, (long long)ids.size()))) return rc;
   }
-  CK(cudaMemcpy(R.grid, grid.data(), nb * 4, cudaMemcpyHostToDevice));
+  // on the handle's stream: a plain copy may return before its bytes have arrived, and waits for no other stream
+  CK(cudaMemcpyAsync(R.grid, grid.data(), nb * 4, cudaMemcpyHostToDevice, h->stream));
   ring[3 * si + 2] = 0;
-  CK(cudaMemcpy(R.ring, ring.data(), ring.size() * 4, cudaMemcpyHostToDevice));
-  return build_dense(h);
+  CK(cudaMemcpyAsync(R.ring, ring.data(), ring.size() * 4, cudaMemcpyHostToDevice, h->stream));
+  if ((rc = build_dense(h))) return rc;
+  CK(cudaStreamSynchronize(h->stream));
+  return VF_OK;
 }
 
 uint64_t next_pow2(uint64_t v) {
@@ -859,7 +862,7 @@ int vf_fluid_shift(vf_fluid* h, int32_t dx, int32_t dz) {  // fluid.rs:696-720
     ring[i] -= dx / 128;
     ring[i + 1] -= dz / 128;
   }
-  CK(cudaMemcpy(R.ring, ring.data(), ring.size() * 4, cudaMemcpyHostToDevice));
+  CK(cudaMemcpyAsync(R.ring, ring.data(), ring.size() * 4, cudaMemcpyHostToDevice, h->stream));
   for (DetachedPartial& e : h->det) {  // PartialField re-keyed (fluid.rs:697-701); ids are domain-relative
     e.x -= dx;
     e.z -= dz;
@@ -888,9 +891,7 @@ int vf_fluid_ring_evict(vf_fluid* h, int32_t cx, int32_t cz) {  // sparse_volume
   const int w = h->R.ring_w;
   std::vector<int32_t> ring(3 * w * w);
   CK(cudaMemcpy(ring.data(), h->R.ring, ring.size() * 4, cudaMemcpyDeviceToHost));
-  if ((rc = ring_evict_slot(h, (cz & (w - 1)) * w + (cx & (w - 1)), ring))) return rc;
-  CK(cudaStreamSynchronize(h->stream));
-  return VF_OK;
+  return ring_evict_slot(h, (cz & (w - 1)) * w + (cx & (w - 1)), ring);
 }
 
 int vf_fluid_ring_paste(vf_fluid* h, const uint32_t* chunk_grid, const uint8_t* chunk_bricks, uint64_t chunk_nbricks, int32_t chunk_bricks_y,
@@ -977,13 +978,13 @@ int vf_fluid_ring_paste(vf_fluid* h, const uint32_t* chunk_grid, const uint8_t* 
   }
   if (used != h->hctl->atlas_used) {
     h->hctl->atlas_used = used;
-    CK(cudaMemcpy(&R.ctl->atlas_used, &used, 4, cudaMemcpyHostToDevice));
+    CK(cudaMemcpyAsync(&R.ctl->atlas_used, &h->hctl->atlas_used, 4, cudaMemcpyHostToDevice, h->stream));
   }
-  CK(cudaMemcpy(R.grid, grid.data(), nb * 4, cudaMemcpyHostToDevice));
+  CK(cudaMemcpyAsync(R.grid, grid.data(), nb * 4, cudaMemcpyHostToDevice, h->stream));
   ring[3 * si] = cx;
   ring[3 * si + 1] = cz;
   ring[3 * si + 2] = 1;
-  CK(cudaMemcpy(R.ring, ring.data(), ring.size() * 4, cudaMemcpyHostToDevice));
+  CK(cudaMemcpyAsync(R.ring, ring.data(), ring.size() * 4, cudaMemcpyHostToDevice, h->stream));
   // the returned entries live in the atlas again; erased ones are gone for good
   if ((rc = detached_bits(h, back, 0))) return rc;
   if ((rc = detached_count(h, -(long long)back.size()))) return rc;
@@ -1303,7 +1304,9 @@ int vf_batch_create(vf_fluid* const* hs, int32_t n, vf_batch** out) {
     delete b;
     return VF_ERR_OOM;
   }
-  if (cudaMemcpy(b->dregs, regs.data(), sizeof(Region) * n, cudaMemcpyHostToDevice) != cudaSuccess) {
+  // (the copy may return before its bytes have arrived, and the ticks' stream does not wait for the default one)
+  if (cudaMemcpy(b->dregs, regs.data(), sizeof(Region) * n, cudaMemcpyHostToDevice) != cudaSuccess ||
+      cudaStreamSynchronize(cudaStreamLegacy) != cudaSuccess) {
     cudaFree(b->dregs);
     delete b;
     return VF_ERR_CUDA;
