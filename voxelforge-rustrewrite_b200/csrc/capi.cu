@@ -120,12 +120,24 @@ void free_world(vf_fluid* h) {
   h->uploaded = false;
 }
 
-// The dense words in step with the grid and the atlas again.
-int build_dense(vf_fluid* h) {
-  k_dense<<<(unsigned)std::min<uint64_t>(((uint64_t)h->R.ncells + 255) / 256, 148 * 32), 256, 0, h->stream>>>(h->R);
+// The dense words of the domain's columns [x0, x1) x [z0, z1) in step with the grid and the atlas again.
+int build_dense(vf_fluid* h, int64_t x0, int64_t z0, int64_t x1, int64_t z1) {
+  const Region& R = h->R;
+  x0 = std::max<int64_t>(x0, R.px0);
+  z0 = std::max<int64_t>(z0, R.pz0);
+  x1 = std::min<int64_t>(x1, (int64_t)R.px0 + R.PX);
+  z1 = std::min<int64_t>(z1, (int64_t)R.pz0 + R.PZ);
+  if (x0 >= x1 || z0 >= z1) return VF_OK;
+  const int sx = (int)(x1 - x0), sz = (int)(z1 - z0);
+  const uint64_t rows = (uint64_t)sz * R.PY;
+  k_dense<<<(unsigned)std::min<uint64_t>(rows, 148 * 64), std::min(256, (sx + 31) / 32 * 32), 0, h->stream>>>(R, (int)x0, (int)z0, sx, sz);
   CK(cudaGetLastError());
   return VF_OK;
 }
+int build_dense_chunk(vf_fluid* h, int32_t cx, int32_t cz) {
+  return build_dense(h, (int64_t)cx * 128, (int64_t)cz * 128, (int64_t)cx * 128 + 128, (int64_t)cz * 128 + 128);
+}
+int build_dense_all(vf_fluid* h) { return build_dense(h, INT32_MIN, INT32_MIN, INT32_MAX, INT32_MAX); }
 
 int ensure_scratch(vf_fluid* h, size_t bytes) {
   if (h->scratch_bytes >= bytes) return VF_OK;
@@ -262,7 +274,7 @@ int ring_evict_slot(vf_fluid* h, int si, std::vector<int32_t>& ring) {
   CK(cudaMemcpyAsync(R.grid, grid.data(), nb * 4, cudaMemcpyHostToDevice, h->stream));
   ring[3 * si + 2] = 0;
   CK(cudaMemcpyAsync(R.ring, ring.data(), ring.size() * 4, cudaMemcpyHostToDevice, h->stream));
-  if ((rc = build_dense(h))) return rc;
+  if ((rc = build_dense_chunk(h, ocx, ocz))) return rc;
   CK(cudaStreamSynchronize(h->stream));
   return VF_OK;
 }
@@ -475,7 +487,7 @@ int vf_fluid_upload_world(vf_fluid* h, int32_t nx, int32_t ny, int32_t nz, int32
   if ((rc = dalloc(h, &h->dR, 1, false))) return rc;
   CK(cudaMemcpyAsync(h->dR, &R, sizeof(Region), cudaMemcpyHostToDevice, h->stream));
   h->R = R;
-  if ((rc = build_dense(h))) return rc;
+  if ((rc = build_dense_all(h))) return rc;
   CK(cudaStreamSynchronize(h->stream));
   h->uploaded = true;
   h->acc = 0.0f;
@@ -989,7 +1001,7 @@ int vf_fluid_ring_paste(vf_fluid* h, const uint32_t* chunk_grid, const uint8_t* 
   if ((rc = detached_bits(h, back, 0))) return rc;
   if ((rc = detached_count(h, -(long long)back.size()))) return rc;
   h->det.swap(keep);
-  if ((rc = build_dense(h))) return rc;
+  if ((rc = build_dense_chunk(h, cx, cz))) return rc;
   CK(cudaStreamSynchronize(h->stream));
   return VF_OK;
 }
@@ -1031,7 +1043,7 @@ int vf_fluid_reset(vf_fluid* h) {  // fluid.rs:318-320: the fluid's tables only
   std::memcpy(z.prof, c.prof, sizeof(z.prof));
   CK(cudaMemcpyAsync(R.ctl, &z, sizeof(Ctl), cudaMemcpyHostToDevice, h->stream));
   h->acc = 0.0f;
-  if ((rc = build_dense(h))) return rc;
+  if ((rc = build_dense_all(h))) return rc;
   return sync_ctl(h);
 }
 
