@@ -76,6 +76,8 @@ struct DeviceScope {
   }
 };
 
+constexpr uint32_t EV_ACT_CAP = 1u << 22;  // entries of a handle's activation log
+
 // The tick kernel for `nreg` regions: one CTA per region.
 constexpr int PAR_SMEM_BYTES = (int)((sizeof(TickSmem) + 127) / 128 * 128);
 static_assert(PAR_SMEM_BYTES + 2048 + 1024 <= 132 * 1024, "the tick fits the 132 KB carve-out, static arrays and the system's 1 KB included");
@@ -137,7 +139,6 @@ int build_dense(vf_fluid* h, int64_t x0, int64_t z0, int64_t x1, int64_t z1) {
 int build_dense_chunk(vf_fluid* h, int32_t cx, int32_t cz) {
   return build_dense(h, (int64_t)cx * 128, (int64_t)cz * 128, (int64_t)cx * 128 + 128, (int64_t)cz * 128 + 128);
 }
-int build_dense_all(vf_fluid* h) { return build_dense(h, INT32_MIN, INT32_MIN, INT32_MAX, INT32_MAX); }
 
 int ensure_scratch(vf_fluid* h, size_t bytes) {
   if (h->scratch_bytes >= bytes) return VF_OK;
@@ -449,10 +450,10 @@ int vf_fluid_upload_world(vf_fluid* h, int32_t nx, int32_t ny, int32_t nz, int32
   if ((rc = dalloc(h, &R.mark_list, tiles))) return rc;
   if ((rc = dalloc(h, &R.mark_tflag, tiles))) return rc;
   // per-tick event logs: <= 50 activations and 7 writes per swept cell, plus levelling's
-  R.ev_act_cap = 1u << 22;
+  R.ev_act_cap = EV_ACT_CAP;
   R.ev_seed_cap = 1u << 18;
   R.ev_chg_cap = 1u << 21;
-  if ((rc = dalloc(h, &R.ev_act, R.ev_act_cap, false))) return rc;
+  if ((rc = dalloc(h, &R.ev_act, EV_ACT_CAP, false))) return rc;
   if ((rc = dalloc(h, &R.ev_seed, R.ev_seed_cap, false))) return rc;
   if ((rc = dalloc(h, &R.ev_chg, R.ev_chg_cap, false))) return rc;
   if ((rc = dalloc(h, &R.stamp, ncells, false))) return rc;
@@ -487,7 +488,7 @@ int vf_fluid_upload_world(vf_fluid* h, int32_t nx, int32_t ny, int32_t nz, int32
   if ((rc = dalloc(h, &h->dR, 1, false))) return rc;
   CK(cudaMemcpyAsync(h->dR, &R, sizeof(Region), cudaMemcpyHostToDevice, h->stream));
   h->R = R;
-  if ((rc = build_dense_all(h))) return rc;
+  if ((rc = build_dense(h, R.px0, R.pz0, (int64_t)R.px0 + R.PX, (int64_t)R.pz0 + R.PZ))) return rc;
   CK(cudaStreamSynchronize(h->stream));
   h->uploaded = true;
   h->acc = 0.0f;
@@ -1020,8 +1021,6 @@ int vf_fluid_reset(vf_fluid* h) {  // fluid.rs:318-320: the fluid's tables only
   const uint64_t tiles = (uint64_t)R.TX * R.PY * R.TZ;
   CK(cudaMemsetAsync(R.marks, 0, tiles * 128 * 4, h->stream));
   CK(cudaMemsetAsync(R.mark_tflag, 0, tiles * 4, h->stream));
-  // per-tick maps a failed tick may have left set (cell positions, rows, pull-written cells)
-  CK(cudaMemsetAsync(R.stamp, 0xFF, (size_t)R.ncells * 4, h->stream));
   if (R.detbits) CK(cudaMemsetAsync(R.detbits, 0, words * 4, h->stream));  // kept entries go with the rest
   h->det.clear();
   Ctl c = *h->hctl;
@@ -1043,7 +1042,20 @@ int vf_fluid_reset(vf_fluid* h) {  // fluid.rs:318-320: the fluid's tables only
   std::memcpy(z.prof, c.prof, sizeof(z.prof));
   CK(cudaMemcpyAsync(R.ctl, &z, sizeof(Ctl), cudaMemcpyHostToDevice, h->stream));
   h->acc = 0.0f;
-  if ((rc = build_dense_all(h))) return rc;
+  // A handle whose tick or edit failed does not get here: the words were in step with the grid and the atlas, and the
+  // maps that a tick uses (stamp, rb) are idle.
+  if (used) {
+    int* map = (int*)R.ev_act;  // idle between ticks
+    if (used > EV_ACT_CAP) {
+      if ((rc = ensure_scratch(h, (size_t)used * 4))) return rc;
+      map = (int*)h->scratch;
+    }
+    const uint64_t nb = (uint64_t)R.bx * R.by * R.bz;
+    CK(cudaMemsetAsync(map, 0xFF, (size_t)used * 4, h->stream));
+    k_slot_map<<<(unsigned)std::min<uint64_t>((nb + 255) / 256, 8192), 256, 0, h->stream>>>(R, map, used);
+    k_dense_slots<<<std::min((used + 7) / 8, 148u * 16), 256, 0, h->stream>>>(R, map, used);
+    CK(cudaGetLastError());
+  }
   return sync_ctl(h);
 }
 
@@ -1234,7 +1246,7 @@ int vf_fluid_set_sweep(vf_fluid* h, int32_t engine, int32_t gate, uint64_t spin_
 int vf_fluid_set_log_caps(vf_fluid* h, uint32_t act, uint32_t seed, uint32_t chg) {
   int rc = check(h);
   if (rc) return rc;
-  if (act < 1 || act > (1u << 22) || seed < 1 || seed > (1u << 18) || chg < 1 || chg > (1u << 21)) return VF_ERR_INVALID;
+  if (act < 1 || act > EV_ACT_CAP || seed < 1 || seed > (1u << 18) || chg < 1 || chg > (1u << 21)) return VF_ERR_INVALID;
   DeviceScope scope(h->device);
   if (scope.err != cudaSuccess) return VF_ERR_CUDA;
   if ((rc = sync_ctl(h))) return rc;

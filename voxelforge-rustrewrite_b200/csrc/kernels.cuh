@@ -2118,8 +2118,23 @@ __global__ void __launch_bounds__(32) k_edit(Region R, int kind, const int* xyz,
   if (lane == 0 && out_count) *out_count = cnt;
 }
 
+// The first cell of the brick at grid index gi; false where a ring world's slot holds no chunk.
+__device__ __forceinline__ bool brick_origin(const Region& R, unsigned gi, int& x, int& y, int& z) {
+  int bx = (int)(gi % (unsigned)R.bx), bz = (int)(gi / ((unsigned)R.bx * (unsigned)R.by));
+  y = (int)((gi / (unsigned)R.bx) % (unsigned)R.by) * 8;
+  if (R.ring_w) {
+    const int* s = R.ring + 3 * ((bz >> 4) * R.ring_w + (bx >> 4));
+    if (!s[2]) return false;
+    bx = s[0] * 16 + (bx & 15);
+    bz = s[1] * 16 + (bz & 15);
+  }
+  x = bx * 8;
+  z = bz * 8;
+  return true;
+}
+
 // The dense words of a box of columns from the grid and the atlas, a row of cells per CTA: the whole domain
-// after an upload and a reset, one chunk's 128 x 128 columns when it comes or goes. Bound by the words' stores
+// after an upload, one chunk's 128 x 128 columns when it comes or goes. Bound by the words' stores
 // (a 576 x 160 x 576 domain: 212 MB; a chunk of 256 layers: 19 MB, where the whole domain of 9 x 9 chunks is 1.7 GB:
 // an eviction and a paste there 6.3 ms with it, 4.2 with the chunk).
 __global__ void __launch_bounds__(256) k_dense(Region R, int x0, int z0, int sx, int sz) {
@@ -2128,6 +2143,29 @@ __global__ void __launch_bounds__(256) k_dense(Region R, int x0, int z0, int sx,
     for (int x = x0 + (int)threadIdx.x; x < x0 + sx; x += (int)blockDim.x) {
       const CD c = load_cell(R, R.ring, x, y, z);
       R.dense[dom_id(R, x, y, z)] = dense_code(c.out, c.mat, __float_as_uint(c.part));
+    }
+  }
+}
+
+// The dense words after a reset: the partial volumes are gone, the materials stand, so that only the cells of
+// bricks with a slot can differ (slot_gi: k_slot_map's), a warp each. Latency: a brick is one round of loads and 64
+// sectors of stores.
+__global__ void __launch_bounds__(256) k_dense_slots(Region R, const int* slot_gi, unsigned nslots) {
+  const unsigned lane = lane_id();
+  for (unsigned s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; s < nslots; s += (gridDim.x * blockDim.x) >> 5) {
+    const int gi = slot_gi[s];
+    int x0, y0, z0;
+    if (gi < 0 || !brick_origin(R, (unsigned)gi, x0, y0, z0)) continue;
+    const bool held = !R.ring_w || chunk_loaded(R, R.ring, x0 >> 7, z0 >> 7);
+    unsigned char mat[16];
+#pragma unroll
+    for (int k = 0; k < 16; ++k) mat[k] = R.amat[(size_t)s * 512u + 32u * k + lane];
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+      const unsigned v = 32u * k + lane;
+      const int x = x0 + (int)(v & 7u), y = y0 + (int)((v >> 3) & 7u), z = z0 + (int)(v >> 6);
+      const bool out = !held || y >= R.ny || (!R.ring_w && (x >= R.nx || z >= R.nz));
+      if (in_dom(R, x, y, z)) R.dense[dom_id(R, x, y, z)] = dense_code(out, mat[k], 0u);
     }
   }
 }
