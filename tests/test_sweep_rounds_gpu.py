@@ -144,3 +144,26 @@ def test_partial_block_past_the_attempt_budget(vf, orc):
     run(sim, o, 4)
     assert sim.stats().pull_attempts >= 4096
     sim.close()
+
+
+@pytest.mark.parametrize("n", [33, 128, 700])  # 96 x 97 .. 764 x 96 rows; tiles cut short, chunks of several tiles past 524,288 rows
+def test_partials_in_order_over_chunks_of_rows(vf, n):
+    ny = 65 if n < 700 else 760
+    w = vf.World(n, ny, n)
+    w.fill_box(0, 0, 0, n - 1, 3, n - 1, STONE)
+    sim = vf.FluidSim(w, device=0, atlas_bricks=1 << 17)
+    rng = np.random.default_rng(n)
+    c = np.unique(np.concatenate([rng.integers((0, 4, 0), (n, ny, n), (9000, 3)), [[0, 4, 0], [n - 1, ny - 1, n - 1], [n - 1, 4, 0], [0, ny - 1, n - 1]],
+                                  [[x, 9, n // 2] for x in range(n)], [[5, y, 7] for y in range(4, ny)]]), axis=0).astype(np.int32)
+    assert len(sim.partials()[1]) == 0
+    sim.emit(c, 0.3)
+    xyz, vol = sim.partials()
+    assert np.array_equal(xyz, c[np.lexsort((c[:, 0], c[:, 1], c[:, 2]))]) and np.all(vol == np.float32(0.3))
+    assert sim.partial_count() == len(c)
+    import ctypes as C
+
+    take, total = len(c) // 3, C.c_uint64()  # fewer than there are: the first ones
+    part, few = np.zeros((take, 3), np.int32), np.zeros(take, np.float32)
+    assert vf.lib().vf_fluid_export_partials(sim.h, part.ctypes.data_as(C.POINTER(C.c_int32)), few.ctypes.data_as(C.POINTER(C.c_float)), take, C.byref(total)) == 0
+    assert total.value == len(c) and np.array_equal(part, xyz[:take]) and np.all(few == np.float32(0.3))
+    sim.close()

@@ -802,20 +802,36 @@ int vf_fluid_export_partials(vf_fluid* h, int32_t* xyz, float* vol, uint64_t cap
   if (rc) return rc;
   DeviceScope scope(h->device);  // the caller's current device is given back on return
   if ((rc = sync_ctl(h))) return rc;
-  const unsigned spans = (h->R.ncells + PART_SPAN - 1) / PART_SPAN;
-  cap = std::min<uint64_t>(cap, (uint64_t)h->R.ncells + h->det.size());  // there are no more
-  const size_t o_count = align16((size_t)spans * 4), o_xyz = o_count + 64, o_vol = o_xyz + align16(cap * 12);
+  if (!cap) {  // how many there are stands in the control block, kept ones included
+    if (n) *n = (uint64_t)h->hctl->partial_count;
+    return VF_OK;
+  }
+  const Region& R = h->R;
+  const unsigned nslots = std::min(h->hctl->atlas_used, R.atlas_cap), nrows = (unsigned)R.PY * (unsigned)R.PZ;
+  const unsigned per = ((nrows + PART_CHUNKS - 1) / PART_CHUNKS + PART_TILE - 1) / PART_TILE * PART_TILE, chunks = (nrows + per - 1) / per;
+  cap = std::min<uint64_t>(cap, (uint64_t)R.ncells + h->det.size());  // there are no more
+  const size_t o_rows = align16((size_t)nslots * 4), o_sums = o_rows + align16((size_t)nrows * 4), o_xyz = o_sums + align16((size_t)chunks * 4),
+               o_vol = o_xyz + align16(cap * 12);
   if ((rc = ensure_scratch(h, o_vol + align16(cap * 4) + 16))) return rc;
-  unsigned* counts = (unsigned*)h->scratch;
-  unsigned long long* dcount = (unsigned long long*)((char*)h->scratch + o_count);
+  int* map = (int*)h->scratch;
+  unsigned *rows = (unsigned*)((char*)h->scratch + o_rows), *sums = (unsigned*)((char*)h->scratch + o_sums);
   int* dxyz = (int*)((char*)h->scratch + o_xyz);
   float* dvol = (float*)((char*)h->scratch + o_vol);
-  k_part_count<<<spans, 256, 0, h->stream>>>(h->R, counts);
-  k_part_write<<<spans, 256, 0, h->stream>>>(h->R, counts, dxyz, dvol, cap, dcount);
+  CK(cudaMemsetAsync(rows, 0, (size_t)nrows * 4, h->stream));
+  if (nslots) {
+    const uint64_t nb = (uint64_t)R.bx * R.by * R.bz;
+    CK(cudaMemsetAsync(map, 0xFF, (size_t)nslots * 4, h->stream));
+    k_slot_map<<<(unsigned)std::min<uint64_t>((nb + 255) / 256, 8192), 256, 0, h->stream>>>(R, map, nslots);
+    k_part_rows<<<std::min((nslots + 7) / 8, 148u * 16), 256, 0, h->stream>>>(R, map, nslots, rows);
+  }
+  k_part_sums<<<chunks, PART_TILE, 0, h->stream>>>(rows, nrows, per, sums);
+  k_part_write<<<chunks, PART_TILE, 0, h->stream>>>(R, rows, nrows, per, sums, dxyz, dvol, cap);
   CK(cudaGetLastError());
-  unsigned long long cnt = 0;
-  CK(cudaMemcpyAsync(&cnt, dcount, 8, cudaMemcpyDeviceToHost, h->stream));
+  std::vector<unsigned> in_chunk(chunks);
+  CK(cudaMemcpyAsync(in_chunk.data(), sums, (size_t)chunks * 4, cudaMemcpyDeviceToHost, h->stream));
   CK(cudaStreamSynchronize(h->stream));
+  unsigned long long cnt = 0;
+  for (const unsigned c : in_chunk) cnt += c;
   uint64_t take = std::min<uint64_t>(cnt, cap);
   if (take && xyz) CK(cudaMemcpy(xyz, dxyz, take * 12, cudaMemcpyDeviceToHost));
   if (take && vol) CK(cudaMemcpy(vol, dvol, take * 4, cudaMemcpyDeviceToHost));

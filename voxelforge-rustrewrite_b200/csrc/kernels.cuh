@@ -2296,20 +2296,13 @@ __global__ void k_gather_changes(Region R, unsigned long long n, Voxel* out) {
   }
 }
 
-// Partial entries in (z, y, x) order, which is the order of domain ids: a count per span of PART_SPAN dense
-// words, then every span writes behind the ones before it. Bound by reading the dense words twice (a
-// 320 x 160 x 320 domain: 66 MB, 12 us each); entries gathered by atlas slot had to be sorted on the host (9,656
-// of them: 0.4 ms).
-constexpr unsigned PART_SPAN = 8192;
+// Partial entries in (z, y, x) order, which is the order of domain ids: a count per row of cells from the bricks that
+// have a slot (no other cell has an entry), sums over chunks of rows, and every chunk writes its rows behind the
+// ones before it. What is read follows the bricks and the rows with entries, not the domain: passes over all its dense
+// words took 700 us a call on the world of 9 x 9 chunks, entries gathered by slot and sorted on the host 180 us with
+// hardly an entry and 610 with 9,656 (dam break).
+constexpr unsigned PART_TILE = 128, PART_CHUNKS = 4096;  // rows of a chunk: a multiple of the tile, so few chunks that each adds up those before it
 __device__ __forceinline__ bool dc_has_part(unsigned u) { return dc_solid(u) ? u == DC_SOLID_PART : dc_volume(u) > 0.0f && dc_volume(u) < 1.0f; }
-__device__ __forceinline__ uint4 dense_quad(const Region& R, unsigned id) {
-  if (id + 4u <= R.ncells) return *reinterpret_cast<const uint4*>(R.dense + id);
-  uint4 u = make_uint4(0u, 0u, 0u, 0u);
-  if (id < R.ncells) u.x = R.dense[id];
-  if (id + 1u < R.ncells) u.y = R.dense[id + 1u];
-  if (id + 2u < R.ncells) u.z = R.dense[id + 2u];
-  return u;
-}
 __device__ __forceinline__ unsigned block_sum(unsigned v) {
   __shared__ unsigned s[32];
   v = __reduce_add_sync(FULLMASK, v);
@@ -2318,54 +2311,97 @@ __device__ __forceinline__ unsigned block_sum(unsigned v) {
   __syncthreads();
   return __reduce_add_sync(FULLMASK, (threadIdx.x & 31u) < (blockDim.x >> 5) ? s[threadIdx.x & 31u] : 0u);
 }
-__global__ void __launch_bounds__(256) k_part_count(Region R, unsigned* counts) {
-  unsigned c = 0;
+// Entries per row (z - pz0) * PY + y; a warp per slot, eight lanes per row of its brick.
+__global__ void __launch_bounds__(256) k_part_rows(Region R, const int* slot_gi, unsigned nslots, unsigned* rows) {
+  const unsigned lane = lane_id();
+  for (unsigned s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; s < nslots; s += (gridDim.x * blockDim.x) >> 5) {
+    const int gi = slot_gi[s];
+    int x0, y0, z0;
+    if (gi < 0 || !brick_origin(R, (unsigned)gi, x0, y0, z0)) continue;
+    unsigned u[16];
 #pragma unroll
-  for (unsigned r = 0; r < PART_SPAN / 1024u; ++r) {
-    const uint4 u = dense_quad(R, blockIdx.x * PART_SPAN + r * 1024u + threadIdx.x * 4u);
-    c += (dc_has_part(u.x) ? 1u : 0u) + (dc_has_part(u.y) ? 1u : 0u) + (dc_has_part(u.z) ? 1u : 0u) + (dc_has_part(u.w) ? 1u : 0u);
+    for (int k = 0; k < 16; ++k) {
+      const unsigned v = 32u * k + lane;
+      const int x = x0 + (int)(v & 7u), y = y0 + (int)((v >> 3) & 7u), z = z0 + (int)(v >> 6);
+      u[k] = in_dom(R, x, y, z) ? R.dense[dom_id(R, x, y, z)] : 0u;
+    }
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+      const unsigned c = (unsigned)__popc((__ballot_sync(FULLMASK, dc_has_part(u[k])) >> (lane & 24u)) & 0xFFu);
+      const unsigned v = 32u * k + lane;
+      if (c && (lane & 7u) == 0u) atomicAdd(rows + (size_t)(z0 + (int)(v >> 6) - R.pz0) * (unsigned)R.PY + (unsigned)(y0 + (int)((v >> 3) & 7u)), c);
+    }
   }
-  c = block_sum(c);
-  if (threadIdx.x == 0) counts[blockIdx.x] = c;
 }
-__global__ void __launch_bounds__(256) k_part_write(Region R, const unsigned* counts, int* xyz, float* vol, unsigned long long cap, unsigned long long* count) {
-  const unsigned tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-  __shared__ unsigned s[8];
-  if (counts[blockIdx.x] == 0u && blockIdx.x != gridDim.x - 1u) return;
+__global__ void __launch_bounds__(PART_TILE) k_part_sums(const unsigned* rows, unsigned nrows, unsigned per, unsigned* sums) {
+  unsigned c = 0;
+  const unsigned r0 = blockIdx.x * per, r1 = min(nrows, r0 + per);
+  for (unsigned r = r0 + threadIdx.x; r < r1; r += PART_TILE) c += rows[r];
+  c = block_sum(c);
+  if (threadIdx.x == 0) sums[blockIdx.x] = c;
+}
+__global__ void __launch_bounds__(PART_TILE) k_part_write(Region R, const unsigned* rows, unsigned nrows, unsigned per, const unsigned* sums, int* xyz, float* vol,
+                                                          unsigned long long cap) {
+  __shared__ unsigned s_cnt[PART_TILE / 32], s_nz[PART_TILE / 32], s_row[PART_TILE], s_at[PART_TILE];
+  const unsigned tid = threadIdx.x, lane = lane_id(), warp = tid >> 5;
+  if (sums[blockIdx.x] == 0u) return;
   unsigned before = 0;
-  for (unsigned b = tid; b < blockIdx.x; b += 256u) before += counts[b];
+  for (unsigned b = tid; b < blockIdx.x; b += PART_TILE) before += sums[b];
   before = block_sum(before);
-  if (blockIdx.x == gridDim.x - 1u && tid == 0u) *count = before + counts[blockIdx.x];
-  for (unsigned r = 0; r < PART_SPAN / 1024u; ++r) {
-    const unsigned id = blockIdx.x * PART_SPAN + r * 1024u + tid * 4u;
-    const uint4 q = dense_quad(R, id);
-    const unsigned u[4] = {q.x, q.y, q.z, q.w};
-    unsigned c = 0;
-#pragma unroll
-    for (int e = 0; e < 4; ++e) c += dc_has_part(u[e]) ? 1u : 0u;
+  const unsigned r0 = blockIdx.x * per, r1 = min(nrows, r0 + per);
+  for (unsigned base = r0; base < r1; base += PART_TILE) {
+    // ---- the tile's rows with entries, and where each one's begin
+    const unsigned c = base + tid < r1 ? rows[base + tid] : 0u;
     unsigned pre = c;
     for (int o = 1; o < 32; o <<= 1) {
       const unsigned v = __shfl_up_sync(FULLMASK, pre, o);
       if (lane >= (unsigned)o) pre += v;
     }
+    const unsigned b = __ballot_sync(FULLMASK, c != 0u);
     __syncthreads();
-    if (lane == 31u) s[warp] = pre;
+    if (lane == 31u) {
+      s_cnt[warp] = pre;
+      s_nz[warp] = (unsigned)__popc(b);
+    }
     __syncthreads();
-    const unsigned w = lane < 8u ? s[lane] : 0u;
-    unsigned long long k = before + __reduce_add_sync(FULLMASK, lane < warp ? w : 0u) + pre - c;
-    before += __reduce_add_sync(FULLMASK, w);
+    unsigned at = before + pre - c, k0 = (unsigned)__popc(b & lanemask_lt()), full = 0;
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      if (!dc_has_part(u[e])) continue;
-      if (k < cap) {
-        int x, y, z;
-        dom_xyz(R, id + e, x, y, z);
-        xyz[3 * k] = x;
-        xyz[3 * k + 1] = y;
-        xyz[3 * k + 2] = z;
-        vol[k] = dc_solid(u[e]) ? load_cell(R, R.ring, x, y, z).part : dc_volume(u[e]);
+    for (unsigned w = 0; w < PART_TILE / 32; ++w) {
+      at += w < warp ? s_cnt[w] : 0u;
+      k0 += w < warp ? s_nz[w] : 0u;
+      before += s_cnt[w];
+      full += s_nz[w];
+    }
+    if (c) {
+      s_row[k0] = base + tid;
+      s_at[k0] = at;
+    }
+    __syncthreads();
+    // ---- a row per warp
+    for (unsigned k = warp; k < full; k += PART_TILE / 32) {
+      const unsigned row = s_row[k];
+      const unsigned id0 = row * (unsigned)R.PX;
+      unsigned long long p = s_at[k];
+      for (unsigned x0 = 0; x0 < (unsigned)R.PX; x0 += 128u) {  // four loads under way at a time
+        unsigned u[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) u[e] = x0 + 32u * e + lane < (unsigned)R.PX ? R.dense[id0 + x0 + 32u * e + lane] : 0u;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const bool has = dc_has_part(u[e]);
+          const unsigned m = __ballot_sync(FULLMASK, has);
+          const unsigned long long i = p + (unsigned)__popc(m & lanemask_lt());
+          if (has && i < cap) {
+            int x, y, z;
+            dom_xyz(R, id0 + x0 + 32u * e + lane, x, y, z);
+            xyz[3 * i] = x;
+            xyz[3 * i + 1] = y;
+            xyz[3 * i + 2] = z;
+            vol[i] = dc_solid(u[e]) ? load_cell(R, R.ring, x, y, z).part : dc_volume(u[e]);
+          }
+          p += (unsigned)__popc(m);
+        }
       }
-      ++k;
     }
   }
 }
