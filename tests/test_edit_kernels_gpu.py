@@ -103,3 +103,26 @@ def test_displaced_water_rises_past_a_full_column(vf, orc, depth):
     assert_same_state(sim, o, (-1, 0, -1, 18, 105, 18))
     assert sim.partial_count() == o.partial_count()
     sim.close()
+
+
+# one cell, or a few in turn, many times: over the levels where water shows and hides, until it is full or gone
+@pytest.mark.parametrize("n", [2, 1023, 1024, 1025, 3000])
+@pytest.mark.parametrize("cells", [1, 8])
+@pytest.mark.parametrize("amount", [0.3, 0.013, 1e-4, 1e-7, -0.013, -0.3])
+def test_emitters_of_the_same_cells(vf, orc, n, cells, amount):
+    sim, o, box = lake(vf, orc)
+    some = np.array([[20, 12, 20], [20, 13, 20], [5, 12, 5], [30, 20, 30], [11, 20, 11], [0, 4, 0], [20, 14, 20], [39, 27, 39]], np.int32)[:cells]
+    lists = np.ascontiguousarray(np.resize(some, (n, 3)))
+    for s in (sim, o):
+        s.set_partial(20, 13, 20, 0.49)
+        s.set_partial(5, 12, 5, 0.31)
+    for _ in range(2):
+        sim.emit(lists, amount)
+        o.emit(lists, amount)
+        assert_same_state(sim, o, box)
+        assert sim.partial_count() == o.partial_count()
+    assert all(m == o.get_voxel(x, y, z) for x, y, z, m in sim.download_changes().tolist())
+    sim.tick(2)
+    o.tick(2)
+    assert_same_state(sim, o, box)
+    sim.close()

@@ -1642,10 +1642,12 @@ __device__ __forceinline__ unsigned edit_scan(unsigned* cnt, bool f, unsigned* t
 
 // Rain emitters in list order (for each cell: vol' = min(1, vol + amount) through set_volume, then
 // activate it), one CTA. Cells of the list that differ do not touch each other, so a chunk of 1024
-// runs at once; a cell listed again in the chunk waits for its earlier entry (claims in rb) and the
-// activations join the FIFO in list order by a scan. One warp in order spent ~1.6 us per emitter.
+// runs at once; the first entry of a cell (claims in rb) takes the later ones of the chunk with it, one
+// after another in registers, and the activations join the FIFO in list order by a scan. One warp in order
+// spent ~0.8 us per emitter of a cell listed before and 1.2 per new one (1,024 of one cell: 845 us; in rounds of the
+// chunk, one entry of each cell a round, 1.4 ms).
 __global__ void __launch_bounds__(EDIT_THREADS) k_emit(Region R, const int* xyz, unsigned long long n, float amount) {
-  __shared__ unsigned cnt[32];
+  __shared__ unsigned cnt[32], s_more[EDIT_THREADS];
   __shared__ int s_pd, s_ch;
   const unsigned tid = threadIdx.x;
   if (tid == 0) s_pd = s_ch = 0;
@@ -1655,41 +1657,48 @@ __global__ void __launch_bounds__(EDIT_THREADS) k_emit(Region R, const int* xyz,
   for (unsigned long long base = 0; base < n; base += blockDim.x) {
     const unsigned long long i = base + tid;
     int x = 0, y = 0, z = 0;
-    bool pend = false;
+    bool open = false;
     unsigned id = 0;
+    CD c = CD{0.0f, NOSLOT, 0u, 0, true};
     if (i < n) {
       x = xyz[3 * i];
       y = xyz[3 * i + 1];
       z = xyz[3 * i + 2];
-      pend = !cd_solid(load_cell_par(R, R.ring, x, y, z));  // a cell's solidity does not change here
-      if (pend) id = dom_id(R, x, y, z);
+      c = load_cell_par(R, R.ring, x, y, z);
+      open = !cd_solid(c);
+      if (open) id = dom_id(R, x, y, z);
     }
-    bool act = false;
+    s_more[tid] = 0u;
+    if (open) atomicMin(R.rb + id, tid);
+    __syncthreads();
+    const unsigned first = open ? __ldcg(R.rb + id) : tid;  // set by atomics (in L2): read past L1
+    const bool act = open && first == tid;
+    if (first != tid) atomicAdd(&s_more[first], 1u);
+    __syncthreads();
+    // (an entry that needs no slot changes nothing, and so do the later ones of its cell)
+    materialize_cta(R, act && set_volume_needs_slot(c, fminf(1.0f, __fadd_rn(cd_volume(c), amount))), c.gi, c.slot);
     int pd = 0;
-    for (bool first = true;; first = false) {
-      if (pend) atomicMin(R.rb + id, tid);
-      __syncthreads();
-      const bool win = pend && __ldcg(R.rb + id) == tid;  // set by atomics (in L2): read past L1
-      __syncthreads();
-      CD c = CD{0.0f, NOSLOT, 0u, 0, true};
-      float nv = 0.0f;
-      if (win) {
-        c = load_cell_par(R, R.ring, x, y, z);
-        nv = fminf(1.0f, __fadd_rn(cd_volume(c), amount));
-      }
-      const bool need = win && set_volume_needs_slot(c, nv);
-      materialize_cta(R, need, c.gi, c.slot);
-      if (win) {
-        const SVPlan p = sv_plan(c.part, c.mat, c.slot != NOSLOT, nv);
-        if (c.slot != NOSLOT) sv_apply(R, c, id, local_index(x, y, z), p);
-        if (p.wmat) record_change(R, id);
-        if (p.ch) s_ch = 1;
+    if (act) {
+      bool wpart = false, wmat = false, ch = false;
+      for (unsigned k = s_more[tid] + 1u; k; --k) {
+        const SVPlan p = sv_plan(c.part, c.mat, c.slot != NOSLOT, fminf(1.0f, __fadd_rn(cd_volume(c), amount)));
+        wpart |= p.wpart;
+        wmat |= p.wmat;
+        ch |= p.ch;
         pd += p.dp;
-        R.rb[id] = 0xFFFFFFFFu;
-        pend = false;
-        act = first;
+        if (!p.wmat && !(p.wpart && __float_as_uint(p.npart) != __float_as_uint(c.part))) break;  // the later ones do the same
+        if (p.wpart) c.part = p.npart;
+        if (p.wmat) c.mat = p.nmat;
       }
-      if (!__syncthreads_or(pend ? 1 : 0)) break;
+      if (c.slot != NOSLOT) {
+        const size_t o = (size_t)c.slot * 512u + local_index(x, y, z);
+        if (wpart) R.avol[o] = c.part;
+        if (wmat) R.amat[o] = c.mat;
+        dense_put(R, id, c.mat, c.part);
+      }
+      if (wmat) record_change(R, id);
+      if (ch) s_ch = 1;
+      R.rb[id] = 0xFFFFFFFFu;
     }
     if (pd) atomicAdd(&s_pd, pd);
     const bool isnew = act && !((__ldcg(&R.active[id >> 5]) >> (id & 31u)) & 1u);
