@@ -115,3 +115,24 @@ def test_lists_in_no_order(vf, orc, order):
     assert sim.apply_brush(cells, STONE) == o.apply_brush(cells, STONE)
     same(sim, o, 2)
     sim.close()
+
+
+# cells without water touch nothing but themselves and may come in any order: columns that reach as far below and
+# above their first cell as one walk goes, and one row further, in air and with water at the bottom
+@pytest.mark.parametrize("first", [60, 100, 20])
+@pytest.mark.parametrize("order", ["listed", "down", "shuffled"])
+def test_dry_columns_in_any_order(vf, orc, first, order):
+    sim, o = pool(vf, orc, 200, 40)
+    ys = [first] + [y for y in (first - 31, first - 32, first - 33, first + 95, first + 96, first - 1, first + 1, first + 40, first - 20, 39, 41) if 4 <= y < 200]
+    if order == "down":
+        ys = sorted(set(ys))[::-1]
+    elif order == "shuffled":
+        ys = np.random.default_rng(first).permutation(sorted(set(ys))).tolist()
+    cells = np.array([[x, y, 20] for x in range(10, 20) for y in ys], np.int32)
+    assert sim.apply_brush(cells, STONE) == o.apply_brush(cells, STONE)
+    same(sim, o)
+    cells = np.random.default_rng(7).permutation(sphere((24, 70, 24), 7))  # all dry
+    cells = np.ascontiguousarray(cells)
+    assert sim.apply_brush(cells, STONE) == o.apply_brush(cells, STONE)
+    same(sim, o, 2)
+    sim.close()

@@ -208,6 +208,7 @@ __host__ __device__ inline unsigned dense_code(bool out, unsigned mat, unsigned 
   return mat == WATER ? DC_FULL : 0u;
 }
 __host__ __device__ inline bool dc_solid(unsigned u) { return (int)u >= (int)DC_SOLID; }
+__host__ __device__ inline bool dc_water(unsigned u) { return (int)u > 0 && !dc_solid(u); }  // the material
 
 // One cell as the atlas holds it.
 struct __align__(16) CD {

@@ -1767,29 +1767,32 @@ __global__ void __launch_bounds__(EDIT_THREADS) k_carve(Region R, const int* xyz
 
 // apply_brush with a solid material (src/edit/brush.rs:93-111) over a long list, one CTA. A listed water
 // cell's water goes up its own column (FluidSim::displace, fluid.rs:370-408), so the columns of a stroke
-// are independent as long as every column's cells are listed upwards and its water finds room above: a
+// are independent as long as the cells of a column with water are listed upwards and it finds room above: a
 // warp then takes a column, in registers. In chunks of the list: the voxels and columns are claimed (rb, stamp); every
 // column is tried without writing, up to its first cell that does not fit (water that goes to the sides, a
-// cell listed after one above it or twice, a column of more than 128 cells, water that
+// cell of such a column after one above it, a voxel listed twice, a column of more than 96 rows, water that
 // goes to more than three cells). What the list holds before the first of those commits to the dense words and logs what
 // each listed cell did, and the log is followed in list order: slots, the atlas, and the
 // activations (27 around a displaced cell, then those that took its water), 16 cells at a time, each cell
 // activated by its first mention. That first cell then takes its turn as brush_warp does (up to 64 cells when
 // the next chunks stop early too), and the rest is the next chunk. One warp in list order spent 3.2 us
-// on each displaced cell.
+// on each displaced cell and 1.2 on a dry one: 257 dry cells 375 us in any order (here 80; 410 in an order that goes
+// down while such columns had to be listed upwards too).
 constexpr int BRUSH_THREADS = 512;
 constexpr unsigned BRUSH_CHUNK = 4096, BRUSH_MIN = 12;
 constexpr int BRUSH_ROWS = 4, BRUSH_TARGETS = 3;
+constexpr int BRUSH_BELOW = 32;  // rows of a column that may lie below its first cell
 static_assert(BRUSH_CHUNK * sizeof(uint4) <= MAX_CELLS_PER_TICK * sizeof(LvCell), "the log lies where a tick keeps its records");
 // A log entry: .x = cells that took water | 4 placed | 8 it was water | 16 << t: cell t's voxel changed |
 // 128 it keeps an entry; .y, .z, .w those cells, or the entry's volume.
 
-// The listed cells of a column before entry `limit`, from its first (the lowest) up, by one warp. Returns the
+// The listed cells before entry `limit` of the column of entry `lead`, from the lowest up, by one warp. Returns the
 // first entry that does not fit, or `limit` (nothing is written unless `commit`).
 __device__ __forceinline__ unsigned brush_column(const Region& R, const int* xyz, unsigned lead, unsigned limit, bool commit, uint4* log, int& pd,
                                                  unsigned& placed) {
   const unsigned lane = lane_id();
-  const int x = xyz[3 * lead], y = xyz[3 * lead + 1], z = xyz[3 * lead + 2];
+  const int x = xyz[3 * lead], z = xyz[3 * lead + 2];
+  const int y = min(xyz[3 * lead + 1], (int)(__ldcg(R.stamp + dom_id(R, x, 1, z)) >> 1));  // (idle: 2^31 - 1)
   const unsigned id0 = dom_id(R, x, y, z);
   unsigned u[BRUSH_ROWS], at[BRUSH_ROWS], dirty = 0;
 #pragma unroll
@@ -1799,9 +1802,13 @@ __device__ __forceinline__ unsigned brush_column(const Region& R, const int* xyz
     u[k] = in ? R.dense[id0 + (unsigned)(up * R.PX)] : DC_SOLID;
     at[k] = in ? __ldcg(R.rb + id0 + (unsigned)(up * R.PX)) : NOSLOT;
   }
-  // Up to `limit` the column is listed upwards: it ends before the first entry with an earlier one above it. A later
-  // end then only takes the column's last cells away, so the commit finds what the try found.
-  if (!commit) {
+  // A column with water to displace is listed upwards up to `limit`: it ends before the first entry with an earlier
+  // one above it. A later end then only takes the column's last cells away, so the commit finds what the try found.
+  // (Cells without water touch nothing but themselves: their order is free.)
+  bool wet = false;
+#pragma unroll
+  for (int k = 0; k < BRUSH_ROWS; ++k) wet |= at[k] < limit && dc_water(u[k]);
+  if (!commit && __any_sync(FULLMASK, wet)) {
     unsigned above = NOSLOT, bad = NOSLOT;  // the earliest entry of the rows above
 #pragma unroll
     for (int k = BRUSH_ROWS - 1; k >= 0; --k) {
@@ -1915,7 +1922,7 @@ __global__ void __launch_bounds__(BRUSH_THREADS) k_brush(Region R, const int* li
     const unsigned all = (unsigned)min((unsigned long long)size, n - base);
     if (tid == 0) s_limit = all;
     __syncthreads();
-    // ---- claims: a voxel's first entry, a column's first entry
+    // ---- claims: a voxel's first entry, a column's first entry (at its layer 0), its lowest cell below that one (layer 1)
     for (unsigned i = tid; i < all; i += BRUSH_THREADS) {
       const int x = xyz[3 * i], y = xyz[3 * i + 1], z = xyz[3 * i + 2];
       log[i] = make_uint4(0u, 0u, 0u, 0u);
@@ -1927,9 +1934,14 @@ __global__ void __launch_bounds__(BRUSH_THREADS) k_brush(Region R, const int* li
     for (unsigned i = tid; i < all; i += BRUSH_THREADS) {
       const int x = xyz[3 * i], y = xyz[3 * i + 1], z = xyz[3 * i + 2];
       if (outside(R, ring, x, y, z)) continue;
-      const unsigned lead = __ldcg(R.stamp + dom_id(R, x, 0, z));
+      const unsigned id = dom_id(R, x, y, z), lead = __ldcg(R.stamp + dom_id(R, x, 0, z));
       const int yl = xyz[3 * lead + 1];
-      if (__ldcg(R.rb + dom_id(R, x, y, z)) != i || y < yl || y - yl >= 32 * BRUSH_ROWS) atomicMin(&s_limit, i);
+      bool end = __ldcg(R.rb + id) != i || y - yl >= 32 * BRUSH_ROWS - BRUSH_BELOW || yl - y > BRUSH_BELOW;
+      if (y < yl && !end) {  // (water in one of the two: the try would find it too, after trying more)
+        end = dc_water(R.dense[id]) || dc_water(R.dense[dom_id(R, x, yl, z)]);
+        if (!end) atomicMin(R.stamp + dom_id(R, x, 1, z), 2u * (unsigned)y + 1u);
+      }
+      if (end) atomicMin(&s_limit, i);
     }
     __syncthreads();
     // ---- the columns: tried, then committed
@@ -1940,15 +1952,15 @@ __global__ void __launch_bounds__(BRUSH_THREADS) k_brush(Region R, const int* li
       pd = 0;
       placed = 0;
       __syncthreads();
-      for (unsigned b0 = warp * 32u; b0 < len; b0 += BRUSH_THREADS) {
-        const unsigned i = b0 + lane;
+      for (unsigned b0 = warp; b0 < len; b0 += BRUSH_THREADS) {  // neighbours in the list to different warps: often a row of columns
+        const unsigned i = b0 + lane * (BRUSH_THREADS / 32);
         bool lead = false;
         if (i < len) {
           const int x = xyz[3 * i], y = xyz[3 * i + 1], z = xyz[3 * i + 2];
           lead = !outside(R, ring, x, y, z) && __ldcg(R.stamp + dom_id(R, x, 0, z)) == i;
         }
         for (unsigned mask = __ballot_sync(FULLMASK, lead); mask; mask &= mask - 1u) {
-          const unsigned fit = brush_column(R, xyz, b0 + (unsigned)__ffs(mask) - 1u, len, commit != 0, log, pd, placed);
+          const unsigned fit = brush_column(R, xyz, b0 + ((unsigned)__ffs(mask) - 1u) * (BRUSH_THREADS / 32), len, commit != 0, log, pd, placed);
           if (lane == 0u && fit < len) atomicMin(&s_limit, fit);
         }
       }
@@ -1959,6 +1971,7 @@ __global__ void __launch_bounds__(BRUSH_THREADS) k_brush(Region R, const int* li
       if (outside(R, ring, x, y, z)) continue;
       R.rb[dom_id(R, x, y, z)] = 0xFFFFFFFFu;
       R.stamp[dom_id(R, x, 0, z)] = 0xFFFFFFFFu;
+      R.stamp[dom_id(R, x, 1, z)] = 0xFFFFFFFFu;
     }
     __syncthreads();
     if (pd) atomicAdd(&s_pd, pd);
