@@ -42,3 +42,40 @@ def test_gradients_at_tile_edges(vf, n):
     for _ in range(2):
         assert np.abs(mlp.grads(xd, yd) - ref).max() <= tol
     mlp.close()
+
+
+def test_a_refused_call_leaves_the_handle_as_it_was():
+    """Gradients wait for the host, which a stream under capture refuses: the call fails, and the next one is right
+    (in a process of its own, for the broken capture)."""
+    import subprocess
+    import sys
+    from pathlib import Path
+
+    code = """
+import numpy as np, torch
+import __graft_entry__ as ge
+vf = ge.load_package()
+from vfwater import proposal
+mlp = proposal.MLP(seed=4)
+x = torch.rand(200, 32, device="cuda").half()
+y = (torch.rand(200, device="cuda") < 0.5).float()
+want = mlp.grads(x, y)
+graph, stream = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+refused = []
+try:
+    with torch.cuda.graph(graph, stream=stream):
+        for call in (lambda: mlp.grads(x, y, stream=stream.cuda_stream), lambda: mlp.train_step(x, y, 0.0, stream=stream.cuda_stream, want_loss=True)):
+            try:
+                call()
+            except vf.VfError:
+                refused.append(1)
+except RuntimeError:
+    pass
+assert len(refused) == 2, refused
+torch.cuda.synchronize()
+for _ in range(2):
+    assert np.allclose(mlp.grads(x, y), want, rtol=1e-5, atol=1e-9)
+print("ok")
+"""
+    r = subprocess.run([sys.executable, "-c", code], cwd=Path(__file__).resolve().parents[1], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and r.stdout.strip().endswith("ok"), r.stdout + r.stderr

@@ -468,6 +468,14 @@ void release(vf_mlp* h) {
   if (h->hgrad) cudaFreeHost(h->hgrad);
   delete h;
 }
+// The sums' reader empties them; where a call failed it may not have run, so the call that says so does it, and
+// takes its error with it (the next call asks for errors of its own).
+int failed(vf_mlp* h, cudaStream_t st) {
+  cudaMemsetAsync(h->d.g, 0, NPARAM * 4, st);
+  cudaMemsetAsync(h->d.ticket, 0, 4, st);
+  cudaGetLastError();
+  return VF_ERR_CUDA;
+}
 unsigned blocks_for(uint64_t n) { return (unsigned)((n + 16 * WARPS - 1) / (16 * WARPS)); }
 }  // namespace
 
@@ -549,7 +557,7 @@ int vf_mlp_grads(vf_mlp* h, const void* dev_x, const float* dev_y, uint64_t n, f
   cudaStream_t st = (cudaStream_t)stream;
   // (d.g is empty between calls: its reader empties it)
   k_backward<<<std::min(blocks_for(n), (unsigned)h->ctas), 32 * WARPS, sizeof(BackSmem), st>>>(h->d, (const __half*)dev_x, dev_y, (int)n, 1.0f / (float)n, h->dgrad);
-  if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(st) != cudaSuccess) return VF_ERR_CUDA;
+  if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(st) != cudaSuccess) return failed(h, st);
   std::memcpy(grads, h->hgrad, NPARAM * 4);
   return VF_OK;
 }
@@ -570,10 +578,10 @@ int vf_mlp_train_step(vf_mlp* h, const void* dev_x, const float* dev_y, uint64_t
   k_adam<<<(NPARAM + 255) / 256, 256, 0, st>>>(h->d, lr, b1, b2, 1e-8f, c1, c2);
   k_refresh<<<32, 256, 0, st>>>(h->d);
   if (loss) {
-    if (cudaMemcpyAsync(loss, h->d.loss, 4, cudaMemcpyDeviceToHost, st) != cudaSuccess) return VF_ERR_CUDA;
-    if (cudaStreamSynchronize(st) != cudaSuccess) return VF_ERR_CUDA;
+    if (cudaMemcpyAsync(loss, h->d.loss, 4, cudaMemcpyDeviceToHost, st) != cudaSuccess) return failed(h, st);
+    if (cudaStreamSynchronize(st) != cudaSuccess) return failed(h, st);
   }
-  return cudaGetLastError() == cudaSuccess ? VF_OK : VF_ERR_CUDA;
+  return cudaGetLastError() == cudaSuccess ? VF_OK : failed(h, st);
 }
 
 }  // extern "C"
