@@ -184,9 +184,8 @@ int vf_fluid_export_box(vf_fluid* h, int32_t x0, int32_t y0, int32_t z0, int32_t
 int vf_fluid_digest(vf_fluid* h, uint64_t* state, uint64_t* queue, uint64_t* seeds);
 
 /* Cycle counters per tick phase, summed over all ticks (SM clock of the region's CTA): 0 drain,
- * 1 sort, 2 sweep, 3 sweep waiting on prefetch, 4 pressure pulls, 5 activation logging, 6 voxel
- * writes, 7 seed commit, 8 levelling, 9 FIFO commit, 10 change commit, 11 mark clearing,
- * 15 between ticks. */
+ * 1 sort, 2 sweep, 7 seed commit, 8 levelling, 9 FIFO commit, 10 change commit, 11 mark clearing,
+ * 15 between ticks; the others zero. */
 int vf_fluid_profile(vf_fluid* h, uint64_t* out16);
 
 /* ---- learned wake proposal (pattern (4)). Rows are atlas slots (materialised bricks).

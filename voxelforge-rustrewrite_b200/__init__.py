@@ -399,23 +399,22 @@ class FluidSim:
         """Lower the per-tick event-log capacities (a tick that overflows one fails with VF_ERR_OOM)."""
         self._check(lib().vf_fluid_set_log_caps(self.h, act, seed, chg), "set_log_caps")
 
-    SWEEP_PROFILE = ("prepass", "segments", "rollbacks", "logs", "dep_wait", "start_wait", "footprint", "pulls", "writes", "cells",
-                     "row_fetch", "worker_total", "cone_wait", "gate_wait", "searches", "rounds", "search_reads",
-                     "source_writes")
+    # counters of vf_fluid_sweep_profile: SM cycles of the parts of a sweep, then counts (the other entries are zero)
+    SWEEP_PROFILE = {"prepass": 0, "rounds_and_pulls": 1, "atlas_and_logs": 3, "cta_searches": 7, "wide_rounds": 8, "cells": 9, "searches": 14, "rounds": 15}
 
     def sweep_profile(self) -> dict:
-        """Sweep counters summed over ticks (vf_fluid_sweep_profile: SM cycles, and counts of cells, searches, rounds)."""
+        """Sweep counters summed over ticks: SM cycles of the prepass, of rounds and pulls (of which: searches by all
+        warps, rounds by all warps), of the atlas and the event logs; drained cells, pressure searches, rounds."""
         a = (C.c_uint64 * 18)()
         self._check(lib().vf_fluid_sweep_profile(self.h, a), "sweep_profile")
-        return dict(zip(self.SWEEP_PROFILE, map(int, a)))
+        return {k: int(a[i]) for k, i in self.SWEEP_PROFILE.items()}
 
     def sweep_stats(self) -> dict:
-        """Sweep counters over all ticks: rounds (segments), searches run again (rollbacks), searches (replayed)."""
+        """Sweep counters over all ticks: rounds, pressure searches, and those run again because an earlier cell had yet
+        to write what they read."""
         a, b, c = C.c_uint64(), C.c_uint64(), C.c_uint64()
-        k = (C.c_uint64 * 3)()
-        self._check(lib().vf_fluid_sweep_stats(self.h, C.byref(a), C.byref(b), C.byref(c), k), "sweep_stats")
-        return {"segments": a.value, "rollbacks": b.value, "replayed": c.value,
-                "conflicts": {"reader_started": k[0], "pull_read": k[1], "new_attempter": k[2]}}
+        self._check(lib().vf_fluid_sweep_stats(self.h, C.byref(a), C.byref(b), C.byref(c), None), "sweep_stats")
+        return {"rounds": a.value, "searches": c.value, "searches_again": b.value}
 
     def emit_device_async(self, dev_xyz_ptr: int, n: int, amount: float):
         self._check(lib().vf_fluid_emit_device_async(self.h, C.c_void_p(dev_xyz_ptr), n, amount), "emit_device_async")
@@ -485,14 +484,14 @@ class FluidSim:
     def last_tick_cells(self) -> int:
         return self.stats().last_tick_cells
 
-    PROFILE_PHASES = ("drain", "sort", "sweep", "sweep_wait", "pulls", "act_log", "writes", "seed_commit", "level", "fifo_commit",
-                      "chg_commit", "mark_clear", "sweep_top", "sweep_cell", "sweep_tail", "between")
+    # entries of vf_fluid_profile (the others are zero)
+    PROFILE_PHASES = {"drain": 0, "sort": 1, "sweep": 2, "seed_commit": 7, "level": 8, "fifo_commit": 9, "chg_commit": 10, "mark_clear": 11, "between": 15}
 
     def profile(self) -> dict:
         """SM cycles per tick phase, summed over all ticks so far."""
         a = (C.c_uint64 * 16)()
         self._check(lib().vf_fluid_profile(self.h, a), "profile")
-        return {k: int(v) for k, v in zip(self.PROFILE_PHASES, a) if k != "-"}
+        return {k: int(a[i]) for k, i in self.PROFILE_PHASES.items()}
 
     def shift(self, dx, dz):
         self._check(lib().vf_fluid_shift(self.h, dx, dz), "shift")
