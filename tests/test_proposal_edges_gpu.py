@@ -79,3 +79,39 @@ print("ok")
 """
     r = subprocess.run([sys.executable, "-c", code], cwd=Path(__file__).resolve().parents[1], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and r.stdout.strip().endswith("ok"), r.stdout + r.stderr
+
+
+@pytest.mark.parametrize("ring", [False, True])
+@pytest.mark.parametrize("rows", [1, 300, 100000])  # fewer rows than slots, more than the atlas holds
+def test_staging_counts_rows_and_changes_nothing(vf, ring, rows):
+    import torch
+
+    from vfwater import proposal
+
+    if ring:
+        w = vf.World.ring(4, 64)
+        chunk = vf.World(128, 64, 128)
+        chunk.fill_box(0, 0, 0, 127, 7, 127, 3)
+        for cx in (-1, 0):
+            w.ring_paste(chunk, cx, 0)
+        w.fill_box(-20, 8, 40, 19, 30, 59, 5)
+        box = (-24, 7, 36, 23, 34, 63)
+    else:
+        w = vf.World(61, 43, 77)  # bricks that reach past the world on every side
+        w.fill_box(0, 0, 0, 60, 3, 76, 3)
+        w.fill_box(30, 4, 40, 60, 30, 76, 5)
+        box = (0, 0, 0, 60, 42, 76)
+    sim = vf.FluidSim(w, atlas_bricks=2000)
+    sim.wake(*box)
+    sim.tick(5)
+    if ring:
+        sim.ring_evict(0, 0)
+    before = sim.digest()
+    p = torch.rand(rows, device="cuda")
+    p[0] = 0.5
+    n = min(rows, max(2000, sim.stats().atlas_used + 64))
+    staged = proposal.stage(sim, p, 0.5)
+    assert staged <= int((p >= 0.5).sum()) and (rows > 1000 or staged == int((p[:n] >= 0.5).sum()))
+    assert sim.digest() == before
+    sim.tick(2)
+    sim.close()

@@ -1230,7 +1230,8 @@ int vf_fluid_stage_bricks(vf_fluid* h, const float* dev_prob, uint64_t nslots, f
   if (!nslots) return VF_OK;
   const unsigned n = (unsigned)std::min<uint64_t>(nslots, h->R.atlas_cap);
   CK(cudaMemsetAsync(h->staged, 0, 4, h->stream));
-  k_stage<<<(n + 255) / 256, 256, 0, h->stream>>>(h->R, n, dev_prob, threshold, h->staged);
+  const uint64_t threads = std::max<uint64_t>(n, (uint64_t)h->R.bx * h->R.by * h->R.bz);
+  k_stage<<<(unsigned)std::min<uint64_t>((threads + 255) / 256, 148 * 8), 256, 0, h->stream>>>(h->R, n, dev_prob, threshold, h->staged);
   CK(cudaGetLastError());
   if (n_staged) {
     unsigned c = 0;

@@ -134,8 +134,7 @@ __device__ void materialize_lanes(const Region& R, bool need, unsigned gi, unsig
     }
   }
   __syncwarp();
-  // publish the slot after its fill (release): prefetching warps read the grid word first and
-  // then the atlas, with a fence in between
+  // publish the slot after its fill (release)
   __threadfence_block();
   if (leader && s != NOSLOT && g < 256u) *(volatile unsigned*)(R.grid + gi) = 256u + s;
   int src = need ? (__ffs(peers) - 1) : (int)lane;

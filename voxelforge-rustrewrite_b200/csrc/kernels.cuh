@@ -1389,7 +1389,7 @@ __global__ void __launch_bounds__(PAR_THREADS, 1) k_tick_par(Region* regs, int n
   extern __shared__ __align__(16) unsigned char smraw[];
   TickSmem& sm = *reinterpret_cast<TickSmem*>(smraw);
   // The region's constants (sizes, array bases): a copy in shared memory keeps them off the L1, which
-  // the sweep's records and atlas lines stream through.
+  // the sweep's records and dense words stream through.
   __shared__ Region s_reg;
   for (int r = blockIdx.x; r < nreg; r += gridDim.x) {
     if (threadIdx.x == 0) s_reg = regs[r];
@@ -2588,15 +2588,23 @@ __global__ void k_slot_labels(Region R, unsigned nslots, unsigned since, unsigne
   }
 }
 
-// Pre-stage the bricks the proposal expects to wake: their material and volume lines into L2.
+// Pre-stage the bricks the proposal expects to wake: what the sweep and its searches read of their cells, the dense
+// words (64 rows of one sector), into L2. `staged` counts the slots, a thread each; a thread per grid word finds
+// their bricks. It gains little, for most of a region's words are in L2: 40 ticks of the ring world 117.2 ms, 117.7
+// when it fetched the atlas, which the sweep no longer reads.
 __global__ void k_stage(Region R, unsigned nslots, const float* prob, float thr, unsigned* staged) {
-  for (unsigned s = blockIdx.x * blockDim.x + threadIdx.x; s < nslots; s += gridDim.x * blockDim.x) {
-    if (!(prob[s] >= thr)) continue;
-    const char* m = reinterpret_cast<const char*>(R.amat + (size_t)s * 512u);
-    const char* v = reinterpret_cast<const char*>(R.avol + (size_t)s * 512u);
-    for (int k = 0; k < 4; ++k) asm volatile("prefetch.global.L2 [%0];" ::"l"(m + 128 * k));
-    for (int k = 0; k < 16; ++k) asm volatile("prefetch.global.L2 [%0];" ::"l"(v + 128 * k));
-    atomicAdd(staged, 1u);
+  const unsigned t0 = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
+  for (unsigned s = t0; s < nslots; s += nt)
+    if (prob[s] >= thr) atomicAdd(staged, 1u);
+  const unsigned nb = (unsigned)R.bx * (unsigned)R.by * (unsigned)R.bz;
+  for (unsigned long long gi = t0; gi < nb; gi += nt) {
+    const unsigned g = R.grid[gi];
+    if (g < 256u || g - 256u >= nslots || !(prob[g - 256u] >= thr)) continue;
+    int x, y, z;
+    if (!brick_origin(R, (unsigned)gi, x, y, z) || !in_dom(R, x, y, z) || !in_dom(R, x + 7, y + 7, z + 7)) continue;
+    const unsigned* row = R.dense + dom_id(R, x, y, z);
+    for (int lz = 0; lz < 8; ++lz)
+      for (int ly = 0; ly < 8; ++ly) asm volatile("prefetch.global.L2 [%0];" ::"l"(row + (unsigned)((lz * R.PY + ly) * R.PX)));
   }
 }
 

@@ -7,7 +7,7 @@ the last four ticks (own and the faces': the flux proxy), wake recency, height, 
 is whether any cell of the brick is drained by the exact scheduler in ticks (t, t+k]. The network
 (32 -> 64 -> 64 -> 1) trains on the GPU with the library's own fp16 forward/backward kernels.
 
-At run time the proposal's positives are pre-staged (L2 prefetch of their atlas lines) before the
+At run time the proposal's positives are pre-staged (L2 prefetch of their dense words) before the
 tick; the exact FIFO still decides what runs, so a miss costs time and never correctness.
 """
 from __future__ import annotations

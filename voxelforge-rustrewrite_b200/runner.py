@@ -187,7 +187,7 @@ class LearnedResult:
 def run_learned(vf, wl, sims, t0: int, ticks: int, torch, stream, mlp, stage_every: int = 4, threshold: float = 0.5) -> LearnedResult:
     """Batched execution (one launch per tick run over all regions) with the learned wake
     proposal: every `stage_every` ticks each region's bricks are scored by the network and the
-    positives' atlas lines are pre-staged into L2 before the ticks run. The exact FIFO still
+    positives' dense words are pre-staged into L2 before the ticks run. The exact FIFO still
     decides what runs. Recall/precision are scored against the engine's own wake record
     `proposal.HORIZON` ticks later (outside the timed intervals)."""
     from . import proposal
