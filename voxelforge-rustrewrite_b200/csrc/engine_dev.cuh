@@ -54,17 +54,6 @@ __device__ __forceinline__ CD load_cell(const Region& R, const int* ring, int x,
   return c;
 }
 
-__device__ __forceinline__ CD shfl_cd(const CD& c, int src) {
-  CD r;
-  r.part = __shfl_sync(FULLMASK, c.part, src);
-  r.slot = __shfl_sync(FULLMASK, c.slot, src);
-  r.gi = __shfl_sync(FULLMASK, c.gi, src);
-  unsigned p = __shfl_sync(FULLMASK, (unsigned)c.mat | ((unsigned)c.out << 8), src);
-  r.mat = (unsigned char)(p & 255u);
-  r.out = (p >> 8) != 0;
-  return r;
-}
-
 // Warp-uniform scheduler state of one region: a tick's, or a host edit's.
 struct WS {
   unsigned long long qhead, qtail;

@@ -649,28 +649,6 @@ __device__ __forceinline__ bool mark_test(const Region& R, int x, int y, int z) 
   return (__ldcg(R.marks + (size_t)tile * 128u + (bit >> 5)) >> (bit & 31u)) & 1u;
 }
 
-// Exclusive prefix of a per-thread 64-bit value over the CTA (thread order); *total = the sum.
-__device__ unsigned long long cta_scan_u64(unsigned long long v, unsigned long long* total) {
-  __shared__ unsigned long long s_w[MAX_WARPS];
-  const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-  unsigned long long incl = v;
-  for (int o = 1; o < 32; o <<= 1) {
-    const unsigned long long u = __shfl_up_sync(FULLMASK, incl, o);
-    if (lane >= (unsigned)o) incl += u;
-  }
-  if (lane == 31u) s_w[warp] = incl;
-  __syncthreads();
-  unsigned long long before = 0, all = 0;
-  for (unsigned w = 0; w < NW_; ++w) {
-    const unsigned long long t = s_w[w];
-    if (w < warp) before += t;
-    all += t;
-  }
-  __syncthreads();
-  *total = all;
-  return before + incl - v;
-}
-
 // The flood fill of FluidSim::level_layer (fluid.rs:425-446) continued from queue entry qs of qe,
 // batch by batch over the CTA. The batch is every waiting entry; entry p's side d is tried in the
 // reference's order p-major, d-minor: its rank 4(p - qs) + d claims the cell (the lowest rank is

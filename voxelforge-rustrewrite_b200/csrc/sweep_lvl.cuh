@@ -284,11 +284,6 @@ __device__ __forceinline__ void succ_offset(int q, int s, int& dx, int& dy, int&
   dz = (q >= 2 && q <= 4) ? s : q == 5 ? 2 * s : q == 9 ? 1 : q == 10 ? -1 : 0;
 }
 
-__device__ __forceinline__ unsigned rank_at(const Region& R, int x, int y, int z) {
-  if (!in_dom(R, x, y, z)) return NOSLOT;
-  return R.stamp[dom_id(R, x, y, z)];
-}
-
 // ------------------------------------------------------------------------------- the lists
 // A cell enters a list once and the parked list once, so neither outgrows the tick's cells; the bounds
 // are checked all the same where an entry goes to global memory.
