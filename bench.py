@@ -37,7 +37,7 @@ DAM_BREAK = "dam-break 512x128x512, 4-octave noise terrain, lake y<48, 8-wide ch
 # DRAM bytes (read + write) of one k_tick_par launch of one step (10 dam-break ticks, ticks
 # 51..60, cold L2 as after the bench's flush): a one-off ncu capture, summarised in
 # profiles/k_tick_par_dambreak_step_dram.txt. Compare with roofline.alg_bytes_per_step.
-STEP_DRAM_BYTES = 2570496 + 212480
+STEP_DRAM_BYTES = 1_910_000 + 194_560
 
 
 def parse():
@@ -49,7 +49,7 @@ def parse():
     ap.add_argument("--workload", type=int, default=2)
     ap.add_argument("--scale", type=float, default=1.0)
     ap.add_argument("--engine", type=int, default=1, help="accepted by the library, without effect")
-    ap.add_argument("--gate", type=int, default=4 | (1 << 8), help="same-layer gate | lower-layer cone << 8")
+    ap.add_argument("--gate", type=int, default=4 | (1 << 8), help="bits 16-20: warps of a region's CTA (8..16, 0: 16); the others without effect")
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--no-variants", action="store_true")
     ap.add_argument("--variant-ticks", type=int, default=100)
@@ -190,8 +190,7 @@ VARIANTS = [
     (3, "64 regions, x,z in 32..256, y in 64..128, noise terrain, 1-4 water boxes (one persistent launch)"),
     (4, "ring 9x9 chunks of 128x256x128 (1152x256x1152), sea y<64, 1000 rain emitters, 1 level per 4 ticks"),
 ]
-VARIANT_TUNE = [{"engine": 0, "producers": 7, "depth": 64, "ticks_per_launch": 10}, {"engine": 1, "gate": 4, "ticks_per_launch": 10},
-                {"engine": 1, "gate": 4 | (1 << 8), "ticks_per_launch": 10}]
+VARIANT_TUNE = [{"gate": w << 16, "ticks_per_launch": 10} for w in (0, 8, 12)]  # warps of a region's CTA (0: 16)
 
 
 def _digests(sims):
@@ -210,7 +209,7 @@ def variant_row(vf, torch, stream, wid: int, desc: str, ticks: int, mlp, threads
     if wl.regions > 1:
         knobs, table = autotune.tune(vf, wid, 1.0, torch, warmup=0, ticks=10, candidates=VARIANT_TUNE)
         row["tuned"] = knobs
-        row["tune_table"] = [{k: r[k] for k in ("engine", "gate", "producers", "depth", "cell_steps_per_s")} for r in table]
+        row["tune_table"] = [{"warps": r["gate"] >> 16 & 31 or 16, "cell_steps_per_s": r["cell_steps_per_s"]} for r in table]
     # plain: one region per launch, one tick per launch, the host waiting for every tick; the
     # regions run one after another, so a sample of them gives the mode's rate
     sample = list(range(0, wl.regions, max(1, wl.regions // 8)))
@@ -407,8 +406,8 @@ def ours(args):
         "e2e": {"value": e2e, "unit": UNIT, "h2d_bytes_per_step": h2d // max(args.steps, 1), "d2h_bytes_per_step": d2h // max(args.steps, 1),
                 "steps": args.steps, "timer": "host wall clock", "same_ticks_as_value": True, "same_end_state": bool(e2e_same)},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak, "traffic": STEP_DRAM_BYTES,
-                     "traffic_source": "one-off ncu capture of one step's k_tick_par launch (dram__bytes read + write), taken with the sweep in rows",
-                     "peak_kind": peak_kind, "kernel": "k_tick_par" if args.engine else "k_tick", "alg_bytes_per_step": alg_bytes / args.steps},
+                     "traffic_source": "one-off ncu capture of one step's k_tick_par launch (dram__bytes read + write)",
+                     "peak_kind": peak_kind, "kernel": "k_tick_par", "alg_bytes_per_step": alg_bytes / args.steps},
         "gpu_launches": args.steps,
         "clocks": clk.summary(),
         "cells_per_step": cells / args.steps,
