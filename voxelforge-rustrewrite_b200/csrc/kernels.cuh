@@ -458,7 +458,7 @@ __device__ __noinline__ void sweep_levels(const Region& Rs, TickSmem& sm, WS& sW
   // ---- the later conflicting cells of every cell, and how many earlier ones each waits for
   const int sgn = flip ? -1 : 1;
   for (unsigned i = tid; i < n; i += NT_) {
-    if (cell_done(L, i)) continue;
+    if (cell_done_now(L, i)) continue;
     const unsigned cid = R.lv[i].cid;
     unsigned s[12];
 #pragma unroll

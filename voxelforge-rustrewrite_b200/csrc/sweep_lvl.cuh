@@ -299,14 +299,20 @@ __device__ __forceinline__ void park_put(const Region& R, unsigned b, unsigned t
   if (t < MAX_CELLS_PER_TICK) R.lv_park[(size_t)b * MAX_CELLS_PER_TICK + t] = (unsigned short)i;
   else set_status(R, ST_RANGE, 52);
 }
-// Four cells' bytes share a word, and in a round one warp finishes a cell while others count down its
-// neighbours: during the rounds every access is to the whole word, and every change an atomic one.
-__device__ __forceinline__ unsigned dep_byte(const LvSmem& L, unsigned i) { return (vld(&L.dep[i >> 2]) >> ((i & 3u) * 8u)) & 0xFFu; }
-__device__ __forceinline__ void cell_finish(LvSmem& L, unsigned i, unsigned slots) {  // (the byte of a cell that runs is 0)
-  atomicOr(&L.dep[i >> 2], (DONE | slots) << ((i & 3u) * 8u));
-}
+// Four cells' bytes share a word, and in a round of the CTA one warp finishes a cell while others count down its
+// neighbours: there every access is to the whole word, and every change an atomic one (cell_done_now, cell_finish;
+// bit_now for pp). Where nobody else is at work, warp 0 between rounds and code between barriers, bytes are read and
+// written as such (words everywhere: +3% of the sweep's cycles, on warp 0's chain).
+__device__ __forceinline__ unsigned dep_byte(const LvSmem& L, unsigned i) { return reinterpret_cast<const volatile unsigned char*>(L.dep)[i]; }
 __device__ __forceinline__ bool cell_done(const LvSmem& L, unsigned i) { return dep_byte(L, i) >= DONE; }
-__device__ __forceinline__ bool bit_of(const unsigned* w, unsigned i) { return (vld(w + (i >> 5)) >> (i & 31u)) & 1u; }  // (a round's other warps clear pp bits)
+__device__ __forceinline__ bool cell_done_now(const LvSmem& L, unsigned i) { return (vld(&L.dep[i >> 2]) >> ((i & 3u) * 8u)) & DONE; }
+template <bool SOLO>
+__device__ __forceinline__ void cell_finish(LvSmem& L, unsigned i, unsigned slots) {  // (the byte of a cell that runs is 0)
+  if (SOLO) reinterpret_cast<volatile unsigned char*>(L.dep)[i] = (unsigned char)(DONE | slots);
+  else atomicOr(&L.dep[i >> 2], (DONE | slots) << ((i & 3u) * 8u));
+}
+__device__ __forceinline__ bool bit_of(const unsigned* w, unsigned i) { return (w[i >> 5] >> (i & 31u)) & 1u; }
+__device__ __forceinline__ bool bit_now(const unsigned* w, unsigned i) { return (vld(w + (i >> 5)) >> (i & 31u)) & 1u; }
 // att bits before position i
 __device__ __forceinline__ unsigned attempts_before(const LvSmem& L, unsigned i) {
   return (unsigned)L.gpre[i >> 5] + (unsigned)__popc(L.att[i >> 5] & ((1u << (i & 31u)) - 1u));
@@ -383,7 +389,7 @@ __device__ __forceinline__ float lv_cells(const Region& R, LvSmem& L, const Lane
   const unsigned i = c.i, w = c.w, u = c.u;
   const uint2 ce = c.ce;
   bool has = c.has;
-  const bool pp = has && i < kp && bit_of(L.pp, i);
+  const bool pp = has && i < kp && (SOLO ? bit_of(L.pp, i) : bit_now(L.pp, i));
   const int y = (int)(ce.y & YE_Y), at = (int)ce.x + S.off;
   // ---- a cell that attempts a pull and has a start cell waits for the pull
   if (__any_sync(FULLMASK, pp && !pulled)) {
@@ -477,9 +483,10 @@ __device__ __forceinline__ float lv_cells(const Region& R, LvSmem& L, const Lane
     if (r0 && !p0) park_put(R, pb, t + (unsigned)__popc(h0 & lanemask_lt()), a);
     if (r1 && !p1) park_put(R, pb, t + (unsigned)(__popc(h0) + __popc(h1 & lanemask_lt())), b);
   }
+  if (SOLO) __syncwarp();  // the counts are down before a byte beside them is written
   if (has && l == 0u) {
     R.lv_ev[i] = ev | (am & 0xFCu) | ((am & 0x80u) << 9) | ((cm & 0x7Fu) << 8);  // bit 16: seeds itself
-    cell_finish(L, i, pm & 0x7Fu);
+    cell_finish<SOLO>(L, i, pm & 0x7Fu);
     if (pp) atomicAnd(&L.pp[i >> 5], ~(1u << (i & 31u)));
   }
   __syncwarp();
@@ -502,7 +509,7 @@ __device__ __forceinline__ void lv_cell_thread(const Region& R, LvSmem& L, bool 
   }
   const unsigned w[6] = {ra.x, ra.y, ra.z, ra.w, rb.x, rb.y}, ye = rb.w;
   const int cid = (int)rb.z, y = (int)(ye & YE_Y);
-  const bool pp = has && i < kp && bit_of(L.pp, i);
+  const bool pp = has && i < kp && bit_now(L.pp, i);
   unsigned u[7];
 #pragma unroll
   for (int l = 0; l < 7; ++l) {
@@ -579,7 +586,7 @@ __device__ __forceinline__ void lv_cell_thread(const Region& R, LvSmem& L, bool 
   }
   if (has) {
     R.lv_ev[i] = (am & 0xFCu) | ((am & 0x80u) << 9) | cm << 8;
-    cell_finish(L, i, pm);
+    cell_finish<false>(L, i, pm);
     if (pp) atomicAnd(&L.pp[i >> 5], ~(1u << (i & 31u)));
   }
   // ---- the ready ones to the next list, or parked above the gate: places by a scan over the warp
@@ -1284,7 +1291,7 @@ __device__ __noinline__ int lv_long(const Region& Rs, LvSmem& L, unsigned n, int
     if (tid == 0) L.cnt[zc] = 0u;
     for (unsigned at = tid & ~31u; at < fcount; at += blockDim.x) {
       const unsigned t = at + lane_id(), i = t < fcount ? list_get(R, L, cur, t) : 0u;
-      lv_cell_thread(R, L, t < fcount && !cell_done(L, i), i, gate, kp, cur ^ 1u, nc, pb, pd);
+      lv_cell_thread(R, L, t < fcount && !cell_done_now(L, i), i, gate, kp, cur ^ 1u, nc, pb, pd);
     }
     __syncthreads();
     cur ^= 1u;
@@ -1320,7 +1327,7 @@ __device__ __noinline__ int lv_wide(const Region& Rs, LvSmem& L, unsigned n, int
     if (tid == 0) L.cnt[zc] = 0u;
     auto record = [&](unsigned at) {
       const unsigned t = at + (lane >> 3), i = t < fcount ? list_get(R, L, cur, t) : 0u;
-      return cell_record(R, t < fcount && !cell_done(L, i), i);
+      return cell_record(R, t < fcount && !cell_done_now(L, i), i);
     };
     if (fcount <= step) {
       if (t0 < fcount) {
