@@ -913,7 +913,8 @@ __device__ __forceinline__ void search_solo(const Region& R, LvSmem& L) {
 // reached within 13 steps it makes the cell below it a surface, which is the safe side. True: hopeless.
 // All threads of a CTA of 16 warps; ends with a barrier. ~7,000 cycles.
 // It is asked after a search that examined 512 entries for nothing, until it says no: regions of 50% size, 32 of
-// them, 206 -> 174 ms (4,071 of 4,557 searches hopeless), with edits 248 -> 223; a quarter dam asks 3 times.
+// them, 206 -> 174 ms (asked for 4,557 of the busiest
+// region's 5,651 searches, 4,071 times yes), with edits 248 -> 223 (4,352 of 8,780, 3,949); a quarter dam asks 3 times.
 constexpr int FLOOD_STEPS = 13;  // 9 steps hold 670 cells of open water; a corner of it takes a few more
 __device__ __noinline__ bool search_hopeless(const Region& Rs, LvSmem& L) {
   const Region R = Rs;
