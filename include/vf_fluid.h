@@ -165,7 +165,7 @@ int vf_fluid_shift(vf_fluid* h, int32_t dx, int32_t dz);
  * into the slot as chunk (cx, cz); kept entries of its cells come back into its bricks. The FIFO,
  * the level seeds and the marks are untouched, as in the reference. The chunk must lie inside the
  * handle's cell domain (the box of the chunks loaded at upload, moved by shifts): VF_ERR_RANGE
- * otherwise; VF_ERR_OOM when the atlas is full. A paste refused after that check has evicted the slot's chunk. */
+ * otherwise; VF_ERR_OOM when the atlas is full (the slot's chunk has been evicted then). */
 int vf_fluid_ring_evict(vf_fluid* h, int32_t cx, int32_t cz);
 int vf_fluid_ring_paste(vf_fluid* h, const uint32_t* chunk_grid, const uint8_t* chunk_bricks, uint64_t chunk_nbricks, int32_t chunk_bricks_y,
                         int32_t cx, int32_t cz);

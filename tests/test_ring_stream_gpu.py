@@ -90,12 +90,15 @@ def test_chunks_come_and_go(vf, orc):
         for s in (sim, o):
             s.tick(2)
         assert_same_digest(sim, o, t)
+        xyz, vol = sim.partials()  # kept entries among them
+        assert o.partial_count() == len(np.unique(xyz, axis=0)) and np.all(vol > 0)
         sim.ring_paste(chunk, cx, cz)
         o.ring_paste(grid, bricks, chunk.info.bricks_y, cx, cz)
         for s in (sim, o):
             s.tick(2)
         assert_same_digest(sim, o, t)
-        assert sim.partial_count() == o.partial_count() == len(sim.partials()[1])
+        xyz, vol = sim.partials()
+        assert sim.partial_count() == o.partial_count() == len(np.unique(xyz, axis=0)) and np.all(vol > 0)
     sim.close()
 
 
